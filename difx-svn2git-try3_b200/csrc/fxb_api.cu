@@ -485,30 +485,17 @@ static fxb_status setup_device(fxb_ctx *ctx)
 		d.nrow = p.nrow;
 		d.nchan = p.nchan;
 		if(p.nrow == 0) continue;
-		d.ntr = (p.nrow + kTile - 1) / kTile;
-		d.npair = d.ntr * (d.ntr + 1) / 2;
 		d.spec_off = p.spec_off;
 		d.acc_off = p.acc_off;
 		d.acc_cstride = 1;
 		d.acc_ostride = p.nchan;
 		int32_t *dA, *dB;
-		int16_t *pairs;
 		CK(ctx, dalloc(ctx, &dA, p.destA.size()));
 		CK(ctx, dalloc(ctx, &dB, p.destB.size()));
 		CK(ctx, cudaMemcpyAsync(dA, p.destA.data(), sizeof(int32_t) * p.destA.size(), cudaMemcpyHostToDevice, ctx->stream));
 		CK(ctx, cudaMemcpyAsync(dB, p.destB.data(), sizeof(int32_t) * p.destB.size(), cudaMemcpyHostToDevice, ctx->stream));
-		std::vector<int16_t> hp;
-		for(int i = 0; i < d.ntr; i++)
-			for(int j = i; j < d.ntr; j++)
-			{
-				hp.push_back((int16_t)i);
-				hp.push_back((int16_t)j);
-			}
-		CK(ctx, dalloc(ctx, &pairs, hp.size()));
-		CK(ctx, cudaMemcpyAsync(pairs, hp.data(), sizeof(int16_t) * hp.size(), cudaMemcpyHostToDevice, ctx->stream));
 		d.destA = dA;
 		d.destB = dB;
-		d.pairs = pairs;
 		// inverse of destA / destB: which input pair (and whether conjugated) feeds each output
 		{
 			std::vector<int32_t> src((size_t)std::max(p.nout, 1), -1);
@@ -1387,7 +1374,8 @@ static void launch_xmac_weights(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, u
 		if(ctx->tc)
 			launch_xmac_tc(g.tmap, sh, ctx->d_plans, g.d_idx, g.nf, ctx->nsm, ctx->d_err, ctx->d_acc, st);
 		else
-			launch_xmac_fp32v2(ctx->h_plans[g.plan0], ctx->d_plans, g.d_idx, g.nf, ctx->T, ctx->d_spec, ctx->d_acc, st);
+			launch_xmac_fp32(ctx->h_plans[g.plan0], ctx->d_plans, g.d_idx, g.nf, ctx->T, ctx->nsm, ctx->d_spec, ctx->d_acc,
+			                 st);
 	}
 	if(tuning)
 		cudaEventRecord(tn.ev[nk + 1 + ctx->xgroups.size()], st);

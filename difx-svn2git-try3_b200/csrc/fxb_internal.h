@@ -14,7 +14,6 @@ constexpr int kMaxStations = 64;
 constexpr int kMaxBandsPerStation = 64;
 constexpr int kMaxPolyOrder = 5;          // MAX_POLY_ORDER of the .im reader
 constexpr int kMaxPolys = 64;
-constexpr int kTile = 4;                  // rows per register tile in the FP32 XMAC
 
 // FFT status codes written by the delay kernel (why Mode::process zeroes an FFT).
 enum FftStatus : int32_t {

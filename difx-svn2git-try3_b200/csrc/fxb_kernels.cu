@@ -207,124 +207,6 @@ cudaError_t launch_fstage(const DevStation *st, const DevSubintStation *sub, con
 	return cudaGetLastError();
 }
 
-// FP32 cross-multiply-accumulate (core.cpp:877-972 with the autocorrelations
-// of mode.cpp:1293-1369).  For one frequency, V[i][j] = sum_t X_i X_j^* over
-// all input rows is evaluated in 4x4 register tiles (a complex Hermitian
-// rank-T update per channel): one warp = one tile pair, 32 channels per CTA.
-// Each (output, channel) is owned by one thread, which adds its subint sum
-// into the accumulator.
-__global__ void __launch_bounds__(256) k_xmac_fp32(const DevFreqPlan *__restrict__ plan, int T, int TC,
-                                                   const float2 *__restrict__ spec, float2 *__restrict__ acc)
-{
-	extern __shared__ float2 sxm[];
-	const DevFreqPlan P = *plan;
-	constexpr int CB = 32;
-	const int c0 = blockIdx.y * CB;
-	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const int pairidx = blockIdx.x * 8 + warp;
-	const bool active = pairidx < P.npair;
-	int ti = 0, tj = 0;
-	if(active)
-	{
-		ti = P.pairs[2 * pairidx];
-		tj = P.pairs[2 * pairidx + 1];
-	}
-	const int nrowpad = P.ntr * kTile;
-	const float2 *X = spec + P.spec_off;
-	float vr[4][4], vi[4][4];
-#pragma unroll
-	for(int i = 0; i < 4; i++)
-#pragma unroll
-		for(int j = 0; j < 4; j++)
-		{
-			vr[i][j] = 0.0f;
-			vi[i][j] = 0.0f;
-		}
-	for(int t0 = 0; t0 < T; t0 += TC)
-	{
-		const int tcnt = min(TC, T - t0);
-		const int nel = TC * nrowpad * CB;
-		for(int e = threadIdx.x; e < nel; e += blockDim.x)
-		{
-			int c = e % CB;
-			int r = (e / CB) % nrowpad;
-			int tt = e / (CB * nrowpad);
-			float2 v = make_float2(0.0f, 0.0f);
-			if(tt < tcnt && r < P.nrow && c0 + c < P.nchan)
-				v = X[((int64_t)(t0 + tt) * P.nrow + r) * P.nchan + c0 + c];
-			sxm[e] = v;
-		}
-		__syncthreads();
-		if(active)
-		{
-			for(int tt = 0; tt < tcnt; tt++)
-			{
-				const float2 *row = sxm + (int64_t)tt * nrowpad * CB;
-				float2 a[4], b[4];
-#pragma unroll
-				for(int i = 0; i < 4; i++)
-				{
-					a[i] = row[(ti * 4 + i) * CB + lane];
-					b[i] = row[(tj * 4 + i) * CB + lane];
-				}
-#pragma unroll
-				for(int i = 0; i < 4; i++)
-#pragma unroll
-					for(int j = 0; j < 4; j++)
-					{
-						vr[i][j] = fmaf(a[i].x, b[j].x, fmaf(a[i].y, b[j].y, vr[i][j]));
-						vi[i][j] = fmaf(a[i].y, b[j].x, fmaf(-a[i].x, b[j].y, vi[i][j]));
-					}
-			}
-		}
-		__syncthreads();
-	}
-	if(!active)
-		return;
-	const int c = c0 + lane;
-	if(c >= P.nchan)
-		return;
-#pragma unroll
-	for(int i = 0; i < 4; i++)
-#pragma unroll
-		for(int j = 0; j < 4; j++)
-		{
-			int ri = ti * 4 + i, rj = tj * 4 + j;
-			if(ri >= P.nrow || rj >= P.nrow || (ti == tj && i > j))
-				continue;
-			int dA = P.destA[ri * P.nrow + rj];
-			int dB = P.destB[ri * P.nrow + rj];
-			if(dA >= 0)
-			{
-				float2 *d = acc + P.acc_off + (int64_t)dA * P.nchan + c;
-				float2 o = *d;
-				*d = make_float2(o.x + vr[i][j], o.y + vi[i][j]);
-			}
-			if(dB >= 0)
-			{
-				float2 *d = acc + P.acc_off + (int64_t)dB * P.nchan + c;
-				float2 o = *d;
-				*d = make_float2(o.x + vr[i][j], o.y - vi[i][j]);
-			}
-		}
-}
-
-void launch_xmac_fp32(const DevFreqPlan &plan, const DevFreqPlan *dplan, int T, const float2 *spec, float2 *acc,
-                      cudaStream_t stream)
-{
-	constexpr int CB = 32;
-	const int nrowpad = plan.ntr * kTile;
-	int TC = (96 * 1024) / (nrowpad * CB * (int)sizeof(float2));
-	if(TC > 32) TC = 32;
-	if(TC < 1) TC = 1;
-	size_t smem = (size_t)TC * nrowpad * CB * sizeof(float2);
-	// per-device attribute: raised on every call
-	if(cudaFuncSetAttribute(k_xmac_fp32, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024) != cudaSuccess)
-		return;
-	dim3 grid((plan.npair + 7) / 8, (plan.nchan + CB - 1) / CB);
-	k_xmac_fp32<<<grid, 256, smem, stream>>>(dplan, T, TC, spec, acc);
-}
-
 // Baseline weights sum_t w1*w2 (core.cpp:998-1045) and autocorrelation
 // weights sum_t w (mode.cpp:1304-1307), each as a sequential float sum in FFT
 // order, added to the running totals (core.cpp:1068-1086, 1310-1363).

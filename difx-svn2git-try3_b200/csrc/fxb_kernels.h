@@ -10,7 +10,7 @@ namespace fxb {
 
 // Per-frequency XMAC plan on the device.
 struct DevFreqPlan {
-	int32_t nrow, nchan, ntr, npair;  // rows, channels, 4-row tiles, tile pairs
+	int32_t nrow, nchan;              // rows, channels
 	int32_t tcb;                      // tensor-core form: channels per spectra block (0: spectra [t][row][chan])
 	int32_t tnblk;                    // tensor-core form: blocks per time, spectra [t][block][row][tcb]
 	int32_t acc_cstride;              // accumulator stride between channels (1: [out][chan], nout: [chan][out])
@@ -19,7 +19,6 @@ struct DevFreqPlan {
 	int64_t acc_off;                  // complex offset of accumulators [nout][nchan]
 	const int32_t *destA;             // [nrow*nrow]
 	const int32_t *destB;             // [nrow*nrow]
-	const int16_t *pairs;             // [npair*2] tile pairs (ti <= tj)
 	const int32_t *outsrc;            // [nout] source of each output: a | b << 8 | conj << 16 (a <= b), or -1
 	int64_t spec8_off;                // FP8 form: offset (16-bit words) of this frequency's e4m3 spectra
 	float *iscale;                    // FP8 form: [nchan][nrow] 1 / quantisation scale of the subint
@@ -223,10 +222,10 @@ cudaError_t launch_fstage_tc(const FKind &k, FsArgs a, int nsm, cudaStream_t str
 // twiddles of FFT length N, FKind::twn entries
 void make_fstage_twiddles(int N, float2 *out32);
 
-// FP32 XMAC v2 over a set of frequencies with equal (rows, channels):
-// plan_idx[0..nf) index dplans.
-void launch_xmac_fp32v2(const DevFreqPlan &plan0, const DevFreqPlan *dplans, const int32_t *plan_idx, int nf, int T,
-                        const float2 *spec, float2 *acc, cudaStream_t stream);
+// FP32 cross-multiply-accumulate into acc over a set of frequencies with
+// equal (rows, channels): plan_idx[0..nf) index dplans.
+void launch_xmac_fp32(const DevFreqPlan &plan0, const DevFreqPlan *dplans, const int32_t *plan_idx, int nf, int T,
+                      int nsm, const float2 *spec, float2 *acc, cudaStream_t stream);
 
 // Tensor-core XMAC (csrc/fxb_xmac_tc.cu) over one group of equally shaped
 // subbands whose bf16x2 spectra lie in one block [subband][Tpad][nrow][nchan].
@@ -279,10 +278,6 @@ void launch_xmac_tc_multi(const XMultiArgs &xm, const TcShape &s, int nsm, int32
 // subint's T times maps to 240; writes 1 / scale to iscale[channel][input]
 void launch_quant_fp8(const TcShape &s, const DevFreqPlan *dplans, const int32_t *plan_idx, int nf, int T,
                       const uint32_t *spec16, uint16_t *spec8, cudaStream_t stream);
-
-// FP32 cross-multiply-accumulate of one frequency into acc.
-void launch_xmac_fp32(const DevFreqPlan &plan, const DevFreqPlan *dplan, int T, const float2 *spec, float2 *acc,
-                      cudaStream_t stream);
 
 // Phase cal (csrc/fxb_pcal.cu).  A group is up to kPcalGroupBands recorded
 // bands of one station with the same bin count; a band is one band's tones.
