@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <array>
 #include <tuple>
 #include <cmath>
 #include <cstdio>
@@ -88,11 +89,11 @@ struct fxb_ctx {
 	int nbm = 0;
 	float2 *d_spec = nullptr;
 	float2 *d_acc = nullptr;
-	float *d_bwacc = nullptr, *d_acwacc = nullptr;
-	DevBWeight *d_bw = nullptr;
-	DevACWeight *d_acw = nullptr;
+	float *d_wacc = nullptr, *d_wts = nullptr;   // weight sums; packed data weights [station][FFT]
+	DevWeightSum *d_wsum = nullptr;
+	DevWeightOut *d_wout = nullptr;
 	DevOutMap *d_om = nullptr;
-	int nbw = 0, nacw = 0, nom = 0;
+	int nwsum = 0, nwout = 0, nom = 0;
 	DevZoomCopy *d_zoom = nullptr;       // zoom-band rows gathered after the F stage
 	int nzoom = 0;
 	// phase cal: binning groups, bands, and the FP64 bins of the integration
@@ -826,19 +827,34 @@ static fxb_status setup_device(fxb_ctx *ctx)
 	CK(ctx, dalloc(ctx, &ctx->d_spec, job.xmac_kind == FXB_XMAC_FP32 ? (size_t)job.spec_total : 1));
 	CK(ctx, dalloc(ctx, &ctx->d_acc, (size_t)job.acc_total));
 	CK(ctx, dalloc(ctx, &ctx->d_core, (size_t)job.corelen));
-	ctx->nbw = (int)job.bweights.size();
-	ctx->nacw = (int)job.acweights.size();
 	ctx->nom = (int)job.outmap.size();
-	CK(ctx, dalloc(ctx, &ctx->d_bwacc, ctx->nbw));
-	CK(ctx, dalloc(ctx, &ctx->d_acwacc, ctx->nacw));
 	{
-		std::vector<DevBWeight> hbw(ctx->nbw);
-		for(int i = 0; i < ctx->nbw; i++)
-			hbw[i] = DevBWeight{job.bweights[i].s1, job.bweights[i].s2, job.bweights[i].b1, job.bweights[i].b2,
-			                    job.bweights[i].dst_float};
-		std::vector<DevACWeight> hacw(ctx->nacw);
-		for(int i = 0; i < ctx->nacw; i++)
-			hacw[i] = DevACWeight{job.acweights[i].s, job.acweights[i].band, job.acweights[i].dst_float};
+		// the distinct weight sums, and the sum each core-result slot shows
+		std::vector<DevWeightSum> sums;
+		std::vector<DevWeightOut> wout;
+		std::map<std::array<int, 4>, int> seen;
+		auto slot = [&](int64_t dst, int s1, int s2, int b1, int b2) {
+			if(job.stations[s1].mux_threads == 0)
+				b1 = -1;
+			if(s2 < 0 || job.stations[s2].mux_threads == 0)
+				b2 = -1;
+			const auto r = seen.emplace(std::array<int, 4>{s1, s2, b1, b2}, (int)sums.size());
+			if(r.second)
+				sums.push_back(DevWeightSum{s1, s2, b1, b2});
+			wout.push_back(DevWeightOut{dst, r.first->second, 0});
+		};
+		for(const auto &w : job.bweights)
+			slot(w.dst_float, w.s1, w.s2, w.b1, w.b2);
+		for(const auto &w : job.acweights)
+			slot(w.dst_float, w.s, -1, w.band, -1);
+		ctx->nwsum = (int)sums.size();
+		ctx->nwout = (int)wout.size();
+		CK(ctx, dalloc(ctx, &ctx->d_wacc, ctx->nwsum));
+		CK(ctx, dalloc(ctx, &ctx->d_wts, (size_t)ctx->S * ctx->T));
+		CK(ctx, dalloc(ctx, &ctx->d_wsum, ctx->nwsum));
+		CK(ctx, dalloc(ctx, &ctx->d_wout, ctx->nwout));
+		if(ctx->nwsum) CK(ctx, cudaMemcpyAsync(ctx->d_wsum, sums.data(), sizeof(DevWeightSum) * ctx->nwsum, cudaMemcpyHostToDevice, ctx->stream));
+		if(ctx->nwout) CK(ctx, cudaMemcpyAsync(ctx->d_wout, wout.data(), sizeof(DevWeightOut) * ctx->nwout, cudaMemcpyHostToDevice, ctx->stream));
 		std::vector<DevOutMap> hom(ctx->nom);
 		for(int i = 0; i < ctx->nom; i++)
 		{
@@ -852,11 +868,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 			}
 			hom[i] = DevOutMap{a, m.core, m.nchan, m.avg, cs, 0};
 		}
-		CK(ctx, dalloc(ctx, &ctx->d_bw, ctx->nbw));
-		CK(ctx, dalloc(ctx, &ctx->d_acw, ctx->nacw));
 		CK(ctx, dalloc(ctx, &ctx->d_om, ctx->nom));
-		if(ctx->nbw) CK(ctx, cudaMemcpyAsync(ctx->d_bw, hbw.data(), sizeof(DevBWeight) * ctx->nbw, cudaMemcpyHostToDevice, ctx->stream));
-		if(ctx->nacw) CK(ctx, cudaMemcpyAsync(ctx->d_acw, hacw.data(), sizeof(DevACWeight) * ctx->nacw, cudaMemcpyHostToDevice, ctx->stream));
 		if(ctx->nom) CK(ctx, cudaMemcpyAsync(ctx->d_om, hom.data(), sizeof(DevOutMap) * ctx->nom, cudaMemcpyHostToDevice, ctx->stream));
 		// phase cal: binning groups, every band's tones for the DFT, and one
 		// slice of FP64 bins per chunk of FFTs
@@ -949,8 +961,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 	}
 	CK(ctx, upload_lut8(ctx->stream));
 	CK(ctx, cudaMemsetAsync(ctx->d_acc, 0, sizeof(float2) * std::max<int64_t>(job.acc_total, 1), ctx->stream));
-	CK(ctx, cudaMemsetAsync(ctx->d_bwacc, 0, sizeof(float) * std::max(ctx->nbw, 1), ctx->stream));
-	CK(ctx, cudaMemsetAsync(ctx->d_acwacc, 0, sizeof(float) * std::max(ctx->nacw, 1), ctx->stream));
+	CK(ctx, cudaMemsetAsync(ctx->d_wacc, 0, sizeof(float) * std::max(ctx->nwsum, 1), ctx->stream));
 	CK(ctx, cudaStreamSynchronize(ctx->stream));
 	return FXB_OK;
 }
@@ -1244,7 +1255,7 @@ static void launch_prep(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, unsigned 
 		fxb::launch_prep(ctx->d_st, sl.d_sub, ctx->S, ctx->T, ctx->d_valid, ctx->d_bandok, ctx->valid_stride, st,
 		                 ctx->d_fillok);
 	launch_fft_params(ctx->d_st, sl.d_sub, sl.d_vflags, ctx->nflagint, ctx->d_valid, ctx->d_bandok, ctx->valid_stride,
-	                  ctx->S, ctx->T, job.fringe_rot_order, ctx->d_params, ctx->d_pbw, ctx->nbm, st, ctx->d_fillok);
+	                  ctx->S, ctx->T, job.fringe_rot_order, ctx->d_params, ctx->d_pbw, ctx->nbm, st, ctx->d_fillok, ctx->d_wts);
 	cudaEventRecordWithFlags(sl.tev[1], st, evf);
 }
 
@@ -1379,8 +1390,7 @@ static void launch_xmac_weights(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, u
 	}
 	if(tuning)
 		cudaEventRecord(tn.ev[nk + 1 + ctx->xgroups.size()], st);
-	launch_weights(ctx->d_bw, ctx->nbw, ctx->d_acw, ctx->nacw, ctx->d_params, ctx->d_pbw, ctx->nbm, ctx->d_st, ctx->T,
-	               ctx->d_bwacc, ctx->d_acwacc, st);
+	launch_weights(ctx->d_wsum, ctx->nwsum, ctx->d_wts, ctx->d_pbw, ctx->nbm, ctx->T, ctx->d_wacc, st);
 	cudaEventRecordWithFlags(sl.tev[3], st, evf);
 	// a launch that could not start (resources, configuration) leaves its
 	// error behind; keep it for the submit to report
@@ -1751,7 +1761,7 @@ fxb_status fxb_job_footprint(const fxb_job_desc *desc, size_t *bytes)
 	double b = (double)job.spec_total * (job.xmac_kind == FXB_XMAC_FP32 ? 8.0
 	                                     : job.xmac_kind != FXB_XMAC_FP8 ? 4.0 * 1.25 * pad32
 	                                                                      : (4.0 * pad64 + 2.0 * pad64 + 0.5) * 1.25);
-	b += (double)job.acc_total * 8.0 + (double)job.corelen * 16.0 + (double)S * T * 64.0 +
+	b += (double)job.acc_total * 8.0 + (double)job.corelen * 16.0 + (double)S * T * 68.0 +
 	     (double)job.pcal_bins * 8.0 * pcal_chunks(job, pcal_groups(job));
 	// raw VDIF staging of the in-flight subints (payload plus headers, 1/8 slack)
 	for(int s = 0; s < S; s++)
@@ -1778,8 +1788,8 @@ fxb_status fxb_read_results(fxb_ctx *ctx, float *coreresult, size_t nfloats)
 		ctx->err = "result buffer too small";
 		return FXB_ERR_ARG;
 	}
-	launch_finalise(ctx->d_om, ctx->nom, 0, ctx->d_acc, ctx->d_bw, ctx->nbw, ctx->d_bwacc, ctx->d_acw, ctx->nacw,
-	                ctx->d_acwacc, ctx->d_core, ctx->job.corelen, ctx->stream);
+	launch_finalise(ctx->d_om, ctx->nom, ctx->d_acc, ctx->d_wout, ctx->nwout, ctx->d_wacc, ctx->d_core,
+	                ctx->job.corelen, ctx->stream);
 	launch_pcal_final(ctx->d_pbands, ctx->npbands, ctx->pchunks, ctx->job.pcal_bins, ctx->d_pbins, ctx->d_core, ctx->stream);
 	CK(ctx, cudaGetLastError());
 	CK(ctx, cudaMemcpyAsync(coreresult, ctx->d_core, sizeof(float2) * ctx->job.corelen, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1793,8 +1803,7 @@ fxb_status fxb_reset(fxb_ctx *ctx)
 		ctx->dirty = true;
 	if(!ctx) return FXB_ERR_ARG;
 	CK(ctx, cudaMemsetAsync(ctx->d_acc, 0, sizeof(float2) * std::max<int64_t>(ctx->job.acc_total, 1), ctx->stream));
-	CK(ctx, cudaMemsetAsync(ctx->d_bwacc, 0, sizeof(float) * std::max(ctx->nbw, 1), ctx->stream));
-	CK(ctx, cudaMemsetAsync(ctx->d_acwacc, 0, sizeof(float) * std::max(ctx->nacw, 1), ctx->stream));
+	CK(ctx, cudaMemsetAsync(ctx->d_wacc, 0, sizeof(float) * std::max(ctx->nwsum, 1), ctx->stream));
 	if(ctx->d_pbins)
 		CK(ctx, cudaMemsetAsync(ctx->d_pbins, 0,
 		                        sizeof(double) * (size_t)ctx->pchunks * (size_t)std::max<int64_t>(ctx->job.pcal_bins, 1),
@@ -1950,8 +1959,8 @@ fxb_status fxb_read_results_device(fxb_ctx *ctx, float *dev_out, size_t nfloats)
 		ctx->err = "result buffer too small";
 		return FXB_ERR_ARG;
 	}
-	launch_finalise(ctx->d_om, ctx->nom, 0, ctx->d_acc, ctx->d_bw, ctx->nbw, ctx->d_bwacc, ctx->d_acw, ctx->nacw,
-	                ctx->d_acwacc, (float2 *)dev_out, ctx->job.corelen, ctx->stream);
+	launch_finalise(ctx->d_om, ctx->nom, ctx->d_acc, ctx->d_wout, ctx->nwout, ctx->d_wacc, (float2 *)dev_out,
+	                ctx->job.corelen, ctx->stream);
 	launch_pcal_final(ctx->d_pbands, ctx->npbands, ctx->pchunks, ctx->job.pcal_bins, ctx->d_pbins, (float2 *)dev_out,
 	                  ctx->stream);
 	CK(ctx, cudaGetLastError());

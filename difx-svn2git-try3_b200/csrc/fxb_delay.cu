@@ -213,7 +213,7 @@ __global__ void k_fft_params(const DevStation *__restrict__ st, const DevSubintS
                              const int32_t *__restrict__ validflags, int nflagint, const uint8_t *__restrict__ valid,
                              const uint32_t *__restrict__ bandok, int64_t valid_stride, int T, int order,
                              FftParam *__restrict__ out, float *__restrict__ pbw, int nbm,
-                             const uint8_t *__restrict__ fillok)
+                             const uint8_t *__restrict__ fillok, float *__restrict__ wts)
 {
 	const int s = blockIdx.y;
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -229,6 +229,12 @@ __global__ void k_fft_params(const DevStation *__restrict__ st, const DevSubintS
 	const DevSubintStation &U = sub[s];
 	const int offsetsec = U.subsec, offsetns = U.subns;
 	const int32_t *vf = validflags + (int64_t)s * nflagint;
+	// the data weight a second time, packed, for the weight sums (k_weights)
+	auto put = [&](const FftParam &r) {
+		out[(int64_t)s * T + i] = r;
+		if(wts)
+			wts[(int64_t)s * T + i] = r.weight;
+	};
 	FftParam p;
 	p.status = kFftZero;
 	p.nearest = 0;
@@ -243,13 +249,13 @@ __global__ void k_fft_params(const DevStation *__restrict__ st, const DevSubintS
 
 	if(U.nbytes <= 1 || U.invalid_subint || !flag_valid(vf, i))
 	{
-		out[(int64_t)s * T + i] = p;
+		put(p);
 		return;
 	}
 	Nearest nr = nearest_sample(S, U, offsetsec, offsetns, i);
 	if(!nr.inrange)
 	{
-		out[(int64_t)s * T + i] = p;
+		put(p);
 		return;
 	}
 	int nearest = nr.nearest;
@@ -268,7 +274,7 @@ __global__ void k_fft_params(const DevStation *__restrict__ st, const DevSubintS
 			int ups = pn - (pn % S.gran);
 			if(!(nearest < ups || nearest > ups))
 			{
-				out[(int64_t)s * T + i] = p;
+				put(p);
 				return;
 			}
 		}
@@ -337,7 +343,7 @@ __global__ void k_fft_params(const DevStation *__restrict__ st, const DevSubintS
 	}
 	if(!(weight > 0.0f))
 	{
-		out[(int64_t)s * T + i] = p;
+		put(p);
 		return;
 	}
 	p.status = kFftOk;
@@ -391,7 +397,7 @@ __global__ void k_fft_params(const DevStation *__restrict__ st, const DevSubintS
 		p.b = b;
 		p.c = c;
 	}
-	out[(int64_t)s * T + i] = p;
+	put(p);
 }
 
 void launch_frame_valid(const DevStation *st, const DevSubintStation *sub, uint8_t *valid, uint32_t *bandok,
@@ -415,11 +421,11 @@ void launch_interpolators(const DevStation *st, DevSubintStation *sub, int S, in
 
 void launch_fft_params(const DevStation *st, const DevSubintStation *sub, const int32_t *validflags, int nflagint,
                        const uint8_t *valid, const uint32_t *bandok, int64_t valid_stride, int S, int T, int order,
-                       FftParam *out, float *pbw, int nbm, cudaStream_t stream, const uint8_t *fillok)
+                       FftParam *out, float *pbw, int nbm, cudaStream_t stream, const uint8_t *fillok, float *wts)
 {
 	dim3 grid((T + 127) / 128, S);
 	k_fft_params<<<grid, 128, 0, stream>>>(st, sub, validflags, nflagint, valid, bandok, valid_stride, T, order, out,
-	                                       pbw, nbm, fillok);
+	                                       pbw, nbm, fillok, wts);
 }
 
 }  // namespace fxb

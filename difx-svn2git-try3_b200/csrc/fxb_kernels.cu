@@ -207,73 +207,78 @@ cudaError_t launch_fstage(const DevStation *st, const DevSubintStation *sub, con
 	return cudaGetLastError();
 }
 
-// Baseline weights sum_t w1*w2 (core.cpp:998-1045) and autocorrelation
-// weights sum_t w (mode.cpp:1304-1307), each as a sequential float sum in FFT
-// order, added to the running totals (core.cpp:1068-1086, 1310-1363).
-// Baseline and autocorrelation weights of one subint: the float sums of
-// w1(t) * w2(t) (baseline) and of w(t) over valid FFTs (autocorrelation), added
-// in FFT order as Core does.  One warp per weight: the lanes load and multiply
-// 256 FFTs at a time in parallel, then lane 0 adds them in order (adding 0 for
-// an invalid FFT leaves a non-negative float sum unchanged).
-// INTERLACEDVDIF stations weigh each band by its own data weight
-// (Mode::getDataWeight, mode.h:168, mode.cpp:1300-1303).
-__global__ void k_weights(const DevBWeight *__restrict__ bw, int nbw, const DevACWeight *__restrict__ acw, int nacw,
-                          const FftParam *__restrict__ params, const float *__restrict__ pbw, int nbm,
-                          const DevStation *__restrict__ st, int T, float *__restrict__ bwacc,
-                          float *__restrict__ acwacc)
+// Weight sums of one subint: sum_t w1(t) w2(t) of a baseline (core.cpp:
+// 998-1045) and sum_t w(t) of a station (mode.cpp:1304-1307; w is zero where
+// the FFT is not valid), each the float sum in FFT order that Core forms,
+// added to the running total (core.cpp:1068-1086, 1310-1363).  INTERLACEDVDIF
+// stations weigh each band by its own data weight (Mode::getDataWeight,
+// mode.h:168, mode.cpp:1300-1303).
+//
+// Bound: latency, of the loads and of a chain of T float additions.  One warp
+// per distinct sum (not per core-result slot: the products of a baseline
+// share one) reads 128 FFTs at a time from the packed weights.  Additions of
+// zeros and ones to an integral sum below 2^23 are exact in any order, so a
+// run of 32 such weights (whole or invalid FFTs) is added by its count; other
+// runs are added one by one.  20 stations x 4 subbands, T = 4096: 87 -> 8 us per
+// subint; 10 stations x 8, T = 250: 7.9 -> 2.9 us.
+__global__ void __launch_bounds__(128) k_weights(const DevWeightSum *__restrict__ sums, int nsum,
+                                                 const float *__restrict__ wts, const float *__restrict__ pbw, int nbm,
+                                                 int T, float *__restrict__ acc)
 {
-	__shared__ float buf[4][256];
+	constexpr int G = 4;                      // runs of 32 in flight
+	__shared__ __align__(16) float buf[4][32];
 	const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 	const int k = blockIdx.x * 4 + w;
-	if(k >= nbw + nacw)
+	if(k >= nsum)
 		return;
-	const bool isb = k < nbw;
-	const FftParam *p1 = params + (int64_t)(isb ? bw[k].s1 : acw[k - nbw].s) * T;
-	const FftParam *p2 = params + (int64_t)(isb ? bw[k].s2 : 0) * T;
-	const int sa = isb ? bw[k].s1 : acw[k - nbw].s, sb = isb ? bw[k].s2 : sa;
-	const int ba = isb ? bw[k].b1 : acw[k - nbw].band, bb = isb ? bw[k].b2 : -1;
-	const float *wa = (pbw && st[sa].mux) ? pbw + (int64_t)sa * T * nbm + ba : nullptr;
-	const float *wb = (pbw && st[sb].mux && bb >= 0) ? pbw + (int64_t)sb * T * nbm + bb : nullptr;
+	const DevWeightSum u = sums[k];
+	const float *wa = u.b1 >= 0 ? pbw + (int64_t)u.s1 * T * nbm + u.b1 : wts + (int64_t)u.s1 * T;
+	const int sa = u.b1 >= 0 ? nbm : 1;
+	const bool two = u.s2 >= 0;
+	const float *wb = !two ? wa : (u.b2 >= 0 ? pbw + (int64_t)u.s2 * T * nbm + u.b2 : wts + (int64_t)u.s2 * T);
+	const int sb = two && u.b2 >= 0 ? nbm : 1;
 	float sum = 0.0f;
-	for(int t0 = 0; t0 < T; t0 += 256)
+	for(int t0 = 0; t0 < T; t0 += 32 * G)
 	{
-		const int n = min(256, T - t0);
-		for(int j = lane; j < n; j += 32)
+		float v[G];
+#pragma unroll
+		for(int g = 0; g < G; g++)
 		{
-			const int t = t0 + j;
-			float v;
-			const float w1 = wa ? wa[(int64_t)t * nbm] : p1[t].weight;
-			if(isb)
-				v = __fmul_rn(w1, wb ? wb[(int64_t)t * nbm] : p2[t].weight);
-			else if(p1[t].status != kFftOk)
-				v = 0.0f;
-			else
-				v = w1;
-			buf[w][j] = v;
+			const int t = t0 + 32 * g + lane;
+			v[g] = t < T ? __ldg(wa + (int64_t)t * sa) : 0.0f;
+			if(two)
+				v[g] = __fmul_rn(v[g], t < T ? __ldg(wb + (int64_t)t * sb) : 0.0f);
 		}
-		__syncwarp();
-		if(lane == 0)
-			for(int j = 0; j < n; j++)
-				sum = __fadd_rn(sum, buf[w][j]);
-		__syncwarp();
+#pragma unroll
+		for(int g = 0; g < G; g++)
+		{
+			// adding 0 (past T, or an invalid FFT) leaves a non-negative sum unchanged
+			const uint32_t ones = __ballot_sync(0xffffffffu, v[g] == 1.0f);
+			if(__all_sync(0xffffffffu, v[g] == 1.0f || v[g] == 0.0f) && sum == rintf(sum) && sum < 8388608.0f)
+			{
+				sum += (float)__popc(ones);
+				continue;
+			}
+			buf[w][lane] = v[g];
+			__syncwarp();
+#pragma unroll
+			for(int j = 0; j < 32; j += 4)
+			{
+				const float4 q = *(const float4 *)(buf[w] + j);
+				sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, q.x), q.y), q.z), q.w);
+			}
+			__syncwarp();
+		}
 	}
 	if(lane == 0)
-	{
-		if(isb)
-			bwacc[k] = __fadd_rn(bwacc[k], sum);
-		else
-			acwacc[k - nbw] = __fadd_rn(acwacc[k - nbw], sum);
-	}
+		acc[k] = __fadd_rn(acc[k], sum);
 }
 
-void launch_weights(const DevBWeight *bw, int nbw, const DevACWeight *acw, int nacw, const FftParam *params,
-                    const float *pbw, int nbm, const DevStation *st, int T, float *bwacc, float *acwacc,
+void launch_weights(const DevWeightSum *sums, int nsum, const float *wts, const float *pbw, int nbm, int T, float *acc,
                     cudaStream_t stream)
 {
-	int n = nbw + nacw;
-	if(n == 0)
-		return;
-	k_weights<<<(n + 3) / 4, 128, 0, stream>>>(bw, nbw, acw, nacw, params, pbw, nbm, st, T, bwacc, acwacc);
+	if(nsum > 0)
+		k_weights<<<(nsum + 3) / 4, 128, 0, stream>>>(sums, nsum, wts, pbw, nbm, T, acc);
 }
 
 // Core-result assembly (core.cpp:1774-1802 channel averaging, 1266-1363):
@@ -306,28 +311,22 @@ __global__ void k_finalise(const DevOutMap *__restrict__ om, const float2 *__res
 	}
 }
 
-__global__ void k_finalise_weights(const DevBWeight *__restrict__ bw, int nbw, const float *__restrict__ bwacc,
-                                   const DevACWeight *__restrict__ acw, int nacw, const float *__restrict__ acwacc,
+__global__ void k_finalise_weights(const DevWeightOut *__restrict__ wout, int n, const float *__restrict__ wacc,
                                    float *__restrict__ corefloat)
 {
-	int k = blockIdx.x * blockDim.x + threadIdx.x;
-	if(k < nbw)
-		corefloat[bw[k].dst] = bwacc[k];
-	else if(k < nbw + nacw)
-		corefloat[acw[k - nbw].dst] = acwacc[k - nbw];
+	const int k = blockIdx.x * blockDim.x + threadIdx.x;
+	if(k < n)
+		corefloat[wout[k].dst] = wacc[wout[k].sum];
 }
 
-void launch_finalise(const DevOutMap *om, int nom, int maxout, const float2 *acc, const DevBWeight *bw, int nbw,
-                     const float *bwacc, const DevACWeight *acw, int nacw, const float *acwacc, float2 *core,
-                     int64_t corelen, cudaStream_t stream)
+void launch_finalise(const DevOutMap *om, int nom, const float2 *acc, const DevWeightOut *wout, int nwout,
+                     const float *wacc, float2 *core, int64_t corelen, cudaStream_t stream)
 {
-	(void)maxout;
 	cudaMemsetAsync(core, 0, sizeof(float2) * corelen, stream);
 	if(nom > 0)
 		k_finalise<<<nom, 256, 0, stream>>>(om, acc, core);
-	int n = nbw + nacw;
-	if(n > 0)
-		k_finalise_weights<<<(n + 127) / 128, 128, 0, stream>>>(bw, nbw, bwacc, acw, nacw, acwacc, (float *)core);
+	if(nwout > 0)
+		k_finalise_weights<<<(nwout + 127) / 128, 128, 0, stream>>>(wout, nwout, wacc, (float *)core);
 }
 
 // Stand-alone decode with mark5_unpack_with_offset's contract

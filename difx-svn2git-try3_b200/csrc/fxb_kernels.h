@@ -30,14 +30,17 @@ struct DevOutMap {
 	int32_t cstride, pad;
 };
 
-struct DevBWeight {
-	int32_t s1, s2, b1, b2;   // stations and recorded bands
-	int64_t dst;
+// A weight sum: stations and, of INTERLACEDVDIF stations, recorded bands (-1:
+// the station's own weight); s2 = -1: the weights of s1 alone.
+struct DevWeightSum {
+	int32_t s1, s2, b1, b2;
 };
 
-struct DevACWeight {
-	int32_t s, band;          // station and band (per-band weights of INTERLACEDVDIF stations)
+// A weight slot of the core result (float index) and the sum it shows.  The
+// products of one baseline share a sum, so do a station's autocorrelations.
+struct DevWeightOut {
 	int64_t dst;
+	int32_t sum, pad;
 };
 
 // One zoom-band row: spectra channels [choff, choff + nchan) of row src_row
@@ -64,7 +67,8 @@ void launch_prep(const DevStation *st, DevSubintStation *sub, int S, int blocksp
                  uint32_t *bandok, int64_t valid_stride, cudaStream_t stream, uint8_t *fillok);
 void launch_fft_params(const DevStation *st, const DevSubintStation *sub, const int32_t *validflags, int nflagint,
                        const uint8_t *valid, const uint32_t *bandok, int64_t valid_stride, int S, int T, int order,
-                       FftParam *out, float *pbw, int nbm, cudaStream_t stream, const uint8_t *fillok = nullptr);
+                       FftParam *out, float *pbw, int nbm, cudaStream_t stream, const uint8_t *fillok = nullptr,
+                       float *wts = nullptr);
 
 // Fused unpack -> fringe rotation -> FFT -> fractional-sample correction.
 // One CTA per (station, FFT); writes FP32 spectra into spec.  Returns the
@@ -319,14 +323,13 @@ void launch_pcal_final(const DevPcalBand *bands, int nbands, int nchunk, int64_t
 void launch_zoom_gather(const DevZoomCopy *zc, int nzc, const DevFreqPlan *plans, int T, bool tc, void *spec,
                         cudaStream_t stream);
 
+// adds the subint's weight sums to acc[nsum].  wts: data weights [station][FFT];
 // pbw: per-band data weights [station][FFT][nbm] of INTERLACEDVDIF stations (null: none)
-void launch_weights(const DevBWeight *bw, int nbw, const DevACWeight *acw, int nacw, const FftParam *params,
-                    const float *pbw, int nbm, const DevStation *st, int T, float *bwacc, float *acwacc,
+void launch_weights(const DevWeightSum *sums, int nsum, const float *wts, const float *pbw, int nbm, int T, float *acc,
                     cudaStream_t stream);
 
-void launch_finalise(const DevOutMap *om, int nom, int maxout, const float2 *acc, const DevBWeight *bw, int nbw,
-                     const float *bwacc, const DevACWeight *acw, int nacw, const float *acwacc, float2 *core,
-                     int64_t corelen, cudaStream_t stream);
+void launch_finalise(const DevOutMap *om, int nom, const float2 *acc, const DevWeightOut *wout, int nwout,
+                     const float *wacc, float2 *core, int64_t corelen, cudaStream_t stream);
 
 void launch_vdif_unpack(const uint8_t *data, int64_t nbytes, int payload, int header, int nchan, int nbits,
                         int64_t offsetsamples, int nsamp, float *out, int *good, cudaStream_t stream);

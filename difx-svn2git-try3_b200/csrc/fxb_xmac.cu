@@ -11,7 +11,7 @@
 // Bound: the FP32 pipe and the shared-memory reads, R R complex products (4
 // R R FFMA) per 2 R eight-byte loads of a warp; the registers (2 R R sums)
 // decide how many warps hide each other's latencies.  20 rows x 1024 channels
-// x 8 subbands x 250 times: R = 5 in 96 registers (20 warps per SM) 147 us,
+// x 8 subbands x 250 times: R = 5 in 96 registers (20 warps per SM) 144 us,
 // R = 4 in 64 (30 warps) 159 us, R = 5 in 80 161 us, R = 5 in 128 (10 warps)
 // 210 us; the FFMAs alone take 53 us.  Packed FFMA2 (fma.rn.f32x2) runs at half
 // the rate of FFMA and needs twice the sums: 160 us.  60 rows x 2048 x 2 x 26:
@@ -26,7 +26,7 @@
 // order, so a result depends on the job alone, never on the schedule.
 // Measured: 4 stations, 256 channels, T = 250: 142 -> 12 us; 7 rows x 64
 // channels x 16 subbands, T = 2005: 552 -> 60 us; 10 stations x 8 x 1024
-// channels, T = 250: 198 -> 147 us.
+// channels, T = 250: 198 -> 144 us.
 
 #include <cuda_runtime.h>
 #include <cooperative_groups.h>
