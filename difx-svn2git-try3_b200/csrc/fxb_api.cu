@@ -629,7 +629,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 		{
 			const Job::Station &js = job.stations[s];
 			const int N = ctx->h_st[s].fftchannels;
-			const bool pairs = N <= 2048;
+			const bool pairs = N <= 8192;
 			std::vector<int> done(js.nband, 0);
 			for(int b = 0; b < js.nband; b++)
 			{
@@ -764,8 +764,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 				CK(ctx, cudaMemcpyAsync(d, h.data(), sizeof(float2) * h.size(), cudaMemcpyHostToDevice, ctx->stream));
 				k.tw = d;
 			}
-			bool wide = false;
-			if(out == 1 && !k.tcfft && !k.cplx && fstage_multi_shape(k.N, k.nb, &wide))
+			if(out == 1 && !k.tcfft && !k.cplx && fstage_multi_class(k.N, k.nb) >= 0)
 				k.persist = 1;
 			hg.insert(hg.end(), kv.second.begin(), kv.second.end());
 			ctx->fkinds.push_back(k);
@@ -773,15 +772,11 @@ static fxb_status setup_device(fxb_ctx *ctx)
 		// the persistent launches' work list: per kind tq x fpc FFT times of
 		// one item per unit, times outer and items inner
 		{
-			// classes: wide, two-band narrow, one-band narrow units of plain
-			// VDIF, then of raw reads
 			std::vector<FsMultiUnit> cls[kFsMultiClasses];
 			for(const FKind &k : ctx->fkinds)
 			{
 				if(!k.persist)
 					continue;
-				bool w = false;
-				fstage_multi_shape(k.N, k.nb, &w);
 				FsMultiKind mk;
 				memset(&mk, 0, sizeof(mk));
 				mk.tw = k.tw;
@@ -794,7 +789,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 				const int ki = (int)ctx->pkinds.size();
 				ctx->pkinds.push_back(mk);
 				const int per = mk.tq * k.fpc, nt = (ctx->T + per - 1) / per;
-				std::vector<FsMultiUnit> &dst = cls[3 * k.muxraw + (w ? 0 : 3 - k.nb)];
+				std::vector<FsMultiUnit> &dst = cls[kFsMultiPer * k.muxraw + fstage_multi_class(k.N, k.nb)];
 				for(int t = 0; t < nt; t++)
 					for(int it = 0; it < k.count; it++)
 						dst.push_back(FsMultiUnit{ki, it, t});

@@ -1,0 +1,728 @@
+// F stage of a work item with both polarisations of a subband (device code;
+// fxb_fstage.cuh has the stage's description and its one-band form).
+//
+// The two bands of a subband share their FFT times, fringe rotation,
+// fractional-sample rotation and twiddles; only their samples differ.  A value
+// is therefore a pair of bands, held as two packed registers (band 0, band 1)
+// of real and of imaginary parts:
+//  - the butterflies' additions are packed FP32 (add.rn.f32x2), half the
+//    instructions; products with a scalar (twiddles, rotators) use the two
+//    halves as plain registers, which costs no moves;
+//  - an exchange element is 16 bytes, so that a shared-memory instruction
+//    carries both bands; element i sits at i + i / 8, free of bank conflicts
+//    for every pass;
+//  - the sideband's half of the last pass alone is computed: its outputs k and
+//    k + N/2 differ by the sign of the odd inputs, which the packed FMA takes
+//    as a factor, so that one code serves both sidebands;
+//  - a thread's four output channels are N/8 apart: their fractional-sample
+//    rotators follow from the first by one step per FFT, computed once;
+//  - the window of a valid FFT in frames of at least N/8 samples is read with
+//    one running bit position; other windows take the general loop.
+// An FFT of up to 256 points lies within a warp and exchanges without CTA
+// barriers, one of 512 or 1024 points synchronises its own threads only.
+//
+// Bound: instruction issue (FFT arithmetic about half of it).  Thread
+// instructions per sample of a band and launch times before and after are
+// with the kernels in fxb_fs_pair_tc.cu.
+#pragma once
+
+#include "fxb_fstage.cuh"
+
+namespace fxb {
+
+namespace {
+
+typedef unsigned long long u64;
+
+__device__ __forceinline__ u64 pk2(float a, float b)
+{
+	u64 d;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+	return d;
+}
+__device__ __forceinline__ float2 up2(u64 v)
+{
+	float2 r;
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+	return r;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b)
+{
+	u64 d;
+	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+	return d;
+}
+__device__ __forceinline__ u64 sub2(u64 a, u64 b)
+{
+	u64 d;
+	asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+	return d;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b)
+{
+	u64 d;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+	return d;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c)
+{
+	u64 d;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+	return d;
+}
+
+// one complex value of both bands: (band 0, band 1) real and imaginary parts
+struct cp {
+	u64 re, im;
+};
+
+__device__ __forceinline__ cp add(cp a, cp b) { return {add2(a.re, b.re), add2(a.im, b.im)}; }
+__device__ __forceinline__ cp sub(cp a, cp b) { return {sub2(a.re, b.re), sub2(a.im, b.im)}; }
+__device__ __forceinline__ cp add_mi(cp a, cp b) { return {add2(a.re, b.im), sub2(a.im, b.re)}; }   // a - i b
+__device__ __forceinline__ cp add_pi(cp a, cp b) { return {sub2(a.re, b.im), add2(a.im, b.re)}; }   // a + i b
+__device__ __forceinline__ cp rot45(cp a)                                                            // a (1 - i) / sqrt2
+{
+	const u64 r = pk2(0.70710678118654752440f, 0.70710678118654752440f);
+	return {mul2(add2(a.re, a.im), r), mul2(sub2(a.im, a.re), r)};
+}
+// rounded in one fixed way, so that every instance of the code agrees
+__device__ __forceinline__ void rot1(float &x, float &y, float c, float s)
+{
+	const float xr = fmaf(x, c, -__fmul_rn(y, s)), xi = fmaf(x, s, __fmul_rn(y, c));
+	x = xr;
+	y = xi;
+}
+__device__ __forceinline__ cp twid(cp a, float2 w)
+{
+	float2 r = up2(a.re), i = up2(a.im);
+	rot1(r.x, i.x, w.x, w.y);
+	rot1(r.y, i.y, w.x, w.y);
+	return {pk2(r.x, r.y), pk2(i.x, i.y)};
+}
+
+// outputs 0 .. R/2 - 1 of the R-point DFT with the odd inputs times sg (1: the
+// first R/2 bins, -1: the second R/2); nsg = -sg
+template <int R>
+__device__ __forceinline__ void dft_half(const cp *x, cp *y, u64 sg, u64 nsg)
+{
+	if constexpr(R == 8)
+	{
+		const cp a0 = add(x[0], x[4]), d0 = sub(x[0], x[4]), a2 = add(x[2], x[6]), d2 = sub(x[2], x[6]);
+		const cp a1 = add(x[1], x[5]), d1 = sub(x[1], x[5]), a3 = add(x[3], x[7]), d3 = sub(x[3], x[7]);
+		const cp b0 = add(a0, a2), b2 = sub(a0, a2), b1 = add(a1, a3), b3 = sub(a1, a3);
+		const cp f0 = add_mi(d0, d2), f2 = add_pi(d0, d2);
+		const cp f1 = rot45(add_mi(d1, d3)), f3 = rot45(add_pi(d1, d3));
+		y[0] = {fma2(b1.re, sg, b0.re), fma2(b1.im, sg, b0.im)};
+		y[1] = {fma2(f1.re, sg, f0.re), fma2(f1.im, sg, f0.im)};
+		y[2] = {fma2(b3.im, sg, b2.re), fma2(b3.re, nsg, b2.im)};
+		y[3] = {fma2(f3.im, sg, f2.re), fma2(f3.re, nsg, f2.im)};
+	}
+	else if constexpr(R == 4)
+	{
+		const cp b0 = add(x[0], x[2]), b2 = sub(x[0], x[2]), b1 = add(x[1], x[3]), b3 = sub(x[1], x[3]);
+		y[0] = {fma2(b1.re, sg, b0.re), fma2(b1.im, sg, b0.im)};
+		y[1] = {fma2(b3.im, sg, b2.re), fma2(b3.re, nsg, b2.im)};
+	}
+	else
+		y[0] = {fma2(x[1].re, sg, x[0].re), fma2(x[1].im, sg, x[0].im)};
+}
+
+__device__ __forceinline__ constexpr int ppad(int i) { return i + (i >> 3); }
+
+__device__ __forceinline__ cp ldx(const ulonglong2 *p)
+{
+	const ulonglong2 v = *p;
+	return {v.x, v.y};
+}
+__device__ __forceinline__ void stx(ulonglong2 *p, cp v) { *p = make_ulonglong2(v.re, v.im); }
+
+// exp(2 pi i x) of a double, rounded once (the float angle's remainder enters
+// to first order)
+__device__ __forceinline__ float2 cispi2(double x)
+{
+	const double y = 2.0 * (x - rint(x));
+	const float yf = (float)y, dy = (float)(y - (double)yf) * 3.14159265358979f;
+	float s, c;
+	sincospif(yf, &s, &c);
+	return make_float2(fmaf(-s, dy, c), fmaf(c, dy, s));
+}
+
+// Threads, slots (FFTs side by side) and exchange buffer of length 2^LOGN.
+template <int LOGN>
+struct PShape {
+	static constexpr int N = 1 << LOGN;
+	static constexpr int TPF = N / 8;                        // threads per FFT, one butterfly each
+	static constexpr int NT = TPF > 256 ? TPF : 256;
+	static constexpr int FPC = NT / TPF;
+	static constexpr int PADN = N + N / 8;                   // elements of 16 bytes
+	static constexpr int NMID = (LOGN % 3 == 0) ? LOGN / 3 - 2 : LOGN / 3 - 1;
+	static constexpr int RL = (LOGN % 3 == 0) ? 8 : (1 << (LOGN % 3));
+	// CTAs per SM: 80 registers up to 2048 points, 64 above
+	static constexpr int MINB = NT == 256 ? 3 : 1024 / NT;
+};
+
+// the threads of one FFT meet
+template <int LOGN>
+__device__ __forceinline__ void slot_sync(int slot)
+{
+	using SH = PShape<LOGN>;
+	if constexpr(SH::TPF <= 32)
+		__syncwarp();
+	else if constexpr(SH::FPC > 1)
+		asm volatile("bar.sync %0, %1;\n" ::"r"(1 + slot), "n"(SH::TPF) : "memory");
+	else
+		__syncthreads();
+}
+
+// One middle radix-8 pass (stride s = 2^LOGS, m = N / (8 s)): x_r = X[q + s (p
+// + r m)], y = DFT8(x), Y[q + s (8 p + r)] = y_r w_N^(r p s).
+template <int LOGN, int LOGS>
+__device__ __forceinline__ void pair_mid(ulonglong2 *side, int slot, int b, const float2 *twp)
+{
+	using SH = PShape<LOGN>;
+	constexpr int N = SH::N, s = 1 << LOGS, np = N / (8 * s);
+	const int q = b & (s - 1), p8 = b >> LOGS;
+	cp x[8];
+#pragma unroll
+	for(int r = 0; r < 8; r++)
+	{
+		// N/8 a multiple of 8 (N >= 64): the padding is a constant offset per r
+		if constexpr(N >= 64)
+			x[r] = ldx(side + ppad(b) + r * ppad(N / 8));
+		else
+			x[r] = ldx(side + ppad(b + r * (N / 8)));
+	}
+	float2 w[8];
+#pragma unroll
+	for(int r = 1; r < 8; r++)
+		w[r] = ldtw(twp, (r - 1) * np + p8);
+	dft8(x);
+#pragma unroll
+	for(int r = 1; r < 8; r++)
+		x[r] = twid(x[r], w[r]);
+	slot_sync<LOGN>(slot);
+	// s is a multiple of 8, so is q + 8 s p8 + s r - q: constant offsets again
+	ulonglong2 *o = side + ppad(q + s * 8 * p8);
+#pragma unroll
+	for(int r = 0; r < 8; r++)
+		stx(o + r * ppad(s), x[r]);
+	slot_sync<LOGN>(slot);
+}
+
+template <int LOGN, int PS>
+__device__ __forceinline__ void pair_mids(ulonglong2 *side, int slot, int b, const float2 *tw)
+{
+	if constexpr(PS < PShape<LOGN>::NMID)
+	{
+		pair_mid<LOGN, 3 * (PS + 1)>(side, slot, b, tw + tw_offset(1 << LOGN, PS + 1));
+		pair_mids<LOGN, PS + 1>(side, slot, b, tw);
+	}
+}
+
+// Constants of one FFT, computed by one thread.
+struct PairConst {
+	float P0, alpha, beta, gamma, eps;   // fringe phase (turns): start and per-sample terms
+	float2 st;                           // order 1: rotator step over N/8 samples, exp(-2 pi i alpha N/8)
+	float dhi[2], dlo[2];                // fractional-sample turns per channel of each band (split_turns)
+	float2 os[2];                        // rotator step over N/8 channels of each band
+	float post[2];                       // order-0 post-F turns and the band's phase offset
+	uint32_t fa, so;                     // first frame of the window, window start within it
+	uint32_t fmask;                      // validity of the window's frames (bit k: frame fa + k)
+	int32_t stuck;                       // samples [stuck, N) read as zero
+	int32_t flags;
+	int32_t mi00, mi01, mi10, mi11;      // raw reads: thread frames of the window's first and second frame, per band
+};
+enum : int32_t {
+	kPActive = 1,     // valid FFT
+	kPNarrow = 2,     // fmask covers the window
+	kPBlank = 4,      // a valid frame of the window blanks one of the item's bands
+	kPSame = 8,       // the two bands take the same output rotation
+	kPFast = 16       // every sample of the window counts and the fast read applies
+};
+
+}  // namespace
+
+// One work unit: FFT times [tchunk tq FPC, +tq FPC) of work item gidx (an
+// FGroup of two bands), run by the CTA's PShape<LOGN>::NT threads.
+// VAR 1: raw INTERLACEDVDIF reads; VAR 2: complex sampling.
+template <int LOGN, bool TCO, int VAR>
+__device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx, const int tchunk, const int tq,
+                                                 const float2 *tw, ulonglong2 *fsm, const float *lut8,
+                                                 const u64 *lut4, PairConst *fcs)
+{
+	using SH = PShape<LOGN>;
+	constexpr int N = SH::N, TPF = SH::TPF, FPC = SH::FPC, PADN = SH::PADN, RL = SH::RL;
+	constexpr bool MUX = VAR == 1, CPLX = VAR == 2;
+	constexpr int nchan = CPLX ? N : N / 2;
+	constexpr uint32_t S8 = N / 8;
+	const FGroup &g = a.groups[gidx];
+	const DevStation *Sp = a.st + g.station;
+	const uint32_t fs = (uint32_t)Sp->framesamples;
+	const int nbits = Sp->nbits;
+	constexpr uint32_t cpl = CPLX ? 2u : 1u;
+	const uint32_t bpt = MUX ? (uint32_t)nbits : (uint32_t)(Sp->nband * nbits) * cpl;
+	const int header = Sp->header, framebytes = Sp->framebytes;
+	const uint8_t *buf = a.sub[g.station].buf;
+	const uint8_t *vrow = a.valid + (int64_t)g.station * a.valid_stride;
+	const int32_t *mslot = MUX ? a.sub[g.station].mux_slot : nullptr;
+	const int64_t mk0 = MUX ? a.sub[g.station].mux_k0 : 0;
+	const int mnthr = Sp->nthr, minfb = Sp->inframebytes;
+	const int slot = threadIdx.x / TPF, b = threadIdx.x - slot * TPF;
+	ulonglong2 *const side = fsm + (size_t)slot * PADN;
+	const bool lsb = g.lsb != 0;
+	const int band0 = g.band[0], band1 = g.band[1];
+	const uint32_t boff0 = MUX ? 0u : (uint32_t)(band0 * nbits) * cpl, boff1 = MUX ? 0u : (uint32_t)(band1 * nbits) * cpl;
+	// both bands side by side in one field of 2 nbits, aligned to its size
+	const bool adj = !MUX && !CPLX && boff1 == boff0 + (uint32_t)nbits && boff0 % (2u * (uint32_t)nbits) == 0;
+	const int order = a.order;
+	const int t0 = tchunk * tq * FPC;
+	const int nit = min(tq, (a.T - t0 + FPC - 1) / FPC);
+
+	// ---- constants of the unit's FFTs (FFT f is time t0 + f), one thread per FFT
+	for(int f = threadIdx.x; f < nit * FPC; f += blockDim.x)
+	{
+		const int t = t0 + f;
+		PairConst c;
+		memset(&c, 0, sizeof(c));
+		c.st = c.os[0] = c.os[1] = make_float2(1.0f, 0.0f);
+		const FftParam *pq = a.params + (int64_t)g.station * a.T + t;
+		if(t < a.T && pq->status == kFftOk)
+		{
+			c.flags = kPActive;
+			const uint32_t g0 = (uint32_t)pq->nearest;
+			c.fa = g0 / fs;
+			c.so = g0 - c.fa * fs;
+			c.stuck = pq->stuck;
+			const double invN = 1.0 / N, lo = g.lofreq;
+			const int idl = pq->integerdelay;
+			const double fraclo = a.fraclo ? (lo - (int)lo) * (double)idl : 0.0;
+			// LO offset: seconds since the job start of the FFT's first sample
+			// (mode.cpp:686-694; the scan starts with the job) and the offset's
+			// turns per sample
+			const double walls = (double)a.sub[g.station].subsec + a.sub[g.station].subns / 1.0e9 +
+			                     (double)t * N * Sp->sampletime / 1.0e6;
+			const double low = g.corr ? looff_wall_turns(g.looff, walls) : 0.0;
+			const double los = -g.looff * Sp->sampletime / 1.0e6;
+			double postf = 0.0;
+			if(order == 1)
+			{
+				c.P0 = frac_centered(lo * pq->b + fraclo + low);
+				c.alpha = (float)(lo * pq->a * invN + los);
+				c.st = cispi2(-(double)c.alpha * (double)S8);
+			}
+			else if(order == 2)
+			{
+				const double pa = pq->a, pb = pq->b;
+				const double X1 = (double)Sp->asl * invN;
+				c.P0 = frac_centered(lo * pq->c + fraclo + low);
+				c.alpha = (float)(lo * (pb + pa * X1) * invN + los);
+				c.beta = (float)(lo * 2.0 * pa * X1 * invN);
+				c.gamma = (float)(lo * pb * Sp->asl * invN + los * Sp->asl);
+				c.eps = (float)(lo * pa * X1 * X1);
+			}
+			else
+			{
+				double pr = (pq->averagedelay - idl) * lo;
+				if(a.fraclo)
+					pr += idl * (lo - (int)lo);
+				pr -= walls * g.looff;
+				postf = -(double)(float)(pr - (int)pr);
+			}
+			// per band: fse - clock offset (mode.cpp:1053-1059, 1099-1106); the
+			// channel of an order-0 lower sideband falls with the bin
+			const double sgn = lsb && (order == 0 || CPLX) ? -1.0 : 1.0;
+			c.flags |= kPSame;
+			for(int j = 0; j < 2; j++)
+			{
+				const double D = Sp->bw * (1.0 / nchan) * ((double)pq->fse - g.clk[j]);
+				split_turns(D, c.dhi[j], c.dlo[j]);
+				c.post[j] = (float)postf + g.phase[j];
+				if(j == 0 || g.clk[1] != g.clk[0])
+					c.os[j] = cispi2(sgn * D * (double)S8);
+				else
+					c.os[1] = c.os[0];
+			}
+			if(g.clk[1] != g.clk[0] || g.phase[1] != g.phase[0])
+				c.flags &= ~kPSame;
+			// validity of the window's frames, one bit per frame relative to fa
+			const uint32_t nwf = (c.so + (uint32_t)N - 1) / fs + 1, nm = nwf < 32u ? nwf : 32u;
+			for(uint32_t k = 0; k < nm; k++)
+			{
+				const int64_t fr = (int64_t)c.fa + k;
+				// complex data: the unpack's first frame is checked for fill
+				// pattern only (mark5_stream_unpacker.c:189)
+				const uint8_t *vsrc = (CPLX && k == 0 && a.fillok) ? a.fillok + (int64_t)g.station * a.valid_stride : vrow;
+				if(fr < a.valid_stride && vsrc[fr] != 0)
+					c.fmask |= 1u << k;
+			}
+			if(nwf <= 32)
+				c.flags |= kPNarrow;
+			if(a.bandok)
+			{
+				// EDV4-blanked bands (INTERLACEDVDIF): the general decode path below
+				const uint32_t need = (1u << band0) | (1u << band1);
+				for(uint32_t k = 0; k < nwf; k++)
+				{
+					const int64_t fk = (int64_t)c.fa + k;
+					if(fk < a.valid_stride && vrow[fk] != 0 &&
+					   (a.bandok[(int64_t)g.station * a.valid_stride + fk] & need) != need)
+						c.flags |= kPBlank;
+				}
+			}
+			const bool whole = nwf < 32 && c.fmask == (1u << nwf) - 1u && c.stuck >= N && !(c.flags & kPBlank);
+			if(whole && adj && fs >= S8)
+				c.flags |= kPFast;
+			if(MUX && whole && nwf <= 2)
+			{
+				// valid frames of raw reads are complete slots: every thread is there
+				c.flags |= kPFast;
+				const int32_t *s0 = mslot + (mk0 + (int64_t)c.fa) * mnthr, *s1 = nwf == 2 ? s0 + mnthr : s0;
+				c.mi00 = s0[band0];
+				c.mi01 = s0[band1];
+				c.mi10 = s1[band0];
+				c.mi11 = s1[band1];
+			}
+		}
+		fcs[f] = c;
+	}
+	__syncthreads();
+
+	for(int it = 0; it < nit; it++)
+	{
+		const int t = t0 + it * FPC + slot;
+		const PairConst &fc = fcs[it * FPC + slot];
+		const int flags = fc.flags;
+		// ---- 1. decode: the levels of samples b + r N/8 of both bands
+		u64 lv[8], lu[CPLX ? 8 : 1];        // lu: imaginary parts (complex sampling)
+		const uint32_t so = fc.so, xs = so + (uint32_t)b;
+		if(!CPLX && !MUX && (flags & kPFast))
+		{
+			// one running bit position: a frame boundary skips a header
+			// (so < fs and b < N/8 <= fs: at most one boundary before sample b)
+			uint32_t tin = xs, bit = xs * bpt + boff0;
+			if(tin >= fs)
+			{
+				tin -= fs;
+				bit += (uint32_t)header * 8u;
+			}
+			const uint32_t *wp = (const uint32_t *)(buf + (int64_t)fc.fa * framebytes + header);
+			uint32_t raw[8], sh[8];
+#pragma unroll
+			for(int r = 0; r < 8; r++)
+			{
+				raw[r] = __ldg(wp + (bit >> 5));
+				sh[r] = bit & 31u;
+				tin += S8;
+				bit += S8 * bpt;
+				if(tin >= fs)
+				{
+					tin -= fs;
+					bit += (uint32_t)header * 8u;
+				}
+			}
+			if(nbits == 2)
+			{
+#pragma unroll
+				for(int r = 0; r < 8; r++)
+					lv[r] = lut4[(raw[r] >> sh[r]) & 15u];
+			}
+			else
+			{
+#pragma unroll
+				for(int r = 0; r < 8; r++)
+				{
+					const uint32_t w = raw[r] >> sh[r];
+					lv[r] = pk2(lut8[w & 255u], lut8[(w >> 8) & 255u]);
+				}
+			}
+		}
+		else if(MUX && (flags & kPFast))
+		{
+			const uint8_t *f00 = buf + (int64_t)fc.mi00 * minfb + 32, *f01 = buf + (int64_t)fc.mi01 * minfb + 32;
+			const uint8_t *f10 = buf + (int64_t)fc.mi10 * minfb + 32, *f11 = buf + (int64_t)fc.mi11 * minfb + 32;
+			uint32_t raw0[8], raw1[8], sh[8];
+#pragma unroll
+			for(int r = 0; r < 8; r++)
+			{
+				const uint32_t x = xs + r * S8;
+				const bool second = x >= fs;
+				const uint32_t bit = (second ? x - fs : x) * bpt;
+				raw0[r] = __ldg((const uint32_t *)(second ? f10 : f00) + (bit >> 5));
+				raw1[r] = __ldg((const uint32_t *)(second ? f11 : f01) + (bit >> 5));
+				sh[r] = bit & 31u;
+			}
+#pragma unroll
+			for(int r = 0; r < 8; r++)
+			{
+				const uint32_t w0 = raw0[r] >> sh[r], w1 = raw1[r] >> sh[r];
+				if(nbits == 2)
+					lv[r] = lut4[(w0 & 3u) | ((w1 & 3u) << 2)];
+				else
+					lv[r] = pk2(lut8[w0 & 255u], lut8[w1 & 255u]);
+			}
+		}
+		else
+		{
+			// frames, validity and blanking sample by sample
+			const bool narrow = (flags & kPNarrow) != 0, blank = (flags & kPBlank) != 0;
+			uint32_t kf = xs / fs, tin = xs - kf * fs;
+#pragma unroll
+			for(int r = 0; r < 8; r++)
+			{
+				const int n = b + r * (int)S8;
+				const int64_t fr = (int64_t)fc.fa + kf;
+				bool ok;
+				if(narrow)
+					ok = (fc.fmask >> kf) & 1u;
+				else
+					ok = (flags & kPActive) && fr < a.valid_stride && vrow[fr] != 0;
+				ok = ok && n < fc.stuck;
+				float v0 = 0.0f, v1 = 0.0f, u0 = 0.0f, u1 = 0.0f;
+				if(ok)
+				{
+					const uint32_t bit0 = tin * bpt + boff0, bit1 = tin * bpt + boff1;
+					uint32_t w0, w1;
+					if constexpr(MUX)
+					{
+						const int32_t *slr = mslot + (mk0 + fr) * mnthr;
+						const int i0 = __ldg(slr + band0), i1 = __ldg(slr + band1);
+						w0 = i0 >= 0 ? __ldg((const uint32_t *)(buf + (int64_t)i0 * minfb + 32) + (bit0 >> 5)) : 0u;
+						w1 = i1 >= 0 ? __ldg((const uint32_t *)(buf + (int64_t)i1 * minfb + 32) + (bit1 >> 5)) : 0u;
+					}
+					else
+					{
+						const uint32_t *wp = (const uint32_t *)(buf + fr * framebytes + header);
+						w0 = __ldg(wp + (bit0 >> 5));
+						w1 = __ldg(wp + (bit1 >> 5));
+					}
+					w0 >>= bit0 & 31u;
+					w1 >>= bit1 & 31u;
+					v0 = nbits == 2 ? level2(w0 & 3u) : lut8[w0 & 255u];
+					v1 = nbits == 2 ? level2(w1 & 3u) : lut8[w1 & 255u];
+					if constexpr(CPLX)
+					{
+						u0 = nbits == 2 ? level2((w0 >> 2) & 3u) : lut8[(w0 >> 8) & 255u];
+						u1 = nbits == 2 ? level2((w1 >> 2) & 3u) : lut8[(w1 >> 8) & 255u];
+					}
+					if(blank)
+					{
+						// bands of this sample's frame blanked by its EDV4 validity mask
+						// (blank_vdif_EDV4, format_vdif.c:4699-4780)
+						const uint32_t bo = a.bandok[(int64_t)g.station * a.valid_stride + fr];
+						if(!((bo >> band0) & 1u))
+							v0 = u0 = 0.0f;
+						if(!((bo >> band1) & 1u))
+							v1 = u1 = 0.0f;
+					}
+				}
+				lv[r] = pk2(v0, v1);
+				if constexpr(CPLX)
+					lu[r] = pk2(u0, u1);
+				tin += S8;
+				while(tin >= fs)
+				{
+					tin -= fs;
+					kf++;
+				}
+			}
+		}
+		// ---- 2. fringe rotation (order 1: the rotator of sample b, then one
+		// complex step per N/8 samples), first radix-8 pass (butterfly b, twiddle
+		// w_N^(r b))
+		cp x[8];
+		{
+			float rc = 1.0f, rs = 0.0f;
+			if(order == 1)
+			{
+				float ph = fmaf((float)b, fc.alpha, fc.P0);
+				ph -= rintf(ph);
+				__sincosf(-6.283185307179586f * ph, &rs, &rc);
+			}
+			const float2 st = fc.st;
+#pragma unroll
+			for(int r = 0; r < 8; r++)
+			{
+				if(order == 2)
+				{
+					const int n = b + r * (int)S8, asl = Sp->asl;
+					const int kk = n / asl, jj = n - kk * asl;
+					float ph = fc.P0 + (float)jj * fc.alpha + (float)(kk * jj) * fc.beta + (float)kk * fc.gamma +
+					           (float)(kk * kk) * fc.eps;
+					ph -= rintf(ph);
+					__sincosf(-6.283185307179586f * ph, &rs, &rc);
+				}
+				const float2 v = up2(lv[r]);
+				if constexpr(CPLX)
+				{
+					const float2 u = up2(lu[r]);
+					x[r].re = pk2(fmaf(v.x, rc, -__fmul_rn(u.x, rs)), fmaf(v.y, rc, -__fmul_rn(u.y, rs)));
+					x[r].im = pk2(fmaf(v.x, rs, __fmul_rn(u.x, rc)), fmaf(v.y, rs, __fmul_rn(u.y, rc)));
+				}
+				else
+				{
+					x[r].re = pk2(__fmul_rn(v.x, rc), __fmul_rn(v.y, rc));
+					x[r].im = pk2(__fmul_rn(v.x, rs), __fmul_rn(v.y, rs));
+				}
+				if(order == 1 && r < 7)
+					rot1(rc, rs, st.x, st.y);
+			}
+		}
+		dft8(x);
+#pragma unroll
+		for(int r = 1; r < 8; r++)
+			x[r] = twid(x[r], ldtw(tw, (r - 1) * (N / 8) + b));
+		slot_sync<LOGN>(slot);              // the exchange buffer has been read by the last FFT
+		{
+			ulonglong2 *o = side + ppad(8 * b);
+#pragma unroll
+			for(int r = 0; r < 8; r++)
+				stx(o + r, x[r]);
+		}
+		slot_sync<LOGN>(slot);
+		// ---- 3. middle radix-8 passes through shared memory
+		pair_mids<LOGN, 0>(side, slot, b, tw);
+		// ---- 4. last pass, sideband, fractional-sample rotation, output
+		if(t >= a.T)
+			continue;
+		const DevFreqPlan &P = a.plans[g.freq];
+		constexpr int sL = N / RL, J = 8 / RL;
+		const int row0 = g.row[0], row1 = g.row[1];
+		constexpr float osc = TCO ? 1.0f / (float)(1 << kTcSpecExp) : 1.0f;
+		const bool same = (flags & kPSame) != 0, h16 = a.h16 != 0;
+		// spectra: FP32 form [t][row][chan]; tensor-core form blocked
+		// [t][block][row][tcb] (tcb channels per block; 0: [t][row][chan])
+		const uint32_t tcb = TCO ? (uint32_t)P.tcb : 0u;
+		const uint32_t magic = tcb ? 0xFFFFFFFFu / tcb + 1u : 0u;      // c / tcb = umulhi(c, magic) for c < 2^16
+		const uint32_t rstr = tcb ? tcb : (uint32_t)nchan, bextra = tcb ? (uint32_t)P.nrow * tcb - tcb : 0u;
+		const int64_t tb = P.spec_off + (int64_t)t * (tcb ? (int64_t)P.tnblk * P.nrow * tcb : (int64_t)P.nrow * nchan);
+		auto put = [&](uint32_t c, const cp &y, float cj, float c0, float s0, float c1, float s1) {
+			float2 re = up2(y.re), im = up2(y.im);
+			im.x *= cj;
+			im.y *= cj;
+			rot1(re.x, im.x, c0, s0);
+			rot1(re.y, im.y, c1, s1);
+			const uint32_t off = TCO ? c + __umulhi(c, magic) * bextra : c;
+			if constexpr(TCO)
+			{
+				uint32_t *o = (uint32_t *)a.spec + tb + off;
+				if(row0 >= 0)
+					o[(uint32_t)row0 * rstr] = pack_spec(h16, re.x, im.x);
+				if(row1 >= 0)
+					o[(uint32_t)row1 * rstr] = pack_spec(h16, re.y, im.y);
+			}
+			else
+			{
+				float2 *o = (float2 *)a.spec + tb + off;
+				if(row0 >= 0)
+					o[(uint32_t)row0 * rstr] = make_float2(re.x, im.x);
+				if(row1 >= 0)
+					o[(uint32_t)row1 * rstr] = make_float2(re.y, im.y);
+			}
+		};
+		// rotator exp(2 pi i (ce D + post)) of band j at effective channel ce,
+		// D = hi + lo (ce hi exact), times the spectra's scale
+		auto rotator = [&](int j, int ce) {
+			const float fce = (float)ce;
+			float h = fce * fc.dhi[j];
+			h -= rintf(h);
+			float turns = h + fmaf(fce, fc.dlo[j], fc.post[j]);
+			turns -= rintf(turns);
+			float2 w;
+			__sincosf(6.283185307179586f * turns, &w.y, &w.x);
+			w.x *= osc;
+			w.y *= osc;
+			return w;
+		};
+		if constexpr(CPLX)
+		{
+			// every bin is a channel; the lower sideband keeps bin 0 and mirrors and
+			// conjugates the rest (mode.cpp:1217-1226)
+#pragma unroll
+			for(int jj = 0; jj < J; jj++)
+			{
+				cp y[RL];
+#pragma unroll
+				for(int r = 0; r < RL; r++)
+					y[r] = ldx(side + ppad(b + jj * TPF + sL * r));
+				dftR<RL>(y);
+#pragma unroll
+				for(int r = 0; r < RL; r++)
+				{
+					const int k = b + jj * TPF + sL * r;
+					const int c = !lsb || k == 0 ? k : N - k, ce = lsb ? c - nchan : c;
+					const float2 w0 = rotator(0, ce), w1 = same ? w0 : rotator(1, ce);
+					put((uint32_t)c, y[r], !lsb || k == 0 ? 1.0f : -1.0f, w0.x, w0.y, w1.x, w1.y);
+				}
+			}
+		}
+		else
+		{
+			// the thread's outputs are bins kb + b + m N/8, m = 0 .. 3: channel m N/8 +
+			// b of the sideband; order-0 lower sideband: channel nchan - k, conjugated
+			const bool mirror = lsb && order == 0;
+			const float sgf = lsb && !mirror ? -1.0f : 1.0f;
+			const u64 sg = pk2(sgf, sgf), nsg = pk2(-sgf, -sgf);
+			const int ce = mirror ? -b : (lsb ? b - nchan : b);
+			float2 w0 = rotator(0, ce), w1 = same ? w0 : rotator(1, ce);
+			const float2 os0 = fc.os[0], os1 = fc.os[1];
+			const float cj = mirror ? -1.0f : 1.0f;
+			cp y[4];
+#pragma unroll
+			for(int jj = 0; jj < J; jj++)
+			{
+				cp z[RL], h[RL / 2];
+#pragma unroll
+				for(int r = 0; r < RL; r++)
+				{
+					if constexpr(N >= 64)
+						z[r] = ldx(side + ppad(b) + jj * ppad(TPF) + r * ppad(sL));
+					else
+						z[r] = ldx(side + ppad(b + jj * TPF + sL * r));
+				}
+				dft_half<RL>(z, h, sg, nsg);
+				// output r of group jj is bin b + jj N/8 + r N/RL
+#pragma unroll
+				for(int r = 0; r < RL / 2; r++)
+					y[jj + r * J] = h[r];
+				if(mirror && jj == 0 && b == 0)
+				{
+					// bin N/2, channel 0
+					const float2 m0 = rotator(0, -nchan), m1 = same ? m0 : rotator(1, -nchan);
+					dft_half<RL>(z, h, nsg, sg);
+					put(0u, h[0], -1.0f, m0.x, m0.y, m1.x, m1.y);
+				}
+			}
+#pragma unroll
+			for(int m = 0; m < 4; m++)
+			{
+				const int k = b + m * (int)S8;
+				if(mirror)
+				{
+					if(k > 0)
+						put((uint32_t)(nchan - k), y[m], cj, w0.x, w0.y, w1.x, w1.y);
+				}
+				else
+					put((uint32_t)k, y[m], 1.0f, w0.x, w0.y, w1.x, w1.y);
+				if(m < 3)
+				{
+					rot1(w0.x, w0.y, os0.x, os0.y);
+					if(same)
+						w1 = w0;
+					else
+						rot1(w1.x, w1.y, os1.x, os1.y);
+				}
+			}
+		}
+	}
+}
+
+// the level pairs of two adjacent 2-bit bands, and the 8-bit levels
+__device__ __forceinline__ void fstage_pair_luts(float *lut8, u64 *lut4)
+{
+	for(int i = threadIdx.x; i < 256; i += blockDim.x)
+		lut8[i] = (float)((i - 128) / 3.3);
+	if(threadIdx.x < 16)
+		lut4[threadIdx.x] = pk2(level2(threadIdx.x & 3u), level2(threadIdx.x >> 2u));
+}
+
+}  // namespace fxb

@@ -174,18 +174,28 @@ struct FsArgs {
 };
 
 bool fstage_plan(int N, int nb, int out, FKind *k);
+// the kernels of one-band and two-band items by output form, and the
+// persistent launch of a class (fxb_fs_*.cu)
+struct FsMultiArgs;
+void launch_fs_one_f32(const FKind &k, const FsArgs &a, cudaStream_t stream);
+void launch_fs_pair_f32(const FKind &k, const FsArgs &a, cudaStream_t stream);
+void launch_fs_one_tc(const FKind &k, const FsArgs &a, cudaStream_t stream);
+void launch_fs_pair_tc(const FKind &k, const FsArgs &a, cudaStream_t stream);
+void launch_fs_one_multi(const FsMultiArgs &m, int cls, int nsm, cudaStream_t st);
+void launch_fs_pair_multi(const FsMultiArgs &m, int cls, int nsm, cudaStream_t st);
 void launch_fstage_kind(const FKind &k, FsArgs a, cudaStream_t stream);
 
 // The persistent F-stage launches over the CUDA-core kinds of tensor-core-
 // form contexts (VDIF stations, plain or raw INTERLACEDVDIF reads) of one
 // context or several: CTAs take
 // work units from a list in order, each run as one CTA of launch_fstage_kind
-// runs it (tq x fpc FFT times of one work item).  Narrow units (FFTs of up to
-// 4096 points) run in CTAs of 256 threads, wide units (8192-point FFTs of one
-// band) in CTAs of 512, one launch each.  Every tensor-core-form context runs
-// these kinds this way, alone or in a batch, so results do not depend on it.
+// would run it (tq x fpc FFT times of one work item), one launch per class of
+// units.  Every tensor-core-form context runs these kinds this way, alone or in
+// a batch, so results do not depend on it.
 constexpr int kFsMultiMembers = 16;
-constexpr int kFsMultiFc = 128;          // FFT constants of one narrow unit at most (tq x fpc)
+constexpr int kFsMultiFc = 128;          // FFT constants of one unit of up to 2048 points at most (tq x fpc)
+// classes of units: plain VDIF's (fstage_multi_class), then those of raw reads
+constexpr int kFsMultiPer = 5, kFsMultiClasses = 2 * kFsMultiPer;
 struct FsMultiKind {
 	const void *tw;                      // twiddles of length N
 	int32_t member, code;                // context; 128 x raw INTERLACEDVDIF reads + 32 x bands per item + log2 N
@@ -197,15 +207,15 @@ struct FsMultiUnit {
 struct FsMultiArgs {
 	FsArgs m[kFsMultiMembers];           // per context, with its subint's staging
 	const FsMultiKind *kinds;
-	const FsMultiUnit *units;            // six classes: wide, two-band narrow and one-band narrow units
-	                                     // of plain VDIF, then of raw reads
-	int32_t unit0[6], nunit[6];          // each class's first unit and units
+	const FsMultiUnit *units;            // by class
+	int32_t unit0[kFsMultiClasses], nunit[kFsMultiClasses];   // each class's first unit and units
 	int32_t *ctr;                        // one counter per class, zero before the launch
 };
-constexpr int kFsMultiClasses = 6;
-// whether a kind (FFT length N, bands per item nb) runs in the persistent
-// launches, and as a wide unit; the FFT iterations per unit for a kind's tq
-bool fstage_multi_shape(int N, int nb, bool *wide);
+// class of a kind (FFT length N, bands per item nb) in the persistent launches
+// (0: two bands of 8192 points, 1: one band of 8192, 2: two bands of 4096, 3:
+// two bands of up to 2048, 4: one band of up to 4096; -1: not run there), and
+// the FFT iterations per unit for a kind's tq
+int fstage_multi_class(int N, int nb);
 int fstage_multi_tq(int N, int nb, int tq);
 cudaError_t launch_fstage_multi(const FsMultiArgs &m, int nsm, cudaStream_t stream);
 // the same with the class kernels spread over streams (each kernel on the
