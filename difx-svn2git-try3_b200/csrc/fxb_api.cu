@@ -154,6 +154,8 @@ struct fxb_ctx {
 		TcShape shape{};
 		int64_t spec_base = 0;                    // first bf16x2 value of the group's block
 		int64_t spec8_base = 0;                   // FP8 form: first e4m3x2 word of the group's block
+		float2 *ws = nullptr;                     // sums of the time slices (null: one slice)
+		int maxout = 0;                           // outputs of a subband, at most
 		alignas(64) unsigned char tmap[128];     // CUtensorMap of the block (64-byte aligned)
 	};
 	std::vector<XGroup> xgroups;
@@ -546,7 +548,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 		}
 	}
 	// tensor-core form: bf16x2 spectra, per group one block
-	// [subband][Tpad][nrow][nchan] (times past T stay zero), and
+	// [subband][Tpad][block][trow][CB] (times past T and rows past nrow stay zero), and
 	// [chan][output] accumulators
 	if(ctx->tc)
 	{
@@ -556,7 +558,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 		{
 			fxb_ctx::XGroup &g = ctx->xgroups[gi];
 			const DevFreqPlan &p0 = ctx->h_plans[g.plan0];
-			if(!tc_shape(p0.nrow, p0.nchan, ctx->T, ctx->f8, ctx->h16, &g.shape))
+			if(!tc_shape(p0.nrow, p0.nchan, g.nf, ctx->T, ctx->nsm, ctx->f8, ctx->h16, &g.shape))
 			{
 				ctx->err = "tensor-core XMAC: at most 64 inputs per subband";
 				return FXB_ERR_UNSUPPORTED;
@@ -564,7 +566,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 			g.spec_base = off;
 			g.spec8_base = ctx->spec8_elems;
 			const int nblk = (p0.nchan + g.shape.CB - 1) / g.shape.CB;
-			const int64_t per = (int64_t)g.shape.Tpad * nblk * p0.nrow * g.shape.CB;
+			const int64_t per = (int64_t)g.shape.Tpad * nblk * g.shape.trow * g.shape.CB;
 			const int64_t per8 = (int64_t)g.shape.Tpad * nblk * g.shape.w8;
 			for(size_t i = 0; i < gidx[gi].size(); i++)
 			{
@@ -575,10 +577,16 @@ static fxb_status setup_device(fxb_ctx *ctx)
 				ctx->iscale_elems += (int64_t)d.nchan * d.nrow;
 				d.tcb = g.shape.CB;
 				d.tnblk = nblk;
+				d.trow = g.shape.trow;
+				for(d.pbits = 0; (4 << d.pbits) < d.nchan; d.pbits++)
+					;
+				g.maxout = std::max(g.maxout, job.plan[gidx[gi][i]].nout);
 				d.acc_ostride = 1;
 				d.acc_cstride = job.plan[gidx[gi][i]].nout;
 			}
 			off += per * (int64_t)gidx[gi].size();
+			if(g.xmac && tc_workspace(g.shape, g.nf, g.maxout) > 0)
+				CK(ctx, dalloc(ctx, &g.ws, (size_t)tc_workspace(g.shape, g.nf, g.maxout)));
 			ctx->spec8_elems += per8 * (int64_t)gidx[gi].size();
 		}
 		ctx->specn_elems = off;
@@ -1378,7 +1386,7 @@ static void launch_xmac_weights(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, u
 			}
 		}
 		if(ctx->tc)
-			launch_xmac_tc(g.tmap, sh, ctx->d_plans, g.d_idx, g.nf, ctx->nsm, ctx->d_err, ctx->d_acc, st);
+			launch_xmac_tc(g.tmap, sh, ctx->d_plans, g.d_idx, g.nf, g.ws, g.maxout, ctx->nsm, ctx->d_err, ctx->d_acc, st);
 		else
 			launch_xmac_fp32(ctx->h_plans[g.plan0], ctx->d_plans, g.d_idx, g.nf, ctx->T, ctx->nsm, ctx->d_spec, ctx->d_acc,
 			                 st);
@@ -1555,14 +1563,15 @@ fxb_status fxb_autotune(fxb_ctx *ctx, int32_t rounds)
 	{
 		if(!ctx->xgroups[g].xmac)
 			continue;
-		// one CTA per SM with double-buffered accumulators, or two per SM
-		static const int depth[][3] = {{6, 4, 2}, {6, 3, 2}, {4, 3, 2}, {4, 2, 2}, {3, 2, 2}, {2, 2, 2},
-		                               {4, 2, 1}, {3, 2, 1}, {2, 2, 1}};
-		for(const auto &d : depth)
+		// one CTA per SM, or two per SM: ring depths
+		static const int depth8[][3] = {{6, 4, 2}, {6, 3, 2}, {4, 3, 2}, {4, 2, 2}, {3, 2, 2}, {2, 2, 2},
+		                                {4, 2, 1}, {3, 2, 1}, {2, 2, 1}, {0, 0, 0}};
+		static const int depth16[][3] = {{12, 0, 2}, {8, 0, 2}, {6, 0, 2}, {8, 0, 1}, {6, 0, 1}, {4, 0, 1}, {0, 0, 0}};
+		for(const int(*d)[3] = ctx->f8 ? depth8 : depth16; (*d)[0]; d++)
 		{
 			TcShape sh = ctx->xgroups[g].shape;
-			if(tc_stages(&sh, d[0], d[1], d[2]))
-				t.xc[g].push_back({d[0], d[1], d[2]});
+			if(tc_stages(&sh, (*d)[0], (*d)[1], (*d)[2]))
+				t.xc[g].push_back({(*d)[0], (*d)[1], (*d)[2]});
 		}
 		most = std::max(most, t.xc[g].size());
 	}
@@ -2024,8 +2033,8 @@ fxb_status fxb_read_spectra(fxb_ctx *ctx, int32_t freq, float *out, size_t nfloa
 	CK(ctx, cudaStreamSynchronize(ctx->stream));
 	if(n && ctx->tc)
 	{
-		// half2 or bf16x2 [t][block][row][tcb], scaled by 2^-kTcSpecExp -> FP32 [t][row][chan]
-		const size_t nb = (size_t)ctx->T * p.tnblk * p.nrow * p.tcb;
+		// half2 or bf16x2 [t][block][trow][tcb], scaled by 2^-kTcSpecExp -> FP32 [t][row][chan]
+		const size_t nb = (size_t)ctx->T * p.tnblk * p.trow * p.tcb;
 		std::vector<uint32_t> h(nb);
 		CK(ctx, cudaMemcpy(h.data(), (const uint32_t *)ctx->d_specn + p.spec_off, nb * 4, cudaMemcpyDeviceToHost));
 		const float unscale = (float)(1 << kTcSpecExp);
@@ -2049,7 +2058,8 @@ fxb_status fxb_read_spectra(fxb_ctx *ctx, int32_t freq, float *out, size_t nfloa
 			for(int r = 0; r < p.nrow; r++)
 				for(int c = 0; c < p.nchan; c++)
 				{
-					const uint32_t v = h[(((size_t)t * p.tnblk + c / p.tcb) * p.nrow + r) * p.tcb + c % p.tcb];
+					const int q = chan_pos(p.pbits, c);
+					const uint32_t v = h[(((size_t)t * p.tnblk + q / p.tcb) * p.trow + r) * p.tcb + q % p.tcb];
 					const size_t o = ((size_t)t * p.nrow + r) * p.nchan + c;
 					out[2 * o] = bf(v & 0xFFFFu);
 					out[2 * o + 1] = bf(v >> 16);
@@ -2401,8 +2411,8 @@ static void batch_fused_xmac(fxb_batch *b, int k, cudaStream_t st)
 			if(!common)
 				common = &g.shape;
 			if(g.shape.nrow != common->nrow || g.shape.h16 != common->h16 ||
-			   !xmac_multi_add(&xm, tm, g.shape, c->d_plans, g.d_idx, g.nf, c->d_acc))
-				launch_xmac_tc(tm, g.shape, c->d_plans, g.d_idx, g.nf, c->nsm, c->d_err, c->d_acc, st);
+			   !xmac_multi_add(&xm, tm, g.shape, c->d_plans, g.d_idx, g.nf, g.ws, g.maxout, c->d_acc))
+				launch_xmac_tc(tm, g.shape, c->d_plans, g.d_idx, g.nf, g.ws, g.maxout, c->nsm, c->d_err, c->d_acc, st);
 		}
 	}
 	if(common)

@@ -11,11 +11,12 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB) k_fstage
 	__shared__ float lut8[256];
 	__shared__ u64 lut4[16];
 	__shared__ PairConst fcs[kMaxTQ * PShape<LOGN>::FPC];
+	__shared__ PairOut po;
 	const int item = a.items_fast ? blockIdx.x : blockIdx.y;
 	const int tchunk = a.items_fast ? blockIdx.y : blockIdx.x;
 	fstage_pair_luts(lut8, lut4);
 	__syncthreads();
-	fstage_pair_unit<LOGN, TCO, VAR>(a, a.first + item, tchunk, a.tq, (const float2 *)a.tw, fsp, lut8, lut4, fcs);
+	fstage_pair_unit<LOGN, TCO, VAR>(a, a.first + item, tchunk, a.tq, (const float2 *)a.tw, fsp, lut8, lut4, fcs, &po);
 }
 
 template <int LOGN, bool TCO, int VAR>

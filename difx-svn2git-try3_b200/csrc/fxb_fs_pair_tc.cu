@@ -12,11 +12,12 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB) k_fstage
 	__shared__ float lut8[256];
 	__shared__ u64 lut4[16];
 	__shared__ PairConst fcs[kMaxTQ * PShape<LOGN>::FPC];
+	__shared__ PairOut po;
 	const int item = a.items_fast ? blockIdx.x : blockIdx.y;
 	const int tchunk = a.items_fast ? blockIdx.y : blockIdx.x;
 	fstage_pair_luts(lut8, lut4);
 	__syncthreads();
-	fstage_pair_unit<LOGN, TCO, VAR>(a, a.first + item, tchunk, a.tq, (const float2 *)a.tw, fsp, lut8, lut4, fcs);
+	fstage_pair_unit<LOGN, TCO, VAR>(a, a.first + item, tchunk, a.tq, (const float2 *)a.tw, fsp, lut8, lut4, fcs, &po);
 }
 
 template <int LOGN, bool TCO, int VAR>
@@ -38,6 +39,7 @@ __global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant
 	__shared__ float lut8[256];
 	__shared__ u64 lut4[16];
 	__shared__ PairConst fcs[kFsMultiFc];
+	__shared__ PairOut po;
 	__shared__ int unit_s[2];
 	constexpr int cls = kFsMultiPer * VAR + 3;
 	fstage_pair_luts(lut8, lut4);
@@ -50,13 +52,13 @@ __global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant
 		const int gi = k.first + w.item;
 		switch(k.code & 31)
 		{
-		case 5: fstage_pair_unit<5, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs); break;
-		case 6: fstage_pair_unit<6, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs); break;
-		case 7: fstage_pair_unit<7, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs); break;
-		case 8: fstage_pair_unit<8, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs); break;
-		case 9: fstage_pair_unit<9, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs); break;
-		case 10: fstage_pair_unit<10, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs); break;
-		case 11: fstage_pair_unit<11, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs); break;
+		case 5: fstage_pair_unit<5, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
+		case 6: fstage_pair_unit<6, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
+		case 7: fstage_pair_unit<7, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
+		case 8: fstage_pair_unit<8, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
+		case 9: fstage_pair_unit<9, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
+		case 10: fstage_pair_unit<10, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
+		case 11: fstage_pair_unit<11, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
 		default: break;
 		}
 	}
@@ -71,6 +73,7 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB)
 	__shared__ float lut8[256];
 	__shared__ u64 lut4[16];
 	__shared__ PairConst fcs[kMaxTQ];
+	__shared__ PairOut po;
 	__shared__ int unit_s[2];
 	constexpr int cls = kFsMultiPer * VAR + (LOGN == 12 ? 2 : 0);
 	fstage_pair_luts(lut8, lut4);
@@ -80,7 +83,7 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB)
 		const FsMultiUnit w = m.units[m.unit0[cls] + u];
 		const FsMultiKind k = m.kinds[w.kind];
 		fstage_pair_unit<LOGN, true, VAR>(m.m[k.member], k.first + w.item, w.tchunk, k.tq, (const float2 *)k.tw, fsp, lut8,
-		                                  lut4, fcs);
+		                                  lut4, fcs, &po);
 	}
 }
 

@@ -336,7 +336,7 @@ __device__ __forceinline__ void fstage_unit(const FsArgs &a, const int gidx, con
 	uint2 *const side1 = pp ? side0 + (size_t)FPC * PADN : side0;
 	const uint8_t *vrow = a.valid + (int64_t)g.station * a.valid_stride;
 	const int64_t spec_off = a.plans[g.freq].spec_off;
-	const int prow = a.plans[g.freq].nrow;
+	const int prow = a.plans[g.freq].tcb ? a.plans[g.freq].trow : a.plans[g.freq].nrow, pbits = a.plans[g.freq].pbits;
 	// tensor-core form: spectra blocked [t][block][row][tcb] (tcb channels per block)
 	const uint32_t tcb = (uint32_t)a.plans[g.freq].tcb, tnblk = (uint32_t)a.plans[g.freq].tnblk;
 	const uint32_t tcb_magic = tcb ? 0xFFFFFFFFu / tcb + 1u : 0u;    // c / tcb = umulhi(c, magic) for c < 2^16
@@ -667,7 +667,7 @@ __device__ __forceinline__ void fstage_unit(const FsArgs &a, const int gidx, con
 						uint32_t *o;
 						if(tcb)
 						{
-							const uint32_t blk = __umulhi((uint32_t)c, tcb_magic), cl = (uint32_t)c - blk * tcb;
+							const uint32_t pc = (uint32_t)chan_pos(pbits, c), blk = __umulhi(pc, tcb_magic), cl = pc - blk * tcb;
 							o = (uint32_t *)a.spec + spec_off + (((int64_t)t * tnblk + blk) * prow) * tcb + cl +
 							    (int64_t)row0 * tcb;
 						}

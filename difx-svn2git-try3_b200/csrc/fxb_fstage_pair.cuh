@@ -232,6 +232,17 @@ struct PairConst {
 	int32_t flags;
 	int32_t mi00, mi01, mi10, mi11;      // raw reads: thread frames of the window's first and second frame, per band
 };
+// Where a unit's spectra go: FP32 form [t][row][chan]; tensor-core form blocked
+// [t][block][trow][tcb] in the order of chan_pos.
+struct PairOut {
+	int64_t first, tstride;              // the first band's value of time 0, channel (position) 0; a time
+	int32_t rowd;                        // from the first band's values to the second's
+	uint32_t tcb, magic, bextra;         // channels of a block; p / tcb = umulhi(p, magic) for p < 2^16;
+	                                     // position p sits at p + p / tcb x bextra
+	int32_t pbits, flags;
+};
+enum : int32_t { kORow0 = 1, kORow1 = 2, kOH16 = 4, kOQuad = 8, kOBoth = 16 };
+
 enum : int32_t {
 	kPActive = 1,     // valid FFT
 	kPNarrow = 2,     // fmask covers the window
@@ -248,7 +259,7 @@ enum : int32_t {
 template <int LOGN, bool TCO, int VAR>
 __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx, const int tchunk, const int tq,
                                                  const float2 *tw, ulonglong2 *fsm, const float *lut8,
-                                                 const u64 *lut4, PairConst *fcs)
+                                                 const u64 *lut4, PairConst *fcs, PairOut *po)
 {
 	using SH = PShape<LOGN>;
 	constexpr int N = SH::N, TPF = SH::TPF, FPC = SH::FPC, PADN = SH::PADN, RL = SH::RL;
@@ -275,9 +286,32 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 	// both bands side by side in one field of 2 nbits, aligned to its size
 	const bool adj = !MUX && !CPLX && boff1 == boff0 + (uint32_t)nbits && boff0 % (2u * (uint32_t)nbits) == 0;
 	const int order = a.order;
+	constexpr float osc = TCO ? 1.0f / (float)(1 << kTcSpecExp) : 1.0f;
 	const int t0 = tchunk * tq * FPC;
 	const int nit = min(tq, (a.T - t0 + FPC - 1) / FPC);
 
+	// ---- the unit's place in the spectra, by the CTA's last thread
+	if(threadIdx.x == blockDim.x - 1)
+	{
+		const DevFreqPlan &P = a.plans[g.freq];
+		const int row0 = g.row[0] < 0 ? 0 : g.row[0];
+		PairOut u;
+		u.tcb = TCO ? (uint32_t)P.tcb : 0u;
+		u.magic = TCO ? 0xFFFFFFFFu / u.tcb + 1u : 0u;
+		u.bextra = TCO ? (uint32_t)(P.trow - 1) * u.tcb : 0u;
+		u.pbits = TCO ? P.pbits : 0;
+		const int rstr = TCO ? P.tcb : nchan;
+		u.rowd = (g.row[1] - row0) * rstr;
+		u.tstride = TCO ? (int64_t)P.tnblk * P.trow * P.tcb : (int64_t)P.nrow * nchan;
+		u.first = P.spec_off + (int64_t)row0 * rstr;
+		u.flags = (g.row[0] >= 0 ? kORow0 : 0) | (g.row[1] >= 0 ? kORow1 : 0) | (a.h16 ? kOH16 : 0);
+		// four channels of a thread at once: blocks of a power of two channels
+		if(TCO && !CPLX && (u.tcb == 2 || u.tcb == 4 || u.tcb == 8) && !(lsb && order == 0))
+			u.flags |= kOQuad;
+		if((u.flags & kORow0) && (u.flags & kORow1) && u.rowd == 2 && !(row0 & 1) && TCO && !(P.trow & 1))
+			u.flags |= kOBoth;
+		*po = u;
+	}
 	// ---- constants of the unit's FFTs (FFT f is time t0 + f), one thread per FFT
 	for(int f = threadIdx.x; f < nit * FPC; f += blockDim.x)
 	{
@@ -584,40 +618,40 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 		// ---- 4. last pass, sideband, fractional-sample rotation, output
 		if(t >= a.T)
 			continue;
-		const DevFreqPlan &P = a.plans[g.freq];
 		constexpr int sL = N / RL, J = 8 / RL;
-		const int row0 = g.row[0], row1 = g.row[1];
-		constexpr float osc = TCO ? 1.0f / (float)(1 << kTcSpecExp) : 1.0f;
-		const bool same = (flags & kPSame) != 0, h16 = a.h16 != 0;
-		// spectra: FP32 form [t][row][chan]; tensor-core form blocked
-		// [t][block][row][tcb] (tcb channels per block; 0: [t][row][chan])
-		const uint32_t tcb = TCO ? (uint32_t)P.tcb : 0u;
-		const uint32_t magic = tcb ? 0xFFFFFFFFu / tcb + 1u : 0u;      // c / tcb = umulhi(c, magic) for c < 2^16
-		const uint32_t rstr = tcb ? tcb : (uint32_t)nchan, bextra = tcb ? (uint32_t)P.nrow * tcb - tcb : 0u;
-		const int64_t tb = P.spec_off + (int64_t)t * (tcb ? (int64_t)P.tnblk * P.nrow * tcb : (int64_t)P.nrow * nchan);
-		auto put = [&](uint32_t c, const cp &y, float cj, float c0, float s0, float c1, float s1) {
-			float2 re = up2(y.re), im = up2(y.im);
-			im.x *= cj;
-			im.y *= cj;
-			rot1(re.x, im.x, c0, s0);
-			rot1(re.y, im.y, c1, s1);
-			const uint32_t off = TCO ? c + __umulhi(c, magic) * bextra : c;
+		const bool same = (flags & kPSame) != 0;
+		const int oflags = po->flags;
+		const bool h16 = (oflags & kOH16) != 0;
+		const int rowd = po->rowd;
+		const int64_t base = po->first + (int64_t)t * po->tstride;
+		auto put = [&](int c, const cp &y) {
+			const float2 re = up2(y.re), im = up2(y.im);
 			if constexpr(TCO)
 			{
-				uint32_t *o = (uint32_t *)a.spec + tb + off;
-				if(row0 >= 0)
-					o[(uint32_t)row0 * rstr] = pack_spec(h16, re.x, im.x);
-				if(row1 >= 0)
-					o[(uint32_t)row1 * rstr] = pack_spec(h16, re.y, im.y);
+				const uint32_t p = (uint32_t)chan_pos(po->pbits, c);
+				uint32_t *o = (uint32_t *)a.spec + base + (p + __umulhi(p, po->magic) * po->bextra);
+				if(oflags & kORow0)
+					*o = pack_spec(h16, re.x, im.x);
+				if(oflags & kORow1)
+					o[rowd] = pack_spec(h16, re.y, im.y);
 			}
 			else
 			{
-				float2 *o = (float2 *)a.spec + tb + off;
-				if(row0 >= 0)
-					o[(uint32_t)row0 * rstr] = make_float2(re.x, im.x);
-				if(row1 >= 0)
-					o[(uint32_t)row1 * rstr] = make_float2(re.y, im.y);
+				float2 *o = (float2 *)a.spec + base + c;
+				if(oflags & kORow0)
+					*o = make_float2(re.x, im.x);
+				if(oflags & kORow1)
+					o[rowd] = make_float2(re.y, im.y);
 			}
+		};
+		// y conjugated when cj < 0, times the bands' rotators
+		auto turn = [](const cp &y, float cj, float2 w0, float2 w1) {
+			float2 re = up2(y.re), im = up2(y.im);
+			im.x *= cj;
+			im.y *= cj;
+			rot1(re.x, im.x, w0.x, w0.y);
+			rot1(re.y, im.y, w1.x, w1.y);
+			return cp{pk2(re.x, re.y), pk2(im.x, im.y)};
 		};
 		// rotator exp(2 pi i (ce D + post)) of band j at effective channel ce,
 		// D = hi + lo (ce hi exact), times the spectra's scale
@@ -651,7 +685,7 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 					const int k = b + jj * TPF + sL * r;
 					const int c = !lsb || k == 0 ? k : N - k, ce = lsb ? c - nchan : c;
 					const float2 w0 = rotator(0, ce), w1 = same ? w0 : rotator(1, ce);
-					put((uint32_t)c, y[r], !lsb || k == 0 ? 1.0f : -1.0f, w0.x, w0.y, w1.x, w1.y);
+					put(c, turn(y[r], !lsb || k == 0 ? 1.0f : -1.0f, w0, w1));
 				}
 			}
 		}
@@ -665,7 +699,6 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 			const int ce = mirror ? -b : (lsb ? b - nchan : b);
 			float2 w0 = rotator(0, ce), w1 = same ? w0 : rotator(1, ce);
 			const float2 os0 = fc.os[0], os1 = fc.os[1];
-			const float cj = mirror ? -1.0f : 1.0f;
 			cp y[4];
 #pragma unroll
 			for(int jj = 0; jj < J; jj++)
@@ -689,20 +722,21 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 					// bin N/2, channel 0
 					const float2 m0 = rotator(0, -nchan), m1 = same ? m0 : rotator(1, -nchan);
 					dft_half<RL>(z, h, nsg, sg);
-					put(0u, h[0], -1.0f, m0.x, m0.y, m1.x, m1.y);
+					put(0, turn(h[0], -1.0f, m0, m1));
 				}
 			}
 #pragma unroll
 			for(int m = 0; m < 4; m++)
 			{
-				const int k = b + m * (int)S8;
 				if(mirror)
-				{
-					if(k > 0)
-						put((uint32_t)(nchan - k), y[m], cj, w0.x, w0.y, w1.x, w1.y);
-				}
+					y[m] = turn(y[m], -1.0f, w0, w1);
 				else
-					put((uint32_t)k, y[m], 1.0f, w0.x, w0.y, w1.x, w1.y);
+				{
+					float2 re = up2(y[m].re), im = up2(y[m].im);
+					rot1(re.x, im.x, w0.x, w0.y);
+					rot1(re.y, im.y, w1.x, w1.y);
+					y[m] = cp{pk2(re.x, re.y), pk2(im.x, im.y)};
+				}
 				if(m < 3)
 				{
 					rot1(w0.x, w0.y, os0.x, os0.y);
@@ -710,6 +744,63 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 						w1 = w0;
 					else
 						rot1(w1.x, w1.y, os1.x, os1.y);
+				}
+			}
+			bool stored = false;
+			if constexpr(TCO)
+				if(oflags & kOQuad)
+				{
+					// the four values of each band side by side (chan_pos): blocks of 8 or 4
+					// channels take one 16-byte store per band, blocks of 2 two of 8 bytes, or
+					// both bands at once where their rows are an aligned pair
+					stored = true;
+					uint32_t q0[4], q1[4];
+#pragma unroll
+					for(int m = 0; m < 4; m++)
+					{
+						const float2 re = up2(y[m].re), im = up2(y[m].im);
+						q0[m] = pack_spec(h16, re.x, im.x);
+						q1[m] = pack_spec(h16, re.y, im.y);
+					}
+					const uint32_t tcb = po->tcb, bextra = po->bextra;
+					uint32_t *o = (uint32_t *)a.spec + base +
+					              (4u * (uint32_t)b + (tcb == 2 ? 2u * (uint32_t)b : (tcb == 4 ? (uint32_t)b : (uint32_t)b >> 1)) * bextra);
+					if(tcb >= 4)
+					{
+						if(oflags & kORow0)
+							*(uint4 *)o = make_uint4(q0[0], q0[1], q0[2], q0[3]);
+						if(oflags & kORow1)
+							*(uint4 *)(o + rowd) = make_uint4(q1[0], q1[1], q1[2], q1[3]);
+					}
+					else if(oflags & kOBoth)
+					{
+						*(uint4 *)o = make_uint4(q0[0], q0[1], q1[0], q1[1]);
+						*(uint4 *)(o + bextra + tcb) = make_uint4(q0[2], q0[3], q1[2], q1[3]);
+					}
+					else
+					{
+						if(oflags & kORow0)
+						{
+							*(uint2 *)o = make_uint2(q0[0], q0[1]);
+							*(uint2 *)(o + bextra + tcb) = make_uint2(q0[2], q0[3]);
+						}
+						if(oflags & kORow1)
+						{
+							*(uint2 *)(o + rowd) = make_uint2(q1[0], q1[1]);
+							*(uint2 *)(o + rowd + bextra + tcb) = make_uint2(q1[2], q1[3]);
+						}
+					}
+				}
+			if(!stored)
+			{
+#pragma unroll
+				for(int m = 0; m < 4; m++)
+				{
+					const int k = b + m * (int)S8;
+					if(!mirror)
+						put(k, y[m]);
+					else if(k > 0)
+						put(nchan - k, y[m]);
 				}
 			}
 		}

@@ -204,6 +204,50 @@ __device__ __forceinline__ uint32_t pack_h2(float a, float b)
 	return *(const uint32_t *)&h;
 }
 
+// two FP32 values in one register pair
+typedef unsigned long long u64;
+__device__ __forceinline__ u64 pk2(float a, float b)
+{
+	u64 d;
+	asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+	return d;
+}
+__device__ __forceinline__ float2 up2(u64 v)
+{
+	float2 r;
+	asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+	return r;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b)
+{
+	u64 d;
+	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+	return d;
+}
+__device__ __forceinline__ u64 sub2(u64 a, u64 b)
+{
+	u64 d;
+	asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+	return d;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c)
+{
+	u64 d;
+	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+	return d;
+}
+// complex product of two packed pairs
+__device__ __forceinline__ void cmul2(u64 xr, u64 xi, u64 wr, u64 wi, u64 &zr, u64 &zi)
+{
+	zr = sub2(mul2(xr, wr), mul2(xi, wi));
+	zi = fma2(xr, wi, mul2(xi, wr));
+}
+__device__ __forceinline__ uint32_t pack_h2(u64 v)
+{
+	const float2 f = up2(v);
+	return pack_h2(f.x, f.y);
+}
+
 // one spectral value of the tensor-core forms: (re, im) as half2 or bf16x2
 __device__ __forceinline__ uint32_t pack_spec(bool h16, float re, float im)
 {
@@ -225,7 +269,8 @@ __device__ __forceinline__ float fracc(double x) { return (float)(x - rint(x)); 
 // (one lane per unit, 32 units at a time) into a shared-memory ring.
 struct UnitRec {
 	float P0[2], alpha[2];        // fringe phase (turns) at n = 0 and per sample, per subband
-	float Sr[2], Si[2];           // rotator step per sample exp(-2 pi i alpha)
+	float Sr[2], Si[2];           // rotator step over one sample exp(-2 pi i alpha)
+	float S2r[2], S2i[2];         // and over two
 	uint32_t fmask;               // validity of the window's frames (bit j: frame fa + j)
 	int32_t so, fs;               // window start within frame fa, samples per frame
 	int32_t swbits;               // staged bit of sample 0
@@ -236,11 +281,11 @@ struct UnitRec {
 	int32_t nstage, station;      // staged bytes; station
 	int32_t t;                    // FFT time
 	float dhi[2][2], dlo[2][2];   // fractional-sample turns per channel of [subband][polarisation] (split_turns)
-	float st32[2][2];             // the same over 32 channels, reduced to [-1/2, 1/2)
+	float st32[2][2], st256[2][2];   // the same over 32 and 256 channels, reduced to [-1/2, 1/2)
 	float post[2][2];             // order-0 post-F turns plus the phase-offset rotation, per [subband][polarisation]
 	int32_t row[2][2];            // spectra row of [subband][polarisation] (-1: not written)
-	int64_t spec[2];              // first spectra value of the subband's [t][block][row][tcb] block
-	int32_t tnblk[2], nrow[2], tcb[2];
+	int64_t spec[2];              // first spectra value of the subband's [t][block][trow][tcb] block
+	int32_t nrow[2], tcb[2];      // rows and channels of a block
 };
 enum : int32_t { kOk = 1, kAllValid = 2, kManual = 4, kHas0 = 8, kHas1 = 16, kLsb0 = 32, kLsb1 = 64 };
 constexpr int kRing = 16;         // unit records in flight (>= staging + operand buffers + 2, with margin)
@@ -251,12 +296,9 @@ struct TcLayout {
 	static constexpr int kStgBytes = kN * BPT / 8 + 64;   // one window, 16-byte slack either side
 	static constexpr int kOffStg = kOffOp + kNS * kOpBytes;
 	static constexpr int kOffLut = kOffStg + kNStg * kStgBytes;
-	static constexpr int kOffTw = kOffLut + 256 * 16;     // twiddles w_2048^(n2 k1), float2 [k1][n2]
+	static constexpr int kOffTw = kOffLut + 256 * 16;     // twiddles w_2048^(n2 k1) of two k1, float4 [k1 / 2][n2]
 	static constexpr int kOffRing = kOffTw + kN1 * kN2 * 8;
-	// per output warp and lane: the spectra offset of channel k1 + 32 j (j = 0..31)
-	// in the blocked layout of the last (tcb, nrow) seen
-	static constexpr int kOffOutTab = (kOffRing + kRing * (int)sizeof(UnitRec) + 15) & ~15;
-	static constexpr int kUsed = kOffOutTab + 4 * 32 * 32 * 4;
+	static constexpr int kUsed = kOffRing + kRing * (int)sizeof(UnitRec);
 	static constexpr size_t kSmem = 1024 + (size_t)kUsed;
 	static_assert(kOffStg % 16 == 0 && kStgBytes % 16 == 0, "staging must be 16-aligned");
 	static_assert(kSmem <= 227 * 1024, "shared memory");
@@ -269,7 +311,7 @@ __device__ __forceinline__ UnitRec build_unit(const FsArgs &a, const int32_t *pa
 	constexpr int nchan = kN / 2;
 	UnitRec r;
 	memset(&r, 0, sizeof(r));
-	r.Sr[0] = r.Sr[1] = 1.0f;
+	r.Sr[0] = r.Sr[1] = r.S2r[0] = r.S2r[1] = 1.0f;
 	const int pi = u % npairs;
 	r.t = u / npairs;
 	const int gi[2] = {pairs[2 * pi], pairs[2 * pi + 1]};
@@ -291,9 +333,8 @@ __device__ __forceinline__ UnitRec build_unit(const FsArgs &a, const int32_t *pa
 		r.nib[sb] = g.band[0] >> 1;
 		r.row[sb][0] = g.row[0];
 		r.row[sb][1] = g.row[1];
-		r.spec[sb] = P.spec_off + (int64_t)r.t * P.tnblk * P.nrow * P.tcb;
-		r.tnblk[sb] = P.tnblk;
-		r.nrow[sb] = P.nrow;
+		r.spec[sb] = P.spec_off + (int64_t)r.t * P.tnblk * P.trow * P.tcb;
+		r.nrow[sb] = P.trow;
 		r.tcb[sb] = P.tcb;
 		if(p.status != kFftOk)
 			continue;
@@ -314,6 +355,9 @@ __device__ __forceinline__ UnitRec build_unit(const FsArgs &a, const int32_t *pa
 			sincospif(-2.0f * r.alpha[sb], &sn, &cs);
 			r.Sr[sb] = cs;
 			r.Si[sb] = sn;
+			sincospif(-4.0f * r.alpha[sb], &sn, &cs);
+			r.S2r[sb] = cs;
+			r.S2i[sb] = sn;
 		}
 		else if(a.order == 0)
 		{
@@ -330,6 +374,7 @@ __device__ __forceinline__ UnitRec build_unit(const FsArgs &a, const int32_t *pa
 			const double D = bw * (1.0 / nchan) * ((double)p.fse - g.clk[q]);
 			split_turns(D, r.dhi[sb][q], r.dlo[sb][q]);
 			r.st32[sb][q] = fracc(32.0 * D);
+			r.st256[sb][q] = fracc(256.0 * D);
 			r.post[sb][q] = (float)(postf + (double)g.phase[q]);
 		}
 	}
@@ -378,7 +423,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 	unsigned char *ops = base + kOffOp;
 	unsigned char *stg = base + LY::kOffStg;
 	float4 *lut = (float4 *)(base + LY::kOffLut);
-	float2 *twt = (float2 *)(base + LY::kOffTw);
+	float4 *twt = (float4 *)(base + LY::kOffTw);
 	UnitRec *ring = (UnitRec *)(base + LY::kOffRing);
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 	const int order = a.order;
@@ -391,12 +436,13 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 	// nibble(t + 1) << 4, nibble = code(p0) | code(p1) << 2 (format_vdif.c:78)
 	for(int i = tid; i < 256; i += blockDim.x)
 		lut[i] = make_float4(level2f(i & 3u), level2f((i >> 4) & 3u), level2f((i >> 2) & 3u), level2f((i >> 6) & 3u));
-	for(int i = tid; i < kN1 * kN2; i += blockDim.x)
+	for(int i = tid; i < kN1 / 2 * kN2; i += blockDim.x)
 	{
-		const int k1 = i / kN2, n2 = i - k1 * kN2;
-		float sn, cs;
-		sincospif(-(float)(n2 * k1) / (float)(kN / 2), &sn, &cs);
-		twt[i] = make_float2(cs, sn);
+		const int k1 = 2 * (i / kN2), n2 = i % kN2;
+		float4 w;
+		sincospif(-(float)(n2 * k1) / (float)(kN / 2), &w.z, &w.x);
+		sincospif(-(float)(n2 * (k1 + 1)) / (float)(kN / 2), &w.w, &w.y);
+		twt[i] = w;
 	}
 	if(tid == 0)
 	{
@@ -606,7 +652,21 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 				{
 					const int nsh = 4 * R.nib[sb];
 					const uint32_t vms = (flags & (sb == 0 ? kHas0 : kHas1)) ? vm : 0u;
-					float dv0[8], dv1[8];
+					// fringe rotators exp(-2 pi i (P0 + alpha n)) of two times at once, from n0 on
+					u64 rr = pk2(1.0f, 1.0f), ri = 0ull, s2r = rr, s2i = 0ull;
+					if(order == 1)
+					{
+						float ph = R.P0[sb] + R.alpha[sb] * (float)n0;
+						ph -= rintf(ph);
+						float c0, s0;
+						__sincosf(-6.283185307179586f * ph, &s0, &c0);
+						const float Sr = R.Sr[sb], Si = R.Si[sb];
+						rr = pk2(c0, c0 * Sr - s0 * Si);
+						ri = pk2(s0, c0 * Si + s0 * Sr);
+						s2r = pk2(R.S2r[sb], R.S2r[sb]);
+						s2i = pk2(R.S2i[sb], R.S2i[sb]);
+					}
+					uint32_t re0[4], im0[4], re1[4], im1[4];
 #pragma unroll
 					for(int j = 0; j < 8; j += 2)
 					{
@@ -629,34 +689,27 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 							sa = sb2 = nsh & 31;
 						}
 						const uint32_t idx = ((wa >> sa) & 15u) | (((wb >> sb2) & 15u) << 4);
-						const float4 l = lut[idx];
-						const bool v0 = (vms >> j) & 1u, v1 = (vms >> (j + 1)) & 1u;
-						dv0[j] = v0 ? l.x : 0.0f;
-						dv0[j + 1] = v1 ? l.y : 0.0f;
-						dv1[j] = v0 ? l.z : 0.0f;
-						dv1[j + 1] = v1 ? l.w : 0.0f;
-					}
-					// fringe rotator exp(-2 pi i (P0 + alpha n)) at n = n0 .. n0 + 7
-					const float Sr = R.Sr[sb], Si = R.Si[sb];
-					float rr = 1.0f, ri = 0.0f;
-					if(order == 1)
-					{
-						float ph = R.P0[sb] + R.alpha[sb] * (float)n0;
-						ph -= rintf(ph);
-						__sincosf(-6.283185307179586f * ph, &ri, &rr);
-					}
-					uint32_t re0[4], im0[4], re1[4], im1[4];
-#pragma unroll
-					for(int j = 0; j < 8; j += 2)
-					{
-						const float rr1 = rr * Sr - ri * Si;
-						const float ri1 = rr * Si + ri * Sr;
-						re0[j >> 1] = pack_h2(dv0[j] * rr, dv0[j + 1] * rr1);
-						im0[j >> 1] = pack_h2(dv0[j] * ri, dv0[j + 1] * ri1);
-						re1[j >> 1] = pack_h2(dv1[j] * rr, dv1[j + 1] * rr1);
-						im1[j >> 1] = pack_h2(dv1[j] * ri, dv1[j + 1] * ri1);
-						rr = rr1 * Sr - ri1 * Si;
-						ri = rr1 * Si + ri1 * Sr;
+						float4 l = lut[idx];
+						if(vms != 0xFFu)
+						{
+							const bool v0 = (vms >> j) & 1u, v1 = (vms >> (j + 1)) & 1u;
+							l.x = v0 ? l.x : 0.0f;
+							l.y = v1 ? l.y : 0.0f;
+							l.z = v0 ? l.z : 0.0f;
+							l.w = v1 ? l.w : 0.0f;
+						}
+						const u64 d0 = pk2(l.x, l.y), d1 = pk2(l.z, l.w);
+						re0[j >> 1] = pack_h2(mul2(d0, rr));
+						im0[j >> 1] = pack_h2(mul2(d0, ri));
+						re1[j >> 1] = pack_h2(mul2(d1, rr));
+						im1[j >> 1] = pack_h2(mul2(d1, ri));
+						if(j < 6)
+						{
+							u64 nr, ni;
+							cmul2(rr, ri, s2r, s2i, nr, ni);
+							rr = nr;
+							ri = ni;
+						}
 					}
 					// A1 tile sb: rows m = p 64 + n2 (the 8 times 8g..8g+7 are one 16-byte
 					// run), K = part 32 + n1
@@ -683,7 +736,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 		const int L = tid - 32 * kTwW0;         // tensor-memory lane (p, n2)
 		const int p = L >> 6, n2 = L & 63;
 		const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
-		const float2 *tw = twt + n2;             // w_2048^(n2 k1) at tw[k1 kN2]
+		const float4 *tw = twt + n2;             // w_2048^(n2 k1) of k1, k1 + 1 at tw[k1 / 2 kN2]
 		for(int k = 0; k < nk; k++)
 		{
 			const int b = k & 1, s = k % kNS;
@@ -709,11 +762,12 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 #pragma unroll
 				for(int q = 0; q < 16; q += 2)
 				{
-					const int k1 = 16 * hh + q;
-					const float y0r = v[2 * q], y0i = v[2 * q + 1], y1r = v[2 * q + 2], y1i = v[2 * q + 3];
-					const float2 w0 = tw[k1 * kN2], w1 = tw[(k1 + 1) * kN2];
-					zr[q >> 1] = pack_h2(y0r * w0.x - y0i * w0.y, y1r * w1.x - y1i * w1.y);
-					zi[q >> 1] = pack_h2(y0r * w0.y + y0i * w0.x, y1r * w1.y + y1i * w1.x);
+					// columns: real parts of k1 and k1 + 1, then their imaginary parts
+					const float4 w = tw[(8 * hh + (q >> 1)) * kN2];
+					u64 zrp, zip;
+					cmul2(pk2(v[2 * q], v[2 * q + 1]), pk2(v[2 * q + 2], v[2 * q + 3]), pk2(w.x, w.y), pk2(w.z, w.w), zrp, zip);
+					zr[q >> 1] = pack_h2(zrp);
+					zi[q >> 1] = pack_h2(zip);
 				}
 #pragma unroll
 				for(int c = 0; c < 2; c++)
@@ -740,9 +794,6 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 		const int sb = ch >> 1, p = ch & 1;
 		const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
 		constexpr float osc = 1.0f / (float)(1 << kTcSpecExp);
-		// this lane's offsets, read back only by itself
-		uint32_t *otab = (uint32_t *)(base + LY::kOffOutTab) + ch * 1024 + lane;
-		int tab_tcb = -1, tab_nrow = -1;
 		for(int k = 0; k < nk; k++)
 		{
 			const int b = k & 1;
@@ -752,42 +803,45 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 				break;
 			}
 			asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-			// channels k1 + 32 j, j in [0, 16) then [16, 32): 32 columns each
+			// 32 columns at a time: 8 per j0 = 0 .. 7, channels k1 + 32 j0 + 256 m, m =
+			// 0 .. 3, as (re m 0, 1), (im 0, 1), (re 2, 3), (im 2, 3)
 			float v[32];
 			const uint32_t tcol = tmem + lane_base + (uint32_t)(256 * b + 128);
 			tld32(tcol, v);
-			tld_wait();
 			const UnitRec &R = ring[k % kRing];
 			const int row = R.row[sb][p];
-			// channel c = k1 + 32 j: exp(2 pi i (ce D + post)), ce = c (upper
-			// sideband) or c - nchan (lower), D = hi + lo (ce hi exact), stepped
-			// by exp(2 pi i 32 D)
+			// channel c: exp(2 pi i (ce D + post)), ce = c (upper sideband) or c - nchan
+			// (lower), D = hi + lo (ce hi exact), stepped by exp(2 pi i 256 D) over m
+			// and by exp(2 pi i 32 D) over j0
 			const bool lsb = (R.flags & (sb == 0 ? kLsb0 : kLsb1)) != 0;
 			const float fce = (float)(lsb ? k1 - nchan : k1);
 			float th = fce * R.dhi[sb][p];
 			th -= rintf(th);
 			float turns = th + fmaf(fce, R.dlo[sb][p], R.post[sb][p]);
 			turns -= rintf(turns);
-			float qr, qi;
+			float qr, qi, mr, mi, sr, si;
 			__sincosf(6.283185307179586f * turns, &qi, &qr);
+			__sincosf(6.283185307179586f * R.st256[sb][p], &mi, &mr);
+			__sincosf(6.283185307179586f * R.st32[sb][p], &si, &sr);
 			qr *= osc;
 			qi *= osc;
-			float sr, si;
-			__sincosf(6.283185307179586f * R.st32[sb][p], &si, &sr);
-			const int tcb = R.tcb[sb];
-			uint32_t *o = (uint32_t *)a.spec + R.spec[sb] + (int64_t)(row < 0 ? 0 : row) * tcb;
-			if(row >= 0 && (tcb != tab_tcb || R.nrow[sb] != tab_nrow))
+			const float q1r = qr * mr - qi * mi, q1i = qr * mi + qi * mr;
+			u64 ar = pk2(qr, q1r), ai = pk2(qi, q1i), br, bi;          // m = 0, 1 and m = 2, 3
 			{
-				// channel c = k1 + 32 j sits at (c / tcb) nrow tcb + c % tcb
-				tab_tcb = tcb;
-				tab_nrow = R.nrow[sb];
-				const uint32_t PT = (uint32_t)tab_nrow * (uint32_t)tcb;
-				for(int j = 0; j < 32; j++)
-				{
-					const uint32_t c = (uint32_t)(k1 + 32 * j), blk = c / (uint32_t)tcb;
-					otab[32 * j] = blk * PT + (c - blk * (uint32_t)tcb);
-				}
+				const float m2r = mr * mr - mi * mi, m2i = 2.0f * mr * mi;
+				cmul2(ar, ai, pk2(m2r, m2r), pk2(m2i, m2i), br, bi);
 			}
+			const u64 stepr = pk2(sr, sr), stepi = pk2(si, si);
+			// position of the lane's first four channels (chan_pos: 4 k1) in the blocks
+			// of tcb channels, and the distance of the next four (128 positions on)
+			const uint32_t tcb = (uint32_t)R.tcb[sb], extra = (uint32_t)(R.nrow[sb] - 1) * tcb;
+			uint32_t *o = (uint32_t *)a.spec + R.spec[sb] + (int64_t)(row < 0 ? 0 : row) * (int)tcb;
+			const bool quad = tcb == 2 || tcb == 4 || tcb == 8;
+			const uint32_t magic = 0xFFFFFFFFu / tcb + 1u;
+			const uint32_t jstep = quad ? 128u * (uint32_t)R.nrow[sb] : 0u;
+			if(quad)
+				o += 4u * (uint32_t)k1 + (tcb == 2 ? 2u * (uint32_t)k1 : (tcb == 4 ? (uint32_t)k1 : (uint32_t)k1 >> 1)) * extra;
+			tld_wait();
 #pragma unroll
 			for(int hh = 0; hh < 2; hh++)
 			{
@@ -803,14 +857,47 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 				if(row < 0)
 					continue;
 #pragma unroll
-				for(int q = 0; q < 16; q++)
+				for(int j = 0; j < 4; j++)
 				{
-					const int j = 16 * hh + q;
-					const float xr = v[2 * q], xi = v[2 * q + 1];
-					o[otab[32 * j]] = pack_spec(H16, xr * qr - xi * qi, xr * qi + xi * qr);
-					const float nr = qr * sr - qi * si;
-					qi = qr * si + qi * sr;
-					qr = nr;
+					const float *x = v + 8 * j;
+					u64 zr, zi;
+					uint32_t h[4];
+					cmul2(pk2(x[0], x[1]), pk2(x[2], x[3]), ar, ai, zr, zi);
+					float2 r2 = up2(zr), i2 = up2(zi);
+					h[0] = pack_spec(H16, r2.x, i2.x);
+					h[1] = pack_spec(H16, r2.y, i2.y);
+					cmul2(pk2(x[4], x[5]), pk2(x[6], x[7]), br, bi, zr, zi);
+					r2 = up2(zr);
+					i2 = up2(zi);
+					h[2] = pack_spec(H16, r2.x, i2.x);
+					h[3] = pack_spec(H16, r2.y, i2.y);
+					if(hh < 1 || j < 3)
+					{
+						cmul2(ar, ai, stepr, stepi, zr, zi);
+						ar = zr;
+						ai = zi;
+						cmul2(br, bi, stepr, stepi, zr, zi);
+						br = zr;
+						bi = zi;
+					}
+					if(quad)
+					{
+						if(tcb == 2)
+						{
+							*(uint2 *)o = make_uint2(h[0], h[1]);
+							*(uint2 *)(o + extra + 2) = make_uint2(h[2], h[3]);
+						}
+						else
+							*(uint4 *)o = make_uint4(h[0], h[1], h[2], h[3]);
+						o += jstep;
+					}
+					else
+					{
+						const uint32_t p0 = 4u * (uint32_t)(k1 + 32 * (4 * hh + j));
+#pragma unroll
+						for(uint32_t m = 0; m < 4; m++)
+							o[p0 + m + __umulhi(p0 + m, magic) * extra] = h[m];
+					}
 				}
 			}
 		}
@@ -898,9 +985,10 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 // ---------------------------------------------------------------- host side
 // Constant tables in the kernel's shared-memory byte layout (values in
 // double, rounded once to FP16), K-major with the 128-byte swizzle:
-//   DFT-32: rows j = 2 k1 + part (out), K = part_in 32 + n1;
+//   DFT-32: one row per (k1, part out), K = part_in 32 + n1;
 //   DFT-64 of the upper (k2 in [0, 32)) and lower (k2 in [32, 64)) sideband:
-//          rows j = 2 k2' + part, K = part_in 64 + n2, two K halves of 64.
+//          one row per (k2', part out), K = part_in 64 + n2, two K halves of 64;
+//   the rows (columns of the results) in the order the readers take them.
 // A complex product (x_r + i x_i)(cos t - i sin t) is
 //   re: x_r cos t + x_i sin t,  im: -x_r sin t + x_i cos t.
 size_t fstage_tc_tables_bytes() { return kTablesBytes; }
@@ -920,10 +1008,12 @@ void make_fstage_tc_tables(void *out)
 		{
 			const double th = 2.0 * M_PI * (double)(k1 * n1 % kN1) / kN1;
 			const double c = cos(th), sn = sin(th);
-			put(o + kOffB1, 2 * k1, n1, c);
-			put(o + kOffB1, 2 * k1, 32 + n1, sn);
-			put(o + kOffB1, 2 * k1 + 1, n1, -sn);
-			put(o + kOffB1, 2 * k1 + 1, 32 + n1, c);
+			// columns 4 (k1 / 2): real parts of k1 and k1 + 1, then imaginary parts
+			const int re = 4 * (k1 >> 1) + (k1 & 1), im = re + 2;
+			put(o + kOffB1, re, n1, c);
+			put(o + kOffB1, re, 32 + n1, sn);
+			put(o + kOffB1, im, n1, -sn);
+			put(o + kOffB1, im, 32 + n1, c);
 		}
 	for(int side = 0; side < 2; side++)
 	{
@@ -935,11 +1025,13 @@ void make_fstage_tc_tables(void *out)
 			{
 				const double ph = 2.0 * M_PI * (double)(n2 * k2 % kN2) / kN2;
 				const double c = cos(ph), sn = sin(ph);
+				// columns of k2' = j0 + 8 m: 8 j0 + 4 (m / 2) + m % 2 (real), + 2 (imaginary);
 				// K = part_in 64 + n2: the real part's K half, then the imaginary part's
-				put(t, 2 * j, n2, c);
-				put(t + 8192, 2 * j, n2, sn);
-				put(t, 2 * j + 1, n2, -sn);
-				put(t + 8192, 2 * j + 1, n2, c);
+				const int m = j >> 3, re = 8 * (j & 7) + 4 * (m >> 1) + (m & 1), im = re + 2;
+				put(t, re, n2, c);
+				put(t + 8192, re, n2, sn);
+				put(t, im, n2, -sn);
+				put(t + 8192, im, n2, c);
 			}
 		}
 	}

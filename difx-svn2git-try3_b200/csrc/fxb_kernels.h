@@ -12,7 +12,9 @@ namespace fxb {
 struct DevFreqPlan {
 	int32_t nrow, nchan;              // rows, channels
 	int32_t tcb;                      // tensor-core form: channels per spectra block (0: spectra [t][row][chan])
-	int32_t tnblk;                    // tensor-core form: blocks per time, spectra [t][block][row][tcb]
+	int32_t tnblk;                    // tensor-core form: blocks per time, spectra [t][block][trow][tcb]
+	int32_t trow;                     // tensor-core form: rows of a block (nrow and, in the FP16 / BF16 form, zero rows)
+	int32_t pbits;                    // tensor-core form: log2(nchan / 4), see chan_pos
 	int32_t acc_cstride;              // accumulator stride between channels (1: [out][chan], nout: [chan][out])
 	int32_t acc_ostride;              // accumulator stride between outputs
 	int64_t spec_off;                 // complex offset of this frequency's spectra
@@ -29,6 +31,18 @@ struct DevOutMap {
 	int32_t nchan, avg;
 	int32_t cstride, pad;
 };
+
+// Tensor-core form: channel c sits at position p of its plan's blocks (block p /
+// tcb, p % tcb), the four channels nchan / 4 apart side by side: they are the
+// outputs of one thread of the F stage's last pass, which stores them at once
+// (the XMAC takes the channels of a block in any order).
+#if defined(__CUDACC__)
+__host__ __device__ __forceinline__ int chan_pos(int pbits, int c)
+{
+	return ((c & ((1 << pbits) - 1)) << 2) | (c >> pbits);
+}
+__host__ __device__ __forceinline__ int pos_chan(int pbits, int p) { return ((p & 3) << pbits) | (p >> 2); }
+#endif
 
 // A weight sum: stations and, of INTERLACEDVDIF stations, recorded bands (-1:
 // the station's own weight); s2 = -1: the weights of s1 alone.
@@ -241,30 +255,38 @@ void make_fstage_twiddles(int N, float2 *out32);
 void launch_xmac_fp32(const DevFreqPlan &plan0, const DevFreqPlan *dplans, const int32_t *plan_idx, int nf, int T,
                       int nsm, const float2 *spec, float2 *acc, cudaStream_t stream);
 
-// Tensor-core XMAC (csrc/fxb_xmac_tc.cu) over one group of equally shaped
-// subbands whose bf16x2 spectra lie in one block [subband][Tpad][nrow][nchan].
+// Tensor-core XMAC (csrc/fxb_xmac_h.cu; FP8 form: csrc/fxb_xmac_f8.cu) over one
+// group of equally shaped subbands whose bf16x2 spectra lie in one block
+// [subband][Tpad][block][trow][CB].
 struct TcShape {
 	int32_t f8;                       // FP8 form: e4m3 pairs, K tiles of 64 times
 	int32_t h16;                      // operands (or the FP8 form's source spectra) FP16, else BF16
-	int32_t w8;                       // FP8 form: values per time of a block, nrow * CB padded to 8
-	int32_t nrow, nchan, r2p, G, CB, Tpad;
+	int32_t nrow, nchan, T;
+	int32_t CB, trow, Tpad;           // channels and rows of a block, times padded to whole K tiles
+	int32_t nkt, nslice;              // K tiles; slices of a unit's times summed apart
+	int32_t split;                    // 1: the two operand tiles of a block are units of their own
+	int32_t nrs, nas;                 // ring stages (FP8 form: raw and operand stages)
+	int32_t nb;                       // 2: one CTA per SM, 1: two
+	// FP8 form
+	int32_t w8;                       // values per time of a block, nrow * CB padded to 8
+	int32_t r2p, G;                   // real rows per channel (padded to 8), channels per tile
 	int32_t raw_bytes, raw_stride;    // bytes of one TMA box, stride of the raw stages
-	int32_t nrs, nas;                 // raw and operand stages
-	int32_t nb;                       // accumulator buffers: 2 (one CTA per SM) or 1 (two CTAs per SM)
 	int32_t dstride, dump_off;        // accumulator copy: floats per row, byte offset
 	size_t smem;
 };
-bool tc_shape(int nrow, int nchan, int T, bool f8, bool h16, TcShape *s);
-// set the raw / operand ring depths and accumulator buffers of a shape (and
-// its shared-memory plan); false if they do not fit (227 KB for one CTA per
-// SM, 112 KB each for two)
-bool tc_stages(TcShape *s, int nrs, int nas, int nb = 2);
+bool tc_shape(int nrow, int nchan, int nf, int T, int nsm, bool f8, bool h16, TcShape *s);
+// set the ring depths and CTAs per SM of a shape (and its shared-memory plan);
+// false if they do not fit (227 KB for one CTA per SM, 112 KB each for two)
+bool tc_stages(TcShape *s, int nrs, int nas, int nb);
 bool tc_make_tensormap(void *map_out, const void *spec, const TcShape &s, int nf);
 size_t tc_tensormap_size();
+// complex values of workspace a group needs for its slices' sums (maxout: the
+// most outputs of its subbands)
+int64_t tc_workspace(const TcShape &s, int nf, int maxout);
 void launch_xmac_tc(const void *tmap, const TcShape &s, const DevFreqPlan *dplans, const int32_t *plan_idx, int nf,
-                    int nsm, int32_t *err, float2 *acc, cudaStream_t stream);
+                    float2 *ws, int maxout, int nsm, int32_t *err, float2 *acc, cudaStream_t stream);
 // One launch over several groups (of one context or several) whose shapes
-// share rows, form and ring depths: the CTAs stride over the groups' work
+// share rows and form: the CTAs stride over the groups' work
 // units in turn.  Each product is added to its accumulator once per subint
 // whatever the schedule, so results equal those of a launch per group.
 constexpr int kXMultiGroups = 16;
@@ -275,7 +297,11 @@ struct XGroupRec {
 	const DevFreqPlan *plans;
 	const int32_t *plan_idx;             // [subbands of the group] plan of each
 	float2 *acc;                         // the context's accumulators
+	float2 *ws;                          // sums of each slice [slice][subband][channel][ws_nout]
+	int64_t ws_slice;
+	int32_t ws_nout, nf;
 	int32_t nchan, nkt, nblk, unit0;     // channels, K tiles, channel blocks per subband, first unit
+	int32_t nslice, split;               // 1: an operand tile per unit
 };
 struct XMultiArgs {
 	TmapBytes map[kXMultiGroups];        // CUtensorMap of each group's spectra block
@@ -284,8 +310,13 @@ struct XMultiArgs {
 };
 // appends a group (false when the launch is full)
 bool xmac_multi_add(XMultiArgs *xm, const void *tmap, const TcShape &s, const DevFreqPlan *dplans,
-                    const int32_t *plan_idx, int nf, float2 *acc);
+                    const int32_t *plan_idx, int nf, float2 *ws, int maxout, float2 *acc);
 void launch_xmac_tc_multi(const XMultiArgs &xm, const TcShape &s, int nsm, int32_t *err, cudaStream_t stream);
+// FP8 form (fxb_xmac_f8.cu)
+bool f8_shape(TcShape *s);
+bool f8_stages(TcShape *s, int nrs, int nas, int nb);
+bool f8_tensormap(void *map_out, const void *spec, const TcShape &s, int nf);
+void f8_launch(const XMultiArgs &xm, const TcShape &s, int nsm, int32_t *err, cudaStream_t stream);
 // FP8 form: per subband of the group (plan_idx[nf]), the bf16x2 spectra
 // [Tpad][nblk][nrow][CB] at spec_off -> e4m3x2 [Tpad][nblk][w8] at spec8_off,
 // scaled per (channel, input) so that the input's largest component over the
