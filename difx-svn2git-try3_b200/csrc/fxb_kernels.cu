@@ -214,71 +214,108 @@ cudaError_t launch_fstage(const DevStation *st, const DevSubintStation *sub, con
 // stations weigh each band by its own data weight (Mode::getDataWeight,
 // mode.h:168, mode.cpp:1300-1303).
 //
-// Bound: latency, of the loads and of a chain of T float additions.  One warp
-// per distinct sum (not per core-result slot: the products of a baseline
-// share one) reads 128 FFTs at a time from the packed weights.  Additions of
-// zeros and ones to an integral sum below 2^23 are exact in any order, so a
-// run of 32 such weights (whole or invalid FFTs) is added by its count; other
-// runs are added one by one.  20 stations x 4 subbands, T = 4096: 87 -> 8 us per
-// subint; 10 stations x 8, T = 250: 7.9 -> 2.9 us.
-__global__ void __launch_bounds__(128) k_weights(const DevWeightSum *__restrict__ sums, int nsum,
-                                                 const float *__restrict__ wts, const float *__restrict__ pbw, int nbm,
-                                                 int T, float *__restrict__ acc)
+// Bound: latency, of the loads and of a chain of T float additions.  One CTA per
+// distinct sum (not per core-result slot: the products of a baseline share one)
+// reads 2048 FFTs at a time from the packed weights.  Additions of zeros and ones
+// to an integral sum below 2^23 are exact in any order, so a chunk, or a run of
+// 32, of such weights (whole or invalid FFTs) is added by its count; other runs are
+// added one by one by the first warp.  20 stations x 4 subbands, T = 4096: 87 us
+// with a warp per slot, 53 us with a warp per sum, 9 us now; 5 stations, T =
+// 38622: 740, 331, 58 us.
+__global__ void __launch_bounds__(256) k_weights(const DevWeightSum *__restrict__ sums, const float *__restrict__ wts,
+                                                 const float *__restrict__ pbw, int nbm, int T,
+                                                 float *__restrict__ acc)
 {
-	constexpr int G = 4;                      // runs of 32 in flight
-	__shared__ __align__(16) float buf[4][32];
-	const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-	const int k = blockIdx.x * 4 + w;
-	if(k >= nsum)
-		return;
-	const DevWeightSum u = sums[k];
+	constexpr int G = 8, kChunk = 256 * G;        // values per thread and chunk
+	__shared__ __align__(16) float buf[kChunk];
+	__shared__ int ones_s[kChunk / 32], clean_s[kChunk / 32], count_s[2][8];
+	__shared__ float sum_s;
+	const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+	const DevWeightSum u = sums[blockIdx.x];
 	const float *wa = u.b1 >= 0 ? pbw + (int64_t)u.s1 * T * nbm + u.b1 : wts + (int64_t)u.s1 * T;
 	const int sa = u.b1 >= 0 ? nbm : 1;
 	const bool two = u.s2 >= 0;
 	const float *wb = !two ? wa : (u.b2 >= 0 ? pbw + (int64_t)u.s2 * T * nbm + u.b2 : wts + (int64_t)u.s2 * T);
 	const int sb = two && u.b2 >= 0 ? nbm : 1;
-	float sum = 0.0f;
-	for(int t0 = 0; t0 < T; t0 += 32 * G)
+	float sum = 0.0f;                             // the same in every thread
+	int par = 0;
+	for(int t0 = 0; t0 < T; t0 += kChunk, par ^= 1)
 	{
 		float v[G];
 #pragma unroll
 		for(int g = 0; g < G; g++)
 		{
-			const int t = t0 + 32 * g + lane;
+			const int t = t0 + 256 * g + (int)threadIdx.x;
 			v[g] = t < T ? __ldg(wa + (int64_t)t * sa) : 0.0f;
 			if(two)
 				v[g] = __fmul_rn(v[g], t < T ? __ldg(wb + (int64_t)t * sb) : 0.0f);
 		}
+		int count = 0;
+		bool clean = true;
 #pragma unroll
 		for(int g = 0; g < G; g++)
 		{
-			// adding 0 (past T, or an invalid FFT) leaves a non-negative sum unchanged
-			const uint32_t ones = __ballot_sync(0xffffffffu, v[g] == 1.0f);
-			if(__all_sync(0xffffffffu, v[g] == 1.0f || v[g] == 0.0f) && sum == rintf(sum) && sum < 8388608.0f)
-			{
-				sum += (float)__popc(ones);
-				continue;
-			}
-			buf[w][lane] = v[g];
-			__syncwarp();
-#pragma unroll
-			for(int j = 0; j < 32; j += 4)
-			{
-				const float4 q = *(const float4 *)(buf[w] + j);
-				sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, q.x), q.y), q.z), q.w);
-			}
-			__syncwarp();
+			count += __popc(__ballot_sync(0xffffffffu, v[g] == 1.0f));
+			clean = clean && (v[g] == 1.0f || v[g] == 0.0f);
 		}
+		if(lane == 0)
+			count_s[par][warp] = count;
+		if(__syncthreads_and(clean) && sum == rintf(sum) && sum < 8388608.0f)
+		{
+			int n = 0;
+#pragma unroll
+			for(int w = 0; w < 8; w++)
+				n += count_s[par][w];
+			sum += (float)n;
+			continue;
+		}
+		// run r of the chunk: FFTs t0 + 32 r .. + 31, held by warp r % 8
+#pragma unroll
+		for(int g = 0; g < G; g++)
+		{
+			const uint32_t ones = __ballot_sync(0xffffffffu, v[g] == 1.0f);
+			const bool all = __all_sync(0xffffffffu, v[g] == 1.0f || v[g] == 0.0f);
+			if(lane == 0)
+			{
+				ones_s[8 * g + warp] = __popc(ones);
+				clean_s[8 * g + warp] = all;
+			}
+			buf[256 * g + threadIdx.x] = v[g];
+		}
+		__syncthreads();
+		if(warp == 0)
+		{
+			const int nrun = min(kChunk, T - t0 + 31) / 32;
+			for(int r = 0; r < nrun; r++)
+			{
+				if(clean_s[r] && sum == rintf(sum) && sum < 8388608.0f)
+				{
+					sum += (float)ones_s[r];
+					continue;
+				}
+				// adding 0 (past T, or an invalid FFT) leaves a non-negative sum unchanged
+#pragma unroll
+				for(int j = 0; j < 32; j += 4)
+				{
+					const float4 q = *(const float4 *)(buf + 32 * r + j);
+					sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, q.x), q.y), q.z), q.w);
+				}
+			}
+			if(lane == 0)
+				sum_s = sum;
+		}
+		__syncthreads();
+		sum = sum_s;
 	}
-	if(lane == 0)
-		acc[k] = __fadd_rn(acc[k], sum);
+	if(threadIdx.x == 0)
+		acc[blockIdx.x] = __fadd_rn(acc[blockIdx.x], sum);
 }
 
 void launch_weights(const DevWeightSum *sums, int nsum, const float *wts, const float *pbw, int nbm, int T, float *acc,
                     cudaStream_t stream)
 {
 	if(nsum > 0)
-		k_weights<<<(nsum + 3) / 4, 128, 0, stream>>>(sums, nsum, wts, pbw, nbm, T, acc);
+		k_weights<<<nsum, 256, 0, stream>>>(sums, wts, pbw, nbm, T, acc);
 }
 
 // Core-result assembly (core.cpp:1774-1802 channel averaging, 1266-1363):
