@@ -142,6 +142,8 @@ struct fxb_ctx {
 	int32_t punit0[kFsMultiClasses] = {}, pnunit[kFsMultiClasses] = {};
 	FsMultiKind *d_pkinds = nullptr;
 	FsMultiUnit *d_punits = nullptr;
+	PairItem *d_pitems = nullptr;        // two-band items and the constants of their FFTs
+	PairConst *d_pconst = nullptr;
 	int32_t *d_pctr = nullptr;
 	void *d_specn = nullptr;             // half2 (or bf16x2) spectra of the tensor-core forms, X 2^-kTcSpecExp
 	void *d_tctab = nullptr;             // constant tables of the tensor-core FFT kernel
@@ -370,6 +372,50 @@ static int pcal_chunks(const Job &job, const std::vector<DevPcalGroup> &groups)
 	const int64_t cap = (int64_t)(64 << 20) / (8 * job.pcal_bins);
 	n = (int)std::min<int64_t>(n, std::max<int64_t>(cap, 1));
 	return std::max(n, 1);
+}
+
+// The unchanging part of a two-band work item (k_pair_consts has the rest).
+static PairItem pair_item(const fxb_ctx *ctx, const FGroup &g, int group, bool tc)
+{
+	const DevStation &S = ctx->h_st[g.station];
+	const DevFreqPlan &P = ctx->h_plans[g.freq];
+	const int nchan = P.nchan, row0 = std::max(g.row[0], 0);
+	PairItem u;
+	memset(&u, 0, sizeof(u));
+	u.tcb = tc ? (uint32_t)P.tcb : 0u;
+	u.magic = tc ? 0xFFFFFFFFu / u.tcb + 1u : 0u;
+	u.bextra = tc ? (uint32_t)(P.trow - 1) * u.tcb : 0u;
+	u.pbits = tc ? P.pbits : 0;
+	const int rstr = tc ? P.tcb : nchan;
+	u.rowd = (g.row[1] - row0) * rstr;
+	u.tstride = tc ? (int64_t)P.tnblk * P.trow * P.tcb : (int64_t)P.nrow * nchan;
+	u.first = P.spec_off + (int64_t)row0 * rstr;
+	u.oflags = (g.row[0] >= 0 ? kORow0 : 0) | (g.row[1] >= 0 ? kORow1 : 0) | (ctx->h16 ? kOH16 : 0);
+	// four channels of a thread at once: blocks of a power of two channels
+	if(tc && !S.cplx && (u.tcb == 2 || u.tcb == 4 || u.tcb == 8) && !(g.lsb && ctx->job.fringe_rot_order == 0))
+		u.oflags |= kOQuad;
+	if((u.oflags & kORow0) && (u.oflags & kORow1) && u.rowd == 2 && !(row0 & 1) && tc && !(P.trow & 1))
+		u.oflags |= kOBoth;
+	const uint32_t cpl = S.cplx ? 2u : 1u;
+	u.fs = (uint32_t)S.framesamples;
+	u.bpt = S.muxraw ? (uint32_t)S.nbits : (uint32_t)(S.nband * S.nbits) * cpl;
+	u.boff0 = S.muxraw ? 0u : (uint32_t)(g.band[0] * S.nbits) * cpl;
+	u.boff1 = S.muxraw ? 0u : (uint32_t)(g.band[1] * S.nbits) * cpl;
+	u.hbits = (uint32_t)S.header * 8u;
+	u.nbits = S.nbits;
+	u.header = S.header;
+	u.framebytes = S.framebytes;
+	u.minfb = S.inframebytes;
+	u.mnthr = S.nthr;
+	u.station = g.station;
+	u.band0 = g.band[0];
+	u.band1 = g.band[1];
+	u.lsb = g.lsb;
+	u.asl = S.asl;
+	// both bands side by side in one field of 2 nbits, aligned to its size
+	u.adj = !S.muxraw && !S.cplx && u.boff1 == u.boff0 + (uint32_t)S.nbits && u.boff0 % (2u * (uint32_t)S.nbits) == 0;
+	u.group = group;
+	return u;
 }
 
 static fxb_status setup_device(fxb_ctx *ctx)
@@ -699,6 +745,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 			}
 		}
 		std::vector<FGroup> hg;
+		std::vector<PairItem> pitems;
 		if(out == 1)
 		{
 			// all stations of a subband side by side in the grid: their rows of
@@ -720,6 +767,12 @@ static fxb_status setup_device(fxb_ctx *ctx)
 			k.cplx = (kv.first.second >> 5) & 1;
 			k.first = (int)hg.size();
 			k.count = (int)kv.second.size();
+			if(k.nb == 2)
+			{
+				k.pair0 = (int)pitems.size();
+				for(int i = 0; i < k.count; i++)
+					pitems.push_back(pair_item(ctx, kv.second[i], k.first + i, out == 1));
+			}
 			// FFT iterations per CTA: as many as still leave two CTAs per SM
 			for(int tq : {4, 2, 1})
 			{
@@ -762,6 +815,9 @@ static fxb_status setup_device(fxb_ctx *ctx)
 					k.tcpairs = dp;
 					k.tcnpairs = (int32_t)(pairs.size() / 2);
 					k.tcbpt = bpt;
+					unsigned char *rec = nullptr;
+					CK(ctx, dalloc(ctx, &rec, fstage_tc_rec_bytes(k.tcnpairs, ctx->T)));
+					k.tcrec = rec;
 				}
 			}
 			{
@@ -777,6 +833,11 @@ static fxb_status setup_device(fxb_ctx *ctx)
 			hg.insert(hg.end(), kv.second.begin(), kv.second.end());
 			ctx->fkinds.push_back(k);
 		}
+		CK(ctx, dalloc(ctx, &ctx->d_pitems, pitems.size()));
+		CK(ctx, dalloc(ctx, &ctx->d_pconst, pitems.size() * (size_t)ctx->T));
+		if(!pitems.empty())
+			CK(ctx, cudaMemcpyAsync(ctx->d_pitems, pitems.data(), sizeof(PairItem) * pitems.size(), cudaMemcpyHostToDevice,
+			                        ctx->stream));
 		// the persistent launches' work list: per kind tq x fpc FFT times of
 		// one item per unit, times outer and items inner
 		{
@@ -800,7 +861,21 @@ static fxb_status setup_device(fxb_ctx *ctx)
 				std::vector<FsMultiUnit> &dst = cls[kFsMultiPer * k.muxraw + fstage_multi_class(k.N, k.nb)];
 				for(int t = 0; t < nt; t++)
 					for(int it = 0; it < k.count; it++)
-						dst.push_back(FsMultiUnit{ki, it, t});
+					{
+						FsMultiUnit u;
+						memset(&u, 0, sizeof(u));
+						u.kind = ki;
+						u.item = it;
+						u.tchunk = t;
+						u.t0 = t * per;
+						u.nfc = std::min(per, ctx->T - u.t0);
+						if(k.nb == 2)
+						{
+							u.pitem = ctx->d_pitems + k.pair0 + it;
+							u.consts = ctx->d_pconst + (size_t)(k.pair0 + it) * ctx->T + u.t0;
+						}
+						dst.push_back(u);
+					}
 			}
 			for(int c = 0; c < kFsMultiClasses; c++)
 			{
@@ -1236,32 +1311,6 @@ static fxb_status stage_subint(fxb_ctx *ctx, const uint8_t *const *bufs, const i
 	return FXB_OK;
 }
 
-// Every kernel of one subint whose inputs sit in slot sl, on stream st.  No
-// host synchronisation and no argument that changes between subints (the
-// subint time travels in the slot's records), so that the sequence can be
-// captured once per slot and replayed.  capture: the slot's four timing
-// events become event-record nodes of the graph.
-// Delay interpolators, raw-read placement, frame validity and per-FFT
-// parameters of one subint (Mode::setOffsets, Mk5Mode::unpack's checks).
-static void launch_prep(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, unsigned evf)
-{
-	const Job &job = ctx->job;
-	cudaEventRecordWithFlags(sl.tev[0], st, evf);
-	if(ctx->nraw)
-	{
-		launch_interpolators(ctx->d_st, sl.d_sub, ctx->S, ctx->T, st);
-		launch_mux_raw(ctx->d_st, sl.d_sub, ctx->S, 0, 0, st);
-		launch_frame_valid(ctx->d_st, sl.d_sub, ctx->d_valid, ctx->d_bandok, ctx->valid_stride, ctx->S, st,
-		                   ctx->d_fillok);
-	}
-	else
-		fxb::launch_prep(ctx->d_st, sl.d_sub, ctx->S, ctx->T, ctx->d_valid, ctx->d_bandok, ctx->valid_stride, st,
-		                 ctx->d_fillok);
-	launch_fft_params(ctx->d_st, sl.d_sub, sl.d_vflags, ctx->nflagint, ctx->d_valid, ctx->d_bandok, ctx->valid_stride,
-	                  ctx->S, ctx->T, job.fringe_rot_order, ctx->d_params, ctx->d_pbw, ctx->nbm, st, ctx->d_fillok, ctx->d_wts);
-	cudaEventRecordWithFlags(sl.tev[1], st, evf);
-}
-
 // The F-stage arguments of one subint (every kind but the twiddles and the
 // scheduling fields).
 static FsArgs fs_args(const fxb_ctx *ctx, const Slot &sl)
@@ -1285,7 +1334,41 @@ static FsArgs fs_args(const fxb_ctx *ctx, const Slot &sl)
 	fa.spec = ctx->tc ? ctx->d_specn : (void *)ctx->d_spec;
 	fa.err = ctx->d_err;
 	fa.h16 = ctx->h16 ? 1 : 0;
+	fa.pitems = ctx->d_pitems;
+	fa.pconst = ctx->d_pconst;
 	return fa;
+}
+
+// Every kernel of one subint whose inputs sit in slot sl, on stream st.  No
+// host synchronisation and no argument that changes between subints (the
+// subint time travels in the slot's records), so that the sequence can be
+// captured once per slot and replayed.  capture: the slot's four timing
+// events become event-record nodes of the graph.
+// Delay interpolators, raw-read placement, frame validity and per-FFT
+// parameters of one subint (Mode::setOffsets, Mk5Mode::unpack's checks).
+static void launch_prep(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, unsigned evf)
+{
+	const Job &job = ctx->job;
+	cudaEventRecordWithFlags(sl.tev[0], st, evf);
+	if(ctx->nraw)
+	{
+		launch_interpolators(ctx->d_st, sl.d_sub, ctx->S, ctx->T, st);
+		launch_mux_raw(ctx->d_st, sl.d_sub, ctx->S, 0, 0, st);
+		launch_frame_valid(ctx->d_st, sl.d_sub, ctx->d_valid, ctx->d_bandok, ctx->valid_stride, ctx->S, st,
+		                   ctx->d_fillok);
+	}
+	else
+		fxb::launch_prep(ctx->d_st, sl.d_sub, ctx->S, ctx->T, ctx->d_valid, ctx->d_bandok, ctx->valid_stride, st,
+		                 ctx->d_fillok);
+	launch_fft_params(ctx->d_st, sl.d_sub, sl.d_vflags, ctx->nflagint, ctx->d_valid, ctx->d_bandok, ctx->valid_stride,
+	                  ctx->S, ctx->T, job.fringe_rot_order, ctx->d_params, ctx->d_pbw, ctx->nbm, st, ctx->d_fillok, ctx->d_wts);
+	const FsArgs fa = fs_args(ctx, sl);
+	for(const FKind &k : ctx->fkinds)
+		if(k.tcfft)
+			launch_tc_units(k, fa, st);
+		else if(k.nb == 2)
+			launch_pair_consts(k, fa, st);
+	cudaEventRecordWithFlags(sl.tev[1], st, evf);
 }
 
 static void launch_xmac_weights(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, unsigned evf, bool tuning,
@@ -1757,6 +1840,10 @@ fxb_status fxb_job_footprint(const fxb_job_desc *desc, size_t *bytes)
 	}
 	const int64_t T = job.blockspersend;
 	const int S = (int)job.stations.size();
+	// two-band items, each with constants per FFT (two items a record in the tensor-core FFT)
+	int64_t pairs = 0;
+	for(const Job::Station &js : job.stations)
+		pairs += js.nband / 2;
 	// spectra (the blocked tensor-core layout pads times to 32 -- 64 for the
 	// e4m3 copy of the FP8 form -- and channels to whole blocks: at most
 	// +25 %), accumulators, core result, FFT parameters
@@ -1765,7 +1852,7 @@ fxb_status fxb_job_footprint(const fxb_job_desc *desc, size_t *bytes)
 	double b = (double)job.spec_total * (job.xmac_kind == FXB_XMAC_FP32 ? 8.0
 	                                     : job.xmac_kind != FXB_XMAC_FP8 ? 4.0 * 1.25 * pad32
 	                                                                      : (4.0 * pad64 + 2.0 * pad64 + 0.5) * 1.25);
-	b += (double)job.acc_total * 8.0 + (double)job.corelen * 16.0 + (double)S * T * 68.0 +
+	b += (double)job.acc_total * 8.0 + (double)job.corelen * 16.0 + (double)S * T * 68.0 + (double)pairs * T * 144.0 +
 	     (double)job.pcal_bins * 8.0 * pcal_chunks(job, pcal_groups(job));
 	// raw VDIF staging of the in-flight subints (payload plus headers, 1/8 slack)
 	for(int s = 0; s < S; s++)

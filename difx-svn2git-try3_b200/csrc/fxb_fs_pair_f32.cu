@@ -8,15 +8,18 @@ template <int LOGN, bool TCO, int VAR>
 __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB) k_fstage_pair(const FsArgs a)
 {
 	extern __shared__ __align__(16) ulonglong2 fsp[];
+	constexpr int FPC = PShape<LOGN>::FPC;
 	__shared__ float lut8[256];
 	__shared__ u64 lut4[16];
-	__shared__ PairConst fcs[kMaxTQ * PShape<LOGN>::FPC];
-	__shared__ PairOut po;
-	const int item = a.items_fast ? blockIdx.x : blockIdx.y;
-	const int tchunk = a.items_fast ? blockIdx.y : blockIdx.x;
+	__shared__ PairConst fcs[kMaxTQ * FPC];
+	__shared__ PairItem I;
+	const int item = a.pair0 + (a.items_fast ? blockIdx.x : blockIdx.y);
+	const int t0 = (a.items_fast ? blockIdx.y : blockIdx.x) * a.tq * FPC, nfc = min(a.tq * FPC, a.T - t0);
+	pair_fetch(&I, fcs, a.pitems + item, a.pconst + (int64_t)item * a.T + t0, nfc);
 	fstage_pair_luts(lut8, lut4);
+	pair_cp_wait();
 	__syncthreads();
-	fstage_pair_unit<LOGN, TCO, VAR>(a, a.first + item, tchunk, a.tq, (const float2 *)a.tw, fsp, lut8, lut4, fcs, &po);
+	fstage_pair_unit<LOGN, TCO, VAR>(a, I, fcs, t0, (nfc + FPC - 1) / FPC, (const float2 *)a.tw, fsp, lut8, lut4);
 }
 
 template <int LOGN, bool TCO, int VAR>

@@ -9,15 +9,18 @@ template <int LOGN, bool TCO, int VAR>
 __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB) k_fstage_pair(const FsArgs a)
 {
 	extern __shared__ __align__(16) ulonglong2 fsp[];
+	constexpr int FPC = PShape<LOGN>::FPC;
 	__shared__ float lut8[256];
 	__shared__ u64 lut4[16];
-	__shared__ PairConst fcs[kMaxTQ * PShape<LOGN>::FPC];
-	__shared__ PairOut po;
-	const int item = a.items_fast ? blockIdx.x : blockIdx.y;
-	const int tchunk = a.items_fast ? blockIdx.y : blockIdx.x;
+	__shared__ PairConst fcs[kMaxTQ * FPC];
+	__shared__ PairItem I;
+	const int item = a.pair0 + (a.items_fast ? blockIdx.x : blockIdx.y);
+	const int t0 = (a.items_fast ? blockIdx.y : blockIdx.x) * a.tq * FPC, nfc = min(a.tq * FPC, a.T - t0);
+	pair_fetch(&I, fcs, a.pitems + item, a.pconst + (int64_t)item * a.T + t0, nfc);
 	fstage_pair_luts(lut8, lut4);
+	pair_cp_wait();
 	__syncthreads();
-	fstage_pair_unit<LOGN, TCO, VAR>(a, a.first + item, tchunk, a.tq, (const float2 *)a.tw, fsp, lut8, lut4, fcs, &po);
+	fstage_pair_unit<LOGN, TCO, VAR>(a, I, fcs, t0, (nfc + FPC - 1) / FPC, (const float2 *)a.tw, fsp, lut8, lut4);
 }
 
 template <int LOGN, bool TCO, int VAR>
@@ -38,30 +41,30 @@ __global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant
 	extern __shared__ __align__(16) ulonglong2 fsp[];
 	__shared__ float lut8[256];
 	__shared__ u64 lut4[16];
-	__shared__ PairConst fcs[kFsMultiFc];
-	__shared__ PairOut po;
-	__shared__ int unit_s[2];
-	constexpr int cls = kFsMultiPer * VAR + 3;
+	__shared__ PairFeed<kFsMultiFc> feed;
 	fstage_pair_luts(lut8, lut4);
-	UnitFeed feed(m.ctr + cls, unit_s);
-	for(int u = feed.first(); u < m.nunit[cls]; u = feed.next())
-	{
-		const FsMultiUnit w = m.units[m.unit0[cls] + u];
-		const FsMultiKind k = m.kinds[w.kind];
+	pair_units(feed, m, kFsMultiPer * VAR + 3, [&](const FsMultiUnit &w, const PairItem &I, const PairConst *fcs) {
+		const FsMultiKind &k = m.kinds[w.kind];
 		const float2 *tw = (const float2 *)k.tw;
-		const int gi = k.first + w.item;
+		const FsArgs &a = m.m[k.member];
 		switch(k.code & 31)
 		{
-		case 5: fstage_pair_unit<5, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
-		case 6: fstage_pair_unit<6, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
-		case 7: fstage_pair_unit<7, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
-		case 8: fstage_pair_unit<8, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
-		case 9: fstage_pair_unit<9, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
-		case 10: fstage_pair_unit<10, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
-		case 11: fstage_pair_unit<11, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, tw, fsp, lut8, lut4, fcs, &po); break;
+#define FXB_PAIR_CASE(LOGN)                                                                                            \
+	case LOGN:                                                                                                         \
+		fstage_pair_unit<LOGN, true, VAR>(a, I, fcs, w.t0, (w.nfc + PShape<LOGN>::FPC - 1) / PShape<LOGN>::FPC, tw, fsp, \
+		                                  lut8, lut4);                                                                  \
+		break;
+			FXB_PAIR_CASE(5)
+			FXB_PAIR_CASE(6)
+			FXB_PAIR_CASE(7)
+			FXB_PAIR_CASE(8)
+			FXB_PAIR_CASE(9)
+			FXB_PAIR_CASE(10)
+			FXB_PAIR_CASE(11)
+#undef FXB_PAIR_CASE
 		default: break;
 		}
-	}
+	});
 }
 
 // 4096 points (class 5 VAR + 2) in CTAs of 512 threads, 8192 (class 5 VAR) of 1024
@@ -72,19 +75,14 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB)
 	extern __shared__ __align__(16) ulonglong2 fsp[];
 	__shared__ float lut8[256];
 	__shared__ u64 lut4[16];
-	__shared__ PairConst fcs[kMaxTQ];
-	__shared__ PairOut po;
-	__shared__ int unit_s[2];
-	constexpr int cls = kFsMultiPer * VAR + (LOGN == 12 ? 2 : 0);
+	__shared__ PairFeed<kMaxTQ> feed;
 	fstage_pair_luts(lut8, lut4);
-	UnitFeed feed(m.ctr + cls, unit_s);
-	for(int u = feed.first(); u < m.nunit[cls]; u = feed.next())
-	{
-		const FsMultiUnit w = m.units[m.unit0[cls] + u];
-		const FsMultiKind k = m.kinds[w.kind];
-		fstage_pair_unit<LOGN, true, VAR>(m.m[k.member], k.first + w.item, w.tchunk, k.tq, (const float2 *)k.tw, fsp, lut8,
-		                                  lut4, fcs, &po);
-	}
+	pair_units(feed, m, kFsMultiPer * VAR + (LOGN == 12 ? 2 : 0),
+	           [&](const FsMultiUnit &w, const PairItem &I, const PairConst *fcs) {
+		           const FsMultiKind &k = m.kinds[w.kind];
+		           fstage_pair_unit<LOGN, true, VAR>(m.m[k.member], I, fcs, w.t0, w.nfc, (const float2 *)k.tw, fsp, lut8,
+		                                             lut4);
+	           });
 }
 
 template <int VAR>
@@ -104,6 +102,138 @@ void launch_fs_pair_multi(const FsMultiArgs &m, int cls, int nsm, cudaStream_t s
 		launch_cls<1>(m, cls - kFsMultiPer, nsm, st);
 	else
 		launch_cls<0>(m, cls, nsm, st);
+}
+
+// The constants of one FFT per thread (grid: FFTs, items): FP64 terms, frames of
+// the window and, of raw reads, their place.  On their own so that the FFT
+// kernels start from finished constants: formed inside them, a unit of four
+// 2048-point FFTs spent about as long on this chain of loads and FP64
+// operations as on one FFT.
+__global__ void __launch_bounds__(128) k_pair_consts(const FsArgs a, int N, int mux, int cplx)
+{
+	const int t = blockIdx.x * blockDim.x + threadIdx.x;
+	if(t >= a.T)
+		return;
+	const int item = a.pair0 + blockIdx.y;
+	const PairItem &I = a.pitems[item];
+	const FGroup &g = a.groups[I.group];
+	const DevStation *Sp = a.st + I.station;
+	const uint32_t fs = I.fs;
+	const int nchan = cplx ? N : N / 2, S8 = N / 8, order = a.order;
+	const uint8_t *vrow = a.valid + (int64_t)I.station * a.valid_stride;
+	PairConst c;
+	memset(&c, 0, sizeof(c));
+	c.st = c.os[0] = c.os[1] = make_float2(1.0f, 0.0f);
+	c.wp = a.sub[I.station].buf;
+	const FftParam *pq = a.params + (int64_t)I.station * a.T + t;
+	if(pq->status == kFftOk)
+	{
+		c.flags = kPActive | kPSame;
+		const uint32_t g0 = (uint32_t)pq->nearest;
+		c.fa = g0 / fs;
+		c.so = g0 - c.fa * fs;
+		c.stuck = pq->stuck;
+		if(!mux)
+			c.wp += (int64_t)c.fa * I.framebytes + I.header;
+		const double invN = 1.0 / N, lo = g.lofreq;
+		const int idl = pq->integerdelay;
+		const double fraclo = a.fraclo ? (lo - (int)lo) * (double)idl : 0.0;
+		// LO offset: seconds since the job start of the FFT's first sample
+		// (mode.cpp:686-694; the scan starts with the job) and the offset's
+		// turns per sample
+		const double walls = (double)a.sub[I.station].subsec + a.sub[I.station].subns / 1.0e9 +
+		                     (double)t * N * Sp->sampletime / 1.0e6;
+		const double low = g.corr ? looff_wall_turns(g.looff, walls) : 0.0;
+		const double los = -g.looff * Sp->sampletime / 1.0e6;
+		double postf = 0.0;
+		if(order == 1)
+		{
+			c.P0 = frac_centered(lo * pq->b + fraclo + low);
+			c.alpha = (float)(lo * pq->a * invN + los);
+			c.st = cispi2(-(double)c.alpha * (double)S8);
+		}
+		else if(order == 2)
+		{
+			const double pa = pq->a, pb = pq->b;
+			const double X1 = (double)Sp->asl * invN;
+			c.P0 = frac_centered(lo * pq->c + fraclo + low);
+			c.alpha = (float)(lo * (pb + pa * X1) * invN + los);
+			c.beta = (float)(lo * 2.0 * pa * X1 * invN);
+			c.gamma = (float)(lo * pb * Sp->asl * invN + los * Sp->asl);
+			c.eps = (float)(lo * pa * X1 * X1);
+		}
+		else
+		{
+			double pr = (pq->averagedelay - idl) * lo;
+			if(a.fraclo)
+				pr += idl * (lo - (int)lo);
+			pr -= walls * g.looff;
+			postf = -(double)(float)(pr - (int)pr);
+		}
+		// per band: fse - clock offset (mode.cpp:1053-1059, 1099-1106); the
+		// channel of an order-0 lower sideband falls with the bin
+		const double sgn = I.lsb && (order == 0 || cplx) ? -1.0 : 1.0;
+		for(int j = 0; j < 2; j++)
+		{
+			const double D = Sp->bw * (1.0 / nchan) * ((double)pq->fse - g.clk[j]);
+			split_turns(D, c.dhi[j], c.dlo[j]);
+			c.post[j] = (float)postf + g.phase[j];
+			if(j == 0 || g.clk[1] != g.clk[0])
+				c.os[j] = cispi2(sgn * D * (double)S8);
+			else
+				c.os[1] = c.os[0];
+		}
+		if(g.clk[1] != g.clk[0] || g.phase[1] != g.phase[0])
+			c.flags &= ~kPSame;
+		// validity of the window's frames, one bit per frame relative to fa
+		const uint32_t nwf = (c.so + (uint32_t)N - 1) / fs + 1, nm = nwf < 32u ? nwf : 32u;
+		for(uint32_t k = 0; k < nm; k++)
+		{
+			const int64_t fr = (int64_t)c.fa + k;
+			// complex data: the unpack's first frame is checked for fill
+			// pattern only (mark5_stream_unpacker.c:189)
+			const uint8_t *vsrc = (cplx && k == 0 && a.fillok) ? a.fillok + (int64_t)I.station * a.valid_stride : vrow;
+			if(fr < a.valid_stride && vsrc[fr] != 0)
+				c.fmask |= 1u << k;
+		}
+		if(nwf <= 32)
+			c.flags |= kPNarrow;
+		if(a.bandok)
+		{
+			// EDV4-blanked bands (INTERLACEDVDIF): the general decode path
+			const uint32_t need = (1u << I.band0) | (1u << I.band1);
+			for(uint32_t k = 0; k < nwf; k++)
+			{
+				const int64_t fk = (int64_t)c.fa + k;
+				if(fk < a.valid_stride && vrow[fk] != 0 &&
+				   (a.bandok[(int64_t)I.station * a.valid_stride + fk] & need) != need)
+					c.flags |= kPBlank;
+			}
+		}
+		const bool whole = nwf < 32 && c.fmask == (1u << nwf) - 1u && c.stuck >= N && !(c.flags & kPBlank);
+		if(whole && I.adj && fs >= (uint32_t)S8)
+			c.flags |= kPFast;
+		if(mux && whole && nwf <= 2)
+		{
+			// valid frames of raw reads are complete slots: every thread is there
+			c.flags |= kPFast;
+			const int32_t *s0 = a.sub[I.station].mux_slot + (a.sub[I.station].mux_k0 + (int64_t)c.fa) * I.mnthr;
+			const int32_t *s1 = nwf == 2 ? s0 + I.mnthr : s0;
+			c.mi00 = s0[I.band0];
+			c.mi01 = s0[I.band1];
+			c.mi10 = s1[I.band0];
+			c.mi11 = s1[I.band1];
+		}
+	}
+	a.pconst[(int64_t)item * a.T + t] = c;
+}
+
+void launch_pair_consts(const FKind &k, const FsArgs &a0, cudaStream_t stream)
+{
+	FsArgs a = a0;
+	a.pair0 = k.pair0;
+	if(k.count > 0 && a.T > 0)
+		k_pair_consts<<<dim3((a.T + 127) / 128, k.count), 128, 0, stream>>>(a, k.N, k.muxraw, k.cplx);
 }
 
 void launch_fs_pair_tc(const FKind &k, const FsArgs &a, cudaStream_t stream)

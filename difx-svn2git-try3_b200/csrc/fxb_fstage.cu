@@ -121,6 +121,7 @@ void launch_fstage_kind(const FKind &k, FsArgs a, cudaStream_t stream)
 	if(k.count <= 0 || a.T <= 0)
 		return;
 	a.first = k.first;
+	a.pair0 = k.pair0;
 	a.tq = k.tq;
 	a.pp = k.pp;
 	a.tw = k.tw;

@@ -219,227 +219,51 @@ __device__ __forceinline__ void pair_mids(ulonglong2 *side, int slot, int b, con
 	}
 }
 
-// Constants of one FFT, computed by one thread.
-struct PairConst {
-	float P0, alpha, beta, gamma, eps;   // fringe phase (turns): start and per-sample terms
-	float2 st;                           // order 1: rotator step over N/8 samples, exp(-2 pi i alpha N/8)
-	float dhi[2], dlo[2];                // fractional-sample turns per channel of each band (split_turns)
-	float2 os[2];                        // rotator step over N/8 channels of each band
-	float post[2];                       // order-0 post-F turns and the band's phase offset
-	uint32_t fa, so;                     // first frame of the window, window start within it
-	uint32_t fmask;                      // validity of the window's frames (bit k: frame fa + k)
-	int32_t stuck;                       // samples [stuck, N) read as zero
-	int32_t flags;
-	int32_t mi00, mi01, mi10, mi11;      // raw reads: thread frames of the window's first and second frame, per band
-};
-// Where a unit's spectra go: FP32 form [t][row][chan]; tensor-core form blocked
-// [t][block][trow][tcb] in the order of chan_pos.
-struct PairOut {
-	int64_t first, tstride;              // the first band's value of time 0, channel (position) 0; a time
-	int32_t rowd;                        // from the first band's values to the second's
-	uint32_t tcb, magic, bextra;         // channels of a block; p / tcb = umulhi(p, magic) for p < 2^16;
-	                                     // position p sits at p + p / tcb x bextra
-	int32_t pbits, flags;
-};
-enum : int32_t { kORow0 = 1, kORow1 = 2, kOH16 = 4, kOQuad = 8, kOBoth = 16 };
-
-enum : int32_t {
-	kPActive = 1,     // valid FFT
-	kPNarrow = 2,     // fmask covers the window
-	kPBlank = 4,      // a valid frame of the window blanks one of the item's bands
-	kPSame = 8,       // the two bands take the same output rotation
-	kPFast = 16       // every sample of the window counts and the fast read applies
-};
-
 }  // namespace
 
-// One work unit: FFT times [tchunk tq FPC, +tq FPC) of work item gidx (an
-// FGroup of two bands), run by the CTA's PShape<LOGN>::NT threads.
+// One work unit: FFT times t0 .. of an item of two bands, run by the CTA's
+// PShape<LOGN>::NT threads in nit rounds.  I: the item, fcs: the constants of its
+// FFTs from t0 on, both in shared memory.
 // VAR 1: raw INTERLACEDVDIF reads; VAR 2: complex sampling.
 template <int LOGN, bool TCO, int VAR>
-__device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx, const int tchunk, const int tq,
-                                                 const float2 *tw, ulonglong2 *fsm, const float *lut8,
-                                                 const u64 *lut4, PairConst *fcs, PairOut *po)
+__device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem &I, const PairConst *fcs, const int t0,
+                                                 const int nit, const float2 *tw, ulonglong2 *fsm, const float *lut8,
+                                                 const u64 *lut4)
 {
 	using SH = PShape<LOGN>;
 	constexpr int N = SH::N, TPF = SH::TPF, FPC = SH::FPC, PADN = SH::PADN, RL = SH::RL;
 	constexpr bool MUX = VAR == 1, CPLX = VAR == 2;
 	constexpr int nchan = CPLX ? N : N / 2;
 	constexpr uint32_t S8 = N / 8;
-	const FGroup &g = a.groups[gidx];
-	const DevStation *Sp = a.st + g.station;
-	const uint32_t fs = (uint32_t)Sp->framesamples;
-	const int nbits = Sp->nbits;
-	constexpr uint32_t cpl = CPLX ? 2u : 1u;
-	const uint32_t bpt = MUX ? (uint32_t)nbits : (uint32_t)(Sp->nband * nbits) * cpl;
-	const int header = Sp->header, framebytes = Sp->framebytes;
-	const uint8_t *buf = a.sub[g.station].buf;
-	const uint8_t *vrow = a.valid + (int64_t)g.station * a.valid_stride;
-	const int32_t *mslot = MUX ? a.sub[g.station].mux_slot : nullptr;
-	const int64_t mk0 = MUX ? a.sub[g.station].mux_k0 : 0;
-	const int mnthr = Sp->nthr, minfb = Sp->inframebytes;
+	const uint32_t fs = I.fs, bpt = I.bpt;
+	const int nbits = I.nbits;
 	const int slot = threadIdx.x / TPF, b = threadIdx.x - slot * TPF;
 	ulonglong2 *const side = fsm + (size_t)slot * PADN;
-	const bool lsb = g.lsb != 0;
-	const int band0 = g.band[0], band1 = g.band[1];
-	const uint32_t boff0 = MUX ? 0u : (uint32_t)(band0 * nbits) * cpl, boff1 = MUX ? 0u : (uint32_t)(band1 * nbits) * cpl;
-	// both bands side by side in one field of 2 nbits, aligned to its size
-	const bool adj = !MUX && !CPLX && boff1 == boff0 + (uint32_t)nbits && boff0 % (2u * (uint32_t)nbits) == 0;
+	const bool lsb = I.lsb != 0;
 	const int order = a.order;
 	constexpr float osc = TCO ? 1.0f / (float)(1 << kTcSpecExp) : 1.0f;
-	const int t0 = tchunk * tq * FPC;
-	const int nit = min(tq, (a.T - t0 + FPC - 1) / FPC);
-
-	// ---- the unit's place in the spectra, by the CTA's last thread
-	if(threadIdx.x == blockDim.x - 1)
-	{
-		const DevFreqPlan &P = a.plans[g.freq];
-		const int row0 = g.row[0] < 0 ? 0 : g.row[0];
-		PairOut u;
-		u.tcb = TCO ? (uint32_t)P.tcb : 0u;
-		u.magic = TCO ? 0xFFFFFFFFu / u.tcb + 1u : 0u;
-		u.bextra = TCO ? (uint32_t)(P.trow - 1) * u.tcb : 0u;
-		u.pbits = TCO ? P.pbits : 0;
-		const int rstr = TCO ? P.tcb : nchan;
-		u.rowd = (g.row[1] - row0) * rstr;
-		u.tstride = TCO ? (int64_t)P.tnblk * P.trow * P.tcb : (int64_t)P.nrow * nchan;
-		u.first = P.spec_off + (int64_t)row0 * rstr;
-		u.flags = (g.row[0] >= 0 ? kORow0 : 0) | (g.row[1] >= 0 ? kORow1 : 0) | (a.h16 ? kOH16 : 0);
-		// four channels of a thread at once: blocks of a power of two channels
-		if(TCO && !CPLX && (u.tcb == 2 || u.tcb == 4 || u.tcb == 8) && !(lsb && order == 0))
-			u.flags |= kOQuad;
-		if((u.flags & kORow0) && (u.flags & kORow1) && u.rowd == 2 && !(row0 & 1) && TCO && !(P.trow & 1))
-			u.flags |= kOBoth;
-		*po = u;
-	}
-	// ---- constants of the unit's FFTs (FFT f is time t0 + f), one thread per FFT
-	for(int f = threadIdx.x; f < nit * FPC; f += blockDim.x)
-	{
-		const int t = t0 + f;
-		PairConst c;
-		memset(&c, 0, sizeof(c));
-		c.st = c.os[0] = c.os[1] = make_float2(1.0f, 0.0f);
-		const FftParam *pq = a.params + (int64_t)g.station * a.T + t;
-		if(t < a.T && pq->status == kFftOk)
-		{
-			c.flags = kPActive;
-			const uint32_t g0 = (uint32_t)pq->nearest;
-			c.fa = g0 / fs;
-			c.so = g0 - c.fa * fs;
-			c.stuck = pq->stuck;
-			const double invN = 1.0 / N, lo = g.lofreq;
-			const int idl = pq->integerdelay;
-			const double fraclo = a.fraclo ? (lo - (int)lo) * (double)idl : 0.0;
-			// LO offset: seconds since the job start of the FFT's first sample
-			// (mode.cpp:686-694; the scan starts with the job) and the offset's
-			// turns per sample
-			const double walls = (double)a.sub[g.station].subsec + a.sub[g.station].subns / 1.0e9 +
-			                     (double)t * N * Sp->sampletime / 1.0e6;
-			const double low = g.corr ? looff_wall_turns(g.looff, walls) : 0.0;
-			const double los = -g.looff * Sp->sampletime / 1.0e6;
-			double postf = 0.0;
-			if(order == 1)
-			{
-				c.P0 = frac_centered(lo * pq->b + fraclo + low);
-				c.alpha = (float)(lo * pq->a * invN + los);
-				c.st = cispi2(-(double)c.alpha * (double)S8);
-			}
-			else if(order == 2)
-			{
-				const double pa = pq->a, pb = pq->b;
-				const double X1 = (double)Sp->asl * invN;
-				c.P0 = frac_centered(lo * pq->c + fraclo + low);
-				c.alpha = (float)(lo * (pb + pa * X1) * invN + los);
-				c.beta = (float)(lo * 2.0 * pa * X1 * invN);
-				c.gamma = (float)(lo * pb * Sp->asl * invN + los * Sp->asl);
-				c.eps = (float)(lo * pa * X1 * X1);
-			}
-			else
-			{
-				double pr = (pq->averagedelay - idl) * lo;
-				if(a.fraclo)
-					pr += idl * (lo - (int)lo);
-				pr -= walls * g.looff;
-				postf = -(double)(float)(pr - (int)pr);
-			}
-			// per band: fse - clock offset (mode.cpp:1053-1059, 1099-1106); the
-			// channel of an order-0 lower sideband falls with the bin
-			const double sgn = lsb && (order == 0 || CPLX) ? -1.0 : 1.0;
-			c.flags |= kPSame;
-			for(int j = 0; j < 2; j++)
-			{
-				const double D = Sp->bw * (1.0 / nchan) * ((double)pq->fse - g.clk[j]);
-				split_turns(D, c.dhi[j], c.dlo[j]);
-				c.post[j] = (float)postf + g.phase[j];
-				if(j == 0 || g.clk[1] != g.clk[0])
-					c.os[j] = cispi2(sgn * D * (double)S8);
-				else
-					c.os[1] = c.os[0];
-			}
-			if(g.clk[1] != g.clk[0] || g.phase[1] != g.phase[0])
-				c.flags &= ~kPSame;
-			// validity of the window's frames, one bit per frame relative to fa
-			const uint32_t nwf = (c.so + (uint32_t)N - 1) / fs + 1, nm = nwf < 32u ? nwf : 32u;
-			for(uint32_t k = 0; k < nm; k++)
-			{
-				const int64_t fr = (int64_t)c.fa + k;
-				// complex data: the unpack's first frame is checked for fill
-				// pattern only (mark5_stream_unpacker.c:189)
-				const uint8_t *vsrc = (CPLX && k == 0 && a.fillok) ? a.fillok + (int64_t)g.station * a.valid_stride : vrow;
-				if(fr < a.valid_stride && vsrc[fr] != 0)
-					c.fmask |= 1u << k;
-			}
-			if(nwf <= 32)
-				c.flags |= kPNarrow;
-			if(a.bandok)
-			{
-				// EDV4-blanked bands (INTERLACEDVDIF): the general decode path below
-				const uint32_t need = (1u << band0) | (1u << band1);
-				for(uint32_t k = 0; k < nwf; k++)
-				{
-					const int64_t fk = (int64_t)c.fa + k;
-					if(fk < a.valid_stride && vrow[fk] != 0 &&
-					   (a.bandok[(int64_t)g.station * a.valid_stride + fk] & need) != need)
-						c.flags |= kPBlank;
-				}
-			}
-			const bool whole = nwf < 32 && c.fmask == (1u << nwf) - 1u && c.stuck >= N && !(c.flags & kPBlank);
-			if(whole && adj && fs >= S8)
-				c.flags |= kPFast;
-			if(MUX && whole && nwf <= 2)
-			{
-				// valid frames of raw reads are complete slots: every thread is there
-				c.flags |= kPFast;
-				const int32_t *s0 = mslot + (mk0 + (int64_t)c.fa) * mnthr, *s1 = nwf == 2 ? s0 + mnthr : s0;
-				c.mi00 = s0[band0];
-				c.mi01 = s0[band1];
-				c.mi10 = s1[band0];
-				c.mi11 = s1[band1];
-			}
-		}
-		fcs[f] = c;
-	}
-	__syncthreads();
 
 	for(int it = 0; it < nit; it++)
 	{
 		const int t = t0 + it * FPC + slot;
 		const PairConst &fc = fcs[it * FPC + slot];
-		const int flags = fc.flags;
+		// constants past T are not there: such slots take part in the barriers only
+		const int flags = t < a.T ? fc.flags : 0;
 		// ---- 1. decode: the levels of samples b + r N/8 of both bands
 		u64 lv[8], lu[CPLX ? 8 : 1];        // lu: imaginary parts (complex sampling)
-		const uint32_t so = fc.so, xs = so + (uint32_t)b;
+		const uint32_t xs = fc.so + (uint32_t)b;
 		if(!CPLX && !MUX && (flags & kPFast))
 		{
 			// one running bit position: a frame boundary skips a header
 			// (so < fs and b < N/8 <= fs: at most one boundary before sample b)
-			uint32_t tin = xs, bit = xs * bpt + boff0;
+			const uint32_t hbits = I.hbits;
+			uint32_t tin = xs, bit = xs * bpt + I.boff0;
 			if(tin >= fs)
 			{
 				tin -= fs;
-				bit += (uint32_t)header * 8u;
+				bit += hbits;
 			}
-			const uint32_t *wp = (const uint32_t *)(buf + (int64_t)fc.fa * framebytes + header);
+			const uint32_t *wp = (const uint32_t *)fc.wp;
 			uint32_t raw[8], sh[8];
 #pragma unroll
 			for(int r = 0; r < 8; r++)
@@ -451,7 +275,7 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 				if(tin >= fs)
 				{
 					tin -= fs;
-					bit += (uint32_t)header * 8u;
+					bit += hbits;
 				}
 			}
 			if(nbits == 2)
@@ -472,8 +296,10 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 		}
 		else if(MUX && (flags & kPFast))
 		{
-			const uint8_t *f00 = buf + (int64_t)fc.mi00 * minfb + 32, *f01 = buf + (int64_t)fc.mi01 * minfb + 32;
-			const uint8_t *f10 = buf + (int64_t)fc.mi10 * minfb + 32, *f11 = buf + (int64_t)fc.mi11 * minfb + 32;
+			const uint8_t *buf = fc.wp + 32;
+			const int minfb = I.minfb;
+			const uint8_t *f00 = buf + (int64_t)fc.mi00 * minfb, *f01 = buf + (int64_t)fc.mi01 * minfb;
+			const uint8_t *f10 = buf + (int64_t)fc.mi10 * minfb, *f11 = buf + (int64_t)fc.mi11 * minfb;
 			uint32_t raw0[8], raw1[8], sh[8];
 #pragma unroll
 			for(int r = 0; r < 8; r++)
@@ -499,6 +325,10 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 		{
 			// frames, validity and blanking sample by sample
 			const bool narrow = (flags & kPNarrow) != 0, blank = (flags & kPBlank) != 0;
+			const int station = I.station, band0 = I.band0, band1 = I.band1, minfb = I.minfb;
+			const uint8_t *buf = a.sub[station].buf, *vrow = a.valid + (int64_t)station * a.valid_stride;
+			const int32_t *mslot = MUX ? a.sub[station].mux_slot : nullptr;
+			const int64_t mk0 = MUX ? a.sub[station].mux_k0 : 0;
 			uint32_t kf = xs / fs, tin = xs - kf * fs;
 #pragma unroll
 			for(int r = 0; r < 8; r++)
@@ -514,18 +344,18 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 				float v0 = 0.0f, v1 = 0.0f, u0 = 0.0f, u1 = 0.0f;
 				if(ok)
 				{
-					const uint32_t bit0 = tin * bpt + boff0, bit1 = tin * bpt + boff1;
+					const uint32_t bit0 = tin * bpt + I.boff0, bit1 = tin * bpt + I.boff1;
 					uint32_t w0, w1;
 					if constexpr(MUX)
 					{
-						const int32_t *slr = mslot + (mk0 + fr) * mnthr;
+						const int32_t *slr = mslot + (mk0 + fr) * I.mnthr;
 						const int i0 = __ldg(slr + band0), i1 = __ldg(slr + band1);
 						w0 = i0 >= 0 ? __ldg((const uint32_t *)(buf + (int64_t)i0 * minfb + 32) + (bit0 >> 5)) : 0u;
 						w1 = i1 >= 0 ? __ldg((const uint32_t *)(buf + (int64_t)i1 * minfb + 32) + (bit1 >> 5)) : 0u;
 					}
 					else
 					{
-						const uint32_t *wp = (const uint32_t *)(buf + fr * framebytes + header);
+						const uint32_t *wp = (const uint32_t *)(buf + fr * I.framebytes + I.header);
 						w0 = __ldg(wp + (bit0 >> 5));
 						w1 = __ldg(wp + (bit1 >> 5));
 					}
@@ -542,7 +372,7 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 					{
 						// bands of this sample's frame blanked by its EDV4 validity mask
 						// (blank_vdif_EDV4, format_vdif.c:4699-4780)
-						const uint32_t bo = a.bandok[(int64_t)g.station * a.valid_stride + fr];
+						const uint32_t bo = a.bandok[(int64_t)station * a.valid_stride + fr];
 						if(!((bo >> band0) & 1u))
 							v0 = u0 = 0.0f;
 						if(!((bo >> band1) & 1u))
@@ -578,7 +408,7 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 			{
 				if(order == 2)
 				{
-					const int n = b + r * (int)S8, asl = Sp->asl;
+					const int n = b + r * (int)S8, asl = I.asl;
 					const int kk = n / asl, jj = n - kk * asl;
 					float ph = fc.P0 + (float)jj * fc.alpha + (float)(kk * jj) * fc.beta + (float)kk * fc.gamma +
 					           (float)(kk * kk) * fc.eps;
@@ -620,16 +450,16 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 			continue;
 		constexpr int sL = N / RL, J = 8 / RL;
 		const bool same = (flags & kPSame) != 0;
-		const int oflags = po->flags;
+		const int oflags = I.oflags;
 		const bool h16 = (oflags & kOH16) != 0;
-		const int rowd = po->rowd;
-		const int64_t base = po->first + (int64_t)t * po->tstride;
+		const int rowd = I.rowd;
+		const int64_t base = I.first + (int64_t)t * I.tstride;
 		auto put = [&](int c, const cp &y) {
 			const float2 re = up2(y.re), im = up2(y.im);
 			if constexpr(TCO)
 			{
-				const uint32_t p = (uint32_t)chan_pos(po->pbits, c);
-				uint32_t *o = (uint32_t *)a.spec + base + (p + __umulhi(p, po->magic) * po->bextra);
+				const uint32_t p = (uint32_t)chan_pos(I.pbits, c);
+				uint32_t *o = (uint32_t *)a.spec + base + (p + __umulhi(p, I.magic) * I.bextra);
 				if(oflags & kORow0)
 					*o = pack_spec(h16, re.x, im.x);
 				if(oflags & kORow1)
@@ -762,7 +592,7 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 						q0[m] = pack_spec(h16, re.x, im.x);
 						q1[m] = pack_spec(h16, re.y, im.y);
 					}
-					const uint32_t tcb = po->tcb, bextra = po->bextra;
+					const uint32_t tcb = I.tcb, bextra = I.bextra;
 					uint32_t *o = (uint32_t *)a.spec + base +
 					              (4u * (uint32_t)b + (tcb == 2 ? 2u * (uint32_t)b : (tcb == 4 ? (uint32_t)b : (uint32_t)b >> 1)) * bextra);
 					if(tcb >= 4)
@@ -804,6 +634,65 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const int gidx
 				}
 			}
 		}
+	}
+}
+
+__device__ __forceinline__ void pair_cp16(void *dst, const void *src)
+{
+	asm volatile("cp.async.ca.shared.global [%0], [%1], 16;\n" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src));
+}
+__device__ __forceinline__ void pair_cp_wait() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
+// a unit's item and constants into shared memory (pair_cp_wait and a barrier
+// before they are read)
+__device__ __forceinline__ void pair_fetch(PairItem *I, PairConst *fcs, const void *item, const void *consts, int nfc)
+{
+	for(int i = threadIdx.x; i < nfc * (int)(sizeof(PairConst) / 16); i += blockDim.x)
+		pair_cp16((char *)fcs + 16 * i, (const char *)consts + 16 * i);
+	if(threadIdx.x < sizeof(PairItem) / 16)
+		pair_cp16((char *)I + 16 * threadIdx.x, (const char *)item + 16 * threadIdx.x);
+}
+
+// The units of a persistent launch's work-list class, CTAs striding over them
+// (the units of a class cost about the same).  Fetched ahead: while unit k runs, the
+// constants of k + 1 and the record of k + 2 are on their way, so that no unit
+// waits for a chain of loads.
+template <int NFC>
+struct PairFeed {
+	FsMultiUnit rec[3];
+	PairItem item[2];
+	PairConst fcs[2][NFC];
+};
+
+template <int NFC, class F>
+__device__ __forceinline__ void pair_units(PairFeed<NFC> &s, const FsMultiArgs &m, const int cls, F &&run)
+{
+	static_assert(sizeof(FsMultiUnit) % 16 == 0 && sizeof(PairItem) % 16 == 0 && sizeof(PairConst) % 16 == 0, "copies");
+	const FsMultiUnit *units = m.units + m.unit0[cls];
+	const int n = m.nunit[cls], step = gridDim.x;
+	constexpr int R16 = sizeof(FsMultiUnit) / 16;
+	auto record = [&](int k, int u) {
+		if(u < n && threadIdx.x < R16)
+			pair_cp16((char *)&s.rec[k % 3] + 16 * threadIdx.x, (const char *)(units + u) + 16 * threadIdx.x);
+	};
+	auto consts = [&](int k, int u) {
+		const FsMultiUnit &r = s.rec[k % 3];
+		if(u < n)
+			pair_fetch(&s.item[k & 1], s.fcs[k & 1], r.pitem, r.consts, r.nfc);
+	};
+	int u = blockIdx.x;
+	record(0, u);
+	record(1, u + step);
+	pair_cp_wait();
+	__syncthreads();
+	consts(0, u);
+	for(int k = 0; u < n; k++, u += step)
+	{
+		pair_cp_wait();
+		__syncthreads();
+		consts(k + 1, u + step);
+		record(k + 2, u + 2 * step);
+		run(s.rec[k % 3], s.item[k & 1], s.fcs[k & 1]);
 	}
 }
 

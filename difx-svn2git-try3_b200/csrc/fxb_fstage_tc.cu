@@ -25,11 +25,10 @@
 //
 // Persistent CTAs (one per SM, 18 warps at 96 registers: an SM sub-partition
 // holds at most five of them in its 16384 registers), warp-specialised:
-//   warp 17     producer: builds the records of 32 units at a time (one lane
-//               per unit: pair, FFT parameters, fringe and fractional-sample
-//               constants, output offsets) into a shared-memory ring and
-//               stages each unit's VDIF window into shared memory (bulk
-//               copies of the valid frames),
+//   warp 17     producer: passes the units' records (k_tc_units: FFT parameters,
+//               fringe and fractional-sample constants, output offsets) on
+//               through a shared-memory ring and stages each unit's VDIF
+//               window into shared memory (bulk copies of the valid frames),
 //   warps 0-7   decode: 8 consecutive times -> the fringe-rotated FP16
 //               samples of the unit's four channels (two-time lookup of
 //               both polarisations, FP32 rotation),
@@ -265,9 +264,9 @@ __device__ __forceinline__ float level2f(uint32_t code)
 
 __device__ __forceinline__ float fracc(double x) { return (float)(x - rint(x)); }
 
-// Everything the roles need of one work unit, built by the producer warp
-// (one lane per unit, 32 units at a time) into a shared-memory ring.
-struct UnitRec {
+// Everything the roles need of one work unit, built by k_tc_units and passed on by
+// the producer warp through a shared-memory ring.
+struct alignas(16) UnitRec {
 	float P0[2], alpha[2];        // fringe phase (turns) at n = 0 and per sample, per subband
 	float Sr[2], Si[2];           // rotator step over one sample exp(-2 pi i alpha)
 	float S2r[2], S2i[2];         // and over two
@@ -279,6 +278,8 @@ struct UnitRec {
 	uint32_t fa;                  // first frame of the window
 	int64_t a0;                   // first staged byte of the payloads from frame fa on
 	int32_t nstage, station;      // staged bytes; station
+	const uint8_t *src;           // payload of frame fa
+	int32_t payload, framebytes;
 	int32_t t;                    // FFT time
 	float dhi[2][2], dlo[2][2];   // fractional-sample turns per channel of [subband][polarisation] (split_turns)
 	float st32[2][2], st256[2][2];   // the same over 32 and 256 channels, reduced to [-1/2, 1/2)
@@ -304,9 +305,8 @@ struct TcLayout {
 	static_assert(kSmem <= 227 * 1024, "shared memory");
 };
 
-// the producer lane's record of unit k (u = blockIdx.x + k gridDim.x)
-template <int BPT>
-__device__ __forceinline__ UnitRec build_unit(const FsArgs &a, const int32_t *pairs, int npairs, int u)
+// the record of unit u; BPT: bits per time of the stations' VDIF words
+__device__ __forceinline__ UnitRec build_unit(const FsArgs &a, const int32_t *pairs, int npairs, int BPT, int u)
 {
 	constexpr int nchan = kN / 2;
 	UnitRec r;
@@ -394,23 +394,33 @@ __device__ __forceinline__ UnitRec build_unit(const FsArgs &a, const int32_t *pa
 		const int64_t a1 = (((b1 + 7) >> 3) + 15) & ~(int64_t)15;
 		r.swbits = (int32_t)(b0 - 8 * r.a0);
 		r.nstage = (int32_t)(a1 - r.a0);
+		r.src = a.sub[s].buf + (int64_t)r.fa * Sp->framebytes + Sp->header;
+		r.payload = Sp->payload;
+		r.framebytes = Sp->framebytes;
 		if(((uintptr_t)a.sub[s].buf & 15u) != 0)
 			r.flags |= kManual;
 	}
 	return r;
 }
 
+// Records of a subint's units, one thread each.  On their own because the FP64
+// terms and their chain of loads made the producer warp the slowest role.
+__global__ void __launch_bounds__(64) k_tc_units(const FsArgs a, const int32_t *__restrict__ pairs, int npairs, int bpt,
+                                                 int nunits, UnitRec *__restrict__ rec)
+{
+	const int u = blockIdx.x * blockDim.x + threadIdx.x;
+	if(u < nunits)
+		rec[u] = build_unit(a, pairs, npairs, bpt, u);
+}
+
 }  // namespace
 
 // tables: DFT-32 (B of MMA 1), DFT-64 upper and lower sideband (B of MMA 2),
-// in their shared-memory byte layouts.  pairs: [npairs][2] FGroup indices of
-// the two subbands of a work unit (-1: none); unit u = pair u % npairs at
-// FFT time u / npairs.  BPT: bits per time of the stations' VDIF words
-// (2-bit bands: 2 x bands).
+// in their shared-memory byte layouts.  recs: the subint's units.  BPT: bits
+// per time of the stations' VDIF words (2-bit bands: 2 x bands).
 template <int BPT, bool H16>
 __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, const uint4 *__restrict__ tables,
-                                                          const int32_t *__restrict__ pairs, int npairs, int nunits,
-                                                          int32_t *err)
+                                                          const UnitRec *__restrict__ recs, int nunits, int32_t *err)
 {
 	using LY = TcLayout<BPT>;
 	extern __shared__ __align__(1024) unsigned char fsm_tc[];
@@ -490,7 +500,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 		{
 			UnitRec r;
 			if(kb + lane < nk)
-				r = build_unit<BPT>(a, pairs, npairs, (int)blockIdx.x + (kb + lane) * (int)gridDim.x);
+				r = recs[(int)blockIdx.x + (kb + lane) * (int)gridDim.x];
 			for(int i = 0; i < 32 && kb + i < nk; i++)
 			{
 				const int k = kb + i, slot = k % kNStg;
@@ -508,8 +518,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 					uint32_t want = 0;
 					const bool copy = (r.flags & kOk) && !(r.flags & kManual);
 					const int nwf = (r.so + kN - 1) / r.fs + 1;
-					const DevStation *Sp = a.st + r.station;
-					const int P = Sp->payload;
+					const int P = r.payload;
 					const int64_t a1 = r.a0 + r.nstage;
 					for(int j = 0; copy && j < nwf && j < 32; j++)
 					{
@@ -522,13 +531,12 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 						// the byte count is armed before the copies that complete it
 						mbar_expect_tx(&stg_full[slot], want);
 						unsigned char *dst = stg + slot * LY::kStgBytes;
-						const uint8_t *buf = a.sub[r.station].buf;
 						for(int j = 0; j < nwf && j < 32; j++)
 						{
 							const int64_t f0 = (int64_t)j * P, lo_ = r.a0 > f0 ? r.a0 : f0, hi_ = a1 < f0 + P ? a1 : f0 + P;
 							if(hi_ <= lo_ || !((r.fmask >> j) & 1u))
 								continue;
-							const uint8_t *src = buf + ((int64_t)r.fa + j) * Sp->framebytes + Sp->header + (lo_ - f0);
+							const uint8_t *src = r.src + (int64_t)j * r.framebytes + (lo_ - f0);
 							bulk_g2s(dst + (lo_ - r.a0), src, (uint32_t)(hi_ - lo_), &stg_full[slot]);
 						}
 					}
@@ -1042,9 +1050,18 @@ bool fstage_tc_eligible(int N, int order, bool any_lsb)
 	return N == kN && (order == 1 || (order == 0 && !any_lsb));
 }
 
+size_t fstage_tc_rec_bytes(int npairs, int T) { return sizeof(UnitRec) * (size_t)npairs * T; }
+
+void launch_tc_units(const FKind &k, const FsArgs &a, cudaStream_t stream)
+{
+	const int nunits = k.tcnpairs * a.T;
+	if(k.tcrec && nunits > 0)
+		k_tc_units<<<(nunits + 63) / 64, 64, 0, stream>>>(a, k.tcpairs, k.tcnpairs, k.tcbpt, nunits, (UnitRec *)k.tcrec);
+}
+
 cudaError_t launch_fstage_tc(const FKind &k, FsArgs a, int nsm, cudaStream_t stream)
 {
-	if(k.count <= 0 || a.T <= 0 || !k.tctab || !k.tcpairs || k.tcnpairs <= 0)
+	if(k.count <= 0 || a.T <= 0 || !k.tctab || !k.tcrec || k.tcnpairs <= 0)
 		return cudaSuccess;
 	a.first = k.first;
 	const int nunits = k.tcnpairs * a.T;
@@ -1053,7 +1070,7 @@ cudaError_t launch_fstage_tc(const FKind &k, FsArgs a, int nsm, cudaStream_t str
 		grid = nunits;
 	auto go = [&](auto kern, size_t smem) {
 		cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-		kern<<<grid, kThreadsTc, smem, stream>>>(a, (const uint4 *)k.tctab, k.tcpairs, k.tcnpairs, nunits, a.err);
+		kern<<<grid, kThreadsTc, smem, stream>>>(a, (const uint4 *)k.tctab, (const UnitRec *)k.tcrec, nunits, a.err);
 	};
 	const bool h = a.h16 != 0;
 	switch(k.tcbpt)

@@ -155,10 +155,12 @@ struct FKind {
 	const void *tw;          // twiddle table of length N (make_fstage_twiddles layout)
 	const void *tctab;       // constant tables of the tensor-core FFT kernel
 	const int32_t *tcpairs;  // tensor-core FFT: [tcnpairs][2] FGroup indices of each work unit's two subbands
+	void *tcrec;             // tensor-core FFT: records of the subint's work units (launch_tc_units)
 	int32_t tcnpairs;
 	int32_t tcbpt;           // tensor-core FFT: bits per time of the stations' VDIF words
 	int32_t muxraw;          // 1: the items' stations hand over raw INTERLACEDVDIF reads
 	int32_t cplx;            // 1: the items' stations sample complex (N = nchan points)
+	int32_t pair0;           // two-band kinds: first PairItem
 	int32_t persist;         // 1: run by the persistent launches (launch_fstage_multi), not launch_fstage_kind
 };
 
@@ -167,6 +169,46 @@ struct FKind {
 // |X| <= 16384 x 38.8) stays inside the FP16 range; the XMAC epilogue scales
 // the products back by 2^(2 kTcSpecExp), exactly.
 constexpr int kTcSpecExp = 5;
+
+// Two-band items (csrc/fxb_fstage_pair.cuh).  Constants of one FFT of one item,
+// computed by k_pair_consts with the subint's FFT parameters.
+struct alignas(16) PairConst {
+	float P0, alpha, beta, gamma;        // fringe phase (turns): start and per-sample terms
+	float eps;
+	float2 st;                           // order 1: rotator step over N/8 samples, exp(-2 pi i alpha N/8)
+	int32_t flags;
+	float dhi[2], dlo[2];                // fractional-sample turns per channel of each band (split_turns)
+	float2 os[2];                        // rotator step over N/8 channels of each band
+	float post[2];                       // order-0 post-F turns and the band's phase offset
+	const uint8_t *wp;                   // first payload byte of the window's first frame (raw reads: the buffer)
+	uint32_t fa, so;                     // first frame of the window, window start within it
+	uint32_t fmask;                      // validity of the window's frames (bit k: frame fa + k)
+	int32_t stuck;                       // samples [stuck, N) read as zero
+	int32_t mi00, mi01, mi10, mi11;      // raw reads: thread frames of the window's first and second frame, per band
+};
+// What does not change from subint to subint: the samples' place in the frames
+// and the spectra's place.  FP32 form [t][row][chan]; tensor-core form blocked
+// [t][block][trow][tcb] in the order of chan_pos.
+struct alignas(16) PairItem {
+	int64_t first, tstride;              // the first band's value of time 0, channel (position) 0; a time
+	int32_t rowd;                        // from the first band's values to the second's
+	uint32_t tcb, magic, bextra;         // channels of a block; p / tcb = umulhi(p, magic) for p < 2^16;
+	                                     // position p sits at p + p / tcb x bextra
+	int32_t pbits, oflags;
+	uint32_t fs, bpt, boff0, boff1;      // samples per frame, bits per time, first bit of each band
+	uint32_t hbits;                      // header bits
+	int32_t nbits, header, framebytes, minfb, mnthr;
+	int32_t station, band0, band1, lsb, asl, adj;   // adj: both bands side by side in one aligned field
+	int32_t group, pad_[3];
+};
+enum : int32_t { kORow0 = 1, kORow1 = 2, kOH16 = 4, kOQuad = 8, kOBoth = 16 };
+enum : int32_t {
+	kPActive = 1,     // valid FFT
+	kPNarrow = 2,     // fmask covers the window
+	kPBlank = 4,      // a valid frame of the window blanks one of the item's bands
+	kPSame = 8,       // the two bands take the same output rotation
+	kPFast = 16       // every sample of the window counts and the fast read applies
+};
 
 struct FsArgs {
 	const DevStation *st;
@@ -184,8 +226,12 @@ struct FsArgs {
 	void *spec;              // [t][row][chan]: float2 (out 0), or half2 / bf16x2 (out 1) scaled by 2^-kTcSpecExp
 	int32_t *err;            // device error flag (bounded waits of the tensor-core FFT kernel)
 	int32_t h16;             // out 1: spectra as FP16 (else BF16)
-	int32_t pad_;
+	int32_t pair0;           // set from FKind::pair0 by launch_fstage_kind
+	const PairItem *pitems;  // two-band items, and the constants of their FFTs [item][T]
+	PairConst *pconst;
 };
+// constants of the subint's FFTs of a two-band kind's items
+void launch_pair_consts(const FKind &k, const FsArgs &a, cudaStream_t stream);
 
 bool fstage_plan(int N, int nb, int out, FKind *k);
 // the kernels of one-band and two-band items by output form, and the
@@ -207,7 +253,7 @@ void launch_fstage_kind(const FKind &k, FsArgs a, cudaStream_t stream);
 // units.  Every tensor-core-form context runs these kinds this way, alone or in
 // a batch, so results do not depend on it.
 constexpr int kFsMultiMembers = 16;
-constexpr int kFsMultiFc = 128;          // FFT constants of one unit of up to 2048 points at most (tq x fpc)
+constexpr int kFsMultiFc = 64;           // FFT constants of one unit of up to 2048 points at most (tq x fpc)
 // classes of units: plain VDIF's (fstage_multi_class), then those of raw reads
 constexpr int kFsMultiPer = 5, kFsMultiClasses = 2 * kFsMultiPer;
 struct FsMultiKind {
@@ -215,8 +261,11 @@ struct FsMultiKind {
 	int32_t member, code;                // context; 128 x raw INTERLACEDVDIF reads + 32 x bands per item + log2 N
 	int32_t first, tq;                   // first FGroup of the kind, FFT iterations per unit
 };
-struct FsMultiUnit {
+struct alignas(16) FsMultiUnit {
 	int32_t kind, item, tchunk;
+	int32_t t0, nfc, pad_;               // two-band units: first FFT, FFTs
+	const PairItem *pitem;
+	const PairConst *consts;             // of FFT t0
 };
 struct FsMultiArgs {
 	FsArgs m[kFsMultiMembers];           // per context, with its subint's staging
@@ -244,6 +293,9 @@ cudaError_t launch_fstage_multi_on(const FsMultiArgs &m, int nsm, const cudaStre
 size_t fstage_tc_tables_bytes();
 void make_fstage_tc_tables(void *out);
 bool fstage_tc_eligible(int N, int order, bool any_lsb);
+size_t fstage_tc_rec_bytes(int npairs, int T);
+// the subint's unit records, before launch_fstage_tc
+void launch_tc_units(const FKind &k, const FsArgs &a, cudaStream_t stream);
 // returns the launch's error
 cudaError_t launch_fstage_tc(const FKind &k, FsArgs a, int nsm, cudaStream_t stream);
 

@@ -1,7 +1,7 @@
 """The corner turn of fxb_vdif_mux against numpy, byte for byte: the index
 permutation (2, 4, 8, 16 threads of 1, 2, 4, 8-bit fields) and the general form
-(other thread counts and widths), payloads of 16- and 32-byte alignment and
-without, and word counts that leave a CTA partly filled."""
+(other thread counts and widths), output buffers of 32-, 16- and 4-byte
+alignment, and word counts that leave a CTA partly filled."""
 import numpy as np
 import pytest
 import torch
@@ -11,18 +11,19 @@ from fxb200.native import vdif_mux_device
 
 pytestmark = pytest.mark.gpu
 
-CASES = [(nt, nb, 1000) for nt in (2, 4, 8, 16) for nb in (1, 2, 4, 8) if nt * nb <= 32] + \
-        [(1, 2, 1000), (3, 2, 1000), (5, 4, 1000), (32, 1, 1000), (16, 2, 4), (16, 2, 8), (16, 2, 520), (8, 2, 12), (4, 2, 5000)]
+CASES = [(nt, nb, 1000, 0) for nt in (2, 4, 8, 16) for nb in (1, 2, 4, 8) if nt * nb <= 32] + \
+        [(1, 2, 1000, 0), (3, 2, 1000, 0), (5, 4, 1000, 0), (32, 1, 1000, 0), (16, 2, 8, 0), (16, 2, 520, 16),
+         (16, 2, 24, 4), (8, 2, 40, 16), (4, 2, 5000, 4)]
 
 
-@pytest.mark.parametrize("nthreads,nbits,payload", CASES)
-def test_corner_turn(nthreads, nbits, payload):
+@pytest.mark.parametrize("nthreads,nbits,payload,off", CASES)
+def test_corner_turn(nthreads, nbits, payload, off):
     nframes, fps = 5, 1000
     data = synth.interlaced_vdif(nthreads=nthreads, nframes=nframes, payload=payload, nbits=nbits, fps=fps, seed=payload + nthreads)
     fb = payload + 32
     din = torch.from_numpy(data).cuda()
     ofb = payload * nthreads + 32
-    dout = torch.full((nframes * ofb,), 0xAB, dtype=torch.uint8, device="cuda")
+    dout = torch.full((nframes * ofb + off,), 0xAB, dtype=torch.uint8, device="cuda")[off:]
     n = vdif_mux_device(din.data_ptr(), data.size, list(range(nthreads)), fb, fps, nbits, dout.data_ptr(), dout.numel())
     assert n == nframes * ofb
     got = dout.cpu().numpy().reshape(nframes, ofb)
