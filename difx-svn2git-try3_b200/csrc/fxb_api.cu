@@ -144,6 +144,8 @@ struct fxb_ctx {
 	FsMultiUnit *d_punits = nullptr;
 	PairItem *d_pitems = nullptr;        // two-band items and the constants of their FFTs
 	PairConst *d_pconst = nullptr;
+	PairTwist *d_ptwist = nullptr;       // of the items from ptwist0 on
+	int ptwist0 = 0;
 	int32_t *d_pctr = nullptr;
 	void *d_specn = nullptr;             // half2 (or bf16x2) spectra of the tensor-core forms, X 2^-kTcSpecExp
 	void *d_tctab = nullptr;             // constant tables of the tensor-core FFT kernel
@@ -387,7 +389,8 @@ static PairItem pair_item(const fxb_ctx *ctx, const FGroup &g, int group, bool t
 	u.bextra = tc ? (uint32_t)(P.trow - 1) * u.tcb : 0u;
 	u.pbits = tc ? P.pbits : 0;
 	const int rstr = tc ? P.tcb : nchan;
-	u.rowd = (g.row[1] - row0) * rstr;
+	u.rowd = ctx->h_plans[g.freq1].spec_off - P.spec_off + (int64_t)(g.row[1] - row0) * rstr;
+	u.two = g.freq1 != g.freq;
 	u.tstride = tc ? (int64_t)P.tnblk * P.trow * P.tcb : (int64_t)P.nrow * nchan;
 	u.first = P.spec_off + (int64_t)row0 * rstr;
 	u.oflags = (g.row[0] >= 0 ? kORow0 : 0) | (g.row[1] >= 0 ? kORow1 : 0) | (ctx->h16 ? kOH16 : 0);
@@ -685,6 +688,8 @@ static fxb_status setup_device(fxb_ctx *ctx)
 			const int N = ctx->h_st[s].fftchannels;
 			const bool pairs = N <= 8192;
 			std::vector<int> done(js.nband, 0);
+			FGroup single;
+			bool waiting = false;
 			for(int b = 0; b < js.nband; b++)
 			{
 				if(done[b] || job.band_row[s][b] < 0)
@@ -711,10 +716,12 @@ static fxb_status setup_device(fxb_ctx *ctx)
 				g.nb = b1 >= 0 ? 2 : 1;
 				g.lsb = job.freqs[f].lower_sideband;
 				g.lofreq = job.freqs[f].freq_mhz;
+				g.freq1 = f;
 				// complex lower sideband: the effective LO is at negative
 				// frequency (mode.cpp:899-903)
 				if(js.cplx && g.lsb)
 					g.lofreq = -g.lofreq;
+				g.lofreq1 = g.lofreq;
 				if(js.has_corr)
 				{
 					// the phase offset rotates the non-R band of the frequency's
@@ -741,8 +748,35 @@ static fxb_status setup_device(fxb_ctx *ctx)
 				}
 				// raw INTERLACEDVDIF reads and complex sampling take their own
 				// kernel instantiations
-				bykind[{N, g.nb + (ctx->h_st[s].muxraw ? 16 : 0) + (ctx->h_st[s].cplx ? 32 : 0)}].push_back(g);
+				const int var = (ctx->h_st[s].muxraw ? 16 : 0) + (ctx->h_st[s].cplx ? 32 : 0);
+				// a single band pairs with the next single one of another subband of
+				// equal sideband and spectra shape (64: kinds of their own)
+				if(g.nb == 1 && pairs && !js.has_corr)
+				{
+					const DevFreqPlan &q = ctx->h_plans[f];
+					const DevFreqPlan *p = waiting ? &ctx->h_plans[single.freq] : nullptr;
+					if(p && single.lsb == g.lsb && p->nrow == q.nrow && p->nchan == q.nchan && p->tcb == q.tcb &&
+					   p->trow == q.trow && p->tnblk == q.tnblk)
+					{
+						single.band[1] = g.band[0];
+						single.row[1] = g.row[0];
+						single.nb = 2;
+						single.freq1 = f;
+						single.lofreq1 = g.lofreq;
+						bykind[{N, 2 + var + 64}].push_back(single);
+						waiting = false;
+						continue;
+					}
+					if(waiting)
+						bykind[{N, 1 + var}].push_back(single);
+					single = g;
+					waiting = true;
+					continue;
+				}
+				bykind[{N, g.nb + var}].push_back(g);
 			}
+			if(waiting)
+				bykind[{N, 1 + (ctx->h_st[s].muxraw ? 16 : 0) + (ctx->h_st[s].cplx ? 32 : 0)}].push_back(single);
 		}
 		std::vector<FGroup> hg;
 		std::vector<PairItem> pitems;
@@ -754,7 +788,14 @@ static fxb_status setup_device(fxb_ctx *ctx)
 				std::stable_sort(kv.second.begin(), kv.second.end(),
 				                 [](const FGroup &x, const FGroup &y) { return x.freq < y.freq; });
 		}
-		for(const auto &kv : bykind)
+		// kinds of mixed subbands (64) last: their items have twists
+		std::vector<std::pair<std::pair<int, int>, std::vector<FGroup>>> ordered;
+		for(int mixed = 0; mixed < 2; mixed++)
+			for(const auto &kv : bykind)
+				if(((kv.first.second >> 6) & 1) == mixed)
+					ordered.push_back(kv);
+		int ntwist = 0;
+		for(const auto &kv : ordered)
 		{
 			FKind k;
 			memset(&k, 0, sizeof(k));
@@ -770,6 +811,11 @@ static fxb_status setup_device(fxb_ctx *ctx)
 			if(k.nb == 2)
 			{
 				k.pair0 = (int)pitems.size();
+				k.two = (kv.first.second >> 6) & 1;
+				if(k.two && ntwist == 0)
+					ctx->ptwist0 = k.pair0;
+				if(k.two)
+					ntwist += k.count;
 				for(int i = 0; i < k.count; i++)
 					pitems.push_back(pair_item(ctx, kv.second[i], k.first + i, out == 1));
 			}
@@ -791,7 +837,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 					any_lsb = any_lsb || gg.lsb;
 				const char *env = getenv("FXB_TC_FFT");
 				// no EDV4 band blanking and no complex sampling there
-				const bool allow = !(env && env[0] == '0') && ctx->nbm == 0 && !k.cplx;
+				const bool allow = !(env && env[0] == '0') && ctx->nbm == 0 && !k.cplx && !(kv.first.second & 64);
 				std::vector<int32_t> pairs;
 				int bpt = 0;
 				if(allow && fstage_tc_eligible(k.N, job.fringe_rot_order, any_lsb) &&
@@ -835,6 +881,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 		}
 		CK(ctx, dalloc(ctx, &ctx->d_pitems, pitems.size()));
 		CK(ctx, dalloc(ctx, &ctx->d_pconst, pitems.size() * (size_t)ctx->T));
+		CK(ctx, dalloc(ctx, &ctx->d_ptwist, (size_t)ntwist * ctx->T));
 		if(!pitems.empty())
 			CK(ctx, cudaMemcpyAsync(ctx->d_pitems, pitems.data(), sizeof(PairItem) * pitems.size(), cudaMemcpyHostToDevice,
 			                        ctx->stream));
@@ -873,6 +920,8 @@ static fxb_status setup_device(fxb_ctx *ctx)
 						{
 							u.pitem = ctx->d_pitems + k.pair0 + it;
 							u.consts = ctx->d_pconst + (size_t)(k.pair0 + it) * ctx->T + u.t0;
+							if(k.two)
+								u.twists = ctx->d_ptwist + (size_t)(k.pair0 - ctx->ptwist0 + it) * ctx->T + u.t0;
 						}
 						dst.push_back(u);
 					}
@@ -1336,6 +1385,8 @@ static FsArgs fs_args(const fxb_ctx *ctx, const Slot &sl)
 	fa.h16 = ctx->h16 ? 1 : 0;
 	fa.pitems = ctx->d_pitems;
 	fa.pconst = ctx->d_pconst;
+	fa.ptwist = ctx->d_ptwist;
+	fa.ptwist0 = ctx->ptwist0;
 	return fa;
 }
 

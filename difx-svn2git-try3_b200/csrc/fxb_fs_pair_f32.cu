@@ -12,14 +12,16 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB) k_fstage
 	__shared__ float lut8[256];
 	__shared__ u64 lut4[16];
 	__shared__ PairConst fcs[kMaxTQ * FPC];
+	__shared__ PairTwist tws[kMaxTQ * FPC];
 	__shared__ PairItem I;
 	const int item = a.pair0 + (a.items_fast ? blockIdx.x : blockIdx.y);
 	const int t0 = (a.items_fast ? blockIdx.y : blockIdx.x) * a.tq * FPC, nfc = min(a.tq * FPC, a.T - t0);
-	pair_fetch(&I, fcs, a.pitems + item, a.pconst + (int64_t)item * a.T + t0, nfc);
+	pair_fetch(&I, fcs, tws, a.pitems + item, a.pconst + (int64_t)item * a.T + t0,
+	           a.two ? a.ptwist + (int64_t)(item - a.ptwist0) * a.T + t0 : nullptr, nfc);
 	fstage_pair_luts(lut8, lut4);
 	pair_cp_wait();
 	__syncthreads();
-	fstage_pair_unit<LOGN, TCO, VAR>(a, I, fcs, t0, (nfc + FPC - 1) / FPC, (const float2 *)a.tw, fsp, lut8, lut4);
+	fstage_pair_unit<LOGN, TCO, VAR>(a, I, fcs, tws, t0, (nfc + FPC - 1) / FPC, (const float2 *)a.tw, fsp, lut8, lut4);
 }
 
 template <int LOGN, bool TCO, int VAR>

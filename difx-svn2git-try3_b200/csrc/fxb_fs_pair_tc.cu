@@ -13,14 +13,16 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB) k_fstage
 	__shared__ float lut8[256];
 	__shared__ u64 lut4[16];
 	__shared__ PairConst fcs[kMaxTQ * FPC];
+	__shared__ PairTwist tws[kMaxTQ * FPC];
 	__shared__ PairItem I;
 	const int item = a.pair0 + (a.items_fast ? blockIdx.x : blockIdx.y);
 	const int t0 = (a.items_fast ? blockIdx.y : blockIdx.x) * a.tq * FPC, nfc = min(a.tq * FPC, a.T - t0);
-	pair_fetch(&I, fcs, a.pitems + item, a.pconst + (int64_t)item * a.T + t0, nfc);
+	pair_fetch(&I, fcs, tws, a.pitems + item, a.pconst + (int64_t)item * a.T + t0,
+	           a.two ? a.ptwist + (int64_t)(item - a.ptwist0) * a.T + t0 : nullptr, nfc);
 	fstage_pair_luts(lut8, lut4);
 	pair_cp_wait();
 	__syncthreads();
-	fstage_pair_unit<LOGN, TCO, VAR>(a, I, fcs, t0, (nfc + FPC - 1) / FPC, (const float2 *)a.tw, fsp, lut8, lut4);
+	fstage_pair_unit<LOGN, TCO, VAR>(a, I, fcs, tws, t0, (nfc + FPC - 1) / FPC, (const float2 *)a.tw, fsp, lut8, lut4);
 }
 
 template <int LOGN, bool TCO, int VAR>
@@ -43,7 +45,8 @@ __global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant
 	__shared__ u64 lut4[16];
 	__shared__ PairFeed<kFsMultiFc> feed;
 	fstage_pair_luts(lut8, lut4);
-	pair_units(feed, m, kFsMultiPer * VAR + 3, [&](const FsMultiUnit &w, const PairItem &I, const PairConst *fcs) {
+	pair_units(feed, m, kFsMultiPer * VAR + 3,
+	           [&](const FsMultiUnit &w, const PairItem &I, const PairConst *fcs, const PairTwist *tws) {
 		const FsMultiKind &k = m.kinds[w.kind];
 		const float2 *tw = (const float2 *)k.tw;
 		const FsArgs &a = m.m[k.member];
@@ -51,8 +54,8 @@ __global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant
 		{
 #define FXB_PAIR_CASE(LOGN)                                                                                            \
 	case LOGN:                                                                                                         \
-		fstage_pair_unit<LOGN, true, VAR>(a, I, fcs, w.t0, (w.nfc + PShape<LOGN>::FPC - 1) / PShape<LOGN>::FPC, tw, fsp, \
-		                                  lut8, lut4);                                                                  \
+		fstage_pair_unit<LOGN, true, VAR>(a, I, fcs, tws, w.t0, (w.nfc + PShape<LOGN>::FPC - 1) / PShape<LOGN>::FPC, tw, \
+		                                  fsp, lut8, lut4);                                                             \
 		break;
 			FXB_PAIR_CASE(5)
 			FXB_PAIR_CASE(6)
@@ -78,9 +81,9 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB)
 	__shared__ PairFeed<kMaxTQ> feed;
 	fstage_pair_luts(lut8, lut4);
 	pair_units(feed, m, kFsMultiPer * VAR + (LOGN == 12 ? 2 : 0),
-	           [&](const FsMultiUnit &w, const PairItem &I, const PairConst *fcs) {
+	           [&](const FsMultiUnit &w, const PairItem &I, const PairConst *fcs, const PairTwist *tws) {
 		           const FsMultiKind &k = m.kinds[w.kind];
-		           fstage_pair_unit<LOGN, true, VAR>(m.m[k.member], I, fcs, w.t0, w.nfc, (const float2 *)k.tw, fsp, lut8,
+		           fstage_pair_unit<LOGN, true, VAR>(m.m[k.member], I, fcs, tws, w.t0, w.nfc, (const float2 *)k.tw, fsp, lut8,
 		                                             lut4);
 	           });
 }
@@ -135,9 +138,8 @@ __global__ void __launch_bounds__(128) k_pair_consts(const FsArgs a, int N, int 
 		c.stuck = pq->stuck;
 		if(!mux)
 			c.wp += (int64_t)c.fa * I.framebytes + I.header;
-		const double invN = 1.0 / N, lo = g.lofreq;
+		const double invN = 1.0 / N;
 		const int idl = pq->integerdelay;
-		const double fraclo = a.fraclo ? (lo - (int)lo) * (double)idl : 0.0;
 		// LO offset: seconds since the job start of the FFT's first sample
 		// (mode.cpp:686-694; the scan starts with the job) and the offset's
 		// turns per sample
@@ -145,30 +147,60 @@ __global__ void __launch_bounds__(128) k_pair_consts(const FsArgs a, int N, int 
 		                     (double)t * N * Sp->sampletime / 1.0e6;
 		const double low = g.corr ? looff_wall_turns(g.looff, walls) : 0.0;
 		const double los = -g.looff * Sp->sampletime / 1.0e6;
-		double postf = 0.0;
-		if(order == 1)
+		double postf[2] = {0.0, 0.0};
+		for(int j = 0; j < (I.two ? 2 : 1); j++)
 		{
-			c.P0 = frac_centered(lo * pq->b + fraclo + low);
-			c.alpha = (float)(lo * pq->a * invN + los);
-			c.st = cispi2(-(double)c.alpha * (double)S8);
-		}
-		else if(order == 2)
-		{
-			const double pa = pq->a, pb = pq->b;
-			const double X1 = (double)Sp->asl * invN;
-			c.P0 = frac_centered(lo * pq->c + fraclo + low);
-			c.alpha = (float)(lo * (pb + pa * X1) * invN + los);
-			c.beta = (float)(lo * 2.0 * pa * X1 * invN);
-			c.gamma = (float)(lo * pb * Sp->asl * invN + los * Sp->asl);
-			c.eps = (float)(lo * pa * X1 * X1);
-		}
-		else
-		{
-			double pr = (pq->averagedelay - idl) * lo;
-			if(a.fraclo)
-				pr += idl * (lo - (int)lo);
-			pr -= walls * g.looff;
-			postf = -(double)(float)(pr - (int)pr);
+			const double lo = j ? g.lofreq1 : g.lofreq;
+			const double fraclo = a.fraclo ? (lo - (int)lo) * (double)idl : 0.0;
+			float P0 = 0.0f, alpha = 0.0f, beta = 0.0f, gamma = 0.0f, eps = 0.0f;
+			float2 st = make_float2(1.0f, 0.0f);
+			if(order == 1)
+			{
+				P0 = frac_centered(lo * pq->b + fraclo + low);
+				alpha = (float)(lo * pq->a * invN + los);
+				st = cispi2(-(double)alpha * (double)S8);
+			}
+			else if(order == 2)
+			{
+				const double pa = pq->a, pb = pq->b;
+				const double X1 = (double)Sp->asl * invN;
+				P0 = frac_centered(lo * pq->c + fraclo + low);
+				alpha = (float)(lo * (pb + pa * X1) * invN + los);
+				beta = (float)(lo * 2.0 * pa * X1 * invN);
+				gamma = (float)(lo * pb * Sp->asl * invN + los * Sp->asl);
+				eps = (float)(lo * pa * X1 * X1);
+			}
+			else
+			{
+				double pr = (pq->averagedelay - idl) * lo;
+				if(a.fraclo)
+					pr += idl * (lo - (int)lo);
+				pr -= walls * g.looff;
+				postf[j] = -(double)(float)(pr - (int)pr);
+			}
+			if(j == 0)
+			{
+				c.P0 = P0;
+				c.alpha = alpha;
+				c.beta = beta;
+				c.gamma = gamma;
+				c.eps = eps;
+				c.st = st;
+				postf[1] = postf[0];
+			}
+			else
+			{
+				PairTwist w;
+				w.P0 = P0;
+				w.alpha = alpha;
+				w.beta = beta;
+				w.gamma = gamma;
+				w.eps = eps;
+				w.st = st;
+				w.pad_ = 0;
+				a.ptwist[(int64_t)(item - a.ptwist0) * a.T + t] = w;
+				c.flags |= kPTwo;
+			}
 		}
 		// per band: fse - clock offset (mode.cpp:1053-1059, 1099-1106); the
 		// channel of an order-0 lower sideband falls with the bin
@@ -177,13 +209,13 @@ __global__ void __launch_bounds__(128) k_pair_consts(const FsArgs a, int N, int 
 		{
 			const double D = Sp->bw * (1.0 / nchan) * ((double)pq->fse - g.clk[j]);
 			split_turns(D, c.dhi[j], c.dlo[j]);
-			c.post[j] = (float)postf + g.phase[j];
+			c.post[j] = (float)postf[j] + g.phase[j];
 			if(j == 0 || g.clk[1] != g.clk[0])
 				c.os[j] = cispi2(sgn * D * (double)S8);
 			else
 				c.os[1] = c.os[0];
 		}
-		if(g.clk[1] != g.clk[0] || g.phase[1] != g.phase[0])
+		if(g.clk[1] != g.clk[0] || c.post[1] != c.post[0])
 			c.flags &= ~kPSame;
 		// validity of the window's frames, one bit per frame relative to fa
 		const uint32_t nwf = (c.so + (uint32_t)N - 1) / fs + 1, nm = nwf < 32u ? nwf : 32u;

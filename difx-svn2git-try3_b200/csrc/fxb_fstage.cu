@@ -122,6 +122,7 @@ void launch_fstage_kind(const FKind &k, FsArgs a, cudaStream_t stream)
 		return;
 	a.first = k.first;
 	a.pair0 = k.pair0;
+	a.two = k.two;
 	a.tq = k.tq;
 	a.pp = k.pp;
 	a.tw = k.tw;

@@ -21,9 +21,16 @@
 // An FFT of up to 256 points lies within a warp and exchanges without CTA
 // barriers, one of 512 or 1024 points synchronises its own threads only.
 //
-// Bound: instruction issue (FFT arithmetic about half of it).  Thread
-// instructions per sample of a band and launch times before and after are
-// with the kernels in fxb_fs_pair_tc.cu.
+// Subbands of one polarisation pair up two by two, if they agree in sideband and
+// spectra and carry no corrections of their own: the fringe rotations then differ
+// too (kPTwo) and cost one packed product more per sample pair, against a whole
+// second pass over the FFT.
+//
+// Bound: shared-memory data pipe (about 70 % busy) and instruction issue.  Launch
+// times in us, one band a unit and now: 10 stations x 16 bands x 250 FFTs of 2048
+// points FP32 342 and 239; 20 x 2 x 8192 points x 128 FFTs of 8 bits 290 and 220;
+// 20 x 8 x 256 points x 4096 709 and 434; the first in FP16 from raw multi-thread
+// reads 523 and 304; 7 x 16 bands of one polarisation x 128 points x 2005 154 and 71.
 #pragma once
 
 #include "fxb_fstage.cuh"
@@ -226,9 +233,9 @@ __device__ __forceinline__ void pair_mids(ulonglong2 *side, int slot, int b, con
 // FFTs from t0 on, both in shared memory.
 // VAR 1: raw INTERLACEDVDIF reads; VAR 2: complex sampling.
 template <int LOGN, bool TCO, int VAR>
-__device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem &I, const PairConst *fcs, const int t0,
-                                                 const int nit, const float2 *tw, ulonglong2 *fsm, const float *lut8,
-                                                 const u64 *lut4)
+__device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem &I, const PairConst *fcs,
+                                                 const PairTwist *tws, const int t0, const int nit, const float2 *tw,
+                                                 ulonglong2 *fsm, const float *lut8, const u64 *lut4)
 {
 	using SH = PShape<LOGN>;
 	constexpr int N = SH::N, TPF = SH::TPF, FPC = SH::FPC, PADN = SH::PADN, RL = SH::RL;
@@ -395,40 +402,70 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 		// w_N^(r b))
 		cp x[8];
 		{
-			float rc = 1.0f, rs = 0.0f;
-			if(order == 1)
-			{
-				float ph = fmaf((float)b, fc.alpha, fc.P0);
+			// rotator of sample n: order 1 the start, order 2 every sample
+			auto start = [&](float P0, float alpha, float &rc, float &rs) {
+				float ph = fmaf((float)b, alpha, P0);
 				ph -= rintf(ph);
 				__sincosf(-6.283185307179586f * ph, &rs, &rc);
-			}
-			const float2 st = fc.st;
-#pragma unroll
-			for(int r = 0; r < 8; r++)
-			{
-				if(order == 2)
-				{
-					const int n = b + r * (int)S8, asl = I.asl;
-					const int kk = n / asl, jj = n - kk * asl;
-					float ph = fc.P0 + (float)jj * fc.alpha + (float)(kk * jj) * fc.beta + (float)kk * fc.gamma +
-					           (float)(kk * kk) * fc.eps;
-					ph -= rintf(ph);
-					__sincosf(-6.283185307179586f * ph, &rs, &rc);
-				}
+			};
+			auto quadr = [&](int n, float P0, float alpha, float beta, float gamma, float eps, float &rc, float &rs) {
+				const int asl = I.asl, kk = n / asl, jj = n - kk * asl;
+				float ph = P0 + (float)jj * alpha + (float)(kk * jj) * beta + (float)kk * gamma + (float)(kk * kk) * eps;
+				ph -= rintf(ph);
+				__sincosf(-6.283185307179586f * ph, &rs, &rc);
+			};
+			auto value = [&](int r, float rc, float rs, float rcb, float rsb) {
 				const float2 v = up2(lv[r]);
 				if constexpr(CPLX)
 				{
 					const float2 u = up2(lu[r]);
-					x[r].re = pk2(fmaf(v.x, rc, -__fmul_rn(u.x, rs)), fmaf(v.y, rc, -__fmul_rn(u.y, rs)));
-					x[r].im = pk2(fmaf(v.x, rs, __fmul_rn(u.x, rc)), fmaf(v.y, rs, __fmul_rn(u.y, rc)));
+					x[r].re = pk2(fmaf(v.x, rc, -__fmul_rn(u.x, rs)), fmaf(v.y, rcb, -__fmul_rn(u.y, rsb)));
+					x[r].im = pk2(fmaf(v.x, rs, __fmul_rn(u.x, rc)), fmaf(v.y, rsb, __fmul_rn(u.y, rcb)));
 				}
 				else
 				{
-					x[r].re = pk2(__fmul_rn(v.x, rc), __fmul_rn(v.y, rc));
-					x[r].im = pk2(__fmul_rn(v.x, rs), __fmul_rn(v.y, rs));
+					x[r].re = pk2(__fmul_rn(v.x, rc), __fmul_rn(v.y, rcb));
+					x[r].im = pk2(__fmul_rn(v.x, rs), __fmul_rn(v.y, rsb));
 				}
-				if(order == 1 && r < 7)
-					rot1(rc, rs, st.x, st.y);
+			};
+			float rc = 1.0f, rs = 0.0f;
+			const float2 st = fc.st;
+			if(order == 1)
+				start(fc.P0, fc.alpha, rc, rs);
+			if(!(flags & kPTwo))
+			{
+#pragma unroll
+				for(int r = 0; r < 8; r++)
+				{
+					if(order == 2)
+						quadr(b + r * (int)S8, fc.P0, fc.alpha, fc.beta, fc.gamma, fc.eps, rc, rs);
+					value(r, rc, rs, rc, rs);
+					if(order == 1 && r < 7)
+						rot1(rc, rs, st.x, st.y);
+				}
+			}
+			else
+			{
+				float rcb = 1.0f, rsb = 0.0f;
+				const PairTwist &ft = tws[it * FPC + slot];
+				const float2 stb = ft.st;
+				if(order == 1)
+					start(ft.P0, ft.alpha, rcb, rsb);
+#pragma unroll
+				for(int r = 0; r < 8; r++)
+				{
+					if(order == 2)
+					{
+						quadr(b + r * (int)S8, fc.P0, fc.alpha, fc.beta, fc.gamma, fc.eps, rc, rs);
+						quadr(b + r * (int)S8, ft.P0, ft.alpha, ft.beta, ft.gamma, ft.eps, rcb, rsb);
+					}
+					value(r, rc, rs, rcb, rsb);
+					if(order == 1 && r < 7)
+					{
+						rot1(rc, rs, st.x, st.y);
+						rot1(rcb, rsb, stb.x, stb.y);
+					}
+				}
 			}
 		}
 		dft8(x);
@@ -452,7 +489,7 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 		const bool same = (flags & kPSame) != 0;
 		const int oflags = I.oflags;
 		const bool h16 = (oflags & kOH16) != 0;
-		const int rowd = I.rowd;
+		const int64_t rowd = I.rowd;
 		const int64_t base = I.first + (int64_t)t * I.tstride;
 		auto put = [&](int c, const cp &y) {
 			const float2 re = up2(y.re), im = up2(y.im);
@@ -645,8 +682,12 @@ __device__ __forceinline__ void pair_cp_wait() { asm volatile("cp.async.wait_all
 
 // a unit's item and constants into shared memory (pair_cp_wait and a barrier
 // before they are read)
-__device__ __forceinline__ void pair_fetch(PairItem *I, PairConst *fcs, const void *item, const void *consts, int nfc)
+__device__ __forceinline__ void pair_fetch(PairItem *I, PairConst *fcs, PairTwist *tws, const void *item,
+                                           const void *consts, const void *twists, int nfc)
 {
+	if(twists)
+		for(int i = threadIdx.x; i < nfc * (int)(sizeof(PairTwist) / 16); i += blockDim.x)
+			pair_cp16((char *)tws + 16 * i, (const char *)twists + 16 * i);
 	for(int i = threadIdx.x; i < nfc * (int)(sizeof(PairConst) / 16); i += blockDim.x)
 		pair_cp16((char *)fcs + 16 * i, (const char *)consts + 16 * i);
 	if(threadIdx.x < sizeof(PairItem) / 16)
@@ -662,6 +703,7 @@ struct PairFeed {
 	FsMultiUnit rec[3];
 	PairItem item[2];
 	PairConst fcs[2][NFC];
+	PairTwist tws[2][NFC];
 };
 
 template <int NFC, class F>
@@ -678,7 +720,7 @@ __device__ __forceinline__ void pair_units(PairFeed<NFC> &s, const FsMultiArgs &
 	auto consts = [&](int k, int u) {
 		const FsMultiUnit &r = s.rec[k % 3];
 		if(u < n)
-			pair_fetch(&s.item[k & 1], s.fcs[k & 1], r.pitem, r.consts, r.nfc);
+			pair_fetch(&s.item[k & 1], s.fcs[k & 1], s.tws[k & 1], r.pitem, r.consts, r.twists, r.nfc);
 	};
 	int u = blockIdx.x;
 	record(0, u);
@@ -692,7 +734,7 @@ __device__ __forceinline__ void pair_units(PairFeed<NFC> &s, const FsMultiArgs &
 		__syncthreads();
 		consts(k + 1, u + step);
 		record(k + 2, u + 2 * step);
-		run(s.rec[k % 3], s.item[k & 1], s.fcs[k & 1]);
+		run(s.rec[k % 3], s.item[k & 1], s.fcs[k & 1], s.tws[k & 1]);
 	}
 }
 

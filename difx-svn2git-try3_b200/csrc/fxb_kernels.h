@@ -110,7 +110,10 @@ struct FGroup {
 	double looff;
 	float phase[2];
 	int32_t corr;            // any correction nonzero
-	int32_t pad_;
+	// two bands of different subbands (equal sideband and spectra shape, no
+	// corrections): the second band's subband; else freq and lofreq again
+	int32_t freq1;
+	double lofreq1;
 };
 
 #if defined(__CUDACC__)
@@ -160,7 +163,7 @@ struct FKind {
 	int32_t tcbpt;           // tensor-core FFT: bits per time of the stations' VDIF words
 	int32_t muxraw;          // 1: the items' stations hand over raw INTERLACEDVDIF reads
 	int32_t cplx;            // 1: the items' stations sample complex (N = nchan points)
-	int32_t pair0;           // two-band kinds: first PairItem
+	int32_t pair0, two;      // two-band kinds: first PairItem; the bands are of different subbands
 	int32_t persist;         // 1: run by the persistent launches (launch_fstage_multi), not launch_fstage_kind
 };
 
@@ -186,12 +189,19 @@ struct alignas(16) PairConst {
 	int32_t stuck;                       // samples [stuck, N) read as zero
 	int32_t mi00, mi01, mi10, mi11;      // raw reads: thread frames of the window's first and second frame, per band
 };
+// kPTwo: the second band's fringe rotation, in an array of its own
+struct alignas(16) PairTwist {
+	float P0, alpha, beta, gamma;
+	float eps;
+	float2 st;
+	int32_t pad_;
+};
 // What does not change from subint to subint: the samples' place in the frames
 // and the spectra's place.  FP32 form [t][row][chan]; tensor-core form blocked
 // [t][block][trow][tcb] in the order of chan_pos.
 struct alignas(16) PairItem {
 	int64_t first, tstride;              // the first band's value of time 0, channel (position) 0; a time
-	int32_t rowd;                        // from the first band's values to the second's
+	int64_t rowd;                        // from the first band's values to the second's
 	uint32_t tcb, magic, bextra;         // channels of a block; p / tcb = umulhi(p, magic) for p < 2^16;
 	                                     // position p sits at p + p / tcb x bextra
 	int32_t pbits, oflags;
@@ -199,7 +209,7 @@ struct alignas(16) PairItem {
 	uint32_t hbits;                      // header bits
 	int32_t nbits, header, framebytes, minfb, mnthr;
 	int32_t station, band0, band1, lsb, asl, adj;   // adj: both bands side by side in one aligned field
-	int32_t group, pad_[3];
+	int32_t group, two;                  // two: the bands' LOs differ
 };
 enum : int32_t { kORow0 = 1, kORow1 = 2, kOH16 = 4, kOQuad = 8, kOBoth = 16 };
 enum : int32_t {
@@ -207,6 +217,7 @@ enum : int32_t {
 	kPNarrow = 2,     // fmask covers the window
 	kPBlank = 4,      // a valid frame of the window blanks one of the item's bands
 	kPSame = 8,       // the two bands take the same output rotation
+	kPTwo = 32,       // the bands take different fringe rotations
 	kPFast = 16       // every sample of the window counts and the fast read applies
 };
 
@@ -229,6 +240,8 @@ struct FsArgs {
 	int32_t pair0;           // set from FKind::pair0 by launch_fstage_kind
 	const PairItem *pitems;  // two-band items, and the constants of their FFTs [item][T]
 	PairConst *pconst;
+	PairTwist *ptwist;       // of the two-band items from ptwist0 on, [item - ptwist0][T]
+	int32_t ptwist0, two;    // two: the launch's items have twists (set by launch_fstage_kind)
 };
 // constants of the subint's FFTs of a two-band kind's items
 void launch_pair_consts(const FKind &k, const FsArgs &a, cudaStream_t stream);
@@ -266,6 +279,7 @@ struct alignas(16) FsMultiUnit {
 	int32_t t0, nfc, pad_;               // two-band units: first FFT, FFTs
 	const PairItem *pitem;
 	const PairConst *consts;             // of FFT t0
+	const PairTwist *twists;             // of FFT t0, or null
 };
 struct FsMultiArgs {
 	FsArgs m[kFsMultiMembers];           // per context, with its subint's staging

@@ -82,3 +82,34 @@ def test_bands_with_their_own_rotations(nchan):
         ref, _, _ = orc.mode_fft(s, buf, dsec, dns, sec, ns, 3)
         for p in range(2):
             assert rel_err(spec[3, 2 * s + p], ref[2 + p]) < TOL["fp32"], (s, p)
+
+
+@pytest.mark.parametrize("xmac", ["fp32", "fp16"])
+@pytest.mark.parametrize("nchan,nfreq,kw", [(16, 2, dict()), (128, 4, dict(fringe_rot_order=2)), (256, 1, dict()),
+                                            (512, 2, dict(sideband="L")), (1024, 4, dict(sideband="L", nbits=8)),
+                                            (1024, 2, dict(fringe_rot_order=0)), (2048, 2, dict(nbits=8)),
+                                            (4096, 4, dict(sideband="L", fringe_rot_order=0))])
+def test_single_bands_of_two_subbands(nchan, nfreq, kw, xmac):
+    """Stations of one polarisation: two subbands of equal sideband make one item,
+    whose bands have fringe rotations of their own (a subband alone and mixed
+    sidebands stay single)."""
+    from fxb200.job import Freq, full_job
+    kw = dict(kw)
+    side = kw.pop("sideband", "U")
+    freqs = [Freq(8400.25 + 16 * k, 16.0, nchan, "U" if k == 3 and nchan == 128 else side) for k in range(nfreq)]
+    job = full_job(2, freqs, pols="R", full_pol=False, subint_ns=3 * nchan * 1000 // 16, **kw)
+    synth.make_delay_polys(job, seed=4)
+    job.validate()
+    sec, ns = 0, 4_000_000
+    inputs = synth.subint_inputs(job, sec, ns, rho=0.05, seed=7)
+    corr = Correlator(job, xmac=xmac)
+    corr.submit(inputs, sec, ns)
+    spec = [corr.spectra(f) for f in range(nfreq)]
+    corr.close()
+    orc = fxoracle.OracleCorrelator(job)
+    for s in range(2):
+        buf, dsec, dns = inputs[s]
+        for t in range(3):
+            ref, _, _ = orc.mode_fft(s, buf, dsec, dns, sec, ns, t)
+            for f in range(nfreq):
+                assert rel_err(spec[f][t, s], ref[f]) < TOL[xmac], (s, t, f)
