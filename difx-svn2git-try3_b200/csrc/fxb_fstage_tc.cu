@@ -30,10 +30,11 @@
 //               through a shared-memory ring and stages each unit's VDIF
 //               window into shared memory (bulk copies of the valid frames),
 //   warps 0-7   decode: 8 consecutive times -> the fringe-rotated FP16
-//               samples of the unit's four channels (two-time lookup of
-//               both polarisations, FP32 rotation),
-//   warps 8-11  twiddle: D1 (tensor memory, 32 columns at a time) -> Z (FP16
-//               operand, in the operand buffer MMA 1 has finished with),
+//               samples of the unit's four channels (lookup of both
+//               polarisations, FP32 rotation),
+//   warps 8-11  twiddle: D1 (tensor memory, 16 columns of both subbands at a
+//               time) -> Z (FP16 operand, in the operand buffer MMA 1 has
+//               finished with),
 //   warps 12-15 output: D2 (32 columns at a time) -> fractional-sample
 //               rotation -> FP16 (or BF16) spectra,
 //   warp 16     MMA issuer (one thread).
@@ -42,6 +43,13 @@
 // Every wait is bounded; a timeout sets the error flag, the CTA stops,
 // waits (bounded) for its copies and MMAs in flight and frees its tensor
 // memory.
+//
+// Bound: the shared-memory data pipe (lookups, operand stores, twiddle loads; 81 %
+// busy before the last step below), with the decode and twiddle warps the longest
+// roles; the tensor cores idle.  10 stations x 16 bands x 250 FFTs a launch: 173 us
+// with the unit records formed by the producer warp, 148 us with k_tc_units ahead of
+// it, 133 us with the conflict-free lookup and the twiddles loaded once for both
+// subbands; 32 stations x 8 bands x 250 FFTs: 348, 337, 309 us.
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -195,6 +203,20 @@ __device__ __forceinline__ void tld32(uint32_t taddr, float *v)
 		v[i] = __uint_as_float(r[i]);
 }
 
+__device__ __forceinline__ void tld16(uint32_t taddr, float *v)
+{
+	uint32_t r[16];
+	asm volatile(
+	    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+	    "%15}, [%16];\n"
+	    : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+	      "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+	    : "r"(taddr));
+#pragma unroll
+	for(int i = 0; i < 16; i++)
+		v[i] = __uint_as_float(r[i]);
+}
+
 __device__ __forceinline__ void tld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
 __device__ __forceinline__ uint32_t pack_h2(float a, float b)
@@ -297,7 +319,7 @@ struct TcLayout {
 	static constexpr int kStgBytes = kN * BPT / 8 + 64;   // one window, 16-byte slack either side
 	static constexpr int kOffStg = kOffOp + kNS * kOpBytes;
 	static constexpr int kOffLut = kOffStg + kNStg * kStgBytes;
-	static constexpr int kOffTw = kOffLut + 256 * 16;     // twiddles w_2048^(n2 k1) of two k1, float4 [k1 / 2][n2]
+	static constexpr int kOffTw = kOffLut + 16 * 8;       // twiddles w_2048^(n2 k1) of two k1, float4 [k1 / 2][n2]
 	static constexpr int kOffRing = kOffTw + kN1 * kN2 * 8;
 	static constexpr int kUsed = kOffRing + kRing * (int)sizeof(UnitRec);
 	static constexpr size_t kSmem = 1024 + (size_t)kUsed;
@@ -432,7 +454,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 	unsigned char *base = (unsigned char *)(((uintptr_t)fsm_tc + 1023) & ~(uintptr_t)1023);
 	unsigned char *ops = base + kOffOp;
 	unsigned char *stg = base + LY::kOffStg;
-	float4 *lut = (float4 *)(base + LY::kOffLut);
+	float2 *lut = (float2 *)(base + LY::kOffLut);
 	float4 *twt = (float4 *)(base + LY::kOffTw);
 	UnitRec *ring = (UnitRec *)(base + LY::kOffRing);
 	const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -442,10 +464,11 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 
 	for(int i = tid; i < kTablesBytes / 16; i += blockDim.x)
 		((uint4 *)base)[i] = __ldg(tables + i);
-	// two times of both polarisations of one subband: index = nibble(t) |
-	// nibble(t + 1) << 4, nibble = code(p0) | code(p1) << 2 (format_vdif.c:78)
-	for(int i = tid; i < 256; i += blockDim.x)
-		lut[i] = make_float4(level2f(i & 3u), level2f((i >> 4) & 3u), level2f((i >> 2) & 3u), level2f((i >> 6) & 3u));
+	// both polarisations of one subband at one time: nibble = code(p0) | code(p1) <<
+	// 2 (format_vdif.c:78).  16 entries of 8 bytes lie in 32 banks, free of conflicts;
+	// a table of two times (256 entries of 16 bytes) took 10 wavefronts a load
+	if(tid < 16)
+		lut[tid] = make_float2(level2f(tid & 3u), level2f(tid >> 2u));
 	for(int i = tid; i < kN1 / 2 * kN2; i += blockDim.x)
 	{
 		const int k1 = 2 * (i / kN2), n2 = i % kN2;
@@ -696,21 +719,20 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 							wb = hi ? w[2 * j + 3] : w[2 * j + 2];
 							sa = sb2 = nsh & 31;
 						}
-						const uint32_t idx = ((wa >> sa) & 15u) | (((wb >> sb2) & 15u) << 4);
-						float4 l = lut[idx];
+						float2 la = lut[(wa >> sa) & 15u], lb = lut[(wb >> sb2) & 15u];
 						if(vms != 0xFFu)
 						{
 							const bool v0 = (vms >> j) & 1u, v1 = (vms >> (j + 1)) & 1u;
-							l.x = v0 ? l.x : 0.0f;
-							l.y = v1 ? l.y : 0.0f;
-							l.z = v0 ? l.z : 0.0f;
-							l.w = v1 ? l.w : 0.0f;
+							la.x = v0 ? la.x : 0.0f;
+							la.y = v0 ? la.y : 0.0f;
+							lb.x = v1 ? lb.x : 0.0f;
+							lb.y = v1 ? lb.y : 0.0f;
 						}
-						const u64 d0 = pk2(l.x, l.y), d1 = pk2(l.z, l.w);
-						re0[j >> 1] = pack_h2(mul2(d0, rr));
-						im0[j >> 1] = pack_h2(mul2(d0, ri));
-						re1[j >> 1] = pack_h2(mul2(d1, rr));
-						im1[j >> 1] = pack_h2(mul2(d1, ri));
+						const float2 r2 = up2(rr), i2 = up2(ri);
+						re0[j >> 1] = pack_h2(la.x * r2.x, lb.x * r2.y);
+						im0[j >> 1] = pack_h2(la.x * i2.x, lb.x * i2.y);
+						re1[j >> 1] = pack_h2(la.y * r2.x, lb.y * r2.y);
+						im1[j >> 1] = pack_h2(la.y * i2.x, lb.y * i2.y);
 						if(j < 6)
 						{
 							u64 nr, ni;
@@ -758,31 +780,37 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 #pragma unroll 1
 			for(int h = 0; h < 4; h++)
 			{
-				// subband sb, channels k1 in [16 hh, 16 hh + 16): 32 columns
-				const int sb = h >> 1, hh = h & 1;
-				float v[32];
-				tld32(tmem + lane_base + (uint32_t)(256 * b + 64 * sb + 32 * hh), v);
+				// k1 in [8 h, 8 h + 8) of both subbands: 16 columns each, one load of their
+				// common twiddles
+				float v[2][16];
+				tld16(tmem + lane_base + (uint32_t)(256 * b + 16 * h), v[0]);
+				tld16(tmem + lane_base + (uint32_t)(256 * b + 64 + 16 * h), v[1]);
 				tld_wait();
 				// Z[k1][n2] = Y[k1][n2] w^(n2 k1); A2 row m = ch 32 + k1 with ch = 2 sb + p,
 				// K = part 64 + n2
-				const int m0 = (2 * sb + p) * 32 + 16 * hh;
-				uint32_t zr[8], zi[8];
+				uint32_t zr[2][4], zi[2][4];
 #pragma unroll
-				for(int q = 0; q < 16; q += 2)
+				for(int q = 0; q < 8; q += 2)
 				{
 					// columns: real parts of k1 and k1 + 1, then their imaginary parts
-					const float4 w = tw[(8 * hh + (q >> 1)) * kN2];
-					u64 zrp, zip;
-					cmul2(pk2(v[2 * q], v[2 * q + 1]), pk2(v[2 * q + 2], v[2 * q + 3]), pk2(w.x, w.y), pk2(w.z, w.w), zrp, zip);
-					zr[q >> 1] = pack_h2(zrp);
-					zi[q >> 1] = pack_h2(zip);
+					const float4 w = tw[(4 * h + (q >> 1)) * kN2];
+					const u64 wr = pk2(w.x, w.y), wi = pk2(w.z, w.w);
+#pragma unroll
+					for(int sb = 0; sb < 2; sb++)
+					{
+						const float *y = v[sb] + 2 * q;
+						u64 zrp, zip;
+						cmul2(pk2(y[0], y[1]), pk2(y[2], y[3]), wr, wi, zrp, zip);
+						zr[sb][q >> 1] = pack_h2(zrp);
+						zi[sb][q >> 1] = pack_h2(zip);
+					}
 				}
 #pragma unroll
-				for(int c = 0; c < 2; c++)
+				for(int sb = 0; sb < 2; sb++)
 				{
-					*(uint4 *)(A2 + mn_off(m0 + 8 * c, n2)) = make_uint4(zr[4 * c], zr[4 * c + 1], zr[4 * c + 2], zr[4 * c + 3]);
-					*(uint4 *)(A2 + mn_off(m0 + 8 * c, 64 + n2)) =
-					    make_uint4(zi[4 * c], zi[4 * c + 1], zi[4 * c + 2], zi[4 * c + 3]);
+					const int m0 = (2 * sb + p) * 32 + 8 * h;
+					*(uint4 *)(A2 + mn_off(m0, n2)) = make_uint4(zr[sb][0], zr[sb][1], zr[sb][2], zr[sb][3]);
+					*(uint4 *)(A2 + mn_off(m0, 64 + n2)) = make_uint4(zi[sb][0], zi[sb][1], zi[sb][2], zi[sb][3]);
 				}
 			}
 			asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
