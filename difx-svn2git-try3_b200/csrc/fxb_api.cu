@@ -101,11 +101,11 @@ struct fxb_ctx {
 	DevPcalGroup *d_pgroups = nullptr;
 	DevPcalBand *d_pbands = nullptr;
 	int npbands = 0;
-	int pchunks = 1;                     // chunks of FFTs, each with its own slice of the bins
+	PcalPlan pplan{1, 1, 1};             // FFT windows in chunks, each with its own slice of the bins
 	struct PcalClass { int first, count, nbits, bpt, shift, maxbins; size_t smem; };
 	std::vector<PcalClass> pclass;       // runs of groups of one sample layout: one launch each
 	size_t psmem = 0;
-	double *d_pbins = nullptr;           // [pchunks][job.pcal_bins]
+	double *d_pbins = nullptr;           // [pplan.chunks][job.pcal_bins]
 	float2 *d_core = nullptr;
 	uint8_t *d_valid = nullptr;          // frame validity [S][valid_stride], then the band masks
 	uint32_t *d_bandok = nullptr;        // [S][valid_stride] in the same allocation
@@ -360,20 +360,16 @@ static std::vector<DevPcalGroup> pcal_groups(const Job &job)
 	return out;
 }
 
-// Chunks of FFTs per subint for the phase-cal binning: about four CTAs per
-// SM, at most one FFT per chunk, and at most 64 MB of bins.
-static int pcal_chunks(const Job &job, const std::vector<DevPcalGroup> &groups)
+static PcalPlan pcal_plan_of(const Job &job, const std::vector<DevPcalGroup> &groups)
 {
-	int64_t ctas = 0;                     // CTAs of one chunk: blocks of 256 bins per group
+	int minfft = INT32_MAX;
 	for(const DevPcalGroup &g : groups)
-		ctas += (g.nbins + 255) / 256;
-	if(ctas == 0 || job.pcal_bins <= 0)
-		return 1;
-	int n = (int)((600 + ctas - 1) / ctas);
-	n = std::min(n, std::max(job.blockspersend, 1));
-	const int64_t cap = (int64_t)(64 << 20) / (8 * job.pcal_bins);
-	n = (int)std::min<int64_t>(n, std::max<int64_t>(cap, 1));
-	return std::max(n, 1);
+	{
+		const Job::Station &js = job.stations[g.station];
+		const int nchan = job.freqs[js.band_freq[0]].nchan;
+		minfft = std::min(minfft, js.cplx ? nchan : 2 * nchan);
+	}
+	return pcal_plan(groups.data(), (int)groups.size(), job.pcal_bins, job.blockspersend, minfft);
 }
 
 // The unchanging part of a two-band work item (k_pair_consts has the rest).
@@ -1010,19 +1006,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 			};
 			std::stable_sort(ctx->h_pgroups.begin(), ctx->h_pgroups.end(),
 			                 [&](const DevPcalGroup &x, const DevPcalGroup &y) { return class_of(x) < class_of(y); });
-			ctx->pchunks = pcal_chunks(job, ctx->h_pgroups);
-			// chunks of a multiple of four FFTs, so that the 2 or 4 lanes of a
-			// bin (bin counts of 128 or 64) share a chunk evenly
-			int tpc = (ctx->T + ctx->pchunks - 1) / ctx->pchunks;
-			tpc = std::min(ctx->T, (tpc + 3) / 4 * 4);
-			// and short enough that the chunk's FFT table and the lane sums fit
-			// one CTA's shared memory
-			size_t lanes = 0;
-			for(const DevPcalGroup &g : ctx->h_pgroups)
-				lanes = std::max(lanes, pcal_group_smem(g));
-			while(tpc > 4 && pcal_smem(lanes, tpc) > kPcalSmemLaunchMax)
-				tpc = (tpc / 2 + 3) / 4 * 4;
-			ctx->pchunks = (ctx->T + tpc - 1) / tpc;
+			ctx->pplan = pcal_plan_of(job, ctx->h_pgroups);
 			for(size_t i = 0; i < ctx->h_pgroups.size(); i++)
 			{
 				const DevPcalGroup &g = ctx->h_pgroups[i];
@@ -1033,7 +1017,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 				fxb_ctx::PcalClass &pc = ctx->pclass.back();
 				pc.count++;
 				pc.maxbins = std::max(pc.maxbins, g.nbins);
-				pc.smem = std::max(pc.smem, pcal_smem(pcal_group_smem(g), tpc));
+				pc.smem = std::max(pc.smem, pcal_smem(pcal_group_smem(g), ctx->pplan.tpc));
 				ctx->psmem = std::max(ctx->psmem, pc.smem);
 			}
 			ctx->npbands = (int)hb.size();
@@ -1047,7 +1031,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 				if(!ctx->h_pgroups.empty())
 					CK(ctx, cudaMemcpyAsync(ctx->d_pgroups, ctx->h_pgroups.data(), sizeof(DevPcalGroup) * ctx->h_pgroups.size(),
 					                        cudaMemcpyHostToDevice, ctx->stream));
-				const size_t nbins = (size_t)ctx->pchunks * (size_t)std::max<int64_t>(job.pcal_bins, 1);
+				const size_t nbins = (size_t)ctx->pplan.chunks * (size_t)std::max<int64_t>(job.pcal_bins, 1);
 				CK(ctx, dalloc(ctx, &ctx->d_pbins, nbins));
 				CK(ctx, cudaMemsetAsync(ctx->d_pbins, 0, sizeof(double) * nbins, ctx->stream));
 			}
@@ -1492,7 +1476,7 @@ static void launch_xmac_weights(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, u
 	Tuner &tn = ctx->tune;
 	const size_t nk = ctx->fkinds.size();
 	for(const auto &pc : ctx->pclass)
-		launch_pcal_bin(ctx->d_pgroups + pc.first, pc.count, pc.maxbins, ctx->pchunks, pc.nbits, pc.bpt, pc.shift != 0,
+		launch_pcal_bin(ctx->d_pgroups + pc.first, pc.count, pc.maxbins, ctx->pplan, pc.nbits, pc.bpt, pc.shift != 0,
 		                pc.smem, ctx->d_st, sl.d_sub, ctx->d_params, ctx->d_valid, ctx->valid_stride, ctx->T,
 		                job.pcal_bins, ctx->d_pbins, st);
 	launch_zoom_gather(ctx->d_zoom, ctx->nzoom, ctx->d_plans, ctx->T, ctx->tc,
@@ -1904,7 +1888,7 @@ fxb_status fxb_job_footprint(const fxb_job_desc *desc, size_t *bytes)
 	                                     : job.xmac_kind != FXB_XMAC_FP8 ? 4.0 * 1.25 * pad32
 	                                                                      : (4.0 * pad64 + 2.0 * pad64 + 0.5) * 1.25);
 	b += (double)job.acc_total * 8.0 + (double)job.corelen * 16.0 + (double)S * T * 68.0 + (double)pairs * T * 144.0 +
-	     (double)job.pcal_bins * 8.0 * pcal_chunks(job, pcal_groups(job));
+	     (double)job.pcal_bins * 8.0 * pcal_plan_of(job, pcal_groups(job)).chunks;
 	// raw VDIF staging of the in-flight subints (payload plus headers, 1/8 slack)
 	for(int s = 0; s < S; s++)
 	{
@@ -1932,7 +1916,7 @@ fxb_status fxb_read_results(fxb_ctx *ctx, float *coreresult, size_t nfloats)
 	}
 	launch_finalise(ctx->d_om, ctx->nom, ctx->d_acc, ctx->d_wout, ctx->nwout, ctx->d_wacc, ctx->d_core,
 	                ctx->job.corelen, ctx->stream);
-	launch_pcal_final(ctx->d_pbands, ctx->npbands, ctx->pchunks, ctx->job.pcal_bins, ctx->d_pbins, ctx->d_core, ctx->stream);
+	launch_pcal_final(ctx->d_pbands, ctx->npbands, ctx->pplan.chunks, ctx->job.pcal_bins, ctx->d_pbins, ctx->d_core, ctx->stream);
 	CK(ctx, cudaGetLastError());
 	CK(ctx, cudaMemcpyAsync(coreresult, ctx->d_core, sizeof(float2) * ctx->job.corelen, cudaMemcpyDeviceToHost, ctx->stream));
 	CK(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1948,7 +1932,7 @@ fxb_status fxb_reset(fxb_ctx *ctx)
 	CK(ctx, cudaMemsetAsync(ctx->d_wacc, 0, sizeof(float) * std::max(ctx->nwsum, 1), ctx->stream));
 	if(ctx->d_pbins)
 		CK(ctx, cudaMemsetAsync(ctx->d_pbins, 0,
-		                        sizeof(double) * (size_t)ctx->pchunks * (size_t)std::max<int64_t>(ctx->job.pcal_bins, 1),
+		                        sizeof(double) * (size_t)ctx->pplan.chunks * (size_t)std::max<int64_t>(ctx->job.pcal_bins, 1),
 		                        ctx->stream));
 	return FXB_OK;
 }
@@ -2103,7 +2087,7 @@ fxb_status fxb_read_results_device(fxb_ctx *ctx, float *dev_out, size_t nfloats)
 	}
 	launch_finalise(ctx->d_om, ctx->nom, ctx->d_acc, ctx->d_wout, ctx->nwout, ctx->d_wacc, (float2 *)dev_out,
 	                ctx->job.corelen, ctx->stream);
-	launch_pcal_final(ctx->d_pbands, ctx->npbands, ctx->pchunks, ctx->job.pcal_bins, ctx->d_pbins, (float2 *)dev_out,
+	launch_pcal_final(ctx->d_pbands, ctx->npbands, ctx->pplan.chunks, ctx->job.pcal_bins, ctx->d_pbins, (float2 *)dev_out,
 	                  ctx->stream);
 	CK(ctx, cudaGetLastError());
 	return FXB_OK;

@@ -405,19 +405,23 @@ struct DevPcalBand {
 	int64_t bin_off, core;
 };
 // shared memory of a group's lane sums (bin counts below the CTA width) and
-// of one launch with tpc FFTs per chunk
+// of one launch with tpc windows per chunk
 size_t pcal_group_smem(const DevPcalGroup &g);
 size_t pcal_smem(size_t group_smem, int tpc);
 constexpr size_t kPcalSmemMax = 96 * 1024;    // lane sums of one group at most
-constexpr size_t kPcalSmemLaunchMax = 200 * 1024;   // a launch's FFT table and lane sums at most
+constexpr size_t kPcalSmemLaunchMax = 200 * 1024;   // a launch's window table and lane sums at most
+// split: windows per FFT; tpc: windows per chunk; chunks: slices of the bins
+struct PcalPlan { int split, tpc, chunks; };
+// nbins: bins (doubles) of a slice; minfft: the groups' shortest FFT
+PcalPlan pcal_plan(const DevPcalGroup *groups, int ngroups, int64_t nbins, int T, int minfft);
 // allows the binning kernels smem bytes of dynamic shared memory (once per context)
 cudaError_t pcal_init(size_t smem);
-// folds the subint's samples into the FP64 bins: the FFTs are split into
-// nchunk chunks, chunk c adds to bins + c * chunk_stride.  Every group of one
+// folds the subint's samples into the FP64 bins: chunk c of the plan adds to
+// bins + c * chunk_stride.  Every group of one
 // launch belongs to stations of nbits-bit samples with bpt bits per time and
 // to one extractor (shift: the shifting extractor's complex bins); maxbins is
 // the launch's largest bin count, smem its pcal_smem.
-void launch_pcal_bin(const DevPcalGroup *groups, int ngroups, int maxbins, int nchunk, int nbits, int bpt, bool shift,
+void launch_pcal_bin(const DevPcalGroup *groups, int ngroups, int maxbins, const PcalPlan &plan, int nbits, int bpt, bool shift,
                      size_t smem, const DevStation *st, const DevSubintStation *sub, const FftParam *params,
                      const uint8_t *valid, int64_t valid_stride, int T, int64_t chunk_stride, double *bins,
                      cudaStream_t stream);

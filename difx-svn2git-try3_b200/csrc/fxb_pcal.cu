@@ -9,14 +9,21 @@
 // summed over every subint of the integration (FP64, one slice per chunk of
 // FFTs) and takes the DFT once, when the core result is read.
 //
-// k_pcal_bin: CTAs over (chunk of FFTs, block of bins, group of a station's
-// bands with the same bin count N).  Samples are decoded as the F stage
+// k_pcal_bin: CTAs over (chunk of FFT windows, block of bins, group of a station's
+// bands with the same bin count N).  Few or long FFTs are cut into split
+// windows of equal length (pcal_plan), so that every lane of a bin has one:
+// a lane that walks a whole window has hundreds of loads in series.  Samples are decoded as the F stage
 // decodes them (zero outside valid frames and past the window's blanking
 // point).  Every bin is summed in a fixed order and each CTA adds its bins,
 // without atomics, into its chunk's own slice of the FP64 bins, so that the
 // result does not depend on scheduling.
-// k_pcal_final: one CTA per band, the chunks summed in order and the DFT at
-// the tone bins, in FP64.
+// k_pcal_final: one CTA per band and tone; its threads take bins and, for bin
+// counts below the CTA width, chunks too: sum and DFT in one pass, in FP64.
+// (One CTA a band with the chunks in series: a chain of chunks x tones loads.)
+//
+// Both are bound by latency.  3 stations x 8 bands, 8 FFTs of 2048 points, 8 bins:
+// about 170 us a launch with whole windows, 7 us now; 7 stations x 16 bands, 2005
+// FFTs of 128 points, 16 bins: k_pcal_final 47 and 9 us.
 
 #include <algorithm>
 
@@ -109,40 +116,44 @@ __global__ void __launch_bounds__(kThreads) k_pcal_bin(const DevPcalGroup *__res
                                                       const DevSubintStation *__restrict__ sub,
                                                       const FftParam *__restrict__ params,
                                                       const uint8_t *__restrict__ valid, int64_t valid_stride, int T,
-                                                      int tpc, int64_t chunk_stride, double *__restrict__ bins)
+                                                      int split, int tpc, int64_t chunk_stride,
+                                                      double *__restrict__ bins)
 {
-	extern __shared__ int4 ftab[];             // per FFT of the chunk: residue of its first sample, first frame, offset, blanking;
-	                                           // then the rotator phase of its first sample (SHIFT), then lane sums
+	extern __shared__ int4 ftab[];             // per window of the chunk: residue of its first sample, first frame, offset, blanking or end
+	                                           // (first sample past it); then the rotator phase of its first sample (SHIFT), then lane sums
 	__shared__ float lut[1 << NBITS];
 	const DevPcalGroup &g = groups[blockIdx.y];
 	const int s = g.station, nb = g.nb, N = g.nbins;
 	const DevStation &S = st[s];
 	const int tid = threadIdx.x;
-	const int L = S.fftchannels;
+	// samples of a window: each FFT's, in split parts
+	const int L = (S.fftchannels + split - 1) / split, TV = T * split;
 	const uint32_t fs = (uint32_t)S.framesamples;
 	// CTAs of bins per chunk: the launch's (gridDim.x / chunks) for its
 	// largest bin count; blocks past this group's bins have nothing to do
-	const int nbb = gridDim.x / ((T + tpc - 1) / tpc);
+	const int nbb = gridDim.x / ((TV + tpc - 1) / tpc);
 	const int chunk = blockIdx.x / nbb, bb = blockIdx.x - chunk * nbb;
 	if(bb * kThreads >= N)
 		return;
-	const int t0 = chunk * tpc, t1 = min(T, t0 + tpc);
+	const int t0 = chunk * tpc, t1 = min(TV, t0 + tpc);
 	const int64_t datasamples = (int)(sub[s].datans / (S.sampletime * 1e3) + 0.5);   // Mode::setData
 	int32_t *fph = reinterpret_cast<int32_t *>(ftab + tpc);   // (offset x first sample) mod fs
 	const int64_t fsi = g.fs, off = g.shift;
 	for(int t = t0 + tid; t < t1; t += kThreads)
 	{
-		const FftParam &p = params[(int64_t)s * T + t];
+		const int f = t / split, first = (t - f * split) * L;
+		const FftParam &p = params[(int64_t)s * T + f];
 		int4 e = make_int4(-1, 0, 0, 0);
-		if(p.status == kFftOk)
+		if(p.status == kFftOk && first < S.fftchannels)
 		{
-			const uint32_t g0 = (uint32_t)p.nearest;
-			e.x = (int)((datasamples + p.nearest) % N);
+			const int64_t n0 = (int64_t)p.nearest + first;
+			const uint32_t g0 = (uint32_t)n0;
+			e.x = (int)((datasamples + n0) % N);
 			e.y = (int)(g0 / fs);
 			e.z = (int)(g0 - (uint32_t)e.y * fs);
-			e.w = p.stuck;
+			e.w = min(p.stuck, S.fftchannels) - first;
 			if(SHIFT)
-				fph[t - t0] = (int32_t)((off * ((datasamples + p.nearest) % fsi)) % fsi);
+				fph[t - t0] = (int32_t)((off * ((datasamples + n0) % fsi)) % fsi);
 		}
 		ftab[t - t0] = e;
 	}
@@ -298,18 +309,23 @@ __global__ void __launch_bounds__(kThreads) k_pcal_final(const DevPcalBand *__re
 	__shared__ double red[2][kThreads / 32];
 	const DevPcalBand b = bands[blockIdx.x];
 	const int N = b.nbins;
-	for(int k = 0; k < b.ntones; k++)
+	// chunk lanes of a bin
+	const int C = N > 0 ? max(1, kThreads / N) : 1;
+	const int c0 = N > 0 && N < kThreads ? threadIdx.x / N : 0;
+	const int m0 = N > 0 && N < kThreads ? threadIdx.x - c0 * N : threadIdx.x;
+	for(int k = blockIdx.y; k < b.ntones; k += gridDim.y)
 	{
 		const int64_t idx = (int64_t)b.first + (int64_t)k * b.step;
 		double re = 0.0, im = 0.0;
-		if(N > 0 && idx < N)
-			for(int m = threadIdx.x; m < N; m += kThreads)
+		if(N > 0 && idx < N && c0 < C)
+			for(int m = m0; m < N; m += kThreads)
 			{
 				// X[idx] = sum_m Z[m] exp(-2 pi i idx m / N), the angle reduced exactly
 				double sn, cs;
 				sincospi(-2.0 * (double)((idx * m) % N) / (double)N, &sn, &cs);
 				double z = 0.0, zi = 0.0;
-				for(int c = 0; c < nchunk; c++)          // the chunks' bins, in chunk order
+#pragma unroll 4
+				for(int c = c0; c < nchunk; c += C)      // the lane's chunks, in order
 				{
 					if(b.shift)
 					{
@@ -356,9 +372,45 @@ size_t pcal_group_smem(const DevPcalGroup &g)
 	return g.nbins < kThreads ? (size_t)g.nb * g.nbins * (kThreads / g.nbins) * sizeof(float) * (g.shift ? 2 : 1) : 0;
 }
 
+// Chunks: about four CTAs per SM and at most 64 MB of bins.  Windows: whole FFTs
+// when every lane of every chunk gets one (the cut costs table entries), else each
+// FFT in parts of at least four samples a bin, so that each lane has a part.
+PcalPlan pcal_plan(const DevPcalGroup *groups, int ngroups, int64_t nbins, int T, int minfft)
+{
+	PcalPlan p{1, 1, std::max(T, 1)};
+	int64_t ctas = 0;                     // CTAs of one chunk: blocks of kThreads bins per group
+	int lanes = 1, maxbins = 1;
+	size_t smem = 0;
+	for(int i = 0; i < ngroups; i++)
+	{
+		const DevPcalGroup &g = groups[i];
+		ctas += (g.nbins + kThreads - 1) / kThreads;
+		lanes = std::max(lanes, kThreads / g.nbins);
+		maxbins = std::max(maxbins, g.nbins);
+		smem = std::max(smem, pcal_group_smem(g));
+	}
+	if(ctas == 0 || nbins <= 0 || T < 1)
+		return p;
+	int64_t n = (600 + ctas - 1) / ctas;
+	n = std::min<int64_t>(n, std::max<int64_t>((int64_t)(64 << 20) / (8 * nbins), 1));
+	p.split = (int)std::max<int64_t>(1, std::min<int64_t>((n * lanes + T - 1) / T, minfft / (4 * maxbins)));
+	const int TV = T * p.split;
+	n = std::min<int64_t>(n, TV);
+	// a multiple of the lanes (at least four), so that they share a chunk evenly
+	const int unit = std::max(lanes, 4);
+	p.tpc = (int)((TV + n - 1) / n);
+	p.tpc = std::min(TV, (p.tpc + unit - 1) / unit * unit);
+	// and short enough that the chunk's table and the lane sums fit one CTA's
+	// shared memory
+	while(p.tpc > 4 && pcal_smem(smem, p.tpc) > kPcalSmemLaunchMax)
+		p.tpc = (p.tpc / 2 + 3) / 4 * 4;
+	p.chunks = (TV + p.tpc - 1) / p.tpc;
+	return p;
+}
+
 size_t pcal_smem(size_t group_smem, int tpc) { return (sizeof(int4) + sizeof(int32_t)) * (size_t)tpc + group_smem; }
 
-void launch_pcal_bin(const DevPcalGroup *groups, int ngroups, int maxbins, int nchunk, int nbits, int bpt, bool shift,
+void launch_pcal_bin(const DevPcalGroup *groups, int ngroups, int maxbins, const PcalPlan &plan, int nbits, int bpt, bool shift,
                      size_t smem, const DevStation *st, const DevSubintStation *sub, const FftParam *params,
                      const uint8_t *valid, int64_t valid_stride, int T, int64_t chunk_stride, double *bins,
                      cudaStream_t stream)
@@ -366,11 +418,10 @@ void launch_pcal_bin(const DevPcalGroup *groups, int ngroups, int maxbins, int n
 	if(ngroups <= 0)
 		return;
 	const bool swar = nbits == 2 && bpt == 32 && !shift, one = bpt <= 32;
-	const int tpc = (T + nchunk - 1) / nchunk;
 	const int nbb = (maxbins + kThreads - 1) / kThreads;
-	const dim3 grid(nbb * ((T + tpc - 1) / tpc), ngroups);
+	const dim3 grid(nbb * plan.chunks, ngroups);
 #define FXB_BIN(B, O, W, S) k_pcal_bin<B, O, W, S><<<grid, kThreads, smem, stream>>>(groups, st, sub, params, valid, \
-	                                                                            valid_stride, T, tpc, chunk_stride, bins)
+	                                                                            valid_stride, T, plan.split, plan.tpc, chunk_stride, bins)
 	if(swar) FXB_BIN(2, true, true, false);
 	else if(!shift && nbits == 2 && one) FXB_BIN(2, true, false, false);
 	else if(!shift && nbits == 2) FXB_BIN(2, false, false, false);
@@ -403,7 +454,7 @@ void launch_pcal_final(const DevPcalBand *bands, int nbands, int nchunk, int64_t
                        float2 *core, cudaStream_t stream)
 {
 	if(nbands > 0)
-		k_pcal_final<<<nbands, kThreads, 0, stream>>>(bands, nchunk, chunk_stride, bins, core);
+		k_pcal_final<<<dim3(nbands, 16), kThreads, 0, stream>>>(bands, nchunk, chunk_stride, bins, core);
 }
 
 }  // namespace fxb

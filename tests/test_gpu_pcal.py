@@ -83,3 +83,21 @@ def test_pcal_long_subint_fine_bins():
     got, ref, layout, n = _run(job, subints=[(0, 0)])
     errs = compare_core(job, layout, n, got, ref)
     assert "pcal" in errs
+
+
+@pytest.mark.parametrize("kw", [
+    dict(nchan=2048, subint_ns=512_000, freq0=8400.1),                              # 320 bins: 3 ragged parts
+    dict(nchan=2048, subint_ns=512_000),                                            # four FFTs in 32 parts
+    dict(nchan=1024, subint_ns=1_024_000, nbits=8, freq0=8400.25),                  # 128 bins: 4 parts, two lanes
+    dict(nchan=1024, subint_ns=1_024_000, nfreq=2, full_pol=True, interval=5.0),    # complex bins
+], ids=["ragged", "long", "8bit", "shifting"])
+def test_pcal_few_long_windows(kw):
+    """Few FFTs: each window is cut into parts, one per lane of a bin.  A part
+    ends inside a frame, beyond the blanking point or in an invalid frame."""
+    job = pcal_job(nstation=3, **kw)
+    subints = [(0, k * kw["subint_ns"]) for k in (1, 2)]
+    f0 = synth.subint_window(job, 0, *subints[0])[0]
+    got, ref, layout, n = _run(job, invalid={0: [f0 + 1], 2: [f0 + 2]}, subints=subints)
+    pc = dict(regions(job, layout, n))["pcal"]
+    e = np.linalg.norm(got[pc] - ref[pc]) / np.linalg.norm(ref[pc])
+    assert e < 1e-5, e
