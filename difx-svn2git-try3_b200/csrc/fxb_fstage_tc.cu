@@ -49,7 +49,10 @@
 // roles; the tensor cores idle.  10 stations x 16 bands x 250 FFTs a launch: 173 us
 // with the unit records formed by the producer warp, 148 us with k_tc_units ahead of
 // it, 133 us with the conflict-free lookup and the twiddles loaded once for both
-// subbands; 32 stations x 8 bands x 250 FFTs: 348, 337, 309 us.
+// subbands; 32 stations x 8 bands x 250 FFTs: 348, 337, 309 us,
+// and 294 with the two subbands' decode interleaved (the first stays at 133).
+// Slower: the lookup's offset by rotating the nibble (294 -> 306), the twiddles by
+// recurrence in registers (133 -> 145, though 294 -> 282), a fourth operand buffer.
 
 #include <cuda.h>
 #include <cuda_runtime.h>
@@ -678,7 +681,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 						vm |= (kf < 32 ? ((fmask >> kf) & 1u) : 0u) << j;
 					}
 				}
-#pragma unroll 1
+#pragma unroll
 				for(int sb = 0; sb < 2; sb++)
 				{
 					const int nsh = 4 * R.nib[sb];
