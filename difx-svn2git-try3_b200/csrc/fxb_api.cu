@@ -38,17 +38,42 @@ struct Slot {
 	int32_t *h_vflags = nullptr;
 	cudaEvent_t copied = nullptr, done = nullptr;
 	bool used = false;
+	// what the preparation kernels hand the others, the slot's own, so that one
+	// subint's run beside the last one's F stage and XMAC: FFT parameters, data
+	// weights (packed [station][FFT]; per band of INTERLACEDVDIF stations
+	// [S][T][nbm]), unit records of the tensor-core FFT
+	FftParam *d_params = nullptr;
+	float *d_wts = nullptr, *d_pbw = nullptr;
+	unsigned char *d_tcrec = nullptr;
+	// frame validity [S][valid_stride], the band masks and the frames without
+	// fill pattern, one allocation
+	uint8_t *d_valid = nullptr;
+	uint32_t *d_bandok = nullptr;
+	uint8_t *d_fillok = nullptr;
+	int64_t valid_stride = 0;
+	// raw INTERLACEDVDIF reads: frame-slot tables, muxed headers and status
+	// words of those stations, carved from one scratch block
+	int32_t *d_mux = nullptr;
+	size_t mux_cap = 0;                // int32 words
+	// end of the preparation kernels on the context's prep_stream, where the slot's
+	// last subint had them there
+	cudaEvent_t prepped = nullptr;
+	bool beside = false;
 	// kernel timing of the slot's last subint: starts of prep, F stage and
 	// XMAC, end of the subint (recorded on every launch, graph nodes included);
 	// tpending: recorded while timing was on and not yet added to the sums
 	cudaEvent_t tev[4] = {nullptr, nullptr, nullptr, nullptr};
 	bool tpending = false;
-	// this slot's subint kernels as one CUDA graph, valid while the
-	// frame-validity array it was captured with is current
-	cudaGraphExec_t gexec = nullptr;
-	const uint8_t *g_valid = nullptr;
-	int64_t g_stride = 0;
-	int g_gen = -1;
+	// this slot's subint kernels as one CUDA graph, and those after the preparation
+	// as another, each valid while the frame-validity array it was captured with is
+	// current
+	struct Graph {
+		cudaGraphExec_t exec = nullptr;
+		const uint8_t *valid = nullptr;
+		int64_t stride = 0;
+		int gen = -1;
+	};
+	Graph whole, after;
 };
 
 // Online autotuner (fxb_autotune): over its first subints a context tries
@@ -71,7 +96,13 @@ struct fxb_ctx {
 	Job job;
 	std::string err;
 	int device = 0;
-	cudaStream_t stream = nullptr, copy_stream = nullptr;
+	// prep_stream: the preparation kernels of a subint that finds the last one
+	// still running (submit)
+	cudaStream_t stream = nullptr, copy_stream = nullptr, prep_stream = nullptr;
+	bool all_tcfft = false;             // every F kind runs the tensor-core FFT
+	cudaEvent_t fork = nullptr;         // of a graph's branch of timing events (mark)
+	bool stations_set = false;          // d_st written on the stream since the last preparation beside it
+	mutable bool exposed = false;       // the caller has the stream (fxb_get_stream)
 	// device memory comes from this pool (a server's, whose memory stays
 	// mapped between jobs) or, when null, the device's default pool; every
 	// allocation and free is stream-ordered, so none synchronises the device
@@ -84,12 +115,10 @@ struct fxb_ctx {
 	std::vector<DevFreqPlan> h_plans;
 	std::vector<void *> owned;          // misc device allocations
 	float2 *d_twiddle = nullptr;
-	FftParam *d_params = nullptr;
-	float *d_pbw = nullptr;              // per-band data weights of INTERLACEDVDIF stations [S][T][nbm]
 	int nbm = 0;
 	float2 *d_spec = nullptr;
 	float2 *d_acc = nullptr;
-	float *d_wacc = nullptr, *d_wts = nullptr;   // weight sums; packed data weights [station][FFT]
+	float *d_wacc = nullptr;             // weight sums
 	DevWeightSum *d_wsum = nullptr;
 	DevWeightOut *d_wout = nullptr;
 	DevOutMap *d_om = nullptr;
@@ -107,15 +136,7 @@ struct fxb_ctx {
 	size_t psmem = 0;
 	double *d_pbins = nullptr;           // [pplan.chunks][job.pcal_bins]
 	float2 *d_core = nullptr;
-	uint8_t *d_valid = nullptr;          // frame validity [S][valid_stride], then the band masks
-	uint32_t *d_bandok = nullptr;        // [S][valid_stride] in the same allocation
-	uint8_t *d_fillok = nullptr;         // [S][valid_stride] frames without fill pattern, same allocation
-	// raw INTERLACEDVDIF reads: frame-slot tables, muxed headers and status
-	// words of those stations, carved per subint from one scratch block
-	int nraw = 0;
-	int32_t *d_mux = nullptr;
-	size_t mux_cap = 0;                  // int32 words
-	int64_t valid_stride = 0;
+	int nraw = 0;                        // stations of raw INTERLACEDVDIF reads
 	std::vector<Slot> slots;
 	int next_slot = 0;
 	int last_slot = -1;              // slot of the last submitted subint
@@ -145,6 +166,7 @@ struct fxb_ctx {
 	PairItem *d_pitems = nullptr;        // two-band items and the constants of their FFTs
 	PairConst *d_pconst = nullptr;
 	PairTwist *d_ptwist = nullptr;       // of the items from ptwist0 on
+	size_t tcrec_bytes = 0;              // unit records of a slot's tensor-core FFT kinds
 	int ptwist0 = 0;
 	int32_t *d_pctr = nullptr;
 	void *d_specn = nullptr;             // half2 (or bf16x2) spectra of the tensor-core forms, X 2^-kTcSpecExp
@@ -291,16 +313,16 @@ static void free_ctx(fxb_ctx *ctx)
 		cudaStreamSynchronize(ctx->stream);
 	if(ctx->copy_stream)
 		cudaStreamSynchronize(ctx->copy_stream);
+	if(ctx->prep_stream)
+		cudaStreamSynchronize(ctx->prep_stream);
 	// every stream is idle: the frees, ordered on the compute stream, return
 	// the memory to its pool
 	for(void *p : ctx->owned)
 		cudaFreeAsync(p, ctx->stream);
-	if(ctx->d_valid)
-		cudaFreeAsync(ctx->d_valid, ctx->stream);
-	if(ctx->d_mux)
-		cudaFreeAsync(ctx->d_mux, ctx->stream);
 	for(auto &s : ctx->slots)
 	{
+		if(s.d_valid) cudaFreeAsync(s.d_valid, ctx->stream);
+		if(s.d_mux) cudaFreeAsync(s.d_mux, ctx->stream);
 		for(auto *p : s.raw)
 			if(p) cudaFreeAsync(p, ctx->stream);
 		if(s.rawall) cudaFreeAsync(s.rawall, ctx->stream);
@@ -311,9 +333,11 @@ static void free_ctx(fxb_ctx *ctx)
 	{
 		std::free(s.h_sub);
 		std::free(s.h_vflags);
-		if(s.gexec) cudaGraphExecDestroy(s.gexec);
+		if(s.whole.exec) cudaGraphExecDestroy(s.whole.exec);
+		if(s.after.exec) cudaGraphExecDestroy(s.after.exec);
 		if(s.copied) cudaEventDestroy(s.copied);
 		if(s.done) cudaEventDestroy(s.done);
+		if(s.prepped) cudaEventDestroy(s.prepped);
 	}
 	for(auto &s : ctx->slots)
 		for(cudaEvent_t e : s.tev)
@@ -322,7 +346,30 @@ static void free_ctx(fxb_ctx *ctx)
 		if(e) cudaEventDestroy(e);
 	if(ctx->stream) cudaStreamDestroy(ctx->stream);
 	if(ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
+	if(ctx->prep_stream) cudaStreamDestroy(ctx->prep_stream);
+	if(ctx->fork) cudaEventDestroy(ctx->fork);
 	delete ctx;
+}
+
+// The slot's frame-validity arrays, for n frames a station.
+static cudaError_t alloc_valid(fxb_ctx *ctx, Slot &sl, int64_t n, cudaStream_t stream)
+{
+	if(sl.d_valid)
+	{
+		const cudaError_t e = cudaFreeAsync(sl.d_valid, stream);
+		if(e != cudaSuccess)
+			return e;
+	}
+	sl.d_valid = nullptr;
+	sl.valid_stride = 0;
+	const size_t vbytes = ((size_t)n * ctx->S + 15) / 16 * 16;
+	const cudaError_t e = pool_alloc(ctx, (void **)&sl.d_valid, 2 * vbytes + sizeof(uint32_t) * n * ctx->S, stream);
+	if(e != cudaSuccess)
+		return e;
+	sl.d_bandok = (uint32_t *)(sl.d_valid + vbytes);
+	sl.d_fillok = sl.d_valid + vbytes + sizeof(uint32_t) * n * ctx->S;
+	sl.valid_stride = n;
+	return cudaSuccess;
 }
 
 // Phase-cal binning groups: a station's bands with tones and equal bin
@@ -424,6 +471,14 @@ static fxb_status setup_device(fxb_ctx *ctx)
 	CK(ctx, cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, ctx->device));
 	CK(ctx, cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
 	CK(ctx, cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking));
+	{
+		// first in line, so that its small kernels get in between those of the F
+		// stage and the XMAC
+		int least = 0, greatest = 0;
+		CK(ctx, cudaDeviceGetStreamPriorityRange(&least, &greatest));
+		CK(ctx, cudaStreamCreateWithPriority(&ctx->prep_stream, cudaStreamNonBlocking, greatest));
+		CK(ctx, cudaEventCreateWithFlags(&ctx->fork, cudaEventDisableTiming));
+	}
 	ctx->S = (int)job.stations.size();
 	ctx->T = job.blockspersend;
 	ctx->F = (int)job.freqs.size();
@@ -790,7 +845,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 			for(const auto &kv : bykind)
 				if(((kv.first.second >> 6) & 1) == mixed)
 					ordered.push_back(kv);
-		int ntwist = 0;
+		size_t ntwist = 0;
 		for(const auto &kv : ordered)
 		{
 			FKind k;
@@ -857,9 +912,8 @@ static fxb_status setup_device(fxb_ctx *ctx)
 					k.tcpairs = dp;
 					k.tcnpairs = (int32_t)(pairs.size() / 2);
 					k.tcbpt = bpt;
-					unsigned char *rec = nullptr;
-					CK(ctx, dalloc(ctx, &rec, fstage_tc_rec_bytes(k.tcnpairs, ctx->T)));
-					k.tcrec = rec;
+					k.tcrec0 = (int64_t)ctx->tcrec_bytes;
+					ctx->tcrec_bytes += (fstage_tc_rec_bytes(k.tcnpairs, ctx->T) + 255) / 256 * 256;
 				}
 			}
 			{
@@ -877,7 +931,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 		}
 		CK(ctx, dalloc(ctx, &ctx->d_pitems, pitems.size()));
 		CK(ctx, dalloc(ctx, &ctx->d_pconst, pitems.size() * (size_t)ctx->T));
-		CK(ctx, dalloc(ctx, &ctx->d_ptwist, (size_t)ntwist * ctx->T));
+		CK(ctx, dalloc(ctx, &ctx->d_ptwist, ntwist * (size_t)ctx->T));
 		if(!pitems.empty())
 			CK(ctx, cudaMemcpyAsync(ctx->d_pitems, pitems.data(), sizeof(PairItem) * pitems.size(), cudaMemcpyHostToDevice,
 			                        ctx->stream));
@@ -943,10 +997,10 @@ static fxb_status setup_device(fxb_ctx *ctx)
 		if(!hg.empty())
 			CK(ctx, cudaMemcpyAsync(ctx->d_groups, hg.data(), sizeof(FGroup) * hg.size(), cudaMemcpyHostToDevice, ctx->stream));
 	}
+	ctx->all_tcfft = !ctx->fkinds.empty();
+	for(const FKind &k : ctx->fkinds)
+		ctx->all_tcfft = ctx->all_tcfft && k.tcfft;
 	// big buffers
-	CK(ctx, dalloc(ctx, &ctx->d_params, (size_t)ctx->S * ctx->T));
-	if(ctx->nbm)
-		CK(ctx, dalloc(ctx, &ctx->d_pbw, (size_t)ctx->S * ctx->T * ctx->nbm));
 	CK(ctx, dalloc(ctx, &ctx->d_spec, job.xmac_kind == FXB_XMAC_FP32 ? (size_t)job.spec_total : 1));
 	CK(ctx, dalloc(ctx, &ctx->d_acc, (size_t)job.acc_total));
 	CK(ctx, dalloc(ctx, &ctx->d_core, (size_t)job.corelen));
@@ -973,7 +1027,6 @@ static fxb_status setup_device(fxb_ctx *ctx)
 		ctx->nwsum = (int)sums.size();
 		ctx->nwout = (int)wout.size();
 		CK(ctx, dalloc(ctx, &ctx->d_wacc, ctx->nwsum));
-		CK(ctx, dalloc(ctx, &ctx->d_wts, (size_t)ctx->S * ctx->T));
 		CK(ctx, dalloc(ctx, &ctx->d_wsum, ctx->nwsum));
 		CK(ctx, dalloc(ctx, &ctx->d_wout, ctx->nwout));
 		if(ctx->nwsum) CK(ctx, cudaMemcpyAsync(ctx->d_wsum, sums.data(), sizeof(DevWeightSum) * ctx->nwsum, cudaMemcpyHostToDevice, ctx->stream));
@@ -1052,12 +1105,28 @@ static fxb_status setup_device(fxb_ctx *ctx)
 
 	// staging slots
 	ctx->slots.resize(job.inflight);
+	// frames of a subint's buffers (an eighth and a few more for windows with
+	// margins; longer ones get a larger array when they come)
+	int64_t frames = 0;
+	for(int s = 0; s < ctx->S; s++)
+	{
+		const Job::Station &js = job.stations[s];
+		const double bits = (double)job.subint_ns * 1e-3 * 2.0 * job.freqs[js.band_freq[0]].bw_mhz * js.nbits * js.nband;
+		frames = std::max(frames, (int64_t)(bits / 8.0 / js.payload * 1.125) + 8);
+	}
 	for(auto &sl : ctx->slots)
 	{
+		CK(ctx, alloc_valid(ctx, sl, frames, ctx->stream));
 		sl.raw.assign(ctx->S, nullptr);
 		sl.rawcap.assign(ctx->S, 0);
 		CK(ctx, dalloc(ctx, &sl.d_sub, ctx->S));
 		CK(ctx, dalloc(ctx, &sl.d_vflags, (size_t)ctx->S * ctx->nflagint));
+		CK(ctx, dalloc(ctx, &sl.d_params, (size_t)ctx->S * ctx->T));
+		CK(ctx, dalloc(ctx, &sl.d_wts, (size_t)ctx->S * ctx->T));
+		if(ctx->nbm)
+			CK(ctx, dalloc(ctx, &sl.d_pbw, (size_t)ctx->S * ctx->T * ctx->nbm));
+		if(ctx->tcrec_bytes)
+			CK(ctx, dalloc(ctx, &sl.d_tcrec, ctx->tcrec_bytes));
 		sl.h_sub = (DevSubintStation *)std::calloc(ctx->S, sizeof(DevSubintStation));
 		sl.h_vflags = (int32_t *)std::calloc((size_t)ctx->S * ctx->nflagint, sizeof(int32_t));
 		if(!sl.h_sub || !sl.h_vflags)
@@ -1067,6 +1136,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 		}
 		CK(ctx, cudaEventCreateWithFlags(&sl.copied, cudaEventDisableTiming));
 		CK(ctx, cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming));
+		CK(ctx, cudaEventCreate(&sl.prepped));
 		for(cudaEvent_t &e : sl.tev)
 			CK(ctx, cudaEventCreate(&e));
 	}
@@ -1153,6 +1223,7 @@ fxb_status fxb_set_delay_poly(fxb_ctx *ctx, int32_t station, int32_t npoly, int3
 	memset(d.coeffs, 0, sizeof(d.coeffs));
 	memcpy(d.coeffs, coeffs, sizeof(double) * npoly * (order + 1));
 	CK(ctx, cudaMemcpyAsync(ctx->d_st + station, &d, sizeof(DevStation), cudaMemcpyHostToDevice, ctx->stream));
+	ctx->stations_set = true;
 	ctx->delay_set[station] = true;
 	return FXB_OK;
 }
@@ -1164,7 +1235,7 @@ static void slot_account(fxb_ctx *ctx, Slot &sl)
 		return;
 	sl.tpending = false;
 	float a = 0, b = 0, c = 0;
-	if(cudaEventElapsedTime(&a, sl.tev[0], sl.tev[1]) == cudaSuccess &&
+	if(cudaEventElapsedTime(&a, sl.tev[0], sl.beside ? sl.prepped : sl.tev[1]) == cudaSuccess &&
 	   cudaEventElapsedTime(&b, sl.tev[1], sl.tev[2]) == cudaSuccess &&
 	   cudaEventElapsedTime(&c, sl.tev[2], sl.tev[3]) == cudaSuccess)
 	{
@@ -1199,6 +1270,7 @@ static fxb_status stage_subint(fxb_ctx *ctx, const uint8_t *const *bufs, const i
 		CK(ctx, cudaEventSynchronize(sl.done));
 	slot_account(ctx, sl);
 	sl.used = true;
+	sl.beside = false;
 
 	// frame-validity array sized for the largest buffer of this subint
 	int64_t need = 0;
@@ -1211,24 +1283,14 @@ static fxb_status stage_subint(fxb_ctx *ctx, const uint8_t *const *bufs, const i
 		}
 		need = std::max<int64_t>(need, nbytes[s] / ctx->h_st[s].payload + 2);
 	}
-	if(need > ctx->valid_stride)
+	if(need > sl.valid_stride)
 	{
-		// stream-ordered: the earlier subints' kernels finish with the old array first
-		if(ctx->d_valid)
-		{
-			CK(ctx, cudaFreeAsync(ctx->d_valid, ctx->stream));
-		ctx->dirty = true;
-			ctx->d_valid = nullptr;
-		}
-		const size_t vbytes = ((size_t)need * ctx->S + 15) / 16 * 16;
-		CK(ctx, pool_alloc(ctx, (void **)&ctx->d_valid, 2 * vbytes + sizeof(uint32_t) * need * ctx->S, ctx->stream));
-		ctx->d_bandok = (uint32_t *)(ctx->d_valid + vbytes);
-		ctx->d_fillok = ctx->d_valid + vbytes + sizeof(uint32_t) * need * ctx->S;
-		ctx->valid_stride = need;
+		// the slot is idle, so the old array can go back at once; the new one is
+		// ordered ahead of the slot's `copied` event
+		CK(ctx, alloc_valid(ctx, sl, need, ctx->copy_stream));
 	}
 
 	// raw INTERLACEDVDIF reads: slot tables, muxed headers and status words
-	// (shared by the staging slots: their kernels run in stream order)
 	std::vector<size_t> mux_off(ctx->S, 0);
 	if(ctx->nraw)
 	{
@@ -1243,14 +1305,14 @@ static fxb_status stage_subint(fxb_ctx *ctx, const uint8_t *const *bufs, const i
 			words += (size_t)(4 * nin / d.nthr) * d.nthr + (size_t)(nin / d.nthr + 1) * 16 + 4;
 			words = (words + 3) & ~(size_t)3;
 		}
-		if(words > ctx->mux_cap)
+		if(words > sl.mux_cap)
 		{
-			if(ctx->d_mux)
-				CK(ctx, cudaFreeAsync(ctx->d_mux, ctx->stream));
-			ctx->dirty = true;
-			ctx->d_mux = nullptr;
-			CK(ctx, pool_alloc(ctx, (void **)&ctx->d_mux, sizeof(int32_t) * words, ctx->stream));
-			ctx->mux_cap = words;
+			if(sl.d_mux)
+				CK(ctx, cudaFreeAsync(sl.d_mux, ctx->copy_stream));
+			sl.d_mux = nullptr;
+			sl.mux_cap = 0;
+			CK(ctx, pool_alloc(ctx, (void **)&sl.d_mux, sizeof(int32_t) * words, ctx->copy_stream));
+			sl.mux_cap = words;
 		}
 	}
 
@@ -1292,7 +1354,7 @@ static fxb_status stage_subint(fxb_ctx *ctx, const uint8_t *const *bufs, const i
 			u.mux_nin = (int32_t)(nbytes[s] / d.inframebytes);
 			u.mux_nproc = u.mux_nin / d.nthr;
 			u.mux_nslot = 4 * u.mux_nin / d.nthr;
-			u.mux_slot = ctx->d_mux + mux_off[s];
+			u.mux_slot = sl.d_mux + mux_off[s];
 			u.mux_hdr = (uint32_t *)(u.mux_slot + (size_t)u.mux_nslot * d.nthr);
 			u.mux_status = (int32_t *)(u.mux_hdr + (size_t)(u.mux_nproc + 1) * 16);
 		}
@@ -1355,11 +1417,11 @@ static FsArgs fs_args(const fxb_ctx *ctx, const Slot &sl)
 	fa.sub = sl.d_sub;
 	fa.groups = ctx->d_groups;
 	fa.plans = ctx->d_plans;
-	fa.valid = ctx->d_valid;
-	fa.bandok = ctx->nbm ? ctx->d_bandok : nullptr;
-	fa.fillok = ctx->d_fillok;
-	fa.valid_stride = ctx->valid_stride;
-	fa.params = ctx->d_params;
+	fa.valid = sl.d_valid;
+	fa.bandok = ctx->nbm ? sl.d_bandok : nullptr;
+	fa.fillok = sl.d_fillok;
+	fa.valid_stride = sl.valid_stride;
+	fa.params = sl.d_params;
 	fa.maxN = ctx->maxN;
 	fa.T = ctx->T;
 	fa.order = job.fringe_rot_order;
@@ -1371,7 +1433,24 @@ static FsArgs fs_args(const fxb_ctx *ctx, const Slot &sl)
 	fa.pconst = ctx->d_pconst;
 	fa.ptwist = ctx->d_ptwist;
 	fa.ptwist0 = ctx->ptwist0;
+	fa.tcrec = sl.d_tcrec;
 	return fa;
+}
+
+// Timing event e at this point of stream st: a record, in a graph an event-record
+// node, which parts the kernels on its sides by 5 us (0.5 us without).  branch: the
+// node goes on a branch of its own (the idle prep_stream carries it while
+// capturing; launch_xmac_weights joins it).  Only for subints in a row: a branch
+// lengthens the start of a graph that the device waits for.
+static void mark(fxb_ctx *ctx, cudaEvent_t e, cudaStream_t st, bool capture, bool branch = false)
+{
+	if(branch)
+	{
+		cudaEventRecord(ctx->fork, st);
+		cudaStreamWaitEvent(ctx->prep_stream, ctx->fork, 0);
+		st = ctx->prep_stream;
+	}
+	cudaEventRecordWithFlags(e, st, capture ? cudaEventRecordExternal : cudaEventRecordDefault);
 }
 
 // Every kernel of one subint whose inputs sit in slot sl, on stream st.  No
@@ -1381,41 +1460,44 @@ static FsArgs fs_args(const fxb_ctx *ctx, const Slot &sl)
 // events become event-record nodes of the graph.
 // Delay interpolators, raw-read placement, frame validity and per-FFT
 // parameters of one subint (Mode::setOffsets, Mk5Mode::unpack's checks).
-static void launch_prep(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, unsigned evf)
+static void launch_prep(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, bool capture)
 {
 	const Job &job = ctx->job;
-	cudaEventRecordWithFlags(sl.tev[0], st, evf);
+	mark(ctx, sl.tev[0], st, capture);
 	if(ctx->nraw)
 	{
 		launch_interpolators(ctx->d_st, sl.d_sub, ctx->S, ctx->T, st);
 		launch_mux_raw(ctx->d_st, sl.d_sub, ctx->S, 0, 0, st);
-		launch_frame_valid(ctx->d_st, sl.d_sub, ctx->d_valid, ctx->d_bandok, ctx->valid_stride, ctx->S, st,
-		                   ctx->d_fillok);
+		launch_frame_valid(ctx->d_st, sl.d_sub, sl.d_valid, sl.d_bandok, sl.valid_stride, ctx->S, st,
+		                   sl.d_fillok);
 	}
 	else
-		fxb::launch_prep(ctx->d_st, sl.d_sub, ctx->S, ctx->T, ctx->d_valid, ctx->d_bandok, ctx->valid_stride, st,
-		                 ctx->d_fillok);
-	launch_fft_params(ctx->d_st, sl.d_sub, sl.d_vflags, ctx->nflagint, ctx->d_valid, ctx->d_bandok, ctx->valid_stride,
-	                  ctx->S, ctx->T, job.fringe_rot_order, ctx->d_params, ctx->d_pbw, ctx->nbm, st, ctx->d_fillok, ctx->d_wts);
+		fxb::launch_prep(ctx->d_st, sl.d_sub, ctx->S, ctx->T, sl.d_valid, sl.d_bandok, sl.valid_stride, st,
+		                 sl.d_fillok);
+	launch_fft_params(ctx->d_st, sl.d_sub, sl.d_vflags, ctx->nflagint, sl.d_valid, sl.d_bandok, sl.valid_stride,
+	                  ctx->S, ctx->T, job.fringe_rot_order, sl.d_params, sl.d_pbw, ctx->nbm, st, sl.d_fillok, sl.d_wts);
 	const FsArgs fa = fs_args(ctx, sl);
 	for(const FKind &k : ctx->fkinds)
 		if(k.tcfft)
 			launch_tc_units(k, fa, st);
 		else if(k.nb == 2)
 			launch_pair_consts(k, fa, st);
-	cudaEventRecordWithFlags(sl.tev[1], st, evf);
 }
 
-static void launch_xmac_weights(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, unsigned evf, bool tuning,
-                                bool xmac = true);
+static void launch_xmac_weights(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, bool capture, bool tuning,
+                                bool xmac = true, bool branch = false);
 
-static void launch_compute(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, bool capture)
+// prep: with the preparation kernels (else they run elsewhere, and the stream
+// already waits for them).
+static void launch_compute(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, bool capture, bool prep = true)
 {
 	Tuner &tn = ctx->tune;
 	const bool tuning = !capture && tn.iter < tn.total;
 	const size_t nk = ctx->fkinds.size();
-	const unsigned evf = capture ? cudaEventRecordExternal : cudaEventRecordDefault;
-	launch_prep(ctx, sl, st, evf);
+	if(prep)
+		launch_prep(ctx, sl, st, capture);
+	const bool branch = capture && !prep;
+	mark(ctx, sl.tev[1], st, capture, branch);
 	{
 		const FsArgs fa = fs_args(ctx, sl);
 		for(size_t i = 0; i < nk; i++)
@@ -1464,24 +1546,25 @@ static void launch_compute(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, bool c
 		if(tuning)
 			cudaEventRecord(tn.ev[nk], st);
 	}
-	launch_xmac_weights(ctx, sl, st, evf, tuning);
+	launch_xmac_weights(ctx, sl, st, capture, tuning, true, branch);
 }
 
 // Phase-cal bins and zoom gathers (after the F stage), the FP8 quantisation,
 // every XMAC group (unless xmac is false: the caller runs them) and the
 // weights of one subint.
-static void launch_xmac_weights(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, unsigned evf, bool tuning, bool xmac)
+static void launch_xmac_weights(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, bool capture, bool tuning, bool xmac,
+                                bool branch)
 {
 	const Job &job = ctx->job;
 	Tuner &tn = ctx->tune;
 	const size_t nk = ctx->fkinds.size();
 	for(const auto &pc : ctx->pclass)
 		launch_pcal_bin(ctx->d_pgroups + pc.first, pc.count, pc.maxbins, ctx->pplan, pc.nbits, pc.bpt, pc.shift != 0,
-		                pc.smem, ctx->d_st, sl.d_sub, ctx->d_params, ctx->d_valid, ctx->valid_stride, ctx->T,
+		                pc.smem, ctx->d_st, sl.d_sub, sl.d_params, sl.d_valid, sl.valid_stride, ctx->T,
 		                job.pcal_bins, ctx->d_pbins, st);
 	launch_zoom_gather(ctx->d_zoom, ctx->nzoom, ctx->d_plans, ctx->T, ctx->tc,
 	                   ctx->tc ? ctx->d_specn : (void *)ctx->d_spec, st);
-	cudaEventRecordWithFlags(sl.tev[2], st, evf);
+	mark(ctx, sl.tev[2], st, capture, branch);
 	if(ctx->f8)
 		for(const auto &g : ctx->xgroups)
 			if(g.xmac)
@@ -1511,8 +1594,13 @@ static void launch_xmac_weights(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, u
 	}
 	if(tuning)
 		cudaEventRecord(tn.ev[nk + 1 + ctx->xgroups.size()], st);
-	launch_weights(ctx->d_wsum, ctx->nwsum, ctx->d_wts, ctx->d_pbw, ctx->nbm, ctx->T, ctx->d_wacc, st);
-	cudaEventRecordWithFlags(sl.tev[3], st, evf);
+	launch_weights(ctx->d_wsum, ctx->nwsum, sl.d_wts, sl.d_pbw, ctx->nbm, ctx->T, ctx->d_wacc, st);
+	if(branch)
+	{
+		cudaEventRecord(ctx->fork, ctx->prep_stream);
+		cudaStreamWaitEvent(st, ctx->fork, 0);
+	}
+	mark(ctx, sl.tev[3], st, capture);
 	// a launch that could not start (resources, configuration) leaves its
 	// error behind; keep it for the submit to report
 	const cudaError_t le = cudaPeekAtLastError();
@@ -1577,36 +1665,37 @@ static void tune_collect(fxb_ctx *ctx)
 	ctx->gen++;
 }
 
-// The slot's graph, captured (again) when missing or when the frame-validity
-// array has been reallocated since.  A capture that fails turns graphs off
-// for the context and leaves the stream as it was.
-static fxb_status slot_graph(fxb_ctx *ctx, Slot &sl)
+// The slot's graph g (with or without the preparation kernels), captured (again)
+// when missing or when the frame-validity array has been reallocated since.  A
+// capture that fails turns graphs off for the context and leaves the stream as it
+// was.
+static fxb_status slot_graph(fxb_ctx *ctx, Slot &sl, Slot::Graph &g, bool prep)
 {
-	if(sl.gexec && sl.g_valid == ctx->d_valid && sl.g_stride == ctx->valid_stride && sl.g_gen == ctx->gen)
+	if(g.exec && g.valid == sl.d_valid && g.stride == sl.valid_stride && g.gen == ctx->gen)
 		return FXB_OK;
-	if(sl.gexec)
+	if(g.exec)
 	{
-		cudaGraphExecDestroy(sl.gexec);
-		sl.gexec = nullptr;
+		cudaGraphExecDestroy(g.exec);
+		g.exec = nullptr;
 	}
 	CK(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-	launch_compute(ctx, sl, ctx->stream, true);
-	cudaGraph_t g = nullptr;
-	cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
+	launch_compute(ctx, sl, ctx->stream, true, prep);
+	cudaGraph_t cg = nullptr;
+	cudaError_t e = cudaStreamEndCapture(ctx->stream, &cg);
 	if(e == cudaSuccess)
-		e = cudaGraphInstantiate(&sl.gexec, g, 0);
-	if(g)
-		cudaGraphDestroy(g);
+		e = cudaGraphInstantiate(&g.exec, cg, 0);
+	if(cg)
+		cudaGraphDestroy(cg);
 	if(e != cudaSuccess)
 	{
 		cudaGetLastError();
-		sl.gexec = nullptr;
+		g.exec = nullptr;
 		ctx->graphs = false;
 		return FXB_OK;
 	}
-	sl.g_valid = ctx->d_valid;
-	sl.g_stride = ctx->valid_stride;
-	sl.g_gen = ctx->gen;
+	g.valid = sl.d_valid;
+	g.stride = sl.valid_stride;
+	g.gen = ctx->gen;
 	return FXB_OK;
 }
 
@@ -1625,18 +1714,47 @@ static fxb_status submit(fxb_ctx *ctx, const uint8_t *const *bufs, const int64_t
 		return rc;
 	Slot &sl = *slp;
 	cudaStream_t st = ctx->stream;
-	CK(ctx, cudaStreamWaitEvent(st, sl.copied, 0));
 	const bool tuning = ctx->tune.iter < ctx->tune.total;
+	// While the subint before the last one (two slots: the last one) still runs, and
+	// the device therefore lags the caller, this one's preparation kernels (latency,
+	// a few blocks each) go beside the F stage and XMAC in progress; a device that
+	// keeps up takes the whole graph, the fewest launches.  Only beside the
+	// tensor-core FFT, which leaves registers to other blocks: the persistent
+	// CUDA-core F launches fill them, and their CTAs that start late behind such a
+	// block end late (20 stations x 8 bands x 256 points: F stage 440 -> 473 us).
+	// The kernels read the station buffers without waiting for the context's stream:
+	// not where the caller may have ordered the buffers' making on that stream.
+	// 10 stations x 16 bands x 250 FFTs: 211 us a subint in line, 193 us beside.
+	const int nsl = (int)ctx->slots.size();
+	const Slot *behind = ctx->last_slot >= 0 ? &ctx->slots[(ctx->last_slot + nsl - (nsl > 2 ? 1 : 0)) % nsl] : nullptr;
+	const bool beside = ctx->graphs && ctx->all_tcfft && !tuning && behind && behind->used && behind != &sl &&
+	                    !(device && ctx->exposed) && cudaEventQuery(behind->done) == cudaErrorNotReady;
+	cudaGetLastError();
+	if(beside)
+	{
+		if(ctx->stations_set)
+		{
+			CK(ctx, cudaEventRecord(sl.prepped, st));
+			CK(ctx, cudaStreamWaitEvent(ctx->prep_stream, sl.prepped, 0));
+			ctx->stations_set = false;
+		}
+		CK(ctx, cudaStreamWaitEvent(ctx->prep_stream, sl.copied, 0));
+		launch_prep(ctx, sl, ctx->prep_stream, false);
+		CK(ctx, cudaEventRecord(sl.prepped, ctx->prep_stream));
+	}
+	CK(ctx, cudaStreamWaitEvent(st, beside ? sl.prepped : sl.copied, 0));
+	sl.beside = beside;
+	Slot::Graph &g = beside ? sl.after : sl.whole;
 	if(ctx->graphs && !tuning)
 	{
-		const fxb_status gs = slot_graph(ctx, sl);
+		const fxb_status gs = slot_graph(ctx, sl, g, !beside);
 		if(gs != FXB_OK)
 			return gs;
 	}
 	if(ctx->graphs && !tuning)
-		CK(ctx, cudaGraphLaunch(sl.gexec, st));
+		CK(ctx, cudaGraphLaunch(g.exec, st));
 	else
-		launch_compute(ctx, sl, st, false);
+		launch_compute(ctx, sl, st, false, !beside);
 	{
 		const fxb_status le = take_launch_err(ctx);
 		if(le != FXB_OK)
@@ -1887,7 +2005,8 @@ fxb_status fxb_job_footprint(const fxb_job_desc *desc, size_t *bytes)
 	double b = (double)job.spec_total * (job.xmac_kind == FXB_XMAC_FP32 ? 8.0
 	                                     : job.xmac_kind != FXB_XMAC_FP8 ? 4.0 * 1.25 * pad32
 	                                                                      : (4.0 * pad64 + 2.0 * pad64 + 0.5) * 1.25);
-	b += (double)job.acc_total * 8.0 + (double)job.corelen * 16.0 + (double)S * T * 68.0 + (double)pairs * T * 144.0 +
+	b += (double)job.acc_total * 8.0 + (double)job.corelen * 16.0 +
+	     (double)S * T * 68.0 * job.inflight + (double)pairs * T * 144.0 * (job.xmac_kind == FXB_XMAC_FP32 ? 1 : job.inflight) +
 	     (double)job.pcal_bins * 8.0 * pcal_plan_of(job, pcal_groups(job)).chunks;
 	// raw VDIF staging of the in-flight subints (payload plus headers, 1/8 slack)
 	for(int s = 0; s < S; s++)
@@ -1987,6 +2106,7 @@ fxb_status fxb_timing_read(fxb_ctx *ctx, int32_t *nsubint, double *prep_ms, doub
 fxb_status fxb_get_stream(const fxb_ctx *ctx, void **stream)
 {
 	if(!ctx || !stream) return FXB_ERR_ARG;
+	ctx->exposed = true;
 	*stream = (void *)ctx->stream;
 	return FXB_OK;
 }
@@ -2203,7 +2323,8 @@ fxb_status fxb_read_fft_weights(fxb_ctx *ctx, float *out, size_t nfloats)
 	if(nfloats < n) return FXB_ERR_ARG;
 	CK(ctx, cudaStreamSynchronize(ctx->stream));
 	std::vector<FftParam> hp(n);
-	CK(ctx, cudaMemcpy(hp.data(), ctx->d_params, sizeof(FftParam) * n, cudaMemcpyDeviceToHost));
+	const FftParam *params = ctx->slots[std::max(ctx->last_slot, 0)].d_params;
+	CK(ctx, cudaMemcpy(hp.data(), params, sizeof(FftParam) * n, cudaMemcpyDeviceToHost));
 	for(size_t i = 0; i < n; i++)
 		out[i] = hp[i].status == kFftOk ? hp[i].weight : 0.0f;
 	return FXB_OK;
@@ -2426,14 +2547,14 @@ static fxb_status batch_fused_plan(fxb_batch *b)
 // then the members' weights as branches.
 static void batch_fused_launch(fxb_batch *b, int k, const std::vector<Slot *> &slots, bool capture)
 {
-	const unsigned evf = capture ? cudaEventRecordExternal : cudaEventRecordDefault;
 	const size_t n = b->m.size();
 	cudaEventRecord(b->fork, b->stream);
 	for(size_t i = 0; i < n; i++)
 	{
 		fxb_ctx *c = b->m[i];
 		cudaStreamWaitEvent(c->stream, b->fork, 0);
-		launch_prep(c, *slots[i], c->stream, evf);
+		launch_prep(c, *slots[i], c->stream, capture);
+		mark(c, slots[i]->tev[1], c->stream, capture);
 	}
 	for(size_t i = 0; i < n; i++)
 	{
@@ -2505,7 +2626,7 @@ static void batch_fused_launch(fxb_batch *b, int k, const std::vector<Slot *> &s
 	{
 		fxb_ctx *c = b->m[i];
 		cudaStreamWaitEvent(c->stream, b->fork, 0);
-		launch_xmac_weights(c, *slots[i], c->stream, evf, false, false);
+		launch_xmac_weights(c, *slots[i], c->stream, capture, false, false);
 	}
 	for(size_t i = 0; i < n; i++)
 	{
@@ -2547,7 +2668,7 @@ static fxb_status batch_graph(fxb_batch *b, int k, const std::vector<Slot *> &sl
 	const size_t n = b->m.size();
 	bool ok = b->gexec[k] != nullptr && b->g_fused[k] == (int)fused;
 	for(size_t i = 0; ok && i < n; i++)
-		ok = b->g_valid[k][i] == b->m[i]->d_valid && b->g_stride[k][i] == b->m[i]->valid_stride &&
+		ok = b->g_valid[k][i] == slots[i]->d_valid && b->g_stride[k][i] == slots[i]->valid_stride &&
 		     b->g_gen[k][i] == b->m[i]->gen;
 	if(ok)
 		return FXB_OK;
@@ -2590,8 +2711,8 @@ static fxb_status batch_graph(fxb_batch *b, int k, const std::vector<Slot *> &sl
 	}
 	for(size_t i = 0; i < n; i++)
 	{
-		b->g_valid[k][i] = b->m[i]->d_valid;
-		b->g_stride[k][i] = b->m[i]->valid_stride;
+		b->g_valid[k][i] = slots[i]->d_valid;
+		b->g_stride[k][i] = slots[i]->valid_stride;
 		b->g_gen[k][i] = b->m[i]->gen;
 	}
 	b->g_fused[k] = (int)fused;

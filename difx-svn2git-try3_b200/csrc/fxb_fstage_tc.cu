@@ -1086,13 +1086,14 @@ size_t fstage_tc_rec_bytes(int npairs, int T) { return sizeof(UnitRec) * (size_t
 void launch_tc_units(const FKind &k, const FsArgs &a, cudaStream_t stream)
 {
 	const int nunits = k.tcnpairs * a.T;
-	if(k.tcrec && nunits > 0)
-		k_tc_units<<<(nunits + 63) / 64, 64, 0, stream>>>(a, k.tcpairs, k.tcnpairs, k.tcbpt, nunits, (UnitRec *)k.tcrec);
+	if(nunits > 0)
+		k_tc_units<<<(nunits + 63) / 64, 64, 0, stream>>>(a, k.tcpairs, k.tcnpairs, k.tcbpt, nunits,
+		                                                  (UnitRec *)(a.tcrec + k.tcrec0));
 }
 
 cudaError_t launch_fstage_tc(const FKind &k, FsArgs a, int nsm, cudaStream_t stream)
 {
-	if(k.count <= 0 || a.T <= 0 || !k.tctab || !k.tcrec || k.tcnpairs <= 0)
+	if(k.count <= 0 || a.T <= 0 || !k.tctab || k.tcnpairs <= 0)
 		return cudaSuccess;
 	a.first = k.first;
 	const int nunits = k.tcnpairs * a.T;
@@ -1101,7 +1102,7 @@ cudaError_t launch_fstage_tc(const FKind &k, FsArgs a, int nsm, cudaStream_t str
 		grid = nunits;
 	auto go = [&](auto kern, size_t smem) {
 		cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-		kern<<<grid, kThreadsTc, smem, stream>>>(a, (const uint4 *)k.tctab, (const UnitRec *)k.tcrec, nunits, a.err);
+		kern<<<grid, kThreadsTc, smem, stream>>>(a, (const uint4 *)k.tctab, (const UnitRec *)(a.tcrec + k.tcrec0), nunits, a.err);
 	};
 	const bool h = a.h16 != 0;
 	switch(k.tcbpt)

@@ -158,7 +158,7 @@ struct FKind {
 	const void *tw;          // twiddle table of length N (make_fstage_twiddles layout)
 	const void *tctab;       // constant tables of the tensor-core FFT kernel
 	const int32_t *tcpairs;  // tensor-core FFT: [tcnpairs][2] FGroup indices of each work unit's two subbands
-	void *tcrec;             // tensor-core FFT: records of the subint's work units (launch_tc_units)
+	int64_t tcrec0;          // tensor-core FFT: first byte of its units' records (launch_tc_units) in FsArgs::tcrec
 	int32_t tcnpairs;
 	int32_t tcbpt;           // tensor-core FFT: bits per time of the stations' VDIF words
 	int32_t muxraw;          // 1: the items' stations hand over raw INTERLACEDVDIF reads
@@ -241,6 +241,7 @@ struct FsArgs {
 	const PairItem *pitems;  // two-band items, and the constants of their FFTs [item][T]
 	PairConst *pconst;
 	PairTwist *ptwist;       // of the two-band items from ptwist0 on, [item - ptwist0][T]
+	unsigned char *tcrec;    // unit records of the tensor-core FFT kinds
 	int32_t ptwist0, two;    // two: the launch's items have twists (set by launch_fstage_kind)
 };
 // constants of the subint's FFTs of a two-band kind's items

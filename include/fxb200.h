@@ -440,7 +440,9 @@ FXB_API void *fxb_host_alloc(size_t bytes, fxb_status *status);
 FXB_API void fxb_host_free(void *p);
 
 /* The cudaStream_t (as void*) on which the context launches its kernels,
- * so that callers can order their own work and events against it. */
+ * so that callers can order their own work and events against it.  (A queue of
+ * subints from host buffers may run preparation kernels on a stream of its own;
+ * this stream waits for them.) */
 FXB_API fxb_status fxb_get_stream(const fxb_ctx *ctx, void **stream);
 
 /* As fxb_read_results, but the core result is written asynchronously (on
