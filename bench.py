@@ -818,7 +818,7 @@ def gpu_arm(args, job):
     f_avg = f_ms / max(nrec, 1)
     x_avg = x_ms / max(nrec, 1)
     tcfft = args.xmac != "fp32" and any("tensor-core FFT" in t for t in tuning)
-    fname = "k_fstage_tc" if tcfft else "k_fstage"
+    fname = "k_fstage_tc" if tcfft else "k_fstage_pair"
     alg = in_bytes + spec_bytes
     achieved = alg / (f_avg * 1e-3) / 1e9
     roofline = {"bound": "hbm", "kernel": fname, "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
@@ -833,7 +833,7 @@ def gpu_arm(args, job):
         I = sum(1 for st in job.stations for fb, _ in st.bands if fb == f)
         useful += 8 * (I * (I + 1) // 2) * job.freqs[f].nchan * T
     tcx = args.xmac != "fp32"
-    xname = "k_xmac_tc" if tcx else "k_xmac_fp32v2"
+    xname = {"fp32": "k_xmac_fp32", "fp8": "k_xmac_f8"}.get(args.xmac, "k_xmac_h")
     xach = useful / (x_avg * 1e-3) / 1e12
     xmac_roofline = {"bound": "tensor" if tcx else "fp32 pipe", "kernel": xname, "achieved": xach, "unit": "TFLOP/s",
                      "peak_burst": tf_peak if tcx else None, "frac_burst": xach / tf_peak if tcx else None,

@@ -153,7 +153,7 @@ struct fxb_ctx {
 	double t_prep = 0, t_f = 0, t_x = 0; // per-stage sums over timed subints (ms)
 	int32_t t_n = 0;
 	std::vector<bool> delay_set;
-	// F-stage work items (by kind) and FP32 XMAC v2 launch groups
+	// F-stage work items (by kind)
 	FGroup *d_groups = nullptr;
 	std::vector<FKind> fkinds;
 	// the kinds of the persistent F launches and their work list (wide units

@@ -38,7 +38,10 @@
 // extents, so a context alone and in a batch agree.
 //
 // Bound: HBM / L2 reads of the spectra at up to about 20 inputs, the epilogue's
-// reductions and the matrix work above.  Measured with launch_xmac_tc_multi.
+// reductions and the matrix work above.  Launch times in us with K-major operands
+// made by transposer warps, and now: 20 inputs x 8 x 1024 channels x 250 FFTs 69 and
+// 47 (the loads alone take 31); 40 x 4 x 128 x 4096 180 and 79; 10 x 2 x 64 x 38622
+// 1720 and 81 (time slices); 64 x 4 x 1024 x 250 125 and 134 (two reads).
 // Every wait is bounded: on timeout the CTA records an error code, drains its
 // TMA loads and MMAs, and still releases its tensor memory.
 
@@ -435,8 +438,8 @@ static bool h_stages(TcShape *s, int nst, int nb)
 // Time slices of a group: rounds of units over the resident CTAs times the K
 // tiles of each, every unit with an epilogue worth about kEpi K tiles, and the
 // sums of more than one slice written and read once more (kMerge K tiles each).
-// 40 inputs x 128 channels x 4 subbands, T = 4096 (256 units): see
-// launch_xmac_tc_multi.
+// 40 inputs x 128 channels x 4 subbands, T = 4096 (256 units): 180 us whole, 79 us
+// in slices.
 static int h_slices(const TcShape &s, int nf, int nsm)
 {
 	constexpr int kEpi = 6, kMerge = 2;
