@@ -1727,9 +1727,20 @@ static fxb_status submit(fxb_ctx *ctx, const uint8_t *const *bufs, const int64_t
 	// 10 stations x 16 bands x 250 FFTs: 211 us a subint in line, 193 us beside.
 	const int nsl = (int)ctx->slots.size();
 	const Slot *behind = ctx->last_slot >= 0 ? &ctx->slots[(ctx->last_slot + nsl - (nsl > 2 ? 1 : 0)) % nsl] : nullptr;
-	const bool beside = ctx->graphs && ctx->all_tcfft && !tuning && behind && behind->used && behind != &sl &&
-	                    !(device && ctx->exposed) && cudaEventQuery(behind->done) == cudaErrorNotReady;
-	cudaGetLastError();
+	bool beside = ctx->graphs && ctx->all_tcfft && !tuning && behind && behind->used && behind != &sl &&
+	              !(device && ctx->exposed);
+	// an error that was pending before the call stays for the check at the end
+	if(beside && cudaPeekAtLastError() != cudaSuccess)
+		beside = false;
+	if(beside)
+	{
+		const cudaError_t q = cudaEventQuery(behind->done);
+		if(q == cudaErrorNotReady)
+			cudaGetLastError();
+		else
+			CK(ctx, q);
+		beside = q == cudaErrorNotReady;
+	}
 	if(beside)
 	{
 		if(ctx->stations_set)
