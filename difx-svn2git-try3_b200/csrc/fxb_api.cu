@@ -2076,7 +2076,16 @@ fxb_status fxb_last_timing(const fxb_ctx *ctx, float *fstage_ms, float *xmac_ms,
 	float a = 0, b = 0, t = 0;
 	CK(c, cudaEventElapsedTime(&a, sl.tev[1], sl.tev[2]));
 	CK(c, cudaEventElapsedTime(&b, sl.tev[2], sl.tev[3]));
-	CK(c, cudaEventElapsedTime(&t, sl.tev[0], sl.tev[3]));
+	if(sl.beside)
+	{
+		// the preparation and the rest run apart, with other subints' kernels between
+		float p = 0;
+		CK(c, cudaEventElapsedTime(&p, sl.tev[0], sl.prepped));
+		CK(c, cudaEventElapsedTime(&t, sl.tev[1], sl.tev[3]));
+		t += p;
+	}
+	else
+		CK(c, cudaEventElapsedTime(&t, sl.tev[0], sl.tev[3]));
 	if(fstage_ms) *fstage_ms = a;
 	if(xmac_ms) *xmac_ms = b;
 	if(total_ms) *total_ms = t;

@@ -312,16 +312,20 @@ FXB_API fxb_status fxb_read_results(fxb_ctx *ctx, float *coreresult, size_t nflo
 FXB_API fxb_status fxb_reset(fxb_ctx *ctx);
 
 /* Device time in ms of the last subint's kernels (F stage, XMAC, total),
- * measured with CUDA events on the context's stream. */
+ * measured with CUDA events on the streams that run them.  The total is the
+ * preparation kernels' interval and the rest's, without the wait between the
+ * two where the preparation ran beside earlier subints (fxb_get_stream). */
 FXB_API fxb_status fxb_last_timing(const fxb_ctx *ctx, float *fstage_ms, float *xmac_ms, float *total_ms);
 
-/* Per-subint kernel timing: every subint records four CUDA events on the
- * stream that runs it (event-record nodes of the graph when graphs are on);
+/* Per-subint kernel timing: every subint records CUDA events on the streams
+ * that run it (event-record nodes of the graph when graphs are on);
  * while timing is enabled their intervals are summed as slots come round
  * again.  fxb_timing_read synchronises and returns the number of subints
  * and the summed device time of the FP64 delay/parameter kernels (prep),
  * the F stage and the XMAC (with the FP8 quantisation and the weight
- * kernels), then clears the sums. */
+ * kernels), then clears the sums.  Preparation that ran beside earlier
+ * subints shares the device with their kernels, and its interval is longer
+ * by what it waits for them. */
 FXB_API fxb_status fxb_timing_enable(fxb_ctx *ctx, int32_t on);
 FXB_API fxb_status fxb_timing_read(fxb_ctx *ctx, int32_t *nsubint, double *prep_ms, double *fstage_ms,
                                    double *xmac_ms);
@@ -440,9 +444,11 @@ FXB_API void *fxb_host_alloc(size_t bytes, fxb_status *status);
 FXB_API void fxb_host_free(void *p);
 
 /* The cudaStream_t (as void*) on which the context launches its kernels,
- * so that callers can order their own work and events against it.  (A queue of
- * subints from host buffers may run preparation kernels on a stream of its own;
- * this stream waits for them.) */
+ * so that callers can order their own work and events against it.  A queue of
+ * subints may run preparation kernels beside earlier subints, on a stream of
+ * the context's own that this one waits for: of subints from host buffers
+ * always, from device buffers only in contexts whose stream was never asked
+ * for, since a caller may order the making of its buffers on it. */
 FXB_API fxb_status fxb_get_stream(const fxb_ctx *ctx, void **stream);
 
 /* As fxb_read_results, but the core result is written asynchronously (on
