@@ -859,17 +859,6 @@ static fxb_status setup_device(fxb_ctx *ctx)
 			k.cplx = (kv.first.second >> 5) & 1;
 			k.first = (int)hg.size();
 			k.count = (int)kv.second.size();
-			if(k.nb == 2)
-			{
-				k.pair0 = (int)pitems.size();
-				k.two = (kv.first.second >> 6) & 1;
-				if(k.two && ntwist == 0)
-					ctx->ptwist0 = k.pair0;
-				if(k.two)
-					ntwist += k.count;
-				for(int i = 0; i < k.count; i++)
-					pitems.push_back(pair_item(ctx, kv.second[i], k.first + i, out == 1));
-			}
 			// FFT iterations per CTA: as many as still leave two CTAs per SM
 			for(int tq : {4, 2, 1})
 			{
@@ -915,6 +904,18 @@ static fxb_status setup_device(fxb_ctx *ctx)
 					k.tcrec0 = (int64_t)ctx->tcrec_bytes;
 					ctx->tcrec_bytes += (fstage_tc_rec_bytes(k.tcnpairs, ctx->T) + 255) / 256 * 256;
 				}
+			}
+			// (the tensor-core FFT has records of its own)
+			if(k.nb == 2 && !k.tcfft)
+			{
+				k.pair0 = (int)pitems.size();
+				k.two = (kv.first.second >> 6) & 1;
+				if(k.two && ntwist == 0)
+					ctx->ptwist0 = k.pair0;
+				if(k.two)
+					ntwist += k.count;
+				for(int i = 0; i < k.count; i++)
+					pitems.push_back(pair_item(ctx, kv.second[i], k.first + i, out == 1));
 			}
 			{
 				std::vector<float2> h((size_t)k.twn);
