@@ -351,6 +351,46 @@ static void free_ctx(fxb_ctx *ctx)
 	delete ctx;
 }
 
+// XMAC launch groups: the subbands of equal rows and channels, by plan index.
+static std::vector<std::vector<int32_t>> subband_groups(const Job &job)
+{
+	std::vector<std::vector<int32_t>> out;
+	for(int f = 0; f < (int)job.plan.size(); f++)
+	{
+		const Job::FreqPlan &p = job.plan[f];
+		if(p.nrow <= 0)
+			continue;
+		auto g = std::find_if(out.begin(), out.end(), [&](const std::vector<int32_t> &idx) {
+			const Job::FreqPlan &q = job.plan[idx[0]];
+			return q.nrow == p.nrow && q.nchan == p.nchan && q.xmac == p.xmac;
+		});
+		if(g == out.end())
+			out.push_back({f});
+		else
+			g->push_back(f);
+	}
+	return out;
+}
+
+// Frames that a slot's validity arrays hold at first: those of a subint's buffers,
+// an eighth and a few more for windows with margins (longer buffers get larger
+// arrays when they come).
+static int64_t valid_frames(const Job &job)
+{
+	int64_t frames = 0;
+	for(const Job::Station &js : job.stations)
+	{
+		const double bits = (double)job.subint_ns * 1e-3 * 2.0 * job.freqs[js.band_freq[0]].bw_mhz * js.nbits * js.nband;
+		frames = std::max(frames, (int64_t)(bits / 8.0 / js.payload * 1.125) + 8);
+	}
+	return frames;
+}
+
+static size_t valid_bytes(int64_t frames, int S)
+{
+	return 2 * (((size_t)frames * S + 15) / 16 * 16) + sizeof(uint32_t) * frames * S;
+}
+
 // The slot's frame-validity arrays, for n frames a station.
 static cudaError_t alloc_valid(fxb_ctx *ctx, Slot &sl, int64_t n, cudaStream_t stream)
 {
@@ -363,7 +403,7 @@ static cudaError_t alloc_valid(fxb_ctx *ctx, Slot &sl, int64_t n, cudaStream_t s
 	sl.d_valid = nullptr;
 	sl.valid_stride = 0;
 	const size_t vbytes = ((size_t)n * ctx->S + 15) / 16 * 16;
-	const cudaError_t e = pool_alloc(ctx, (void **)&sl.d_valid, 2 * vbytes + sizeof(uint32_t) * n * ctx->S, stream);
+	const cudaError_t e = pool_alloc(ctx, (void **)&sl.d_valid, valid_bytes(n, ctx->S), stream);
 	if(e != cudaSuccess)
 		return e;
 	sl.d_bandok = (uint32_t *)(sl.d_valid + vbytes);
@@ -619,33 +659,13 @@ static fxb_status setup_device(fxb_ctx *ctx)
 	ctx->tc = job.xmac_kind == FXB_XMAC_BF16 || job.xmac_kind == FXB_XMAC_FP8 || job.xmac_kind == FXB_XMAC_FP16;
 	ctx->f8 = job.xmac_kind == FXB_XMAC_FP8;
 	ctx->h16 = job.xmac_kind == FXB_XMAC_FP16 || job.xmac_kind == FXB_XMAC_FP8;
-	std::vector<std::vector<int32_t>> gidx;
+	const std::vector<std::vector<int32_t>> gidx = subband_groups(job);
+	for(const std::vector<int32_t> &idx : gidx)
 	{
-		std::vector<int> used;
-		for(int f = 0; f < ctx->F; f++)
-			if(ctx->h_plans[f].nrow > 0) used.push_back(f);
-		std::vector<int> taken(used.size(), 0);
-		for(size_t i = 0; i < used.size(); i++)
-		{
-			if(taken[i]) continue;
-			const DevFreqPlan &a = ctx->h_plans[used[i]];
-			std::vector<int32_t> idx;
-			const bool ax = job.plan[used[i]].xmac;
-			for(size_t j = i; j < used.size(); j++)
-			{
-				const DevFreqPlan &b = ctx->h_plans[used[j]];
-				if(!taken[j] && b.nrow == a.nrow && b.nchan == a.nchan && job.plan[used[j]].xmac == ax)
-				{
-					taken[j] = 1;
-					idx.push_back(used[j]);
-				}
-			}
-			ctx->xgroups.emplace_back();
-			ctx->xgroups.back().plan0 = used[i];
-			ctx->xgroups.back().nf = (int)idx.size();
-			ctx->xgroups.back().xmac = ax;
-			gidx.push_back(idx);
-		}
+		ctx->xgroups.emplace_back();
+		ctx->xgroups.back().plan0 = idx[0];
+		ctx->xgroups.back().nf = (int)idx.size();
+		ctx->xgroups.back().xmac = job.plan[idx[0]].xmac;
 	}
 	// tensor-core form: bf16x2 spectra, per group one block
 	// [subband][Tpad][block][trow][CB] (times past T and rows past nrow stay zero), and
@@ -1106,15 +1126,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 
 	// staging slots
 	ctx->slots.resize(job.inflight);
-	// frames of a subint's buffers (an eighth and a few more for windows with
-	// margins; longer ones get a larger array when they come)
-	int64_t frames = 0;
-	for(int s = 0; s < ctx->S; s++)
-	{
-		const Job::Station &js = job.stations[s];
-		const double bits = (double)job.subint_ns * 1e-3 * 2.0 * job.freqs[js.band_freq[0]].bw_mhz * js.nbits * js.nband;
-		frames = std::max(frames, (int64_t)(bits / 8.0 / js.payload * 1.125) + 8);
-	}
+	const int64_t frames = valid_frames(job);
 	for(auto &sl : ctx->slots)
 	{
 		CK(ctx, alloc_valid(ctx, sl, frames, ctx->stream));
@@ -2005,32 +2017,79 @@ fxb_status fxb_job_footprint(const fxb_job_desc *desc, size_t *bytes)
 	}
 	const int64_t T = job.blockspersend;
 	const int S = (int)job.stations.size();
-	// two-band items, each with constants per FFT (two items a record in the tensor-core FFT)
-	int64_t pairs = 0;
-	for(const Job::Station &js : job.stations)
-		pairs += js.nband / 2;
-	// spectra (the blocked tensor-core layout pads times to 32 -- 64 for the
-	// e4m3 copy of the FP8 form -- and channels to whole blocks: at most
-	// +25 %), accumulators, core result, FFT parameters
-	const double pad32 = (double)((T + 31) / 32 * 32) / (double)std::max<int64_t>(T, 1);
-	const double pad64 = (double)((T + 63) / 64 * 64) / (double)std::max<int64_t>(T, 1);
-	double b = (double)job.spec_total * (job.xmac_kind == FXB_XMAC_FP32 ? 8.0
-	                                     : job.xmac_kind != FXB_XMAC_FP8 ? 4.0 * 1.25 * pad32
-	                                                                      : (4.0 * pad64 + 2.0 * pad64 + 0.5) * 1.25);
-	b += (double)job.acc_total * 8.0 + (double)job.corelen * 16.0 +
-	     (double)S * T * 68.0 * job.inflight + (double)pairs * T * 144.0 * (job.xmac_kind == FXB_XMAC_FP32 ? 1 : job.inflight) +
-	     (double)job.pcal_bins * 8.0 * pcal_plan_of(job, pcal_groups(job)).chunks;
-	// raw VDIF staging of the in-flight subints (payload plus headers, 1/8 slack)
-	for(int s = 0; s < S; s++)
+	int dev = 0, nsm = 148;
+	if(cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
 	{
-		const Job::Station &js = job.stations[s];
+		cudaGetLastError();
+		nsm = 148;
+	}
+	// spectra: the tensor-core forms' blocks with their padded times, rows and
+	// channels, the FP8 form's copy and scales, the sums of the time slices
+	const bool f8 = job.xmac_kind == FXB_XMAC_FP8, h16 = f8 || job.xmac_kind == FXB_XMAC_FP16;
+	const bool tc = f8 || h16 || job.xmac_kind == FXB_XMAC_BF16;
+	double b = tc ? 0.0 : (double)job.spec_total * 8.0;
+	for(const std::vector<int32_t> &idx : subband_groups(job))
+	{
+		const Job::FreqPlan &p = job.plan[idx[0]];
+		int maxout = 0;
+		for(int32_t f : idx)
+		{
+			maxout = std::max(maxout, job.plan[f].nout);
+			b += 8.0 * p.nrow * p.nrow + 4.0 * job.plan[f].nout;
+		}
+		TcShape sh;
+		if(!tc || !tc_shape(p.nrow, p.nchan, (int)idx.size(), (int)T, nsm, f8, h16, &sh))
+			continue;
+		const double blocks = (double)((p.nchan + sh.CB - 1) / sh.CB) * sh.Tpad * (double)idx.size();
+		b += blocks * sh.trow * sh.CB * 4.0;
+		if(f8)
+			b += blocks * sh.w8 * 2.0 + (double)idx.size() * p.nchan * p.nrow * 4.0;
+		if(p.xmac)
+			b += (double)tc_workspace(sh, (int)idx.size(), maxout) * 8.0;
+	}
+	b += (double)job.acc_total * 8.0 + (double)job.corelen * 8.0 + (double)job.outmap.size() * sizeof(DevOutMap) +
+	     (double)(job.bweights.size() + job.acweights.size()) * (sizeof(DevWeightOut) + sizeof(DevWeightSum) + 4.0) +
+	     (double)job.pcal_bins * 8.0 * pcal_plan_of(job, pcal_groups(job)).chunks;
+	// the work items' constants per FFT: once per context in the CUDA-core F stage
+	// (and their work list), per slot and two items a record in the tensor-core FFT
+	int nbm = 0;
+	for(const Job::Station &js : job.stations)
+		nbm = std::max(nbm, js.mux_threads > 0 ? js.nband : 0);
+	for(const Job::Station &js : job.stations)
+	{
+		std::map<int, int> bands;                 // of each recorded subband
+		for(int f : js.band_freq)
+			bands[f]++;
+		int both = 0, single = 0;
+		for(const auto &kv : bands)
+		{
+			both += kv.second / 2;
+			single += kv.second % 2;
+		}
+		// single bands of two subbands share an item, with twists
+		const double pairs = (double)T * ((both + single / 2) * (sizeof(PairConst) + sizeof(FsMultiUnit) / 4) +
+		                                  single / 2 * sizeof(PairTwist));
+		const double recs = (double)job.inflight * fstage_tc_rec_bytes((both + single + 2) / 2, (int)T);
+		const bool rec = tc && !js.cplx && nbm == 0 && js.nbits == 2 && 2 * job.freqs[js.band_freq[0]].nchan == 2048;
+		b += rec ? std::max(pairs, recs) : pairs;
+	}
+	// the in-flight subints: FFT parameters and weights, frame validity, records,
+	// raw VDIF (payload plus headers, 1/8 slack) and raw reads' tables
+	b += (double)job.inflight * ((double)S * T * (sizeof(FftParam) + 4.0 + 4.0 * nbm) + valid_bytes(valid_frames(job), S) +
+	                             (double)S * (sizeof(DevSubintStation) + (T / kFlagsPerInt + 1) * 4.0));
+	for(const Job::Station &js : job.stations)
+	{
 		const fxb_freq &f = job.freqs[js.band_freq[0]];
 		const double sps = 2.0 * f.bw_mhz * 1e6;
+		// a read of threads has a header for each thread's frame
+		const int header = js.mux_raw ? 32 * js.mux_threads : js.header;
 		const double per = (double)job.subint_ns * 1e-9 * sps * js.nbits * js.nband / 8.0 *
-		                   (double)(js.payload + js.header) / js.payload;
-		b += job.inflight * (per * 1.125 + 2.0 * (js.payload + js.header) + 4096.0);
+		                   (double)(js.payload + header) / js.payload;
+		b += job.inflight * (per * 1.125 + 2.0 * (js.payload + header) + 4096.0);
+		if(js.mux_raw)
+			b += job.inflight * (per / (js.payload + header) + 2.0) * (16.0 * js.mux_threads + 64.0);
 	}
-	b += 16.0 * 1024 * 1024;           // plans, tables, validity bytes, alignment
+	b += 8.0 * 1024 * 1024;            // plans, twiddles, alignment
 	*bytes = (size_t)b;
 	return FXB_OK;
 }
