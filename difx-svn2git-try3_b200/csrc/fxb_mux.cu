@@ -22,11 +22,13 @@
 //                  word of every thread and writing nthreads output words.
 // Byte work: HBM-bound by design (every payload byte read once, written once).
 
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <type_traits>
 
 #include "fxb_internal.h"
 #include "fxb_kernels.h"
@@ -605,30 +607,78 @@ void launch_mux_raw(const DevStation *st, DevSubintStation *sub, int S, int maxs
 	k_mr_fix<<<(S + 63) / 64, 64, 0, stream>>>(st, sub, S);
 }
 
+// Unique id of the device's primary context; 0: it is not active or, with mine, not
+// the calling thread's context.  Makes no context.
+static unsigned long long primary_context(int dev, bool mine)
+{
+	struct Api {
+		CUresult (*current)(CUcontext *) = nullptr;
+		CUresult (*state)(CUdevice, unsigned *, int *) = nullptr;
+		CUresult (*retain)(CUcontext *, CUdevice) = nullptr;
+		CUresult (*release)(CUdevice) = nullptr;
+		CUresult (*id)(CUcontext, unsigned long long *) = nullptr;
+		bool ok = false;
+		Api()
+		{
+			auto get = [](const char *name, auto &fn) {
+				void *p = nullptr;
+				cudaDriverEntryPointQueryResult q;
+				const bool found = cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess &&
+				                   q == cudaDriverEntryPointSuccess;
+				fn = (std::remove_reference_t<decltype(fn)>)p;
+				return found;
+			};
+			ok = get("cuCtxGetCurrent", current) && get("cuDevicePrimaryCtxGetState", state) &&
+			     get("cuDevicePrimaryCtxRetain", retain) && get("cuDevicePrimaryCtxRelease", release) && get("cuCtxGetId", id);
+			if(!ok)
+				cudaGetLastError();
+		}
+	};
+	static const Api api;
+	CUcontext cur = nullptr, prim = nullptr;
+	unsigned flags = 0;
+	int active = 0;
+	unsigned long long id = 0;
+	if(!api.ok || api.state(dev, &flags, &active) != CUDA_SUCCESS || !active ||
+	   (mine && api.current(&cur) != CUDA_SUCCESS) || api.retain(&prim, dev) != CUDA_SUCCESS)
+		return 0;
+	const bool ok = (!mine || prim == cur) && api.id(prim, &id) == CUDA_SUCCESS;
+	api.release(dev);
+	return ok ? id : 0;
+}
+
 // The calls' tables come from a pool of the calling thread, one per device, that
 // keeps up to 4 MB mapped between calls and goes with the thread: the default pool
 // gives its memory back at every synchronisation, and mapping it again took from
 // 20 us to tens of milliseconds of a 0.1 ms call (1000 frames of 16 threads: 99 to
-// 617 us a call from run to run, with this pool 91 to 99).
+// 617 us a call from run to run, with this pool 91 to 99; the first call on a
+// thread makes the pool).  A pool belongs to the context it was made in: after a
+// reset of the device it is left alone and another made.
 static cudaMemPool_t mux_pool()
 {
 	constexpr int kMaxDevices = 64;
 	struct Pools {
 		cudaMemPool_t p[kMaxDevices] = {};
+		unsigned long long ctx[kMaxDevices] = {};
 		~Pools()
 		{
 			// frees in flight complete first, the driver sees to that
-			for(cudaMemPool_t q : p)
-				if(q)
-					cudaMemPoolDestroy(q);
+			for(int d = 0; d < kMaxDevices; d++)
+				if(p[d] && primary_context(d, false) == ctx[d])
+					cudaMemPoolDestroy(p[d]);
 		}
 	};
 	static thread_local Pools pools;
 	int dev = 0;
 	if(cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices)
 		return nullptr;
-	if(!pools.p[dev])
+	// (the free brings the context up on the thread's first call)
+	const unsigned long long ctx = cudaFree(nullptr) == cudaSuccess ? primary_context(dev, true) : 0;
+	if(!ctx)
+		return nullptr;
+	if(!pools.p[dev] || pools.ctx[dev] != ctx)
 	{
+		pools.p[dev] = nullptr;
 		cudaMemPoolProps props;
 		memset(&props, 0, sizeof(props));
 		props.allocType = cudaMemAllocationTypePinned;
@@ -643,6 +693,7 @@ static cudaMemPool_t mux_pool()
 		}
 		cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
 		pools.p[dev] = p;
+		pools.ctx[dev] = ctx;
 	}
 	return pools.p[dev];
 }
