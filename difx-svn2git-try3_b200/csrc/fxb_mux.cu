@@ -3,7 +3,7 @@
 // DataStream runs on every read of an INTERLACEDVDIF stream before its frames
 // reach Mode.  One call takes one read: nin frames of the wanted threads
 // (interleaved in any order, other threads skipped) and writes nin / nthreads
-// output frames of nthreads channels each, in three launches:
+// output frames of nthreads channels each, in four launches:
 //   k_mux_index    every input frame finds its place: frame slot (time since
 //                  the first frame of the read, in frames) and thread
 //                  (VDIFMuxer::deinterlace, datamuxer.cpp:765-846); where a
@@ -216,11 +216,45 @@ __global__ void k_mux_headers(const MuxArgs a, int32_t *outidx)
 		a.status[1] = a.nproc - k0;
 }
 
+// NT words side by side, by the alignment of the output (MuxArgs::vec)
+template <int NT>
+__device__ __forceinline__ void store_words(uint32_t *dst, const uint32_t *w, int vec)
+{
+	if constexpr(NT >= 8)
+		if(vec == 2)
+		{
+#pragma unroll
+			for(int j = 0; j < NT; j += 8)
+				asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(dst + j), "r"(w[j]),
+				             "r"(w[j + 1]), "r"(w[j + 2]), "r"(w[j + 3]), "r"(w[j + 4]), "r"(w[j + 5]), "r"(w[j + 6]),
+				             "r"(w[j + 7])
+				             : "memory");
+			return;
+		}
+	if constexpr(NT >= 4)
+		if(vec)
+		{
+#pragma unroll
+			for(int j = 0; j < NT; j += 4)
+				*(uint4 *)(dst + j) = make_uint4(w[j], w[j + 1], w[j + 2], w[j + 3]);
+			return;
+		}
+#pragma unroll
+	for(int j = 0; j < NT; j++)
+		dst[j] = w[j];
+}
+
 // Corner turn: x = input word, y = slot; output word (i nthreads + j) of the
 // slot's output frame packs, for k < spow and thread l, sample j spow + k of
 // thread l at bit (k nthreads + l) nbits.  The general form, field by field, for
 // any thread count up to kMaxMuxThreads and any field width.
-__global__ void k_mux_turn(const MuxArgs a, const int32_t *outidx)
+// NT > 0: the thread count, known to the compiler, so that the words stay in
+// registers (an array of run-time bounds lies in local memory: a whole call of 1
+// thread x 8000 frames of 8000 bytes 425 us, 2 x 16 bits x 4000 199 us, 8 x 3 bits x
+// 1000 180 us; in registers 180, 152
+// and 141 us).  One thread: nothing moves.
+template <int NT>
+__global__ void __launch_bounds__(128) k_mux_turn(const MuxArgs a, const int32_t *outidx)
 {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	const int k = blockIdx.y;
@@ -229,21 +263,37 @@ __global__ void k_mux_turn(const MuxArgs a, const int32_t *outidx)
 	const int o = outidx[k];
 	if(o < 0)
 		return;
-	const int nt = a.nthreads;
+	const int nt = NT > 0 ? NT : a.nthreads;
 	const int32_t *sl = a.slot + (int64_t)k * nt;
-	uint32_t w[kMaxMuxThreads];
+	uint32_t w[NT > 0 ? NT : kMaxMuxThreads];
 #pragma unroll
-	for(int l = 0; l < nt; l++)
+	for(int l = 0; l < (NT > 0 ? NT : nt); l++)
 		w[l] = __ldg((const uint32_t *)(a.in + (int64_t)sl[l] * a.inframebytes + 32) + i);
-	const uint32_t mask = (1u << a.nbits) - 1u;
 	uint32_t *dst = (uint32_t *)(a.out + (int64_t)o * a.outframebytes + 32) + (int64_t)i * nt;
-	for(int j = 0; j < nt; j++)
+	if constexpr(NT == 1)
 	{
-		uint32_t word = 0u;
-		for(int kk = 0; kk < a.spow; kk++)
-			for(int l = 0; l < nt; l++)
-				word |= ((w[l] >> ((j * a.spow + kk) * a.nbits)) & mask) << ((kk * nt + l) * a.nbits);
-		dst[j] = word;
+		const int bits = a.spow * a.nbits;
+		dst[0] = bits < 32 ? w[0] & ((1u << bits) - 1u) : w[0];
+	}
+	else
+	{
+		const uint32_t mask = (1u << a.nbits) - 1u;
+		uint32_t v[NT > 0 ? NT : 1];
+#pragma unroll
+		for(int j = 0; j < (NT > 0 ? NT : nt); j++)
+		{
+			uint32_t word = 0u;
+			for(int kk = 0; kk < a.spow; kk++)
+#pragma unroll
+				for(int l = 0; l < (NT > 0 ? NT : nt); l++)
+					word |= ((w[l] >> ((j * a.spow + kk) * a.nbits)) & mask) << ((kk * nt + l) * a.nbits);
+			if constexpr(NT > 0)
+				v[j] = word;
+			else
+				dst[j] = word;
+		}
+		if constexpr(NT > 0)
+			store_words<NT>(dst, v, a.vec);
 	}
 }
 
@@ -322,53 +372,32 @@ __global__ void __launch_bounds__(128) k_mux_shuffle(const MuxArgs a, const int3
 				w[l] ^= t ^ (t << d);
 			}
 		}
-	uint32_t *dst = (uint32_t *)(a.out + (int64_t)o * a.outframebytes + 32) + (int64_t)i * NT;
-	if constexpr(NT >= 8)
-		if(a.vec == 2)
-		{
-#pragma unroll
-			for(int j = 0; j < NT; j += 8)
-				asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};\n" ::"l"(dst + j), "r"(w[j]),
-				             "r"(w[j + 1]), "r"(w[j + 2]), "r"(w[j + 3]), "r"(w[j + 4]), "r"(w[j + 5]), "r"(w[j + 6]),
-				             "r"(w[j + 7])
-				             : "memory");
-			return;
-		}
-	if constexpr(NT >= 4)
-		if(a.vec)
-		{
-#pragma unroll
-			for(int j = 0; j < NT; j += 4)
-				*(uint4 *)(dst + j) = make_uint4(w[j], w[j + 1], w[j + 2], w[j + 3]);
-			return;
-		}
-#pragma unroll
-	for(int j = 0; j < NT; j++)
-		dst[j] = w[j];
+	store_words<NT>((uint32_t *)(a.out + (int64_t)o * a.outframebytes + 32) + (int64_t)i * NT, w, a.vec);
 }
 
+// 2, 4, 8 or 16 threads: the permutation for fields of 1, 2, 4 and 8 bits, field by
+// field for other widths (at most 2 bits of 16 threads, 4 of 8, 8 of 4)
 template <int NT>
-static bool launch_shuffle(const MuxArgs &a, dim3 grid, const int32_t *outidx, cudaStream_t st)
+static void launch_turn(const MuxArgs &a, dim3 grid, const int32_t *outidx, cudaStream_t st)
 {
-	switch(a.nbits)
+	if(a.nbits == 1)
+		k_mux_shuffle<NT, 1><<<grid, 128, 0, st>>>(a, outidx);
+	else if(a.nbits == 2)
+		k_mux_shuffle<NT, 2><<<grid, 128, 0, st>>>(a, outidx);
+	else if constexpr(NT <= 8)
 	{
-	case 1: k_mux_shuffle<NT, 1><<<grid, 128, 0, st>>>(a, outidx); return true;
-	case 2: k_mux_shuffle<NT, 2><<<grid, 128, 0, st>>>(a, outidx); return true;
-	case 4:
-		if constexpr(NT <= 8)
+		if(a.nbits == 4)
 		{
 			k_mux_shuffle<NT, 4><<<grid, 128, 0, st>>>(a, outidx);
-			return true;
+			return;
 		}
-		return false;
-	case 8:
 		if constexpr(NT <= 4)
-		{
-			k_mux_shuffle<NT, 8><<<grid, 128, 0, st>>>(a, outidx);
-			return true;
-		}
-		return false;
-	default: return false;
+			if(a.nbits == 8)
+			{
+				k_mux_shuffle<NT, 8><<<grid, 128, 0, st>>>(a, outidx);
+				return;
+			}
+		k_mux_turn<NT><<<grid, 128, 0, st>>>(a, outidx);
 	}
 }
 
@@ -764,17 +793,15 @@ fxb_status vdif_mux(const uint8_t *dev_in, int64_t inbytes, int32_t nthreads, co
 			k_mux_first<<<(nproc + 255) / 256, 256, 0, st>>>(a);
 			k_mux_headers<<<(nproc + 127) / 128, 128, 0, st>>>(a, outidx);
 			const dim3 grid((a.wordsin + 127) / 128, nproc);
-			bool done = false;
 			switch(nthreads)
 			{
-			case 2: done = launch_shuffle<2>(a, grid, outidx, st); break;
-			case 4: done = launch_shuffle<4>(a, grid, outidx, st); break;
-			case 8: done = launch_shuffle<8>(a, grid, outidx, st); break;
-			case 16: done = launch_shuffle<16>(a, grid, outidx, st); break;
-			default: break;
+			case 1: k_mux_turn<1><<<grid, 128, 0, st>>>(a, outidx); break;
+			case 2: launch_turn<2>(a, grid, outidx, st); break;
+			case 4: launch_turn<4>(a, grid, outidx, st); break;
+			case 8: launch_turn<8>(a, grid, outidx, st); break;
+			case 16: launch_turn<16>(a, grid, outidx, st); break;
+			default: k_mux_turn<0><<<grid, 128, 0, st>>>(a, outidx); break;
 			}
-			if(!done)
-				k_mux_turn<<<grid, 128, 0, st>>>(a, outidx);
 		}
 		ok = cudaGetLastError() == cudaSuccess &&
 		     cudaMemcpyAsync(hst, a.status, sizeof(hst), cudaMemcpyDeviceToHost, st) == cudaSuccess &&

@@ -13,7 +13,9 @@ pytestmark = pytest.mark.gpu
 
 CASES = [(nt, nb, 1000, 0) for nt in (2, 4, 8, 16) for nb in (1, 2, 4, 8) if nt * nb <= 32] + \
         [(1, 2, 1000, 0), (3, 2, 1000, 0), (5, 4, 1000, 0), (32, 1, 1000, 0), (16, 2, 8, 0), (16, 2, 520, 16),
-         (16, 2, 24, 4), (8, 2, 40, 16), (4, 2, 5000, 4)]
+         (16, 2, 24, 4), (8, 2, 40, 16), (4, 2, 5000, 4)] + \
+        [(1, 1, 1000, 0), (1, 3, 1000, 4), (1, 16, 40, 0), (2, 16, 1000, 0), (2, 3, 1000, 4), (4, 6, 1008, 0),
+         (4, 7, 1000, 4), (8, 3, 992, 0), (8, 3, 1000, 16)]
 
 
 @pytest.mark.parametrize("nthreads,nbits,payload,off", CASES)
