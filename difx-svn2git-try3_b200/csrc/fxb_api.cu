@@ -468,7 +468,7 @@ static PairItem pair_item(const fxb_ctx *ctx, const FGroup &g, int group, bool t
 	PairItem u;
 	memset(&u, 0, sizeof(u));
 	u.tcb = tc ? (uint32_t)P.tcb : 0u;
-	u.magic = tc ? 0xFFFFFFFFu / u.tcb + 1u : 0u;
+	u.magic = P.magic;
 	u.bextra = tc ? (uint32_t)(P.trow - 1) * u.tcb : 0u;
 	u.pbits = tc ? P.pbits : 0;
 	const int rstr = tc ? P.tcb : nchan;
@@ -696,6 +696,7 @@ static fxb_status setup_device(fxb_ctx *ctx)
 				isoff[gidx[gi][i]] = ctx->iscale_elems;
 				ctx->iscale_elems += (int64_t)d.nchan * d.nrow;
 				d.tcb = g.shape.CB;
+				d.magic = 0xFFFFFFFFu / (uint32_t)d.tcb + 1u;
 				d.tnblk = nblk;
 				d.trow = g.shape.trow;
 				for(d.pbits = 0; (4 << d.pbits) < d.nchan; d.pbits++)

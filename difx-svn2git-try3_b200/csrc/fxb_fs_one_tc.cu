@@ -29,10 +29,11 @@ static void launch_t(const FKind &k, const FsArgs &a, cudaStream_t stream)
 	k_fstage<LOGN, TCO, VAR><<<fstage_grid(k, a), k.threads, k.smem, stream>>>(a);
 }
 
-constexpr size_t kNarrowSide = 36864;            // exchange buffer: 4096 points of one band, padded
+constexpr size_t kNarrowSide = 18432;            // exchange buffer: 2048 points of one band, padded
+constexpr size_t kMidSide = 36864;               // 4096 points
 constexpr size_t kWideSmem = 73728;              // 8192 points of one band, padded
 
-// Work-list class 5 VAR + 4: every length up to 4096 points in CTAs of 256
+// Work-list class 6 VAR + 5: every length up to 2048 points in CTAs of 256
 // threads (the shape of k_fstage for those lengths), one exchange buffer per
 // unit (three CTAs per SM): faster than two buffers at two CTAs per SM on every
 // length measured.  VAR 0: plain VDIF, 1: raw INTERLACEDVDIF reads.
@@ -43,7 +44,7 @@ __global__ void __launch_bounds__(256, 3) k_fstage_pn(const __grid_constant__ Fs
 	__shared__ float lut8[256];
 	__shared__ FftConst fcs[kFsMultiFc];
 	__shared__ int unit_s[2];
-	constexpr int cls = kFsMultiPer * VAR + 4;
+	constexpr int cls = kFsMultiPer * VAR + 5;
 	fstage_luts(lut8);
 	UnitFeed feed(m.ctr + cls, unit_s);
 	for(int u = feed.first(); u < m.nunit[cls]; u = feed.next())
@@ -61,49 +62,47 @@ __global__ void __launch_bounds__(256, 3) k_fstage_pn(const __grid_constant__ Fs
 		case 9: fstage_unit<9, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, 0, tw, fsm, lut8, fcs); break;
 		case 10: fstage_unit<10, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, 0, tw, fsm, lut8, fcs); break;
 		case 11: fstage_unit<11, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, 0, tw, fsm, lut8, fcs); break;
-		case 12: fstage_unit<12, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, 0, tw, fsm, lut8, fcs); break;
 		default: break;
 		}
 	}
 }
 
-// work-list class 5 VAR + 1: 8192 points in CTAs of 512 threads
-template <int VAR>
-__global__ void __launch_bounds__(512, 2) k_fstage_pw(const __grid_constant__ FsMultiArgs m)
+// 4096 points (class 6 VAR + 3) in CTAs of 256 threads, 8192 (class 6 VAR + 1) of 512
+template <int VAR, int LOGN>
+__global__ void __launch_bounds__(FShape<LOGN>::NT, LOGN == 12 ? 3 : 2) k_fstage_pw(const __grid_constant__ FsMultiArgs m)
 {
 	extern __shared__ __align__(16) uint2 fsm[];
 	__shared__ float lut8[256];
 	__shared__ FftConst fcs[kMaxTQ];
 	__shared__ int unit_s[2];
-	constexpr int cls = kFsMultiPer * VAR + 1;
+	constexpr int cls = kFsMultiPer * VAR + (LOGN == 12 ? 3 : 1);
 	fstage_luts(lut8);
 	UnitFeed feed(m.ctr + cls, unit_s);
 	for(int u = feed.first(); u < m.nunit[cls]; u = feed.next())
 	{
 		const FsMultiUnit w = m.units[m.unit0[cls] + u];
 		const FsMultiKind k = m.kinds[w.kind];
-		fstage_unit<13, true, VAR>(m.m[k.member], k.first + w.item, w.tchunk, k.tq, 0, (const float2 *)k.tw, fsm, lut8, fcs);
+		fstage_unit<LOGN, true, VAR>(m.m[k.member], k.first + w.item, w.tchunk, k.tq, 0, (const float2 *)k.tw, fsm, lut8, fcs);
 	}
 }
 
 template <int VAR>
-static void narrow(const FsMultiArgs &m, int nsm, cudaStream_t st)
+static void launch_cls(const FsMultiArgs &m, int c, int nsm, cudaStream_t st)
 {
-	fs_launch_persistent(k_fstage_pn<VAR>, m, kFsMultiPer * VAR + 4, 3 * nsm, 256, kNarrowSide, st);
-}
-template <int VAR>
-static void wide(const FsMultiArgs &m, int nsm, cudaStream_t st)
-{
-	fs_launch_persistent(k_fstage_pw<VAR>, m, kFsMultiPer * VAR + 1, 2 * nsm, 512, kWideSmem, st);
+	if(c == 5)
+		fs_launch_persistent(k_fstage_pn<VAR>, m, kFsMultiPer * VAR + c, 3 * nsm, 256, kNarrowSide, st);
+	else if(c == 3)
+		fs_launch_persistent(k_fstage_pw<VAR, 12>, m, kFsMultiPer * VAR + c, 3 * nsm, 256, kMidSide, st);
+	else
+		fs_launch_persistent(k_fstage_pw<VAR, 13>, m, kFsMultiPer * VAR + c, 2 * nsm, 512, kWideSmem, st);
 }
 
 void launch_fs_one_multi(const FsMultiArgs &m, int cls, int nsm, cudaStream_t st)
 {
-	const bool raw = cls >= kFsMultiPer;
-	if(cls % kFsMultiPer == 1)
-		raw ? wide<1>(m, nsm, st) : wide<0>(m, nsm, st);
+	if(cls >= kFsMultiPer)
+		launch_cls<1>(m, cls - kFsMultiPer, nsm, st);
 	else
-		raw ? narrow<1>(m, nsm, st) : narrow<0>(m, nsm, st);
+		launch_cls<0>(m, cls, nsm, st);
 }
 
 void launch_fs_one_tc(const FKind &k, const FsArgs &a, cudaStream_t stream)

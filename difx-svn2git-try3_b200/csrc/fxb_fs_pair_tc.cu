@@ -35,7 +35,7 @@ static void launch_t(const FKind &k, const FsArgs &a, cudaStream_t stream)
 
 constexpr size_t kPairSide = 2304 * 16;          // exchange buffers of 2048 points in all, padded
 
-// Work-list class 5 VAR + 3: every length up to 2048 points in CTAs of 256
+// Work-list class 6 VAR + 4: every length up to 2048 points in CTAs of 256
 // threads.  VAR 0: plain VDIF, 1: raw INTERLACEDVDIF reads.
 template <int VAR>
 __global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant__ FsMultiArgs m)
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant
 	__shared__ u64 lut4[16];
 	__shared__ PairFeed<kFsMultiFc> feed;
 	fstage_pair_luts(lut8, lut4);
-	pair_units(feed, m, kFsMultiPer * VAR + 3,
+	pair_units(feed, m, kFsMultiPer * VAR + 4,
 	           [&](const FsMultiUnit &w, const PairItem &I, const PairConst *fcs, const PairTwist *tws) {
 		const FsMultiKind &k = m.kinds[w.kind];
 		const float2 *tw = (const float2 *)k.tw;
@@ -70,7 +70,7 @@ __global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant
 	});
 }
 
-// 4096 points (class 5 VAR + 2) in CTAs of 512 threads, 8192 (class 5 VAR) of 1024
+// 4096 points (class 6 VAR + 2) in CTAs of 512 threads, 8192 (class 6 VAR) of 1024
 template <int VAR, int LOGN>
 __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB)
     k_fstage_pair_pw(const __grid_constant__ FsMultiArgs m)
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB)
 template <int VAR>
 static void launch_cls(const FsMultiArgs &m, int c, int nsm, cudaStream_t st)
 {
-	if(c == 3)
+	if(c == 4)
 		fs_launch_persistent(k_fstage_pair_pn<VAR>, m, kFsMultiPer * VAR + c, 3 * nsm, 256, kPairSide, st);
 	else if(c == 2)
 		fs_launch_persistent(k_fstage_pair_pw<VAR, 12>, m, kFsMultiPer * VAR + c, 2 * nsm, 512, 2 * kPairSide, st);

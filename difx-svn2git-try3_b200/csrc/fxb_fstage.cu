@@ -36,8 +36,8 @@ int fstage_multi_class(int N, int nb)
 	if(N < 32 || N > 8192)
 		return -1;
 	if(nb == 2)
-		return N == 8192 ? 0 : (N == 4096 ? 2 : 3);
-	return N == 8192 ? 1 : 4;
+		return N == 8192 ? 0 : (N == 4096 ? 2 : 4);
+	return N == 8192 ? 1 : (N == 4096 ? 3 : 5);
 }
 
 int fstage_multi_tq(int N, int nb, int tq)
@@ -63,9 +63,8 @@ cudaError_t launch_fstage_multi_on(const FsMultiArgs &m, int nsm, const cudaStre
 	{
 		if(m.nunit[cls] <= 0)
 			continue;
-		const int c = cls % kFsMultiPer;
 		cudaStream_t st = streams[(next++) % nstream];
-		if(c == 1 || c == 4)
+		if((cls % kFsMultiPer) & 1)
 			launch_fs_one_multi(m, cls, nsm, st);
 		else
 			launch_fs_pair_multi(m, cls, nsm, st);

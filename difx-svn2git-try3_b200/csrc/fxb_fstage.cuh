@@ -197,6 +197,35 @@ __device__ __forceinline__ uint32_t pack_spec(bool h16, float re, float im)
 	return *(const uint32_t *)&b;
 }
 
+// Tensor-core form: the four channels of positions p0 .. p0 + 3 (a multiple of 4)
+// of one row of a time's blocks [block][trow][tcb], o its first.  tcb is even;
+// bextra = (trow - 1) tcb lies between the end of a block's run of the row and the
+// next block's, and p / tcb = umulhi(p, magic) for p < 2^16.
+__device__ __forceinline__ void store_quad(uint32_t *o, uint32_t p0, uint32_t tcb, uint32_t magic, uint32_t bextra,
+                                           uint4 h)
+{
+	uint32_t *q = o + p0 + __umulhi(p0, magic) * bextra;
+	if(tcb & 2u)
+	{
+		*(uint2 *)q = make_uint2(h.x, h.y);
+		*(uint2 *)(o + p0 + 2u + __umulhi(p0 + 2u, magic) * bextra) = make_uint2(h.z, h.w);
+	}
+	else
+		*(uint4 *)q = h;
+}
+
+// A row of the tensor-core spectra: its first value of time 0 and the step of a time
+struct OutRow {
+	int64_t first;
+	int32_t tstride;
+	uint32_t tcb, magic, bextra;
+};
+__device__ __forceinline__ OutRow out_row(const DevFreqPlan &P, int row)
+{
+	return {P.spec_off + (int64_t)max(row, 0) * P.tcb, P.tnblk * P.trow * P.tcb, (uint32_t)P.tcb, P.magic,
+	        (uint32_t)(P.trow - 1) * (uint32_t)P.tcb};
+}
+
 // CTAs per SM the register budget is sized for
 template <int LOGN>
 constexpr int fstage_minb()
@@ -335,11 +364,6 @@ __device__ __forceinline__ void fstage_unit(const FsArgs &a, const int gidx, con
 	uint2 *const side0 = fsm + (size_t)slot * PADN;
 	uint2 *const side1 = pp ? side0 + (size_t)FPC * PADN : side0;
 	const uint8_t *vrow = a.valid + (int64_t)g.station * a.valid_stride;
-	const int64_t spec_off = a.plans[g.freq].spec_off;
-	const int prow = a.plans[g.freq].tcb ? a.plans[g.freq].trow : a.plans[g.freq].nrow, pbits = a.plans[g.freq].pbits;
-	// tensor-core form: spectra blocked [t][block][row][tcb] (tcb channels per block)
-	const uint32_t tcb = (uint32_t)a.plans[g.freq].tcb, tnblk = (uint32_t)a.plans[g.freq].tnblk;
-	const uint32_t tcb_magic = tcb ? 0xFFFFFFFFu / tcb + 1u : 0u;    // c / tcb = umulhi(c, magic) for c < 2^16
 	const bool lsb = g.lsb != 0;
 	const double lo = g.lofreq;
 	const float ph0 = g.phase[0];                      // phase-offset rotation (turns)
@@ -348,6 +372,11 @@ __device__ __forceinline__ void fstage_unit(const FsArgs &a, const int gidx, con
 	const int order = a.order;
 	constexpr float osc = 1.0f / (float)(1 << kTcSpecExp);
 	const bool h16 = a.h16 != 0;
+
+	// where registers are short, read again at each FFT's output
+	OutRow out = {};
+	if constexpr(TCO && N > 8192)
+		out = out_row(a.plans[g.freq], row0);
 
 	const int t0 = tchunk * tq * FPC;
 	const int nit = min(tq, (a.T - t0 + FPC - 1) / FPC);
@@ -595,91 +624,172 @@ __device__ __forceinline__ void fstage_unit(const FsArgs &a, const int gidx, con
 			constexpr int J = (KB * 8) / RL;
 			const uint2 *src = wb ? side1 : side0;
 			wb ^= 1;
-			const int64_t obase = spec_off + (int64_t)t * prow * nchan;
-#pragma unroll
-			for(int jj = 0; jj < J; jj++)
-			{
-				const int q = bt + jj * TPF;
-				cf y[RL];
-#pragma unroll
-				for(int r = 0; r < RL; r++)
-					y[r] = lds(src + st_index<sL, (N >= 8192)>(q, r));
-				dftR<RL>(y);
-				if(!tok)
-					continue;
-#pragma unroll
-				for(int r = 0; r < RL; r++)
+			// one value: fractional-sample (and order-0 fringe) rotation of effective
+			// channel ce, y conjugated when cj < 0
+			auto turned = [&](cf y, int ce, float cj) {
+				const float fce = (float)ce;
+				float th = fce * dhi;               // exact (split_turns)
+				th -= rintf(th);
+				float turns = th + fmaf(fce, dlo, postf + ph0);
+				turns -= rintf(turns);
+				float sn, cs;
+				__sincosf(6.283185307179586f * turns, &sn, &cs);
+				const float xr = y.x, xi = cj * y.y;
+				if constexpr(TCO)
 				{
-					const int k = q + sL * r;
-					int c, ce;
-					float cj = 1.0f;
+					cs *= osc;
+					sn *= osc;
+				}
+				return cf{xr * cs - xi * sn, xr * sn + xi * cs};
+			};
+			// the sideband: order-0 lower bands (and complex ones) mirror their bins
+			const bool mirror = lsb && order == 0;
+			if constexpr(TCO)
+			{
+				// A thread's outputs are N/8 apart, bins q0 + m N/8: the channels of a quad
+				// of positions (chan_pos), stored at once.  One by one, a warp's 4-byte
+				// stores met 32 sectors each: 14 stations x 1 band, 8 bits, F stage of 8192
+				// channels 860 us and 600 now, of 4096 275 and 230, of 2048 (with a launch
+				// of its own) 150 and 124, of 1024 82 and 82, of 256 54 and 49
+				constexpr int JG = 8 / RL;
+				const OutRow O = N > 8192 ? out : out_row(a.plans[g.freq], row0);
+				uint32_t *const orow = (uint32_t *)a.spec + O.first + (int64_t)t * O.tstride;
+				auto packed = [&](cf y, int ce, float cj) {
+					const cf v = turned(y, ce, cj);
+					return pack_spec(h16, v.x, v.y);
+				};
+				auto quad = [&](uint32_t p0, uint32_t h0, uint32_t h1, uint32_t h2, uint32_t h3) {
+					store_quad(orow, p0, O.tcb, O.magic, O.bextra, make_uint4(h0, h1, h2, h3));
+				};
+#pragma unroll 1
+				for(int kb = 0; kb < KB; kb++)
+				{
+					const int q0 = bt + kb * TPF;
+					constexpr int NH = CPLX ? 8 : 4;
+					uint32_t h[NH], edge = 0u;
+#pragma unroll
+					for(int g8 = 0; g8 < JG; g8++)
+					{
+						const int q = q0 + g8 * (N / 8);
+						cf y[RL];
+						if constexpr(N <= 2048)
+							asm volatile("" ::: "memory");        // 80 registers: one group's loads at a time
+#pragma unroll
+						for(int r = 0; r < RL; r++)
+							y[r] = lds(src + st_index<sL, (N >= 8192)>(q, r));
+						dftR<RL>(y);
+						if(!tok || row0 < 0)
+							continue;
+#pragma unroll
+						for(int r = 0; r < (CPLX ? RL : RL / 2); r++)
+						{
+							const int k = q + sL * r;
+							uint32_t &o = h[g8 + r * JG];
+							if constexpr(CPLX)
+								o = packed(y[r], lsb ? (k == 0 ? -N : -k) : k, lsb && k != 0 ? -1.0f : 1.0f);
+							else
+							{
+								const bool upper = lsb && !mirror;             // bins N/2 ..
+								o = packed(cf{upper ? y[r + RL / 2].x : y[r].x, upper ? y[r + RL / 2].y : y[r].y},
+								           mirror ? -k : (lsb ? k - nchan : k), mirror ? -1.0f : 1.0f);
+							}
+						}
+						if constexpr(!CPLX)
+							if(mirror && g8 == 0 && q0 == 0)
+								edge = packed(y[RL / 2], -nchan, -1.0f);        // bin N/2, channel 0
+					}
+					if(!tok || row0 < 0)
+						continue;
+					const uint32_t p = 4u * (uint32_t)q0, pm = (uint32_t)(N / 2) - p, p8 = (uint32_t)(N / 2);
 					if constexpr(CPLX)
 					{
-						// every bin is a channel; the lower sideband keeps bin 0 and
-						// mirrors and conjugates the rest (mode.cpp:1217-1226)
 						if(!lsb)
 						{
+							quad(p, h[0], h[2], h[4], h[6]);
+							quad(p + p8, h[1], h[3], h[5], h[7]);
+						}
+						else if(q0 == 0)
+						{
+							quad(0u, h[0], h[6], h[4], h[2]);
+							quad(p8, h[7], h[5], h[3], h[1]);
+						}
+						else
+						{
+							quad(pm, h[7], h[5], h[3], h[1]);
+							quad(pm + p8, h[6], h[4], h[2], h[0]);
+						}
+					}
+					else if(!mirror)
+						quad(p, h[0], h[1], h[2], h[3]);
+					else if(q0 == 0)
+						quad(0u, edge, h[3], h[2], h[1]);
+					else
+						quad(pm, h[3], h[2], h[1], h[0]);
+				}
+			}
+			else
+			{
+				const int64_t obase = a.plans[g.freq].spec_off + (int64_t)t * a.plans[g.freq].nrow * nchan;
+#pragma unroll
+				for(int jj = 0; jj < J; jj++)
+				{
+					const int q = bt + jj * TPF;
+					cf y[RL];
+#pragma unroll
+					for(int r = 0; r < RL; r++)
+						y[r] = lds(src + st_index<sL, (N >= 8192)>(q, r));
+					dftR<RL>(y);
+					if(!tok)
+						continue;
+#pragma unroll
+					for(int r = 0; r < RL; r++)
+					{
+						const int k = q + sL * r;
+						int c, ce;
+						float cj = 1.0f;
+						if constexpr(CPLX)
+						{
+							// every bin is a channel; the lower sideband keeps bin 0 and
+							// mirrors and conjugates the rest (mode.cpp:1217-1226)
+							if(!lsb)
+							{
+								c = k;
+								ce = k;
+							}
+							else
+							{
+								c = k == 0 ? 0 : N - k;
+								ce = c - nchan;
+								cj = k == 0 ? 1.0f : -1.0f;
+							}
+						}
+						else if(!lsb)
+						{
+							if(r >= RL / 2)
+								continue;                  // bins >= nchan
 							c = k;
 							ce = k;
 						}
-						else
+						else if(!mirror)
 						{
-							c = k == 0 ? 0 : N - k;
+							if(r < RL / 2)
+								continue;
+							c = k - nchan;
 							ce = c - nchan;
-							cj = k == 0 ? 1.0f : -1.0f;
-						}
-					}
-					else if(!lsb)
-					{
-						if(r >= RL / 2)
-							continue;                  // bins >= nchan
-						c = k;
-						ce = k;
-					}
-					else if(order != 0)
-					{
-						if(r < RL / 2)
-							continue;
-						c = k - nchan;
-						ce = c - nchan;
-					}
-					else
-					{
-						if(!(k >= 1 && k <= nchan))
-							continue;
-						c = nchan - k;
-						ce = c - nchan;
-						cj = -1.0f;
-					}
-					// fractional-sample (and order-0 fringe) rotation
-					if(row0 < 0)
-						continue;
-					const float fce = (float)ce;
-					float th = fce * dhi;               // exact (split_turns)
-					th -= rintf(th);
-					float turns = th + fmaf(fce, dlo, postf + ph0);
-					turns -= rintf(turns);
-					float sn, cs;
-					__sincosf(6.283185307179586f * turns, &sn, &cs);
-					const float xr = y[r].x, xi = cj * y[r].y;
-					if constexpr(TCO)
-					{
-						uint32_t *o;
-						if(tcb)
-						{
-							const uint32_t pc = (uint32_t)chan_pos(pbits, c), blk = __umulhi(pc, tcb_magic), cl = pc - blk * tcb;
-							o = (uint32_t *)a.spec + spec_off + (((int64_t)t * tnblk + blk) * prow) * tcb + cl +
-							    (int64_t)row0 * tcb;
 						}
 						else
-							o = (uint32_t *)a.spec + obase + c + (int64_t)row0 * nchan;
-						cs *= osc;
-						sn *= osc;
-						*o = pack_spec(h16, xr * cs - xi * sn, xr * sn + xi * cs);
+						{
+							if(!(k >= 1 && k <= nchan))
+								continue;
+							c = nchan - k;
+							ce = c - nchan;
+							cj = -1.0f;
+						}
+						if(row0 < 0)
+							continue;
+						const cf v = turned(y[r], ce, cj);
+						((float2 *)a.spec + obase + c)[(int64_t)row0 * nchan] = make_float2(v.x, v.y);
 					}
-					else
-						((float2 *)a.spec + obase + c)[(int64_t)row0 * nchan] =
-						    make_float2(xr * cs - xi * sn, xr * sn + xi * cs);
 				}
 			}
 		}

@@ -15,6 +15,7 @@ struct DevFreqPlan {
 	int32_t tnblk;                    // tensor-core form: blocks per time, spectra [t][block][trow][tcb]
 	int32_t trow;                     // tensor-core form: rows of a block (nrow and, in the FP16 / BF16 form, zero rows)
 	int32_t pbits;                    // tensor-core form: log2(nchan / 4), see chan_pos
+	uint32_t magic;                   // tensor-core form: p / tcb = umulhi(p, magic) for p < 2^16
 	int32_t acc_cstride;              // accumulator stride between channels (1: [out][chan], nout: [chan][out])
 	int32_t acc_ostride;              // accumulator stride between outputs
 	int64_t spec_off;                 // complex offset of this frequency's spectra
@@ -269,7 +270,7 @@ void launch_fstage_kind(const FKind &k, FsArgs a, cudaStream_t stream);
 constexpr int kFsMultiMembers = 16;
 constexpr int kFsMultiFc = 64;           // FFT constants of one unit of up to 2048 points at most (tq x fpc)
 // classes of units: plain VDIF's (fstage_multi_class), then those of raw reads
-constexpr int kFsMultiPer = 5, kFsMultiClasses = 2 * kFsMultiPer;
+constexpr int kFsMultiPer = 6, kFsMultiClasses = 2 * kFsMultiPer;
 struct FsMultiKind {
 	const void *tw;                      // twiddles of length N
 	int32_t member, code;                // context; 128 x raw INTERLACEDVDIF reads + 32 x bands per item + log2 N
@@ -290,9 +291,9 @@ struct FsMultiArgs {
 	int32_t *ctr;                        // one counter per class, zero before the launch
 };
 // class of a kind (FFT length N, bands per item nb) in the persistent launches
-// (0: two bands of 8192 points, 1: one band of 8192, 2: two bands of 4096, 3:
-// two bands of up to 2048, 4: one band of up to 4096; -1: not run there), and
-// the FFT iterations per unit for a kind's tq
+// (0: two bands of 8192 points, 1: one band of 8192, 2: two bands of 4096, 3: one
+// band of 4096, 4: two bands of up to 2048, 5: one band of up to 2048; -1: not run
+// there), and the FFT iterations per unit for a kind's tq
 int fstage_multi_class(int N, int nb);
 int fstage_multi_tq(int N, int nb, int tq);
 cudaError_t launch_fstage_multi(const FsMultiArgs &m, int nsm, cudaStream_t stream);
