@@ -470,16 +470,12 @@ static PairItem pair_item(const fxb_ctx *ctx, const FGroup &g, int group, bool t
 	u.tcb = tc ? (uint32_t)P.tcb : 0u;
 	u.magic = P.magic;
 	u.bextra = tc ? (uint32_t)(P.trow - 1) * u.tcb : 0u;
-	u.pbits = tc ? P.pbits : 0;
 	const int rstr = tc ? P.tcb : nchan;
 	u.rowd = ctx->h_plans[g.freq1].spec_off - P.spec_off + (int64_t)(g.row[1] - row0) * rstr;
 	u.two = g.freq1 != g.freq;
 	u.tstride = tc ? (int64_t)P.tnblk * P.trow * P.tcb : (int64_t)P.nrow * nchan;
 	u.first = P.spec_off + (int64_t)row0 * rstr;
 	u.oflags = (g.row[0] >= 0 ? kORow0 : 0) | (g.row[1] >= 0 ? kORow1 : 0) | (ctx->h16 ? kOH16 : 0);
-	// four channels of a thread at once: blocks of a power of two channels
-	if(tc && !S.cplx && (u.tcb == 2 || u.tcb == 4 || u.tcb == 8) && !(g.lsb && ctx->job.fringe_rot_order == 0))
-		u.oflags |= kOQuad;
 	if((u.oflags & kORow0) && (u.oflags & kORow1) && u.rowd == 2 && !(row0 & 1) && tc && !(P.trow & 1))
 		u.oflags |= kOBoth;
 	const uint32_t cpl = S.cplx ? 2u : 1u;

@@ -493,23 +493,34 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 		const int64_t base = I.first + (int64_t)t * I.tstride;
 		auto put = [&](int c, const cp &y) {
 			const float2 re = up2(y.re), im = up2(y.im);
-			if constexpr(TCO)
+			float2 *o = (float2 *)a.spec + base + c;
+			if(oflags & kORow0)
+				*o = make_float2(re.x, im.x);
+			if(oflags & kORow1)
+				o[rowd] = make_float2(re.y, im.y);
+		};
+		// Tensor-core form: the four values of each band at positions p0 .. p0 + 3
+		// (chan_pos) at once; blocks of two channels whose rows of the two bands are an
+		// aligned pair take both bands in one store.
+		auto quad = [&](uint32_t p0, uint4 v0, uint4 v1) {
+			uint32_t *o = (uint32_t *)a.spec + base;
+			const uint32_t bextra = I.bextra, magic = I.magic;
+			if(oflags & kOBoth)
 			{
-				const uint32_t p = (uint32_t)chan_pos(I.pbits, c);
-				uint32_t *o = (uint32_t *)a.spec + base + (p + __umulhi(p, I.magic) * I.bextra);
-				if(oflags & kORow0)
-					*o = pack_spec(h16, re.x, im.x);
-				if(oflags & kORow1)
-					o[rowd] = pack_spec(h16, re.y, im.y);
+				uint32_t *q = o + p0 + (p0 >> 1) * bextra;
+				*(uint4 *)q = make_uint4(v0.x, v0.y, v1.x, v1.y);
+				*(uint4 *)(q + bextra + 2) = make_uint4(v0.z, v0.w, v1.z, v1.w);
+				return;
 			}
-			else
-			{
-				float2 *o = (float2 *)a.spec + base + c;
-				if(oflags & kORow0)
-					*o = make_float2(re.x, im.x);
-				if(oflags & kORow1)
-					o[rowd] = make_float2(re.y, im.y);
-			}
+			if(oflags & kORow0)
+				store_quad(o, p0, I.tcb, magic, bextra, v0);
+			if(oflags & kORow1)
+				store_quad(o + rowd, p0, I.tcb, magic, bextra, v1);
+		};
+		auto packed = [&](const cp &y, uint32_t &h0, uint32_t &h1) {
+			const float2 re = up2(y.re), im = up2(y.im);
+			h0 = pack_spec(h16, re.x, im.x);
+			h1 = pack_spec(h16, re.y, im.y);
 		};
 		// y conjugated when cj < 0, times the bands' rotators
 		auto turn = [](const cp &y, float cj, float2 w0, float2 w1) {
@@ -537,22 +548,70 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 		if constexpr(CPLX)
 		{
 			// every bin is a channel; the lower sideband keeps bin 0 and mirrors and
-			// conjugates the rest (mode.cpp:1217-1226)
-#pragma unroll
-			for(int jj = 0; jj < J; jj++)
-			{
-				cp y[RL];
+			// conjugates the rest (mode.cpp:1217-1226).  Output m of the thread is bin b +
+			// m N/8: the even ones are the channels of one quad of positions, the odd ones
+			// of another, in descending order in the lower sideband.  Two bands of four
+			// subbands, 1024 channels, 2 bits, 10 stations, F stage: 142 us in the order of
+			// channels, 187 in that of chan_pos one by one, 125 a quad at a time.
+			auto value = [&](const cp &y, int k) {
+				const int ce = lsb ? (k == 0 ? -N : -k) : k;
+				const float2 w0 = rotator(0, ce), w1 = same ? w0 : rotator(1, ce);
+				return turn(y, !lsb || k == 0 ? 1.0f : -1.0f, w0, w1);
+			};
+			auto load = [&](cp *y, int jj) {
 #pragma unroll
 				for(int r = 0; r < RL; r++)
 					y[r] = ldx(side + ppad(b + jj * TPF + sL * r));
 				dftR<RL>(y);
+			};
+			if constexpr(!TCO)
+			{
 #pragma unroll
-				for(int r = 0; r < RL; r++)
+				for(int jj = 0; jj < J; jj++)
 				{
-					const int k = b + jj * TPF + sL * r;
-					const int c = !lsb || k == 0 ? k : N - k, ce = lsb ? c - nchan : c;
-					const float2 w0 = rotator(0, ce), w1 = same ? w0 : rotator(1, ce);
-					put(c, turn(y[r], !lsb || k == 0 ? 1.0f : -1.0f, w0, w1));
+					cp y[RL];
+					load(y, jj);
+#pragma unroll
+					for(int r = 0; r < RL; r++)
+					{
+						const int k = b + jj * TPF + sL * r;
+						put(!lsb || k == 0 ? k : N - k, value(y[r], k));
+					}
+				}
+			}
+			else
+			{
+				cp y[RL];
+#pragma unroll
+				for(int par = 0; par < 2; par++)
+				{
+					uint32_t h0[4], h1[4];
+#pragma unroll
+					for(int g = 0; g < (J + 1) / 2; g++)
+					{
+						// group jj holds the outputs m = jj + r J
+						const int jj = J == 1 ? 0 : par + 2 * g;
+						if(J > 1 || par == 0)
+							load(y, jj);
+#pragma unroll
+						for(int r = 0; r < RL; r++)
+						{
+							const int m = jj + r * J;
+							if((m & 1) == par)
+								packed(value(y[r], b + m * (int)S8), h0[m >> 1], h1[m >> 1]);
+						}
+					}
+					const uint4 up0 = make_uint4(h0[0], h0[1], h0[2], h0[3]), up1 = make_uint4(h1[0], h1[1], h1[2], h1[3]);
+					const uint4 dn0 = make_uint4(h0[3], h0[2], h0[1], h0[0]), dn1 = make_uint4(h1[3], h1[2], h1[1], h1[0]);
+					const uint32_t p = 4u * (uint32_t)b, half = (uint32_t)(N / 2);
+					if(!lsb)
+						quad(p + (par ? half : 0u), up0, up1);
+					else if(b > 0)
+						quad(half - p + (par ? 0u : half), dn0, dn1);
+					else if(par)
+						quad(half, dn0, dn1);
+					else
+						quad(0u, make_uint4(h0[0], h0[3], h0[2], h0[1]), make_uint4(h1[0], h1[3], h1[2], h1[1]));
 				}
 			}
 		}
@@ -589,7 +648,18 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 					// bin N/2, channel 0
 					const float2 m0 = rotator(0, -nchan), m1 = same ? m0 : rotator(1, -nchan);
 					dft_half<RL>(z, h, nsg, sg);
-					put(0, turn(h[0], -1.0f, m0, m1));
+					const cp e = turn(h[0], -1.0f, m0, m1);
+					if constexpr(TCO)
+					{
+						uint32_t *o = (uint32_t *)a.spec + base, e0, e1;
+						packed(e, e0, e1);
+						if(oflags & kORow0)
+							*o = e0;
+						if(oflags & kORow1)
+							o[rowd] = e1;
+					}
+					else
+						put(0, e);
 				}
 			}
 #pragma unroll
@@ -613,52 +683,32 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 						rot1(w1.x, w1.y, os1.x, os1.y);
 				}
 			}
-			bool stored = false;
 			if constexpr(TCO)
-				if(oflags & kOQuad)
-				{
-					// the four values of each band side by side (chan_pos): blocks of 8 or 4
-					// channels take one 16-byte store per band, blocks of 2 two of 8 bytes, or
-					// both bands at once where their rows are an aligned pair
-					stored = true;
-					uint32_t q0[4], q1[4];
+			{
+				uint32_t h0[4], h1[4];
 #pragma unroll
-					for(int m = 0; m < 4; m++)
+				for(int m = 0; m < 4; m++)
+					packed(y[m], h0[m], h1[m]);
+				const uint32_t p = 4u * (uint32_t)b;
+				if(!mirror || b > 0)
+					quad(mirror ? (uint32_t)(N / 2) - p : p,
+					     make_uint4(mirror ? h0[3] : h0[0], mirror ? h0[2] : h0[1], mirror ? h0[1] : h0[2], mirror ? h0[0] : h0[3]),
+					     make_uint4(mirror ? h1[3] : h1[0], mirror ? h1[2] : h1[1], mirror ? h1[1] : h1[2], mirror ? h1[0] : h1[3]));
+				else
+				{
+					// beside channel 0 (bin N/2, above)
+#pragma unroll
+					for(uint32_t m = 1; m < 4; m++)
 					{
-						const float2 re = up2(y[m].re), im = up2(y[m].im);
-						q0[m] = pack_spec(h16, re.x, im.x);
-						q1[m] = pack_spec(h16, re.y, im.y);
-					}
-					const uint32_t tcb = I.tcb, bextra = I.bextra;
-					uint32_t *o = (uint32_t *)a.spec + base +
-					              (4u * (uint32_t)b + (tcb == 2 ? 2u * (uint32_t)b : (tcb == 4 ? (uint32_t)b : (uint32_t)b >> 1)) * bextra);
-					if(tcb >= 4)
-					{
+						uint32_t *o = (uint32_t *)a.spec + base + m + __umulhi(m, I.magic) * I.bextra;
 						if(oflags & kORow0)
-							*(uint4 *)o = make_uint4(q0[0], q0[1], q0[2], q0[3]);
+							*o = h0[4 - m];
 						if(oflags & kORow1)
-							*(uint4 *)(o + rowd) = make_uint4(q1[0], q1[1], q1[2], q1[3]);
-					}
-					else if(oflags & kOBoth)
-					{
-						*(uint4 *)o = make_uint4(q0[0], q0[1], q1[0], q1[1]);
-						*(uint4 *)(o + bextra + tcb) = make_uint4(q0[2], q0[3], q1[2], q1[3]);
-					}
-					else
-					{
-						if(oflags & kORow0)
-						{
-							*(uint2 *)o = make_uint2(q0[0], q0[1]);
-							*(uint2 *)(o + bextra + tcb) = make_uint2(q0[2], q0[3]);
-						}
-						if(oflags & kORow1)
-						{
-							*(uint2 *)(o + rowd) = make_uint2(q1[0], q1[1]);
-							*(uint2 *)(o + rowd + bextra + tcb) = make_uint2(q1[2], q1[3]);
-						}
+							o[rowd] = h1[4 - m];
 					}
 				}
-			if(!stored)
+			}
+			else
 			{
 #pragma unroll
 				for(int m = 0; m < 4; m++)

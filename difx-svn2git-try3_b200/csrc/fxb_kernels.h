@@ -205,14 +205,14 @@ struct alignas(16) PairItem {
 	int64_t rowd;                        // from the first band's values to the second's
 	uint32_t tcb, magic, bextra;         // channels of a block; p / tcb = umulhi(p, magic) for p < 2^16;
 	                                     // position p sits at p + p / tcb x bextra
-	int32_t pbits, oflags;
+	int32_t oflags;
 	uint32_t fs, bpt, boff0, boff1;      // samples per frame, bits per time, first bit of each band
 	uint32_t hbits;                      // header bits
 	int32_t nbits, header, framebytes, minfb, mnthr;
 	int32_t station, band0, band1, lsb, asl, adj;   // adj: both bands side by side in one aligned field
 	int32_t group, two;                  // two: the bands' LOs differ
 };
-enum : int32_t { kORow0 = 1, kORow1 = 2, kOH16 = 4, kOQuad = 8, kOBoth = 16 };
+enum : int32_t { kORow0 = 1, kORow1 = 2, kOH16 = 4, kOBoth = 8 };
 enum : int32_t {
 	kPActive = 1,     // valid FFT
 	kPNarrow = 2,     // fmask covers the window

@@ -61,3 +61,24 @@ def test_blocks(nstation, xmac, nchan):
         rms = np.sqrt(np.mean(np.abs(ref[0]) ** 2))
         for x, y in ((ref[0].real, got[0].real), (ref[0].imag, got[0].imag)):
             assert np.all(np.abs(x - y) <= 2.0 ** -8 * np.abs(x) + 1e-5 * rms)
+
+
+@pytest.mark.parametrize("nstation", [3, 7, 13])
+@pytest.mark.parametrize("nchan", [16, 32, 64, 128, 256, 512, 1024, 2048, 4096])
+@pytest.mark.parametrize("kw", [dict(), dict(sideband="L"), dict(sideband="L", fringe_rot_order=0)])
+def test_two_bands(nstation, nchan, kw, monkeypatch):
+    monkeypatch.setenv("FXB_TC_FFT", "0")
+    compare(*spectra(nstation, nchan, "fp16", pols="RL", **kw))
+
+
+@pytest.mark.parametrize("nstation", [2, 3, 5, 8, 9, 13, 17])
+@pytest.mark.parametrize("kw", [dict(), dict(sideband="L", fringe_rot_order=0), dict(cplx=True)])
+def test_two_bands_of_fp8_blocks(nstation, kw):
+    compare(*spectra(nstation, 64, "fp8", pols="RL", **kw))
+
+
+@pytest.mark.parametrize("nchan", [32, 64, 128, 256, 512, 1024, 2048, 4096, 8192])
+@pytest.mark.parametrize("sideband", ["U", "L"])
+@pytest.mark.parametrize("nstation,pols", [(3, "R"), (7, "RL"), (13, "RL")])
+def test_complex(nchan, sideband, nstation, pols):
+    compare(*spectra(nstation, nchan, "fp16", pols=pols, sideband=sideband, cplx=True))
