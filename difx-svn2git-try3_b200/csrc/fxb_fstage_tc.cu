@@ -50,7 +50,10 @@
 // with the unit records formed by the producer warp, 148 us with k_tc_units ahead of
 // it, 133 us with the conflict-free lookup and the twiddles loaded once for both
 // subbands; 32 stations x 8 bands x 250 FFTs: 348, 337, 309 us,
-// and 294 with the two subbands' decode interleaved (the first stays at 133).
+// and 294 with the two subbands' decode interleaved (the first stays at 133);
+// with both polarisations of a channel in one output warp, whose 8-byte stores (blocks
+// of two channels, above 24 inputs) so meet half the sectors, 64 inputs 298 and 236, 50
+// inputs 267 and 192 (223 before the channels' present order), the first 137 and 135.
 // Slower: the lookup's offset by rotating the nibble (294 -> 306), the twiddles by
 // recurrence in registers (133 -> 145, though 294 -> 282), a fourth operand buffer.
 
@@ -789,8 +792,8 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 				tld16(tmem + lane_base + (uint32_t)(256 * b + 16 * h), v[0]);
 				tld16(tmem + lane_base + (uint32_t)(256 * b + 64 + 16 * h), v[1]);
 				tld_wait();
-				// Z[k1][n2] = Y[k1][n2] w^(n2 k1); A2 row m = ch 32 + k1 with ch = 2 sb + p,
-				// K = part 64 + n2
+				// Z[k1][n2] = Y[k1][n2] w^(n2 k1); A2 row m = sb 64 + (k1 / 8) 16 + p 8 + k1 % 8, so
+				// that a warp of the output role holds both polarisations; K = part 64 + n2
 				uint32_t zr[2][4], zi[2][4];
 #pragma unroll
 				for(int q = 0; q < 8; q += 2)
@@ -811,7 +814,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 #pragma unroll
 				for(int sb = 0; sb < 2; sb++)
 				{
-					const int m0 = (2 * sb + p) * 32 + 8 * h;
+					const int m0 = sb * 64 + 16 * h + 8 * p;
 					*(uint4 *)(A2 + mn_off(m0, n2)) = make_uint4(zr[sb][0], zr[sb][1], zr[sb][2], zr[sb][3]);
 					*(uint4 *)(A2 + mn_off(m0, 64 + n2)) = make_uint4(zi[sb][0], zi[sb][1], zi[sb][2], zi[sb][3]);
 				}
@@ -829,8 +832,10 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 	else if(warp < kMmaW)
 	{
 		// ================================================================ output
-		const int ch = warp - kOutW0, k1 = lane;
-		const int sb = ch >> 1, p = ch & 1;
+		// lanes l and l + 8 hold the two polarisations of a k1: rows side by side in the
+		// spectra, which a warp's store puts into the same sectors
+		const int quarter = warp - kOutW0, sb = quarter >> 1, p = (lane >> 3) & 1;
+		const int k1 = 16 * (quarter & 1) + 8 * (lane >> 4) + (lane & 7);
 		const uint32_t lane_base = (uint32_t)(32 * (warp & 3)) << 16;
 		constexpr float osc = 1.0f / (float)(1 << kTcSpecExp);
 		for(int k = 0; k < nk; k++)
@@ -875,10 +880,10 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 			// of tcb channels, and the distance of the next four (128 positions on)
 			const uint32_t tcb = (uint32_t)R.tcb[sb], extra = (uint32_t)(R.nrow[sb] - 1) * tcb;
 			uint32_t *o = (uint32_t *)a.spec + R.spec[sb] + (int64_t)(row < 0 ? 0 : row) * (int)tcb;
-			const bool quad = tcb == 2 || tcb == 4 || tcb == 8;
+			const bool pow2 = tcb == 2 || tcb == 4 || tcb == 8;
 			const uint32_t magic = 0xFFFFFFFFu / tcb + 1u;
-			const uint32_t jstep = quad ? 128u * (uint32_t)R.nrow[sb] : 0u;
-			if(quad)
+			const uint32_t jstep = pow2 ? 128u * (uint32_t)R.nrow[sb] : 0u;
+			if(pow2)
 				o += 4u * (uint32_t)k1 + (tcb == 2 ? 2u * (uint32_t)k1 : (tcb == 4 ? (uint32_t)k1 : (uint32_t)k1 >> 1)) * extra;
 			tld_wait();
 #pragma unroll
@@ -886,6 +891,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 			{
 				if(hh == 1)
 				{
+					__syncwarp();             // the load is the whole warp's
 					tld32(tcol + 32, v);
 					tld_wait();
 					asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
@@ -893,8 +899,6 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 					if(lane == 0)
 						mbar_arrive(&d2_empty[b]);
 				}
-				if(row < 0)
-					continue;
 #pragma unroll
 				for(int j = 0; j < 4; j++)
 				{
@@ -919,24 +923,33 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 						br = zr;
 						bi = zi;
 					}
-					if(quad)
+					if(row >= 0)
 					{
-						if(tcb == 2)
+						if(pow2)
 						{
-							*(uint2 *)o = make_uint2(h[0], h[1]);
-							*(uint2 *)(o + extra + 2) = make_uint2(h[2], h[3]);
+							if(tcb == 2)
+							{
+								*(uint2 *)o = make_uint2(h[0], h[1]);
+								*(uint2 *)(o + extra + 2) = make_uint2(h[2], h[3]);
+							}
+							else
+								*(uint4 *)o = make_uint4(h[0], h[1], h[2], h[3]);
 						}
 						else
-							*(uint4 *)o = make_uint4(h[0], h[1], h[2], h[3]);
-						o += jstep;
+						{
+							// even widths of the FP8 form
+							const uint32_t p0 = 4u * (uint32_t)(k1 + 32 * (4 * hh + j)), p2 = p0 + 2u;
+							uint32_t *q = o + p0 + __umulhi(p0, magic) * extra;
+							if(tcb & 2u)
+							{
+								*(uint2 *)q = make_uint2(h[0], h[1]);
+								*(uint2 *)(o + p2 + __umulhi(p2, magic) * extra) = make_uint2(h[2], h[3]);
+							}
+							else
+								*(uint4 *)q = make_uint4(h[0], h[1], h[2], h[3]);
+						}
 					}
-					else
-					{
-						const uint32_t p0 = 4u * (uint32_t)(k1 + 32 * (4 * hh + j));
-#pragma unroll
-						for(uint32_t m = 0; m < 4; m++)
-							o[p0 + m + __umulhi(p0 + m, magic) * extra] = h[m];
-					}
+					o += jstep;
 				}
 			}
 		}

@@ -82,3 +82,18 @@ def test_two_bands_of_fp8_blocks(nstation, kw):
 @pytest.mark.parametrize("nstation,pols", [(3, "R"), (7, "RL"), (13, "RL")])
 def test_complex(nchan, sideband, nstation, pols):
     compare(*spectra(nstation, nchan, "fp16", pols=pols, sideband=sideband, cplx=True))
+
+
+@pytest.mark.parametrize("nstation,pols,nfreq,xmac", [(2, "RL", 1, "fp16"), (6, "RL", 4, "fp16"), (7, "RL", 8, "fp16"),
+                                                      (13, "RL", 2, "bf16"), (25, "RL", 2, "fp16"), (31, "RL", 1, "fp16"),
+                                                      (32, "RL", 2, "fp16"), (3, "RL", 2, "fp8"), (5, "RL", 2, "fp8"),
+                                                      (9, "RL", 2, "fp8"), (13, "RL", 2, "fp8"), (3, "R", 1, "fp16"),
+                                                      (13, "R", 1, "fp16"), (9, "R", 1, "fp8")])
+def test_tensor_core_fft(nstation, pols, nfreq, xmac):
+    """The tensor-core FFT's stores.  In the 2-norm of each spectrum: FP16 samples,
+    tables (twice), intermediate and output, each within 2^-12 (BF16 output: 2^-9)."""
+    ref, got = spectra(nstation, 1024, xmac, pols=pols, nfreq=nfreq, nbits=2)
+    tol = 5 * 2.0 ** -12 + (2.0 ** -9 if xmac == "bf16" else 0)
+    for r, g in zip(ref, got):
+        err = np.linalg.norm(g - r, axis=2) / np.linalg.norm(r, axis=2)
+        assert err.shape == (3, nstation * len(pols)) and np.all(err <= tol), err.max()
