@@ -494,8 +494,9 @@ static PairItem pair_item(const fxb_ctx *ctx, const FGroup &g, int group, bool t
 	u.band1 = g.band[1];
 	u.lsb = g.lsb;
 	u.asl = S.asl;
-	// both bands side by side in one field of 2 nbits, aligned to its size
-	u.adj = !S.muxraw && !S.cplx && u.boff1 == u.boff0 + (uint32_t)S.nbits && u.boff0 % (2u * (uint32_t)S.nbits) == 0;
+	// both bands side by side in one field of twice their size, aligned to it
+	const uint32_t field = (uint32_t)S.nbits * cpl;
+	u.adj = !S.muxraw && u.boff1 == u.boff0 + field && u.boff0 % (2u * field) == 0;
 	u.group = group;
 	return u;
 }

@@ -243,7 +243,7 @@ __global__ void __launch_bounds__(128) k_pair_consts(const FsArgs a, int N, int 
 			}
 		}
 		const bool whole = nwf < 32 && c.fmask == (1u << nwf) - 1u && c.stuck >= N && !(c.flags & kPBlank);
-		if(whole && I.adj && fs >= (uint32_t)S8)
+		if(!mux && whole && fs >= (uint32_t)S8)
 			c.flags |= kPFast;
 		if(mux && whole && nwf <= 2)
 		{

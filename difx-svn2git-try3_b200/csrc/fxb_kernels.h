@@ -219,7 +219,7 @@ enum : int32_t {
 	kPBlank = 4,      // a valid frame of the window blanks one of the item's bands
 	kPSame = 8,       // the two bands take the same output rotation
 	kPTwo = 32,       // the bands take different fringe rotations
-	kPFast = 16       // every sample of the window counts and the fast read applies
+	kPFast = 16       // every sample of the window counts, frames of at least N/8 samples (raw reads: at most two)
 };
 
 struct FsArgs {
