@@ -677,12 +677,13 @@ static unsigned long long primary_context(int dev, bool mine)
 }
 
 // The calls' tables come from a pool of the calling thread, one per device, that
-// keeps up to 4 MB mapped between calls and goes with the thread: the default pool
-// gives its memory back at every synchronisation, and mapping it again took from
-// 20 us to tens of milliseconds of a 0.1 ms call (1000 frames of 16 threads: 99 to
-// 617 us a call from run to run, with this pool 91 to 99; the first call on a
-// thread makes the pool).  A pool belongs to the context it was made in: after a
-// reset of the device it is left alone and another made.
+// keeps the driver's least reserve (32 MB) mapped between calls and goes with the
+// thread.  The default pool, and one told to keep less than that reserve, gives it
+// back at every synchronisation by anyone, and the next call maps it again: a call
+// after a synchronisation then takes 0.4 ms more at best, and now and then tens of
+// milliseconds (allocate, clear, wait, free: 410 us; from this pool 14 us).  A pool
+// belongs to the context it was made in: after a reset of the device it is left
+// alone and another made.
 static cudaMemPool_t mux_pool()
 {
 	constexpr int kMaxDevices = 64;
@@ -714,7 +715,7 @@ static cudaMemPool_t mux_pool()
 		props.location.type = cudaMemLocationTypeDevice;
 		props.location.id = dev;
 		cudaMemPool_t p = nullptr;
-		uint64_t keep = 4u << 20;
+		uint64_t keep = 32u << 20;
 		if(cudaMemPoolCreate(&p, &props) != cudaSuccess)
 		{
 			cudaGetLastError();
