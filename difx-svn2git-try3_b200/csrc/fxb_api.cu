@@ -478,6 +478,10 @@ static PairItem pair_item(const fxb_ctx *ctx, const FGroup &g, int group, bool t
 	u.oflags = (g.row[0] >= 0 ? kORow0 : 0) | (g.row[1] >= 0 ? kORow1 : 0) | (ctx->h16 ? kOH16 : 0);
 	if((u.oflags & kORow0) && (u.oflags & kORow1) && u.rowd == 2 && !(row0 & 1) && tc && !(P.trow & 1))
 		u.oflags |= kOBoth;
+	for(u.shift = 0; (2u << u.shift) <= u.tcb; u.shift++)
+		;
+	if(u.tcb >= 4 && (1u << u.shift) == u.tcb)
+		u.oflags |= kOWide;
 	const uint32_t cpl = S.cplx ? 2u : 1u;
 	u.fs = (uint32_t)S.framesamples;
 	u.bpt = S.muxraw ? (uint32_t)S.nbits : (uint32_t)(S.nband * S.nbits) * cpl;

@@ -9,7 +9,7 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB) k_fstage
 {
 	extern __shared__ __align__(16) ulonglong2 fsp[];
 	constexpr int FPC = PShape<LOGN>::FPC;
-	__shared__ float lut8[256];
+	__shared__ float lut8[260];
 	__shared__ u64 lut4[16];
 	__shared__ PairConst fcs[kMaxTQ * FPC];
 	__shared__ PairTwist tws[kMaxTQ * FPC];

@@ -10,7 +10,7 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB) k_fstage
 {
 	extern __shared__ __align__(16) ulonglong2 fsp[];
 	constexpr int FPC = PShape<LOGN>::FPC;
-	__shared__ float lut8[256];
+	__shared__ float lut8[260];
 	__shared__ u64 lut4[16];
 	__shared__ PairConst fcs[kMaxTQ * FPC];
 	__shared__ PairTwist tws[kMaxTQ * FPC];
@@ -41,7 +41,7 @@ template <int VAR>
 __global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant__ FsMultiArgs m)
 {
 	extern __shared__ __align__(16) ulonglong2 fsp[];
-	__shared__ float lut8[256];
+	__shared__ float lut8[260];
 	__shared__ u64 lut4[16];
 	__shared__ PairFeed<kFsMultiFc> feed;
 	fstage_pair_luts(lut8, lut4);
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB)
     k_fstage_pair_pw(const __grid_constant__ FsMultiArgs m)
 {
 	extern __shared__ __align__(16) ulonglong2 fsp[];
-	__shared__ float lut8[256];
+	__shared__ float lut8[260];
 	__shared__ u64 lut4[16];
 	__shared__ PairFeed<kMaxTQ> feed;
 	fstage_pair_luts(lut8, lut4);

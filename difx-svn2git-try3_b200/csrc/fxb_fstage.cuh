@@ -373,10 +373,13 @@ __device__ __forceinline__ void fstage_unit(const FsArgs &a, const int gidx, con
 	constexpr float osc = 1.0f / (float)(1 << kTcSpecExp);
 	const bool h16 = a.h16 != 0;
 
-	// where registers are short, read again at each FFT's output
+	// (tensor-core form up to 8192 points, where registers are short: read at each
+	// FFT's output)
 	OutRow out = {};
 	if constexpr(TCO && N > 8192)
 		out = out_row(a.plans[g.freq], row0);
+	const int64_t spec_off = TCO ? 0 : a.plans[g.freq].spec_off;
+	const int prow = TCO ? 0 : a.plans[g.freq].nrow;
 
 	const int t0 = tchunk * tq * FPC;
 	const int nit = min(tq, (a.T - t0 + FPC - 1) / FPC);
@@ -729,7 +732,7 @@ __device__ __forceinline__ void fstage_unit(const FsArgs &a, const int gidx, con
 			}
 			else
 			{
-				const int64_t obase = a.plans[g.freq].spec_off + (int64_t)t * a.plans[g.freq].nrow * nchan;
+				const int64_t obase = spec_off + (int64_t)t * prow * nchan;
 #pragma unroll
 				for(int jj = 0; jj < J; jj++)
 				{
@@ -787,8 +790,15 @@ __device__ __forceinline__ void fstage_unit(const FsArgs &a, const int gidx, con
 						}
 						if(row0 < 0)
 							continue;
-						const cf v = turned(y[r], ce, cj);
-						((float2 *)a.spec + obase + c)[(int64_t)row0 * nchan] = make_float2(v.x, v.y);
+						const float fce = (float)ce;
+						float th = fce * dhi;               // exact (split_turns)
+						th -= rintf(th);
+						float turns = th + fmaf(fce, dlo, postf + ph0);
+						turns -= rintf(turns);
+						float sn, cs;
+						__sincosf(6.283185307179586f * turns, &sn, &cs);
+						const float xr = y[r].x, xi = cj * y[r].y;
+						((float2 *)a.spec + obase + c)[(int64_t)row0 * nchan] = make_float2(xr * cs - xi * sn, xr * sn + xi * cs);
 					}
 				}
 			}

@@ -267,20 +267,14 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 		// every load is on its way before the first value is used.  A word holds the
 		// fields of both bands (adj: side by side), or each band has a word of its own
 		const uint32_t apart = MUX ? 0u : I.boff1 - I.boff0;         // bits from the first band's field to the second's
-		auto levels = [&](int r, uint32_t w0, uint32_t w1) {
-			if(nbits == 2)
-			{
-				lv[r] = lut4[(w0 & 3u) | ((w1 & 3u) << 2)];
-				if constexpr(CPLX)
-					lu[r] = lut4[((w0 >> 2) & 3u) | (w1 & 12u)];
-			}
-			else
-			{
-				lv[r] = pk2(lut8[w0 & 255u], lut8[w1 & 255u]);
-				if constexpr(CPLX)
-					lu[r] = pk2(lut8[(w0 >> 8) & 255u], lut8[(w1 >> 8) & 255u]);
-			}
+		// (the same code for 2 and 8 bits: kernels of many lengths fetch it over and over)
+		auto levels = [&](int r, const float *tab, uint32_t w0, uint32_t w1) {
+			const uint32_t mask = (1u << nbits) - 1u;
+			lv[r] = pk2(tab[w0 & mask], tab[w1 & mask]);
+			if constexpr(CPLX)
+				lu[r] = pk2(tab[(w0 >> nbits) & mask], tab[(w1 >> nbits) & mask]);
 		};
+		auto table = [&]() { return lut8 + (nbits == 2 ? 256 : 0); };
 		if(!MUX && (flags & kPFast))
 		{
 			// one running bit position: a frame boundary skips a header
@@ -312,7 +306,17 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 					sh[r] = bit & 31u;
 					step();
 				}
-				if(!CPLX && nbits == 2)
+				if constexpr(CPLX)
+				{
+					const float *tab = table();
+#pragma unroll
+					for(int r = 0; r < 8; r++)
+					{
+						const uint32_t w = raw[r] >> sh[r];
+						levels(r, tab, w, w >> apart);
+					}
+				}
+				else if(nbits == 2)
 				{
 #pragma unroll
 					for(int r = 0; r < 8; r++)
@@ -324,7 +328,7 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 					for(int r = 0; r < 8; r++)
 					{
 						const uint32_t w = raw[r] >> sh[r];
-						levels(r, w, w >> apart);
+						lv[r] = pk2(lut8[w & 255u], lut8[(w >> 8) & 255u]);
 					}
 				}
 			}
@@ -339,9 +343,10 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 					sh[r] = bit & 31u;
 					step();
 				}
+				const float *tab = table();
 #pragma unroll
 				for(int r = 0; r < 8; r++)
-					levels(r, raw[r] >> sh[r], raw1[r] >> ((sh[r] + apart) & 31u));
+					levels(r, tab, raw[r] >> sh[r], raw1[r] >> ((sh[r] + apart) & 31u));
 			}
 		}
 		else if(MUX && (flags & kPFast))
@@ -361,11 +366,12 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 				raw1[r] = __ldg((const uint32_t *)(second ? f11 : f01) + (bit >> 5));
 				sh[r] = bit & 31u;
 			}
+			const float *tab = table();
 #pragma unroll
 			for(int r = 0; r < 8; r++)
-				levels(r, raw0[r] >> sh[r], raw1[r] >> sh[r]);
+				levels(r, tab, raw0[r] >> sh[r], raw1[r] >> sh[r]);
 		}
-		else
+		else if(flags & kPActive)
 		{
 			// frames, validity and blanking sample by sample
 			const bool narrow = (flags & kPNarrow) != 0, blank = (flags & kPBlank) != 0;
@@ -386,7 +392,7 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 				if(narrow)
 					ok = (fc.fmask >> kf) & 1u;
 				else
-					ok = (flags & kPActive) && fr < a.valid_stride && vrow[fr] != 0;
+					ok = fr < a.valid_stride && vrow[fr] != 0;
 				ok = ok && n < fc.stuck;
 				const uint32_t bit = tin * bpt + I.boff0;
 				if constexpr(MUX)
@@ -411,6 +417,7 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 						fp += I.framebytes;
 				}
 			}
+			const float *tab = table();
 #pragma unroll
 			for(int r = 0; r < 8; r++)
 			{
@@ -420,7 +427,7 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 				if(!(pk[r] & 32u))
 					continue;
 				const uint32_t sh0 = pk[r] & 31u;
-				levels(r, raw0[r] >> sh0, (oneword ? raw0[r] : raw1[r]) >> ((sh0 + apart) & 31u));
+				levels(r, tab, raw0[r] >> sh0, (oneword ? raw0[r] : raw1[r]) >> ((sh0 + apart) & 31u));
 				if(blank)
 				{
 					// bands of this sample's frame blanked by its EDV4 validity mask
@@ -435,6 +442,18 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 						lu[r] = pk2(v0 ? u.x : 0.0f, v1 ? u.y : 0.0f);
 					}
 				}
+			}
+		}
+		else
+		{
+			// no FFT, or past T: nothing to read (as windows without a valid frame these
+			// slots kept the last unit waiting for code that nothing else ran)
+#pragma unroll
+			for(int r = 0; r < 8; r++)
+			{
+				lv[r] = 0ull;
+				if constexpr(CPLX)
+					lu[r] = 0ull;
 			}
 		}
 		// ---- 2. fringe rotation (order 1: the rotator of sample b, then one
@@ -544,18 +563,28 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 		// aligned pair take both bands in one store.
 		auto quad = [&](uint32_t p0, uint4 v0, uint4 v1) {
 			uint32_t *o = (uint32_t *)a.spec + base;
-			const uint32_t bextra = I.bextra, magic = I.magic;
-			if(oflags & kOBoth)
+			const uint32_t bextra = I.bextra;
+			if(oflags & kOWide)
 			{
-				uint32_t *q = o + p0 + (p0 >> 1) * bextra;
-				*(uint4 *)q = make_uint4(v0.x, v0.y, v1.x, v1.y);
-				*(uint4 *)(q + bextra + 2) = make_uint4(v0.z, v0.w, v1.z, v1.w);
-				return;
+				o += p0 + (p0 >> I.shift) * bextra;
+				if(oflags & kORow0)
+					*(uint4 *)o = v0;
+				if(oflags & kORow1)
+					*(uint4 *)(o + rowd) = v1;
 			}
-			if(oflags & kORow0)
-				store_quad(o, p0, I.tcb, magic, bextra, v0);
-			if(oflags & kORow1)
-				store_quad(o + rowd, p0, I.tcb, magic, bextra, v1);
+			else if(oflags & kOBoth)
+			{
+				o += p0 + (p0 >> 1) * bextra;
+				*(uint4 *)o = make_uint4(v0.x, v0.y, v1.x, v1.y);
+				*(uint4 *)(o + bextra + 2) = make_uint4(v0.z, v0.w, v1.z, v1.w);
+			}
+			else
+			{
+				if(oflags & kORow0)
+					store_quad(o, p0, I.tcb, I.magic, bextra, v0);
+				if(oflags & kORow1)
+					store_quad(o + rowd, p0, I.tcb, I.magic, bextra, v1);
+			}
 		};
 		auto packed = [&](const cp &y, uint32_t &h0, uint32_t &h1) {
 			const float2 re = up2(y.re), im = up2(y.im);
@@ -730,10 +759,12 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 				for(int m = 0; m < 4; m++)
 					packed(y[m], h0[m], h1[m]);
 				const uint32_t p = 4u * (uint32_t)b;
-				if(!mirror || b > 0)
-					quad(mirror ? (uint32_t)(N / 2) - p : p,
-					     make_uint4(mirror ? h0[3] : h0[0], mirror ? h0[2] : h0[1], mirror ? h0[1] : h0[2], mirror ? h0[0] : h0[3]),
-					     make_uint4(mirror ? h1[3] : h1[0], mirror ? h1[2] : h1[1], mirror ? h1[1] : h1[2], mirror ? h1[0] : h1[3]));
+				const uint4 up0 = make_uint4(h0[0], h0[1], h0[2], h0[3]), up1 = make_uint4(h1[0], h1[1], h1[2], h1[3]);
+				const uint4 dn0 = make_uint4(h0[3], h0[2], h0[1], h0[0]), dn1 = make_uint4(h1[3], h1[2], h1[1], h1[0]);
+				if(!mirror)
+					quad(p, up0, up1);
+				else if(b > 0)
+					quad((uint32_t)(N / 2) - p, dn0, dn1);
 				else
 				{
 					// beside channel 0 (bin N/2, above)
@@ -828,11 +859,13 @@ __device__ __forceinline__ void pair_units(PairFeed<NFC> &s, const FsMultiArgs &
 	}
 }
 
-// the level pairs of two adjacent 2-bit bands, and the 8-bit levels
+// the level pairs of two adjacent 2-bit bands, and the 8-bit and 2-bit levels
 __device__ __forceinline__ void fstage_pair_luts(float *lut8, u64 *lut4)
 {
 	for(int i = threadIdx.x; i < 256; i += blockDim.x)
 		lut8[i] = (float)((i - 128) / 3.3);
+	if(threadIdx.x < 4)
+		lut8[256 + threadIdx.x] = level2(threadIdx.x);
 	if(threadIdx.x < 16)
 		lut4[threadIdx.x] = pk2(level2(threadIdx.x & 3u), level2(threadIdx.x >> 2u));
 }

@@ -15,7 +15,6 @@ struct DevFreqPlan {
 	int32_t tnblk;                    // tensor-core form: blocks per time, spectra [t][block][trow][tcb]
 	int32_t trow;                     // tensor-core form: rows of a block (nrow and, in the FP16 / BF16 form, zero rows)
 	int32_t pbits;                    // tensor-core form: log2(nchan / 4), see chan_pos
-	uint32_t magic;                   // tensor-core form: p / tcb = umulhi(p, magic) for p < 2^16
 	int32_t acc_cstride;              // accumulator stride between channels (1: [out][chan], nout: [chan][out])
 	int32_t acc_ostride;              // accumulator stride between outputs
 	int64_t spec_off;                 // complex offset of this frequency's spectra
@@ -25,6 +24,7 @@ struct DevFreqPlan {
 	const int32_t *outsrc;            // [nout] source of each output: a | b << 8 | conj << 16 (a <= b), or -1
 	int64_t spec8_off;                // FP8 form: offset (16-bit words) of this frequency's e4m3 spectra
 	float *iscale;                    // FP8 form: [nchan][nrow] 1 / quantisation scale of the subint
+	uint32_t magic;                   // tensor-core form: p / tcb = umulhi(p, magic) for p < 2^16
 };
 
 struct DevOutMap {
@@ -205,14 +205,20 @@ struct alignas(16) PairItem {
 	int64_t rowd;                        // from the first band's values to the second's
 	uint32_t tcb, magic, bextra;         // channels of a block; p / tcb = umulhi(p, magic) for p < 2^16;
 	                                     // position p sits at p + p / tcb x bextra
-	int32_t oflags;
+	int32_t shift, oflags;               // shift: log2 tcb (kOWide)
 	uint32_t fs, bpt, boff0, boff1;      // samples per frame, bits per time, first bit of each band
 	uint32_t hbits;                      // header bits
 	int32_t nbits, header, framebytes, minfb, mnthr;
 	int32_t station, band0, band1, lsb, asl, adj;   // adj: both bands side by side in one aligned field
 	int32_t group, two;                  // two: the bands' LOs differ
 };
-enum : int32_t { kORow0 = 1, kORow1 = 2, kOH16 = 4, kOBoth = 8 };
+enum : int32_t {
+	kORow0 = 1,       // the band has a row
+	kORow1 = 2,
+	kOH16 = 4,        // FP16 (else BF16)
+	kOBoth = 8,       // blocks of two channels, the bands' rows an aligned pair
+	kOWide = 16       // blocks of a power of two channels, at least 4
+};
 enum : int32_t {
 	kPActive = 1,     // valid FFT
 	kPNarrow = 2,     // fmask covers the window
