@@ -217,18 +217,10 @@ __global__ void __launch_bounds__(128) k_pair_consts(const FsArgs a, int N, int 
 		}
 		if(g.clk[1] != g.clk[0] || c.post[1] != c.post[0])
 			c.flags &= ~kPSame;
-		// validity of the window's frames, one bit per frame relative to fa
-		const uint32_t nwf = (c.so + (uint32_t)N - 1) / fs + 1, nm = nwf < 32u ? nwf : 32u;
-		for(uint32_t k = 0; k < nm; k++)
-		{
-			const int64_t fr = (int64_t)c.fa + k;
-			// complex data: the unpack's first frame is checked for fill
-			// pattern only (mark5_stream_unpacker.c:189)
-			const uint8_t *vsrc = (cplx && k == 0 && a.fillok) ? a.fillok + (int64_t)I.station * a.valid_stride : vrow;
-			if(fr < a.valid_stride && vsrc[fr] != 0)
-				c.fmask |= 1u << k;
-		}
-		if(nwf <= 32)
+		// validity of the window's frames, one bit per frame relative to fa (k_fft_params)
+		const uint32_t nwf = (c.so + (uint32_t)N - 1) / fs + 1;
+		c.fmask = pq->fmask;
+		if(pq->mflags & 1)
 			c.flags |= kPNarrow;
 		if(a.bandok)
 		{
