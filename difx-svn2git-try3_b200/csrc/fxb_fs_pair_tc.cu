@@ -236,7 +236,7 @@ __global__ void __launch_bounds__(128) k_pair_consts(const FsArgs a, int N, int 
 		}
 		const bool whole = nwf < 32 && c.fmask == (1u << nwf) - 1u && c.stuck >= N && !(c.flags & kPBlank);
 		if(!mux && whole && fs >= (uint32_t)S8)
-			c.flags |= kPFast;
+			c.flags |= I.adj ? kPFast : kPApart;
 		if(mux && whole && nwf <= 2)
 		{
 			// valid frames of raw reads are complete slots: every thread is there

@@ -264,9 +264,8 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 		// ---- 1. decode: the levels of samples b + r N/8 of both bands
 		u64 lv[8], lu[CPLX ? 8 : 1];        // lu: imaginary parts (complex sampling)
 		const uint32_t xs = fc.so + (uint32_t)b;
-		// every load is on its way before the first value is used.  A word holds the
-		// fields of both bands (adj: side by side), or each band has a word of its own
-		const uint32_t apart = MUX ? 0u : I.boff1 - I.boff0;         // bits from the first band's field to the second's
+		// Every load is on its way before the first value is used.  A word holds the
+		// fields of both bands side by side, or each band has a word of its own.
 		// (the same code for 2 and 8 bits: kernels of many lengths fetch it over and over)
 		auto levels = [&](int r, const float *tab, uint32_t w0, uint32_t w1) {
 			const uint32_t mask = (1u << nbits) - 1u;
@@ -286,7 +285,13 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 				tin -= fs;
 				bit += hbits;
 			}
-			auto step = [&]() {
+			const uint32_t *wp = (const uint32_t *)fc.wp;
+			uint32_t raw[8], sh[8];
+#pragma unroll
+			for(int r = 0; r < 8; r++)
+			{
+				raw[r] = __ldg(wp + (bit >> 5));
+				sh[r] = bit & 31u;
 				tin += S8;
 				bit += S8 * bpt;
 				if(tin >= fs)
@@ -294,59 +299,32 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 					tin -= fs;
 					bit += hbits;
 				}
-			};
-			const uint32_t *wp = (const uint32_t *)fc.wp;
-			if(I.adj)
+			}
+			if constexpr(CPLX)
 			{
-				uint32_t raw[8], sh[8];
+				const float *tab = table();
+				const uint32_t apart = I.boff1 - I.boff0;
 #pragma unroll
 				for(int r = 0; r < 8; r++)
 				{
-					raw[r] = __ldg(wp + (bit >> 5));
-					sh[r] = bit & 31u;
-					step();
+					const uint32_t w = raw[r] >> sh[r];
+					levels(r, tab, w, w >> apart);
 				}
-				if constexpr(CPLX)
-				{
-					const float *tab = table();
+			}
+			else if(nbits == 2)
+			{
 #pragma unroll
-					for(int r = 0; r < 8; r++)
-					{
-						const uint32_t w = raw[r] >> sh[r];
-						levels(r, tab, w, w >> apart);
-					}
-				}
-				else if(nbits == 2)
-				{
-#pragma unroll
-					for(int r = 0; r < 8; r++)
-						lv[r] = lut4[(raw[r] >> sh[r]) & 15u];
-				}
-				else
-				{
-#pragma unroll
-					for(int r = 0; r < 8; r++)
-					{
-						const uint32_t w = raw[r] >> sh[r];
-						lv[r] = pk2(lut8[w & 255u], lut8[(w >> 8) & 255u]);
-					}
-				}
+				for(int r = 0; r < 8; r++)
+					lv[r] = lut4[(raw[r] >> sh[r]) & 15u];
 			}
 			else
 			{
-				uint32_t raw[8], raw1[8], sh[8];
 #pragma unroll
 				for(int r = 0; r < 8; r++)
 				{
-					raw[r] = __ldg(wp + (bit >> 5));
-					raw1[r] = __ldg(wp + ((bit + apart) >> 5));
-					sh[r] = bit & 31u;
-					step();
+					const uint32_t w = raw[r] >> sh[r];
+					lv[r] = pk2(lut8[w & 255u], lut8[(w >> 8) & 255u]);
 				}
-				const float *tab = table();
-#pragma unroll
-				for(int r = 0; r < 8; r++)
-					levels(r, tab, raw[r] >> sh[r], raw1[r] >> ((sh[r] + apart) & 31u));
 			}
 		}
 		else if(MUX && (flags & kPFast))
@@ -371,6 +349,37 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 			for(int r = 0; r < 8; r++)
 				levels(r, tab, raw0[r] >> sh[r], raw1[r] >> sh[r]);
 		}
+		else if(!MUX && (flags & kPApart))
+		{
+			// the same with a word for each band
+			const uint32_t hbits = I.hbits, apart = I.boff1 - I.boff0;
+			uint32_t tin = xs, bit = xs * bpt + I.boff0;
+			if(tin >= fs)
+			{
+				tin -= fs;
+				bit += hbits;
+			}
+			const uint32_t *wp = (const uint32_t *)fc.wp;
+			uint32_t raw0[8], raw1[8], sh[8];
+#pragma unroll
+			for(int r = 0; r < 8; r++)
+			{
+				raw0[r] = __ldg(wp + (bit >> 5));
+				raw1[r] = __ldg(wp + ((bit + apart) >> 5));
+				sh[r] = bit & 31u;
+				tin += S8;
+				bit += S8 * bpt;
+				if(tin >= fs)
+				{
+					tin -= fs;
+					bit += hbits;
+				}
+			}
+			const float *tab = table();
+#pragma unroll
+			for(int r = 0; r < 8; r++)
+				levels(r, tab, raw0[r] >> sh[r], raw1[r] >> ((sh[r] + apart) & 31u));
+		}
 		else if(flags & kPActive)
 		{
 			// frames, validity and blanking sample by sample
@@ -380,6 +389,7 @@ __device__ __forceinline__ void fstage_pair_unit(const FsArgs &a, const PairItem
 			const int32_t *mslot = MUX ? a.sub[station].mux_slot : nullptr;
 			const int64_t mk0 = MUX ? a.sub[station].mux_k0 : 0;
 			const bool oneword = !MUX && bpt <= 32;              // all bands of a sample time in one word
+			const uint32_t apart = MUX ? 0u : I.boff1 - I.boff0;
 			uint32_t kf = xs / fs, tin = xs - kf * fs;
 			const uint8_t *fp = MUX ? buf + 32 : buf + ((int64_t)fc.fa + kf) * I.framebytes + I.header;
 			uint32_t raw0[8], raw1[8], pk[8];

@@ -225,7 +225,9 @@ enum : int32_t {
 	kPBlank = 4,      // a valid frame of the window blanks one of the item's bands
 	kPSame = 8,       // the two bands take the same output rotation
 	kPTwo = 32,       // the bands take different fringe rotations
-	kPFast = 16       // every sample of the window counts, frames of at least N/8 samples (raw reads: at most two)
+	kPFast = 16,      // every sample of the window counts, frames of at least N/8 samples, bands side by
+	                  // side; raw reads: at most two frames
+	kPApart = 64      // the same with the bands apart
 };
 
 struct FsArgs {
