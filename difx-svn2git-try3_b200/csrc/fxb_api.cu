@@ -102,6 +102,7 @@ struct fxb_ctx {
 	bool all_tcfft = false;             // every F kind runs the tensor-core FFT
 	cudaEvent_t fork = nullptr;         // of a graph's branch of timing events (mark)
 	bool stations_set = false;          // d_st written on the stream since the last preparation beside it
+	int64_t nsubmit = 0, nbeside = 0;   // subints submitted, and those prepared beside earlier ones
 	mutable bool exposed = false;       // the caller has the stream (fxb_get_stream)
 	// device memory comes from this pool (a server's, whose memory stays
 	// mapped between jobs) or, when null, the device's default pool; every
@@ -1793,6 +1794,8 @@ static fxb_status submit(fxb_ctx *ctx, const uint8_t *const *bufs, const int64_t
 	sl.tpending = ctx->timing_on;
 	ctx->last_slot = (int)(slp - ctx->slots.data());
 	ctx->timed = true;
+	ctx->nsubmit++;
+	ctx->nbeside += beside;
 	return FXB_OK;
 }
 
@@ -1898,6 +1901,12 @@ fxb_status fxb_tuning_report(const fxb_ctx *ctx, char *buf, size_t len, size_t *
 				r += line;
 			}
 		r += "\n";
+	}
+	if(ctx->nsubmit > 0)
+	{
+		snprintf(line, sizeof(line), "preparation: %lld of %lld subints beside earlier ones\n", (long long)ctx->nbeside,
+		         (long long)ctx->nsubmit);
+		r += line;
 	}
 	if(needed)
 		*needed = r.size() + 1;

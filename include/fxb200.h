@@ -238,8 +238,9 @@ FXB_API fxb_status fxb_set_graphs(fxb_ctx *ctx, int32_t on);
  * as many FFT iterations per CTA as leave two CTAs per SM. */
 FXB_API fxb_status fxb_autotune(fxb_ctx *ctx, int32_t rounds);
 /* The current choices (and, after tuning, each candidate's fastest time) as
- * text, one line per F-stage kind and XMAC group; *needed = bytes with the
- * terminating 0. */
+ * text, one line per F-stage kind and XMAC group, and of the submitted subints
+ * how many were prepared beside earlier ones (fxb_get_stream); *needed = bytes
+ * with the terminating 0. */
 FXB_API fxb_status fxb_tuning_report(const fxb_ctx *ctx, char *buf, size_t len, size_t *needed);
 
 /* Batches: contexts whose subints are submitted together, e.g. one context
