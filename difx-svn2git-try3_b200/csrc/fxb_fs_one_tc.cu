@@ -33,7 +33,7 @@ constexpr size_t kNarrowSide = 18432;            // exchange buffer: 2048 points
 constexpr size_t kMidSide = 36864;               // 4096 points
 constexpr size_t kWideSmem = 73728;              // 8192 points of one band, padded
 
-// Work-list class 6 VAR + 5: every length up to 2048 points in CTAs of 256
+// Work-list class 7 VAR + 5: every length up to 2048 points in CTAs of 256
 // threads (the shape of k_fstage for those lengths), one exchange buffer per
 // unit (three CTAs per SM): faster than two buffers at two CTAs per SM on every
 // length measured.  VAR 0: plain VDIF, 1: raw INTERLACEDVDIF reads.
@@ -67,7 +67,7 @@ __global__ void __launch_bounds__(256, 3) k_fstage_pn(const __grid_constant__ Fs
 	}
 }
 
-// 4096 points (class 6 VAR + 3) in CTAs of 256 threads, 8192 (class 6 VAR + 1) of 512
+// 4096 points (class 7 VAR + 3) in CTAs of 256 threads, 8192 (class 7 VAR + 1) of 512
 template <int VAR, int LOGN>
 __global__ void __launch_bounds__(FShape<LOGN>::NT, LOGN == 12 ? 3 : 2) k_fstage_pw(const __grid_constant__ FsMultiArgs m)
 {

@@ -35,7 +35,7 @@ static void launch_t(const FKind &k, const FsArgs &a, cudaStream_t stream)
 
 constexpr size_t kPairSide = 2304 * 16;          // exchange buffers of 2048 points in all, padded
 
-// Work-list class 6 VAR + 4: every length up to 2048 points in CTAs of 256
+// Work-list class 7 VAR + 6: every length up to 1024 points in CTAs of 256
 // threads.  VAR 0: plain VDIF, 1: raw INTERLACEDVDIF reads.
 template <int VAR>
 __global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant__ FsMultiArgs m)
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant
 	__shared__ u64 lut4[16];
 	__shared__ PairFeed<kFsMultiFc> feed;
 	fstage_pair_luts(lut8, lut4);
-	pair_units(feed, m, kFsMultiPer * VAR + 4,
+	pair_units(feed, m, kFsMultiPer * VAR + 6,
 	           [&](const FsMultiUnit &w, const PairItem &I, const PairConst *fcs, const PairTwist *tws) {
 		const FsMultiKind &k = m.kinds[w.kind];
 		const float2 *tw = (const float2 *)k.tw;
@@ -63,14 +63,16 @@ __global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant
 			FXB_PAIR_CASE(8)
 			FXB_PAIR_CASE(9)
 			FXB_PAIR_CASE(10)
-			FXB_PAIR_CASE(11)
 #undef FXB_PAIR_CASE
 		default: break;
 		}
 	});
 }
 
-// 4096 points (class 6 VAR + 2) in CTAs of 512 threads, 8192 (class 6 VAR) of 1024
+// One length: 2048 points (class 7 VAR + 4) in CTAs of 256 threads, 4096 (class 7 VAR +
+// 2) of 512, 8192 (class 7 VAR) of 1024.  (2048 points among the others' code, 10
+// stations x 2 subbands x 2 bands of 8 bits: F stage 89 us, 81 here; 16 threads read raw
+// 311 and 289.)
 template <int VAR, int LOGN>
 __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB)
     k_fstage_pair_pw(const __grid_constant__ FsMultiArgs m)
@@ -80,7 +82,7 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB)
 	__shared__ u64 lut4[16];
 	__shared__ PairFeed<kMaxTQ> feed;
 	fstage_pair_luts(lut8, lut4);
-	pair_units(feed, m, kFsMultiPer * VAR + (LOGN == 12 ? 2 : 0),
+	pair_units(feed, m, kFsMultiPer * VAR + 2 * (13 - LOGN),
 	           [&](const FsMultiUnit &w, const PairItem &I, const PairConst *fcs, const PairTwist *tws) {
 		           const FsMultiKind &k = m.kinds[w.kind];
 		           fstage_pair_unit<LOGN, true, VAR>(m.m[k.member], I, fcs, tws, w.t0, w.nfc, (const float2 *)k.tw, fsp, lut8,
@@ -91,8 +93,10 @@ __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB)
 template <int VAR>
 static void launch_cls(const FsMultiArgs &m, int c, int nsm, cudaStream_t st)
 {
-	if(c == 4)
+	if(c == 6)
 		fs_launch_persistent(k_fstage_pair_pn<VAR>, m, kFsMultiPer * VAR + c, 3 * nsm, 256, kPairSide, st);
+	else if(c == 4)
+		fs_launch_persistent(k_fstage_pair_pw<VAR, 11>, m, kFsMultiPer * VAR + c, 3 * nsm, 256, kPairSide, st);
 	else if(c == 2)
 		fs_launch_persistent(k_fstage_pair_pw<VAR, 12>, m, kFsMultiPer * VAR + c, 2 * nsm, 512, 2 * kPairSide, st);
 	else

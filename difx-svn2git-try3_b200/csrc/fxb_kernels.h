@@ -176,11 +176,14 @@ constexpr int kTcSpecExp = 5;
 
 // Two-band items (csrc/fxb_fstage_pair.cuh).  Constants of one FFT of one item,
 // computed by k_pair_consts with the subint's FFT parameters.
+// In this order without gaps: with gaps they took 128 (twists 48) bytes, written and
+// read once per item and FFT (20 stations x 4 subbands x 4096 FFTs of 256 points: the
+// preparation kernels 41.7 us, 38.8 without).
 struct alignas(16) PairConst {
 	float P0, alpha, beta, gamma;        // fringe phase (turns): start and per-sample terms
 	float eps;
-	float2 st;                           // order 1: rotator step over N/8 samples, exp(-2 pi i alpha N/8)
 	int32_t flags;
+	float2 st;                           // order 1: rotator step over N/8 samples, exp(-2 pi i alpha N/8)
 	float dhi[2], dlo[2];                // fractional-sample turns per channel of each band (split_turns)
 	float2 os[2];                        // rotator step over N/8 channels of each band
 	float post[2];                       // order-0 post-F turns and the band's phase offset
@@ -192,11 +195,12 @@ struct alignas(16) PairConst {
 };
 // kPTwo: the second band's fringe rotation, in an array of its own
 struct alignas(16) PairTwist {
+	float2 st;
 	float P0, alpha, beta, gamma;
 	float eps;
-	float2 st;
 	int32_t pad_;
 };
+static_assert(sizeof(PairConst) == 112 && sizeof(PairTwist) == 32, "no gaps");
 // What does not change from subint to subint: the samples' place in the frames
 // and the spectra's place.  FP32 form [t][row][chan]; tensor-core form blocked
 // [t][block][trow][tcb] in the order of chan_pos.
@@ -276,9 +280,9 @@ void launch_fstage_kind(const FKind &k, FsArgs a, cudaStream_t stream);
 // units.  Every tensor-core-form context runs these kinds this way, alone or in
 // a batch, so results do not depend on it.
 constexpr int kFsMultiMembers = 16;
-constexpr int kFsMultiFc = 64;           // FFT constants of one unit of up to 2048 points at most (tq x fpc)
+constexpr int kFsMultiFc = 64;           // FFT constants of one unit of several lengths' launches at most (tq x fpc)
 // classes of units: plain VDIF's (fstage_multi_class), then those of raw reads
-constexpr int kFsMultiPer = 6, kFsMultiClasses = 2 * kFsMultiPer;
+constexpr int kFsMultiPer = 7, kFsMultiClasses = 2 * kFsMultiPer;
 struct FsMultiKind {
 	const void *tw;                      // twiddles of length N
 	int32_t member, code;                // context; 128 x raw INTERLACEDVDIF reads + 32 x bands per item + log2 N
@@ -299,9 +303,9 @@ struct FsMultiArgs {
 	int32_t *ctr;                        // one counter per class, zero before the launch
 };
 // class of a kind (FFT length N, bands per item nb) in the persistent launches
-// (0: two bands of 8192 points, 1: one band of 8192, 2: two bands of 4096, 3: one
-// band of 4096, 4: two bands of up to 2048, 5: one band of up to 2048; -1: not run
-// there), and the FFT iterations per unit for a kind's tq
+// (two bands of 8192 points: 0, 4096: 2, 2048: 4, up to 1024: 6; one band of 8192: 1,
+// 4096: 3, up to 2048: 5; -1: not run there), and the FFT iterations per unit for a
+// kind's tq
 int fstage_multi_class(int N, int nb);
 int fstage_multi_tq(int N, int nb, int tq);
 cudaError_t launch_fstage_multi(const FsMultiArgs &m, int nsm, cudaStream_t stream);
