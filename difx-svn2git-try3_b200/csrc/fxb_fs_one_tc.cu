@@ -29,53 +29,26 @@ static void launch_t(const FKind &k, const FsArgs &a, cudaStream_t stream)
 	k_fstage<LOGN, TCO, VAR><<<fstage_grid(k, a), k.threads, k.smem, stream>>>(a);
 }
 
-constexpr size_t kNarrowSide = 18432;            // exchange buffer: 2048 points of one band, padded
-constexpr size_t kMidSide = 36864;               // 4096 points
-constexpr size_t kWideSmem = 73728;              // 8192 points of one band, padded
+// CTAs per SM of a persistent launch: one exchange buffer each, three up to 4096
+// points (faster than two buffers at two CTAs per SM on every length measured)
+template <int LOGN>
+struct OneShape {
+	static constexpr int MINB = LOGN <= 12 ? 3 : 2;
+};
 
-// Work-list class 7 VAR + 5: every length up to 2048 points in CTAs of 256
-// threads (the shape of k_fstage for those lengths), one exchange buffer per
-// unit (three CTAs per SM): faster than two buffers at two CTAs per SM on every
-// length measured.  VAR 0: plain VDIF, 1: raw INTERLACEDVDIF reads.
-template <int VAR>
-__global__ void __launch_bounds__(256, 3) k_fstage_pn(const __grid_constant__ FsMultiArgs m)
-{
-	extern __shared__ __align__(16) uint2 fsm[];
-	__shared__ float lut8[256];
-	__shared__ FftConst fcs[kFsMultiFc];
-	__shared__ int unit_s[2];
-	constexpr int cls = kFsMultiPer * VAR + 5;
-	fstage_luts(lut8);
-	UnitFeed feed(m.ctr + cls, unit_s);
-	for(int u = feed.first(); u < m.nunit[cls]; u = feed.next())
-	{
-		const FsMultiUnit w = m.units[m.unit0[cls] + u];
-		const FsMultiKind k = m.kinds[w.kind];
-		const float2 *tw = (const float2 *)k.tw;
-		const int gi = k.first + w.item;
-		switch(k.code & 31)
-		{
-		case 5: fstage_unit<5, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, 0, tw, fsm, lut8, fcs); break;
-		case 6: fstage_unit<6, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, 0, tw, fsm, lut8, fcs); break;
-		case 7: fstage_unit<7, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, 0, tw, fsm, lut8, fcs); break;
-		case 8: fstage_unit<8, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, 0, tw, fsm, lut8, fcs); break;
-		case 9: fstage_unit<9, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, 0, tw, fsm, lut8, fcs); break;
-		case 10: fstage_unit<10, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, 0, tw, fsm, lut8, fcs); break;
-		case 11: fstage_unit<11, true, VAR>(m.m[k.member], gi, w.tchunk, k.tq, 0, tw, fsm, lut8, fcs); break;
-		default: break;
-		}
-	}
-}
-
-// 4096 points (class 7 VAR + 3) in CTAs of 256 threads, 8192 (class 7 VAR + 1) of 512
+// The units of one length (class 2 (13 - LOGN) + 1 of VAR 0: plain VDIF, 1: raw
+// INTERLACEDVDIF reads), each in a kernel of its own: 14 stations x 1 band of 8 bits, F
+// stage among the other lengths' code and alone, 4096 points 137 and 124 us, 2048
+// points 82 and 68.
 template <int VAR, int LOGN>
-__global__ void __launch_bounds__(FShape<LOGN>::NT, LOGN == 12 ? 3 : 2) k_fstage_pw(const __grid_constant__ FsMultiArgs m)
+__global__ void __launch_bounds__(FShape<LOGN>::NT, OneShape<LOGN>::MINB) k_fstage_pw(const __grid_constant__ FsMultiArgs m)
 {
 	extern __shared__ __align__(16) uint2 fsm[];
+	constexpr int FPC = FShape<LOGN>::FPC, NFC = kMaxTQ * FPC < kFsMultiFc ? kMaxTQ * FPC : kFsMultiFc;
 	__shared__ float lut8[256];
-	__shared__ FftConst fcs[kMaxTQ];
+	__shared__ FftConst fcs[NFC];
 	__shared__ int unit_s[2];
-	constexpr int cls = kFsMultiPer * VAR + (LOGN == 12 ? 3 : 1);
+	constexpr int cls = kFsMultiPer * VAR + 2 * (13 - LOGN) + 1;
 	fstage_luts(lut8);
 	UnitFeed feed(m.ctr + cls, unit_s);
 	for(int u = feed.first(); u < m.nunit[cls]; u = feed.next())
@@ -86,15 +59,29 @@ __global__ void __launch_bounds__(FShape<LOGN>::NT, LOGN == 12 ? 3 : 2) k_fstage
 	}
 }
 
+template <int VAR, int LOGN>
+static void launch_len(const FsMultiArgs &m, int nsm, cudaStream_t st)
+{
+	using SH = FShape<LOGN>;
+	fs_launch_persistent(k_fstage_pw<VAR, LOGN>, m, kFsMultiPer * VAR + 2 * (13 - LOGN) + 1, OneShape<LOGN>::MINB * nsm,
+	                     SH::NT, (size_t)SH::FPC * SH::PADN * 8, st);
+}
+
 template <int VAR>
 static void launch_cls(const FsMultiArgs &m, int c, int nsm, cudaStream_t st)
 {
-	if(c == 5)
-		fs_launch_persistent(k_fstage_pn<VAR>, m, kFsMultiPer * VAR + c, 3 * nsm, 256, kNarrowSide, st);
-	else if(c == 3)
-		fs_launch_persistent(k_fstage_pw<VAR, 12>, m, kFsMultiPer * VAR + c, 3 * nsm, 256, kMidSide, st);
-	else
-		fs_launch_persistent(k_fstage_pw<VAR, 13>, m, kFsMultiPer * VAR + c, 2 * nsm, 512, kWideSmem, st);
+	switch(13 - c / 2)
+	{
+	case 5: launch_len<VAR, 5>(m, nsm, st); break;
+	case 6: launch_len<VAR, 6>(m, nsm, st); break;
+	case 7: launch_len<VAR, 7>(m, nsm, st); break;
+	case 8: launch_len<VAR, 8>(m, nsm, st); break;
+	case 9: launch_len<VAR, 9>(m, nsm, st); break;
+	case 10: launch_len<VAR, 10>(m, nsm, st); break;
+	case 11: launch_len<VAR, 11>(m, nsm, st); break;
+	case 12: launch_len<VAR, 12>(m, nsm, st); break;
+	default: launch_len<VAR, 13>(m, nsm, st); break;
+	}
 }
 
 void launch_fs_one_multi(const FsMultiArgs &m, int cls, int nsm, cudaStream_t st)

@@ -33,74 +33,52 @@ static void launch_t(const FKind &k, const FsArgs &a, cudaStream_t stream)
 	k_fstage_pair<LOGN, TCO, VAR><<<fstage_grid(k, a), k.threads, k.smem, stream>>>(a);
 }
 
-constexpr size_t kPairSide = 2304 * 16;          // exchange buffers of 2048 points in all, padded
-
-// Work-list class 7 VAR + 6: every length up to 1024 points in CTAs of 256
-// threads.  VAR 0: plain VDIF, 1: raw INTERLACEDVDIF reads.
-template <int VAR>
-__global__ void __launch_bounds__(256, 3) k_fstage_pair_pn(const __grid_constant__ FsMultiArgs m)
-{
-	extern __shared__ __align__(16) ulonglong2 fsp[];
-	__shared__ float lut8[260];
-	__shared__ u64 lut4[16];
-	__shared__ PairFeed<kFsMultiFc> feed;
-	fstage_pair_luts(lut8, lut4);
-	pair_units(feed, m, kFsMultiPer * VAR + 6,
-	           [&](const FsMultiUnit &w, const PairItem &I, const PairConst *fcs, const PairTwist *tws) {
-		const FsMultiKind &k = m.kinds[w.kind];
-		const float2 *tw = (const float2 *)k.tw;
-		const FsArgs &a = m.m[k.member];
-		switch(k.code & 31)
-		{
-#define FXB_PAIR_CASE(LOGN)                                                                                            \
-	case LOGN:                                                                                                         \
-		fstage_pair_unit<LOGN, true, VAR>(a, I, fcs, tws, w.t0, (w.nfc + PShape<LOGN>::FPC - 1) / PShape<LOGN>::FPC, tw, \
-		                                  fsp, lut8, lut4);                                                             \
-		break;
-			FXB_PAIR_CASE(5)
-			FXB_PAIR_CASE(6)
-			FXB_PAIR_CASE(7)
-			FXB_PAIR_CASE(8)
-			FXB_PAIR_CASE(9)
-			FXB_PAIR_CASE(10)
-#undef FXB_PAIR_CASE
-		default: break;
-		}
-	});
-}
-
-// One length: 2048 points (class 7 VAR + 4) in CTAs of 256 threads, 4096 (class 7 VAR +
-// 2) of 512, 8192 (class 7 VAR) of 1024.  (2048 points among the others' code, 10
-// stations x 2 subbands x 2 bands of 8 bits: F stage 89 us, 81 here; 16 threads read raw
-// 311 and 289.)
+// The units of one length (class 2 (13 - LOGN) of VAR 0: plain VDIF, 1: raw
+// INTERLACEDVDIF reads), each in a kernel of its own: a kernel of several lengths has
+// registers and an order of instructions that suit none.  2048 points among the
+// shorter ones, 10 stations x 2 subbands x 2 bands of 8 bits: F stage 89 us, 81 alone;
+// 16 threads read raw 311 and 289.
 template <int VAR, int LOGN>
 __global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB)
     k_fstage_pair_pw(const __grid_constant__ FsMultiArgs m)
 {
 	extern __shared__ __align__(16) ulonglong2 fsp[];
+	constexpr int FPC = PShape<LOGN>::FPC, NFC = kMaxTQ * FPC < kFsMultiFc ? kMaxTQ * FPC : kFsMultiFc;
 	__shared__ float lut8[260];
 	__shared__ u64 lut4[16];
-	__shared__ PairFeed<kMaxTQ> feed;
+	__shared__ PairFeed<NFC> feed;
 	fstage_pair_luts(lut8, lut4);
 	pair_units(feed, m, kFsMultiPer * VAR + 2 * (13 - LOGN),
 	           [&](const FsMultiUnit &w, const PairItem &I, const PairConst *fcs, const PairTwist *tws) {
 		           const FsMultiKind &k = m.kinds[w.kind];
-		           fstage_pair_unit<LOGN, true, VAR>(m.m[k.member], I, fcs, tws, w.t0, w.nfc, (const float2 *)k.tw, fsp, lut8,
-		                                             lut4);
+		           fstage_pair_unit<LOGN, true, VAR>(m.m[k.member], I, fcs, tws, w.t0, (w.nfc + FPC - 1) / FPC,
+		                                             (const float2 *)k.tw, fsp, lut8, lut4);
 	           });
+}
+
+template <int VAR, int LOGN>
+static void launch_len(const FsMultiArgs &m, int nsm, cudaStream_t st)
+{
+	using SH = PShape<LOGN>;
+	fs_launch_persistent(k_fstage_pair_pw<VAR, LOGN>, m, kFsMultiPer * VAR + 2 * (13 - LOGN), SH::MINB * nsm, SH::NT,
+	                     (size_t)SH::FPC * SH::PADN * 16, st);
 }
 
 template <int VAR>
 static void launch_cls(const FsMultiArgs &m, int c, int nsm, cudaStream_t st)
 {
-	if(c == 6)
-		fs_launch_persistent(k_fstage_pair_pn<VAR>, m, kFsMultiPer * VAR + c, 3 * nsm, 256, kPairSide, st);
-	else if(c == 4)
-		fs_launch_persistent(k_fstage_pair_pw<VAR, 11>, m, kFsMultiPer * VAR + c, 3 * nsm, 256, kPairSide, st);
-	else if(c == 2)
-		fs_launch_persistent(k_fstage_pair_pw<VAR, 12>, m, kFsMultiPer * VAR + c, 2 * nsm, 512, 2 * kPairSide, st);
-	else
-		fs_launch_persistent(k_fstage_pair_pw<VAR, 13>, m, kFsMultiPer * VAR + c, nsm, 1024, 4 * kPairSide, st);
+	switch(13 - c / 2)
+	{
+	case 5: launch_len<VAR, 5>(m, nsm, st); break;
+	case 6: launch_len<VAR, 6>(m, nsm, st); break;
+	case 7: launch_len<VAR, 7>(m, nsm, st); break;
+	case 8: launch_len<VAR, 8>(m, nsm, st); break;
+	case 9: launch_len<VAR, 9>(m, nsm, st); break;
+	case 10: launch_len<VAR, 10>(m, nsm, st); break;
+	case 11: launch_len<VAR, 11>(m, nsm, st); break;
+	case 12: launch_len<VAR, 12>(m, nsm, st); break;
+	default: launch_len<VAR, 13>(m, nsm, st); break;
+	}
 }
 
 void launch_fs_pair_multi(const FsMultiArgs &m, int cls, int nsm, cudaStream_t st)

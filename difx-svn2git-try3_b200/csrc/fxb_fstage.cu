@@ -35,9 +35,7 @@ int fstage_multi_class(int N, int nb)
 {
 	if(N < 32 || N > 8192)
 		return -1;
-	if(nb == 2)
-		return N == 8192 ? 0 : (N == 4096 ? 2 : (N == 2048 ? 4 : 6));
-	return N == 8192 ? 1 : (N == 4096 ? 3 : 5);
+	return 2 * (13 - ilog2(N)) + (nb == 2 ? 0 : 1);
 }
 
 int fstage_multi_tq(int N, int nb, int tq)

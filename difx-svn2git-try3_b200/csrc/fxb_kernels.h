@@ -280,9 +280,10 @@ void launch_fstage_kind(const FKind &k, FsArgs a, cudaStream_t stream);
 // units.  Every tensor-core-form context runs these kinds this way, alone or in
 // a batch, so results do not depend on it.
 constexpr int kFsMultiMembers = 16;
-constexpr int kFsMultiFc = 64;           // FFT constants of one unit of several lengths' launches at most (tq x fpc)
-// classes of units: plain VDIF's (fstage_multi_class), then those of raw reads
-constexpr int kFsMultiPer = 7, kFsMultiClasses = 2 * kFsMultiPer;
+constexpr int kFsMultiFc = 64;           // FFT constants of one unit at most (tq x fpc)
+// classes of units: by length and bands, plain VDIF's (fstage_multi_class), then
+// those of raw reads
+constexpr int kFsMultiPer = 18, kFsMultiClasses = 2 * kFsMultiPer;
 struct FsMultiKind {
 	const void *tw;                      // twiddles of length N
 	int32_t member, code;                // context; 128 x raw INTERLACEDVDIF reads + 32 x bands per item + log2 N
@@ -302,10 +303,9 @@ struct FsMultiArgs {
 	int32_t unit0[kFsMultiClasses], nunit[kFsMultiClasses];   // each class's first unit and units
 	int32_t *ctr;                        // one counter per class, zero before the launch
 };
-// class of a kind (FFT length N, bands per item nb) in the persistent launches
-// (two bands of 8192 points: 0, 4096: 2, 2048: 4, up to 1024: 6; one band of 8192: 1,
-// 4096: 3, up to 2048: 5; -1: not run there), and the FFT iterations per unit for a
-// kind's tq
+// class of a kind (FFT length N = 8192 .. 32, bands per item nb) in the persistent
+// launches: 2 log2(8192 / N), one more for one band; -1: not run there.  And the FFT
+// iterations per unit for a kind's tq
 int fstage_multi_class(int N, int nb);
 int fstage_multi_tq(int N, int nb, int tq);
 cudaError_t launch_fstage_multi(const FsMultiArgs &m, int nsm, cudaStream_t stream);
