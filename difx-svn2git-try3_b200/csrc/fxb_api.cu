@@ -126,6 +126,8 @@ struct fxb_ctx {
 	int nwsum = 0, nwout = 0, nom = 0;
 	DevZoomCopy *d_zoom = nullptr;       // zoom-band rows gathered after the F stage
 	int nzoom = 0;
+	DevZoomGroup *d_zgroups = nullptr;   // the same by zoom frequency
+	int nzgroups = 0, zquads = 0;        // quads of channels of a frequency's rows, at most
 	// phase cal: binning groups, bands, and the FP64 bins of the integration
 	std::vector<DevPcalGroup> h_pgroups;
 	DevPcalGroup *d_pgroups = nullptr;
@@ -1122,6 +1124,18 @@ static fxb_status setup_device(fxb_ctx *ctx)
 				const Job::ZoomCopy &z = job.zooms[i];
 				hz[i] = DevZoomCopy{z.src_freq, z.src_row, z.dst_freq, z.dst_row, z.choff, z.nchan};
 			}
+			std::vector<DevZoomGroup> hg;
+			for(int i = 0; i < ctx->nzoom; i++)
+				if(hg.empty() || hz[i].dst_plan != hz[hg.back().first].dst_plan)
+					hg.push_back({i, 1});
+				else
+					hg.back().count++;
+			ctx->nzgroups = (int)hg.size();
+			for(const DevZoomGroup &g : hg)
+				ctx->zquads = std::max(ctx->zquads, g.count * hz[g.first].nchan / 4);
+			CK(ctx, dalloc(ctx, &ctx->d_zgroups, hg.size()));
+			CK(ctx, cudaMemcpyAsync(ctx->d_zgroups, hg.data(), sizeof(DevZoomGroup) * hg.size(), cudaMemcpyHostToDevice,
+			                        ctx->stream));
 			CK(ctx, dalloc(ctx, &ctx->d_zoom, ctx->nzoom));
 			CK(ctx, cudaMemcpyAsync(ctx->d_zoom, hz.data(), sizeof(DevZoomCopy) * ctx->nzoom, cudaMemcpyHostToDevice, ctx->stream));
 		}
@@ -1578,7 +1592,7 @@ static void launch_xmac_weights(fxb_ctx *ctx, const Slot &sl, cudaStream_t st, b
 		launch_pcal_bin(ctx->d_pgroups + pc.first, pc.count, pc.maxbins, ctx->pplan, pc.nbits, pc.bpt, pc.shift != 0,
 		                pc.smem, ctx->d_st, sl.d_sub, sl.d_params, sl.d_valid, sl.valid_stride, ctx->T,
 		                job.pcal_bins, ctx->d_pbins, st);
-	launch_zoom_gather(ctx->d_zoom, ctx->nzoom, ctx->d_plans, ctx->T, ctx->tc,
+	launch_zoom_gather(ctx->d_zoom, ctx->nzoom, ctx->d_zgroups, ctx->nzgroups, ctx->zquads, ctx->d_plans, ctx->T, ctx->tc,
 	                   ctx->tc ? ctx->d_specn : (void *)ctx->d_spec, st);
 	mark(ctx, sl.tev[2], st, capture, branch);
 	if(ctx->f8)

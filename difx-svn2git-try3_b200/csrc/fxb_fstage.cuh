@@ -197,23 +197,6 @@ __device__ __forceinline__ uint32_t pack_spec(bool h16, float re, float im)
 	return *(const uint32_t *)&b;
 }
 
-// Tensor-core form: the four channels of positions p0 .. p0 + 3 (a multiple of 4)
-// of one row of a time's blocks [block][trow][tcb], o its first.  tcb is even;
-// bextra = (trow - 1) tcb lies between the end of a block's run of the row and the
-// next block's, and p / tcb = umulhi(p, magic) for p < 2^16.
-__device__ __forceinline__ void store_quad(uint32_t *o, uint32_t p0, uint32_t tcb, uint32_t magic, uint32_t bextra,
-                                           uint4 h)
-{
-	uint32_t *q = o + p0 + __umulhi(p0, magic) * bextra;
-	if(tcb & 2u)
-	{
-		*(uint2 *)q = make_uint2(h.x, h.y);
-		*(uint2 *)(o + p0 + 2u + __umulhi(p0 + 2u, magic) * bextra) = make_uint2(h.z, h.w);
-	}
-	else
-		*(uint4 *)q = h;
-}
-
 // A row of the tensor-core spectra: its first value of time 0 and the step of a time
 struct OutRow {
 	int64_t first;

@@ -2,6 +2,7 @@
 // finalisation into the core-result layout, and the stand-alone VDIF decoder.
 
 #include <cuda_runtime.h>
+#include <algorithm>
 #include <cstdint>
 
 #include "fxb_internal.h"
@@ -454,65 +455,91 @@ void launch_vdif_unpack(const uint8_t *data, int64_t nbytes, int payload, int he
 
 // ---------------------------------------------------------------- zoom bands
 // A zoom band's spectra are the channels [choff, choff + nchan) of its parent
-// band's (mode.cpp:169-208): one CTA per (8 FFTs, zoom row) copies them into
-// the zoom frequency's own spectra rows, FP32 [t][row][chan] (float2) or the
-// tensor-core form's blocked [t][block][trow][tcb] (bf16x2 as uint32).  Each
-// thread finds its channel's place in both once and steps the times.
+// band's (mode.cpp:169-208), copied into the zoom frequency's own rows.
 constexpr int kZoomTimes = 8;
 
-// offset of channel c from element (t, row, block 0, offset 0)
-__device__ __forceinline__ uint32_t chan_off(const DevFreqPlan &p, int c)
-{
-	if(p.tcb == 0)
-		return (uint32_t)c;
-	const uint32_t q = (uint32_t)chan_pos(p.pbits, c), blk = q / (uint32_t)p.tcb;
-	return q + blk * (uint32_t)((p.trow - 1) * p.tcb);
-}
-
-// element (t, row, block 0, offset 0)
-__device__ __forceinline__ int64_t row_base(const DevFreqPlan &p, int t, int row)
-{
-	if(p.tcb == 0)
-		return p.spec_off + ((int64_t)t * p.nrow + row) * p.nchan;
-	return p.spec_off + ((int64_t)t * p.tnblk * p.trow + row) * p.tcb;
-}
-
-template <typename V>
+// FP32 form [t][row][chan]: one CTA per (8 FFTs, zoom row), a thread a channel of
+// all eight.
 __global__ void __launch_bounds__(256) k_zoom_gather(const DevZoomCopy *__restrict__ zc,
                                                      const DevFreqPlan *__restrict__ plans, int T,
-                                                     V *__restrict__ spec)
+                                                     float2 *__restrict__ spec)
 {
 	const DevZoomCopy z = zc[blockIdx.y];
-	const DevFreqPlan src = plans[z.src_plan], dst = plans[z.dst_plan];
-	const int t0 = blockIdx.x * kZoomTimes, t1 = min(T, t0 + kZoomTimes);
-	const int64_t sts = row_base(src, 1, z.src_row) - row_base(src, 0, z.src_row);
-	const int64_t dts = row_base(dst, 1, z.dst_row) - row_base(dst, 0, z.dst_row);
+	const DevFreqPlan &src = plans[z.src_plan], &dst = plans[z.dst_plan];
+	const int t0 = blockIdx.x * kZoomTimes;
+	const int64_t sts = (int64_t)src.nrow * src.nchan, dts = (int64_t)dst.nrow * dst.nchan;
+	const float2 *s0 = spec + src.spec_off + t0 * sts + (int64_t)z.src_row * src.nchan + z.choff;
+	float2 *d0 = spec + dst.spec_off + t0 * dts + (int64_t)z.dst_row * dst.nchan;
 	for(int c = threadIdx.x; c < z.nchan; c += blockDim.x)
 	{
-		const V *s = spec + row_base(src, t0, z.src_row) + chan_off(src, z.choff + c);
-		V *d = spec + row_base(dst, t0, z.dst_row) + chan_off(dst, c);
-		V v[kZoomTimes];
+		float2 v[kZoomTimes];
 #pragma unroll
 		for(int k = 0; k < kZoomTimes; k++)
-			if(t0 + k < t1)
-				v[k] = s[k * sts];
+			if(t0 + k < T)
+				v[k] = s0[k * sts + c];
 #pragma unroll
 		for(int k = 0; k < kZoomTimes; k++)
-			if(t0 + k < t1)
-				d[k * dts] = v[k];
+			if(t0 + k < T)
+				d0[k * dts + c] = v[k];
 	}
 }
 
-void launch_zoom_gather(const DevZoomCopy *zc, int nzc, const DevFreqPlan *plans, int T, bool tc, void *spec,
-                        cudaStream_t stream)
+// Tensor-core forms [t][block][trow][tcb], channels in the order of chan_pos: CTAs per
+// (8 FFTs, zoom frequency, share of its quads), a thread the four channels of a quad
+// of positions of one row, the lanes of a warp in neighbouring rows, whose quads lie
+// side by side.
+// Bound by L2: the quads of the parent hold one or two wanted channels of four.  A
+// CTA a row and 4-byte loads and stores met a sector a value: two windows of 256
+// channels on each of 8 subbands, 20 rows x 250 FFTs, F stage and gather 327 us, 185
+// now (244 before the channels' present order).
+__global__ void __launch_bounds__(256) k_zoom_quads(const DevZoomCopy *__restrict__ zc,
+                                                    const DevZoomGroup *__restrict__ groups,
+                                                    const DevFreqPlan *__restrict__ plans, int T,
+                                                    uint32_t *__restrict__ spec)
+{
+	const DevZoomGroup g = groups[blockIdx.y];
+	const int t0 = blockIdx.x * kZoomTimes, nq = zc[g.first].nchan >> 2, n = g.count * nq;
+	for(int w = blockIdx.z * blockDim.x + threadIdx.x; w < n; w += gridDim.z * blockDim.x)
+	{
+		const int i = w / g.count;
+		const DevZoomCopy z = zc[g.first + (w - i * g.count)];
+		const DevFreqPlan &S = plans[z.src_plan], &D = plans[z.dst_plan];
+		const int64_t sts = (int64_t)S.tnblk * S.trow * S.tcb, dts = (int64_t)D.tnblk * D.trow * D.tcb;
+		const uint32_t *s = spec + S.spec_off + t0 * sts + (int64_t)z.src_row * S.tcb;
+		uint32_t *d = spec + D.spec_off + t0 * dts + (int64_t)z.dst_row * D.tcb;
+		const uint32_t sextra = (uint32_t)(S.trow - 1) * (uint32_t)S.tcb, dextra = (uint32_t)(D.trow - 1) * (uint32_t)D.tcb;
+		uint32_t off[4];
+#pragma unroll
+		for(int m = 0; m < 4; m++)
+		{
+			const uint32_t q = (uint32_t)chan_pos(S.pbits, z.choff + i + m * nq);
+			off[m] = q + __umulhi(q, S.magic) * sextra;
+		}
+		const uint32_t dtcb = (uint32_t)D.tcb, dmagic = D.magic;
+		uint4 v[kZoomTimes];
+#pragma unroll
+		for(int k = 0; k < kZoomTimes; k++)
+			if(t0 + k < T)
+				v[k] = make_uint4(s[k * sts + off[0]], s[k * sts + off[1]], s[k * sts + off[2]], s[k * sts + off[3]]);
+#pragma unroll
+		for(int k = 0; k < kZoomTimes; k++)
+			if(t0 + k < T)
+				store_quad(d + k * dts, 4u * (uint32_t)i, dtcb, dmagic, dextra, v[k]);
+	}
+}
+
+void launch_zoom_gather(const DevZoomCopy *zc, int nzc, const DevZoomGroup *groups, int ngroups, int maxquads,
+                        const DevFreqPlan *plans, int T, bool tc, void *spec, cudaStream_t stream)
 {
 	if(nzc <= 0 || T <= 0)
 		return;
-	const dim3 grid((T + kZoomTimes - 1) / kZoomTimes, nzc);
+	const int nt = (T + kZoomTimes - 1) / kZoomTimes;
+	// few FFTs and frequencies: the quads of a frequency over more CTAs
+	const int share = std::max(1, std::min((maxquads + 255) / 256, 1184 / (nt * std::max(ngroups, 1))));
 	if(tc)
-		k_zoom_gather<uint32_t><<<grid, 256, 0, stream>>>(zc, plans, T, (uint32_t *)spec);
+		k_zoom_quads<<<dim3(nt, ngroups, share), 256, 0, stream>>>(zc, groups, plans, T, (uint32_t *)spec);
 	else
-		k_zoom_gather<float2><<<grid, 256, 0, stream>>>(zc, plans, T, (float2 *)spec);
+		k_zoom_gather<<<dim3(nt, nzc), 256, 0, stream>>>(zc, plans, T, (float2 *)spec);
 }
 
 // 8-bit levels (b - 128) / 3.3 (format_vdif.c:122) into the current

@@ -43,6 +43,22 @@ __host__ __device__ __forceinline__ int chan_pos(int pbits, int c)
 	return ((c & ((1 << pbits) - 1)) << 2) | (c >> pbits);
 }
 __host__ __device__ __forceinline__ int pos_chan(int pbits, int p) { return ((p & 3) << pbits) | (p >> 2); }
+// Tensor-core form: the four channels of positions p0 .. p0 + 3 (a multiple of 4)
+// of one row of a time's blocks [block][trow][tcb], o its first.  tcb is even;
+// bextra = (trow - 1) tcb lies between the end of a block's run of the row and the
+// next block's, and p / tcb = umulhi(p, magic) for p < 2^16.
+__device__ __forceinline__ void store_quad(uint32_t *o, uint32_t p0, uint32_t tcb, uint32_t magic, uint32_t bextra,
+                                           uint4 h)
+{
+	uint32_t *q = o + p0 + __umulhi(p0, magic) * bextra;
+	if(tcb & 2u)
+	{
+		*(uint2 *)q = make_uint2(h.x, h.y);
+		*(uint2 *)(o + p0 + 2u + __umulhi(p0 + 2u, magic) * bextra) = make_uint2(h.z, h.w);
+	}
+	else
+		*(uint4 *)q = h;
+}
 #endif
 
 // A weight sum: stations and, of INTERLACEDVDIF stations, recorded bands (-1:
@@ -62,6 +78,10 @@ struct DevWeightOut {
 // of plan src_plan, copied to row dst_row of plan dst_plan.
 struct DevZoomCopy {
 	int32_t src_plan, src_row, dst_plan, dst_row, choff, nchan;
+};
+// consecutive rows of one zoom frequency
+struct DevZoomGroup {
+	int32_t first, count;
 };
 
 // raw INTERLACEDVDIF reads (DevStation::muxraw): frame slots, muxed headers
@@ -445,8 +465,8 @@ void launch_pcal_final(const DevPcalBand *bands, int nbands, int nchunk, int64_t
 
 // Zoom-band spectra from their parents' (after the F stage, before the
 // XMAC): tc selects the tensor-core form's bf16x2 spectra.
-void launch_zoom_gather(const DevZoomCopy *zc, int nzc, const DevFreqPlan *plans, int T, bool tc, void *spec,
-                        cudaStream_t stream);
+void launch_zoom_gather(const DevZoomCopy *zc, int nzc, const DevZoomGroup *groups, int ngroups, int maxquads,
+                        const DevFreqPlan *plans, int T, bool tc, void *spec, cudaStream_t stream);
 
 // adds the subint's weight sums to acc[nsum].  wts: data weights [station][FFT];
 // pbw: per-band data weights [station][FFT][nbm] of INTERLACEDVDIF stations (null: none)

@@ -1,7 +1,7 @@
 """Where the F stage puts its values in the tensor-core spectra: blocks of 2 to 32
 channels, rows of 1 to 50 inputs, four channels stored at once.  Items of one band
-(one polarisation, one subband) at every length, both sidebands, mirrored
-(order-0 lower) bands.
+(one polarisation, one subband) and of two at every length, both sidebands, mirrored
+(order-0 lower) bands, complex sampling, the tensor-core FFT, zoom windows.
 
 Against the FP32 form's spectra of the same job, value by value: the same FP32
 arithmetic in both but for contractions (1e-5 of the rms: five times 2e-6, the FP32
@@ -13,6 +13,7 @@ import pytest
 from fxb200 import synth
 from fxb200.job import Freq, full_job
 from fxb200.native import Correlator
+from helpers import ZOOMS, zoom_job
 
 pytestmark = pytest.mark.gpu
 
@@ -97,3 +98,25 @@ def test_tensor_core_fft(nstation, pols, nfreq, xmac):
     for r, g in zip(ref, got):
         err = np.linalg.norm(g - r, axis=2) / np.linalg.norm(r, axis=2)
         assert err.shape == (3, nstation * len(pols)) and np.all(err <= tol), err.max()
+
+
+@pytest.mark.parametrize("nstation,xmac", [(2, "fp16"), (3, "fp16"), (7, "fp16"), (13, "fp16"), (31, "fp16"), (2, "fp8"),
+                                           (5, "fp8"), (9, "fp8"), (13, "fp8")])
+def test_zoom_windows(nstation, xmac):
+    """Zoom windows (at the start, inside and at the end of their subband) are copies
+    of their parents' channels, in their own blocks."""
+    job = zoom_job(nstation=nstation, subint_ns=16_000 * 11)
+    inputs = synth.subint_inputs(job, 0, 4_000_000, rho=0.05, seed=7)
+    out = []
+    for form in ("fp32", xmac):
+        corr = Correlator(job, xmac=form)
+        corr.submit(inputs, 0, 4_000_000)
+        out.append([corr.spectra(f) for f in range(len(job.freqs))])
+        corr.close()
+    compare(*out)
+    for ref, got in zip(*out):
+        assert ref.shape == got.shape
+    for (parent, off, bw), z in zip(ZOOMS, range(2, 5)):
+        c0, n = int(off * 16), int(bw * 16)
+        for o in out:
+            assert np.array_equal(o[z], o[parent][:, :, c0:c0 + n])
