@@ -507,7 +507,7 @@ def mux_leg(args):
                         % (data.size // 1000000),
             "ms_per_read": ms, "rtf": 0.5 / (ms * 1e-3), "bytes_in": int(data.size), "bytes_out": int(n),
             "achieved_gbs": gbs, "hbm_peak_gbs": hbm_peak, "frac": gbs / hbm_peak, "peak_source": src,
-            "note": "three launches per read (placement, headers, corner turn) plus one 8-byte status read"}
+            "note": "four launches per read (placement, first slots, headers, corner turn) plus one 8-byte status read"}
 
 
 def mux_fused_leg(args):

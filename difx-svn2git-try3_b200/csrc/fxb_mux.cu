@@ -9,14 +9,15 @@
 //                  (VDIFMuxer::deinterlace, datamuxer.cpp:765-846); where a
 //                  slot is filled twice the later input frame wins, as the
 //                  reference's in-order copy does;
-//   k_mux_headers  one thread walks the output frames in order and writes
-//                  their headers (VDIFMuxer::multiplex, datamuxer.cpp:680-763):
-//                  complete slots take thread 0's header with one channel per
-//                  thread, incomplete ones the first present thread's header
-//                  marked invalid, empty ones the previous output header one
-//                  frame later, marked invalid (empty slots before the first
-//                  output frame are dropped);
-//   k_mux_turn     corner turn of the complete slots' payloads
+//   k_mux_first    the first slot that holds any frame;
+//   k_mux_headers  one thread an output frame writes its header
+//                  (VDIFMuxer::multiplex, datamuxer.cpp:680-763): complete slots
+//                  take thread 0's header with one channel per thread, incomplete
+//                  ones the first present thread's marked invalid, empty ones the
+//                  nearest earlier filled slot's advanced one frame per slot,
+//                  marked invalid (empty slots before the first filled one are
+//                  dropped);
+//   k_mux_shuffle, k_mux_turn   corner turn of the complete slots' payloads
 //                  (VDIFMuxer::cornerturn_generic, datamuxer.cpp:253-274):
 //                  one CUDA thread per (output frame, input word), reading the
 //                  word of every thread and writing nthreads output words.

@@ -23,7 +23,8 @@
 // The times are then split over the CTAs of a cluster, and within a CTA over
 // groups of warps where the rows give only a few tile pairs.  The partial
 // sums meet in shared memory and over distributed shared memory in slice
-// order, so a result depends on the job alone, never on the schedule.
+// order, so a result depends on the job and the device's number of SMs (which
+// chooses the slices), never on the schedule.
 // Measured: 4 stations, 256 channels, T = 250: 142 -> 12 us; 7 rows x 64
 // channels x 16 subbands, T = 2005: 552 -> 60 us; 10 stations x 8 x 1024
 // channels, T = 250: 198 -> 144 us.

@@ -35,7 +35,7 @@
 // Few units (few channels, many FFTs): a unit's times are cut into slices, whose
 // sums go to a workspace and are added in slice order by k_xmac_merge, so that a
 // result never depends on the schedule.  Slices are chosen from the group's own
-// extents, so a context alone and in a batch agree.
+// extents and the device's number of SMs, so a context alone and in a batch agree.
 //
 // Bound: HBM / L2 reads of the spectra at up to about 20 inputs, the epilogue's
 // reductions and the matrix work above.  Launch times in us with K-major operands

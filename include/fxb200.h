@@ -254,8 +254,12 @@ FXB_API fxb_status fxb_tuning_report(const fxb_ctx *ctx, char *buf, size_t len, 
  * launches over one work list that spans the members (the N = 2048
  * tensor-core FFT kinds as their own launches), and every XMAC group of
  * every member as one persistent launch on a second stream, beside the next
- * subint's F stage.  Results do not depend on the mode.  A
- * member takes no fxb_submit_subint of its own while it belongs to a batch;
+ * subint's F stage.  Results do not depend on the mode.  A batch keeps
+ * members of one observation in step and costs one graph launch a subint; it
+ * is not the faster form: on a B200, 20 stations with 16 subbands of mixed
+ * widths (4, 16 and 64 MHz), channels and bits run at 7.84 times real time
+ * as contexts submitted by themselves, 7.41 as a batch and 6.98 fused.
+ * A member takes no fxb_submit_subint of its own while it belongs to a batch;
  * its results are read and reset through the usual calls (ordered after the
  * batch's launches).  All members need the same max_subints_in_flight and
  * device; call the batch functions with that device current. */
