@@ -658,8 +658,6 @@ __device__ __forceinline__ void fstage_unit(const FsArgs &a, const int gidx, con
 					{
 						const int q = q0 + g8 * (N / 8);
 						cf y[RL];
-						if constexpr(N <= 2048)
-							asm volatile("" ::: "memory");        // 80 registers: one group's loads at a time
 #pragma unroll
 						for(int r = 0; r < RL; r++)
 							y[r] = lds(src + st_index<sL, (N >= 8192)>(q, r));
