@@ -44,6 +44,7 @@
 
 #include "fxb_internal.h"
 #include "fxb_kernels.h"
+#include "fxb_ptx.cuh"
 
 namespace fxb {
 
@@ -184,18 +185,6 @@ __host__ __device__ inline float level2(uint32_t code)
 }
 
 __device__ __forceinline__ float frac_centered(double x) { return (float)(x - rint(x)); }
-
-// one spectral value of the tensor-core forms: (re, im) as half2 or bf16x2
-__device__ __forceinline__ uint32_t pack_spec(bool h16, float re, float im)
-{
-	if(h16)
-	{
-		const __half2 h = __floats2half2_rn(re, im);
-		return *(const uint32_t *)&h;
-	}
-	const __nv_bfloat162 b = __floats2bfloat162_rn(re, im);
-	return *(const uint32_t *)&b;
-}
 
 // A row of the tensor-core spectra: its first value of time 0 and the step of a time
 struct OutRow {

@@ -44,45 +44,6 @@ namespace fxb {
 
 namespace {
 
-typedef unsigned long long u64;
-
-__device__ __forceinline__ u64 pk2(float a, float b)
-{
-	u64 d;
-	asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
-	return d;
-}
-__device__ __forceinline__ float2 up2(u64 v)
-{
-	float2 r;
-	asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-	return r;
-}
-__device__ __forceinline__ u64 add2(u64 a, u64 b)
-{
-	u64 d;
-	asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-	return d;
-}
-__device__ __forceinline__ u64 sub2(u64 a, u64 b)
-{
-	u64 d;
-	asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-	return d;
-}
-__device__ __forceinline__ u64 mul2(u64 a, u64 b)
-{
-	u64 d;
-	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-	return d;
-}
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c)
-{
-	u64 d;
-	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-	return d;
-}
-
 // one complex value of both bands: (band 0, band 1) real and imaginary parts
 struct cp {
 	u64 re, im;
@@ -878,6 +839,54 @@ __device__ __forceinline__ void fstage_pair_luts(float *lut8, u64 *lut4)
 		lut8[256 + threadIdx.x] = level2(threadIdx.x);
 	if(threadIdx.x < 16)
 		lut4[threadIdx.x] = pk2(level2(threadIdx.x & 3u), level2(threadIdx.x >> 2u));
+}
+
+// One CTA per work unit (grid as k_fstage): the FP32 form, and complex sampling of the
+// tensor-core forms, whose other kinds have persistent launches.
+template <int LOGN, bool TCO, int VAR>
+__global__ void __launch_bounds__(PShape<LOGN>::NT, PShape<LOGN>::MINB) k_fstage_pair(const FsArgs a)
+{
+	extern __shared__ __align__(16) ulonglong2 fsp[];
+	constexpr int FPC = PShape<LOGN>::FPC;
+	__shared__ float lut8[260];
+	__shared__ u64 lut4[16];
+	__shared__ PairConst fcs[kMaxTQ * FPC];
+	__shared__ PairTwist tws[kMaxTQ * FPC];
+	__shared__ PairItem I;
+	const int item = a.pair0 + (a.items_fast ? blockIdx.x : blockIdx.y);
+	const int t0 = (a.items_fast ? blockIdx.y : blockIdx.x) * a.tq * FPC, nfc = min(a.tq * FPC, a.T - t0);
+	pair_fetch(&I, fcs, tws, a.pitems + item, a.pconst + (int64_t)item * a.T + t0,
+	           a.two ? a.ptwist + (int64_t)(item - a.ptwist0) * a.T + t0 : nullptr, nfc);
+	fstage_pair_luts(lut8, lut4);
+	pair_cp_wait();
+	__syncthreads();
+	fstage_pair_unit<LOGN, TCO, VAR>(a, I, fcs, tws, t0, (nfc + FPC - 1) / FPC, (const float2 *)a.tw, fsp, lut8, lut4);
+}
+
+template <int LOGN, bool TCO, int VAR>
+static void launch_t(const FKind &k, const FsArgs &a, cudaStream_t stream)
+{
+	cudaFuncSetAttribute(k_fstage_pair<LOGN, TCO, VAR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
+	cudaFuncSetAttribute(k_fstage_pair<LOGN, TCO, VAR>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+	k_fstage_pair<LOGN, TCO, VAR><<<fstage_grid(k, a), k.threads, k.smem, stream>>>(a);
+}
+
+template <bool TCO, int VAR>
+static void launch_var(const FKind &k, const FsArgs &a, cudaStream_t stream)
+{
+	switch(k.N)
+	{
+	case 32: launch_t<5, TCO, VAR>(k, a, stream); break;
+	case 64: launch_t<6, TCO, VAR>(k, a, stream); break;
+	case 128: launch_t<7, TCO, VAR>(k, a, stream); break;
+	case 256: launch_t<8, TCO, VAR>(k, a, stream); break;
+	case 512: launch_t<9, TCO, VAR>(k, a, stream); break;
+	case 1024: launch_t<10, TCO, VAR>(k, a, stream); break;
+	case 2048: launch_t<11, TCO, VAR>(k, a, stream); break;
+	case 4096: launch_t<12, TCO, VAR>(k, a, stream); break;
+	case 8192: launch_t<13, TCO, VAR>(k, a, stream); break;
+	default: break;
+	}
 }
 
 }  // namespace fxb

@@ -68,6 +68,7 @@
 
 #include "fxb_internal.h"
 #include "fxb_kernels.h"
+#include "fxb_ptx.cuh"
 
 namespace fxb {
 
@@ -88,58 +89,17 @@ constexpr int kDecW = 8;
 constexpr int kTwW0 = kDecW, kOutW0 = kDecW + 4, kMmaW = kDecW + 8, kProdW = kDecW + 9;
 constexpr int kThreadsTc = 32 * (kDecW + 10);
 static_assert(kTwW0 % 4 == 0 && kOutW0 % 4 == 0 && 8 % kDecW == 0, "warp roles");
-constexpr uint32_t kWaitLimitF = 1u << 22;
 constexpr int kTmemCols = 512;
 
 static_assert(kOffOp % 1024 == 0, "operand buffers must be 1024-aligned");
-
-__device__ __forceinline__ uint32_t su32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
-{
-	asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(su32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
-{
-	asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(su32(bar)) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes)
-{
-	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(su32(bar)), "r"(bytes) : "memory");
-}
-
-// bounded wait for the phase with parity `parity`; gives up early once
-// another role has recorded a failure
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *fail)
-{
-	const uint32_t a = su32(bar);
-	for(uint32_t it = 0; it < kWaitLimitF; it++)
-	{
-		uint32_t done;
-		asm volatile(
-		    "{\n\t.reg .pred p;\n\t"
-		    "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-		    "selp.u32 %0, 1, 0, p;\n\t}\n"
-		    : "=r"(done)
-		    : "r"(a), "r"(parity)
-		    : "memory");
-		if(done)
-			return true;
-		if((it & 255u) == 255u && *fail)
-			return false;
-	}
-	return false;
-}
 
 // global -> shared bulk copy (both addresses and the size multiples of 16),
 // completion counted in bytes on the mbarrier
 __device__ __forceinline__ void bulk_g2s(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
 {
 	asm volatile(
-	    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(su32(dst)),
-	    "l"(src), "r"(bytes), "r"(su32(bar))
+	    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(smem_u32(dst)),
+	    "l"(src), "r"(bytes), "r"(smem_u32(bar))
 	    : "memory");
 }
 
@@ -189,7 +149,7 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t adesc, uint64_
 
 __device__ __forceinline__ void commit_to(uint64_t *bar)
 {
-	asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(su32(bar))
+	asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(smem_u32(bar))
 	             : "memory");
 }
 
@@ -225,63 +185,11 @@ __device__ __forceinline__ void tld16(uint32_t taddr, float *v)
 
 __device__ __forceinline__ void tld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::: "memory"); }
 
-__device__ __forceinline__ uint32_t pack_h2(float a, float b)
-{
-	const __half2 h = __floats2half2_rn(a, b);
-	return *(const uint32_t *)&h;
-}
-
-// two FP32 values in one register pair
-typedef unsigned long long u64;
-__device__ __forceinline__ u64 pk2(float a, float b)
-{
-	u64 d;
-	asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
-	return d;
-}
-__device__ __forceinline__ float2 up2(u64 v)
-{
-	float2 r;
-	asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-	return r;
-}
-__device__ __forceinline__ u64 mul2(u64 a, u64 b)
-{
-	u64 d;
-	asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-	return d;
-}
-__device__ __forceinline__ u64 sub2(u64 a, u64 b)
-{
-	u64 d;
-	asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-	return d;
-}
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c)
-{
-	u64 d;
-	asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-	return d;
-}
 // complex product of two packed pairs
 __device__ __forceinline__ void cmul2(u64 xr, u64 xi, u64 wr, u64 wi, u64 &zr, u64 &zi)
 {
 	zr = sub2(mul2(xr, wr), mul2(xi, wi));
 	zi = fma2(xr, wi, mul2(xi, wr));
-}
-__device__ __forceinline__ uint32_t pack_h2(u64 v)
-{
-	const float2 f = up2(v);
-	return pack_h2(f.x, f.y);
-}
-
-// one spectral value of the tensor-core forms: (re, im) as half2 or bf16x2
-__device__ __forceinline__ uint32_t pack_spec(bool h16, float re, float im)
-{
-	if(h16)
-		return pack_h2(re, im);
-	const __nv_bfloat162 b = __floats2bfloat162_rn(re, im);
-	return *(const uint32_t *)&b;
 }
 
 __device__ __forceinline__ float level2f(uint32_t code)
@@ -511,7 +419,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 	}
 	if(warp == kMmaW)
 	{
-		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(su32(&tmem_s)),
+		asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&tmem_s)),
 		             "r"((uint32_t)kTmemCols));
 		asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
 	}
@@ -960,7 +868,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 		// instruction descriptor: D F32 (bit 4), A and B F16, A MN-major (bit 15),
 		// B K-major, N = 64 (bits 17-22: N >> 3), M = 128 (bits 24-28: M >> 4)
 		const uint32_t idesc = (1u << 4) | (1u << 15) | ((64u >> 3) << 17) | ((128u >> 4) << 24);
-		const uint32_t aB1 = su32(base + kOffB1), aB2 = su32(base + kOffB2);
+		const uint32_t aB1 = smem_u32(base + kOffB1), aB2 = smem_u32(base + kOffB2);
 		auto mma2 = [&](int j) -> bool {
 			const int b = j & 1, s = j % kNS;
 			if(!mbar_wait(&a2_full[b], (uint32_t)(j >> 1) & 1u, &fail_s))
@@ -969,7 +877,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 				return false;
 			asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
 			const uint32_t bside = aB2 + ((ring[j % kRing].flags & kLsb0) ? kB2Bytes : 0);
-			const uint32_t aA = su32(ops + s * kOpBytes);
+			const uint32_t aA = smem_u32(ops + s * kOpBytes);
 			const uint32_t dcol = tmem + (uint32_t)(256 * b + 128);
 #pragma unroll
 			for(int ks = 0; ks < 8; ks++)
@@ -992,7 +900,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_fstage_tc(const FsArgs a, con
 				break;
 			}
 			asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-			const uint32_t aA = su32(ops + s * kOpBytes);
+			const uint32_t aA = smem_u32(ops + s * kOpBytes);
 #pragma unroll
 			for(int sb = 0; sb < 2; sb++)
 			{

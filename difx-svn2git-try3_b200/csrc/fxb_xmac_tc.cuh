@@ -1,4 +1,4 @@
-// PTX wrappers shared by the tensor-core XMAC kernels (sm_100a).
+// Device code shared by the tensor-core XMAC kernels (sm_100a).
 #pragma once
 
 #include <cuda.h>
@@ -7,53 +7,11 @@
 
 #include "fxb_internal.h"
 #include "fxb_kernels.h"
+#include "fxb_ptx.cuh"
 
 namespace fxb {
 
 namespace {
-
-constexpr uint32_t kWaitLimit = 1u << 22;
-
-__device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-__device__ __forceinline__ void mbar_init(uint64_t *bar, uint32_t count)
-{
-	asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, uint32_t bytes)
-{
-	asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"(smem_u32(bar)), "r"(bytes)
-	             : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t *bar)
-{
-	asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"(smem_u32(bar)) : "memory");
-}
-
-// bounded wait for the phase with parity `parity`; gives up early once
-// another role has recorded a failure
-__device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volatile int *fail)
-{
-	const uint32_t a = smem_u32(bar);
-	for(uint32_t it = 0; it < kWaitLimit; it++)
-	{
-		uint32_t done;
-		asm volatile(
-		    "{\n\t.reg .pred p;\n\t"
-		    "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-		    "selp.u32 %0, 1, 0, p;\n\t}\n"
-		    : "=r"(done)
-		    : "r"(a), "r"(parity)
-		    : "memory");
-		if(done)
-			return true;
-		if((it & 255u) == 255u && *fail)
-			return false;
-	}
-	return false;
-}
 
 __device__ __forceinline__ void tma_load_3d(void *dst, const CUtensorMap *map, int x, int y, int z, uint64_t *bar)
 {
